@@ -285,7 +285,7 @@ int spgemm_get_stats(spgemm_handle_t h, spgemm_stats* out) {
   const sg::Engine& E = h->eng;
   out->intermediate_products = E.intermediate_products();
   out->nnz_c = E.nnz_c();
-  for (int b = 0; b < sg::FB_COUNT; ++b) out->rows_per_symbolic_bin[b] = E.sym_bin_rows(b);
+  for (int b = 0; b < sg::FB_STAT_COUNT; ++b) out->rows_per_symbolic_bin[b] = E.sym_bin_rows(b);
   out->warp_overflow_rows = E.overflow_rows();
   for (int b = 0; b < sg::NB_COUNT; ++b) out->rows_per_numeric_bin[b] = E.num_bin_rows(b);
   out->long_row_slices = E.slices();

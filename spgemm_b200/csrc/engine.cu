@@ -355,7 +355,7 @@ int Engine::analyze(const cm& A, const cm& B) {
     prof_begin("k_row_analysis");
     k_row_analysis<<<(m + RA_ROWS - 1) / RA_ROWS, RA_THREADS, 0, stream_>>>(
         op_, aoff_.as<int>(), row_p_.as<long long>(), c_cnt_.as<int>(), tcap_.as<int>(),
-        dc->fb_count, sym_rows_.as<int>(), &dc->p_total, &dc->max_row_len, row_span_.as<int2>(),
+        dc->fb_count, dc->may_overflow, sym_rows_.as<int>(), &dc->p_total, &dc->max_row_len, row_span_.as<int2>(),
         &dc->status, tn_);
     SG_LAUNCHED("k_row_analysis");
   }
@@ -370,7 +370,10 @@ int Engine::analyze(const cm& A, const cm& B) {
   SG_CK(cudaStreamSynchronize(stream_), "sync after row analysis");
   if (int r = check_status(host_counters_->status)) return r;
   p_total_ = (long long)host_counters_->p_total;
-  for (int b = 0; b < FB_COUNT; ++b) fb_counts_[b] = host_counters_->fb_count[b];
+  for (int b = 0; b < FB_COUNT; ++b) {
+    fb_counts_[b] = host_counters_->fb_count[b];
+    may_overflow_[b] = host_counters_->may_overflow[b];
+  }
   n_long_sym_ = fb_counts_[FB_LONG];
   max_row_len_ = host_counters_->max_row_len;
   temp_total_ = host_counters_->grand_total;
@@ -506,30 +509,24 @@ int Engine::launch_fused() {
   int* t_col = t_col_.as<int>();
   float* t_val = t_val_.as<float>();
   int* mid_rows = rows + (size_t)FB_MID * m;
-  int* big_rows = rows + (size_t)(FB_BLOCK0 + 2) * m;
-  int overflow_bound = 0;  // rows the warp bins may push to the mid / block lists
 #define SG_FUSED_WARP(L)                                                                      \
   {                                                                                            \
     const int b = L - 6, cnt = fb_counts_[b];                                                  \
     if (cnt > 0) {                                                                             \
-      overflow_bound += cnt;                                                                   \
       const size_t smem = WPB * ((size_t(1) << L) * (VB + 5) + SEG_SCRATCH_BYTES);             \
       SG_CK(smem_attr(k_fused_warp<L, MODE>, smem), "smem attr k_fused_warp");                 \
       prof_begin("k_fused_warp<" #L ">");                                                      \
       k_fused_warp<L, MODE><<<blocks_for(cnt, WPB, (long long)sms_ * 16), SW_THREADS, smem,    \
                               stream_>>>(op, rows + (size_t)b * m, cnt, row_span_.as<int2>(),  \
-                                         toff, c_cnt, t_col, t_val, mid_rows,                  \
-                                         &dc->fb_count[FB_MID], big_rows,                      \
-                                         &dc->fb_count[FB_BLOCK0 + 2], tn_.mid_cols,           \
-                                         rows + (size_t)FB_ESC0 * m, &dc->fb_count[FB_ESC0],   \
-                                         tn_, row_p, &dc->overflow_count);                     \
+                                         toff, c_cnt, t_col, t_val, rows, dc->fb_count, tn_,   \
+                                         row_p, &dc->overflow_count);                          \
       SG_LAUNCHED("k_fused_warp");                                                             \
     }                                                                                          \
   }
   SG_FUSED_WARP(6) SG_FUSED_WARP(7) SG_FUSED_WARP(8) SG_FUSED_WARP(9) SG_FUSED_WARP(10)
 #undef SG_FUSED_WARP
   // mid bitmap rows (and warp overflow with a narrow span)
-  if (fb_counts_[FB_MID] + overflow_bound > 0) {
+  if (fb_counts_[FB_MID] + may_overflow_[FB_MID] > 0) {
     const int width = std::min(n_, tn_.mid_cols) + 32;  // + alignment of lo down to 32
     const int dir_words = (width + 31) / 32;
     const int cap = (int)std::min<long long>(tn_.long_p, n_);
@@ -537,7 +534,7 @@ int Engine::launch_fused() {
                         (size_t)cap * (8 + sizeof(int)) + sizeof(unsigned) * ((dir_words + 31) / 32) +
                         sizeof(int) * (size_t)cap;
     SG_CK(smem_attr(k_num_long<MODE, MID_THREADS, true>, smem), "smem attr k_num_long fused");
-    const int grid = blocks_for(fb_counts_[FB_MID] + overflow_bound, 1, (long long)sms_ * 4);
+    const int grid = blocks_for(fb_counts_[FB_MID] + may_overflow_[FB_MID], 1, (long long)sms_ * 4);
     prof_begin("k_fused_mid");
     k_num_long<MODE, MID_THREADS, true><<<grid, MID_THREADS, smem, stream_>>>(
         op, nullptr, 0, row_p, dir_words, cap, restrict_scratch_.as<int>(), 0,
@@ -548,7 +545,7 @@ int Engine::launch_fused() {
 #define SG_FUSED_BLOCK(L, NT)                                                                 \
   {                                                                                            \
     const int b = L - 11 + FB_BLOCK0;                                                          \
-    const int bound = fb_counts_[b] + (L == 13 ? overflow_bound : 0);                          \
+    const int bound = fb_counts_[b] + may_overflow_[b];                                        \
     if (bound > 0) {                                                                           \
       const size_t smem = (size_t(1) << L) * (VB + 5) + (NT / 32) * SEG_SCRATCH_BYTES;         \
       SG_CK(smem_attr(k_fused_block<L, NT, MODE>, smem), "smem attr k_fused_block");           \
@@ -562,24 +559,36 @@ int Engine::launch_fused() {
   }
   SG_FUSED_BLOCK(11, 256) SG_FUSED_BLOCK(12, 256) SG_FUSED_BLOCK(13, 512)
 #undef SG_FUSED_BLOCK
-  // sorted rows (expand, sort, compress), one block per row; the lists may
-  // also hold warp rows that overflowed their tables
-#define SG_FUSED_ESC(Q, NT, PER_SM)                                                           \
+  // sorted rows (expand, sort, compress); the lists may also hold warp rows
+  // that overflowed their tables. Keys pack (column, position) into 32 bits
+  // when every column of B allows it.
+#define SG_FUSED_ESC_KEY(B, NT, SH, KEY)                                                      \
   {                                                                                            \
-    const int b = FB_ESC0 + Q, cnt = fb_counts_[b] + overflow_bound;                           \
+    const size_t smem = esc_smem_bytes<NT, SH, MODE, KEY>();                                   \
+    SG_CK((smem_attr(k_fused_esc<NT, SH, MODE, KEY>, smem)), "smem attr k_fused_esc");         \
+    constexpr int TEAMS = esc_teams<NT>(), RESIDENT = 2048 / (NT * TEAMS);                     \
+    prof_begin("k_fused_esc<" #NT ">");                                                        \
+    k_fused_esc<NT, SH, MODE, KEY>                                                             \
+        <<<blocks_for(cnt, TEAMS, (long long)sms_ * RESIDENT * 2), NT * TEAMS, smem,           \
+           stream_>>>(op, rows + (size_t)(B) * m, &dc->fb_count[B], row_p, toff,               \
+                      row_span_.as<int2>(), c_cnt, t_col, t_val, status);                      \
+    SG_LAUNCHED("k_fused_esc");                                                                \
+  }
+#define SG_FUSED_ESC(B, NT, SH)                                                               \
+  {                                                                                            \
+    const int cnt = fb_counts_[B] + may_overflow_[B];                                          \
     if (cnt > 0) {                                                                             \
-      const size_t smem = esc_smem_bytes<NT, MODE>();                                          \
-      SG_CK(smem_attr(k_fused_esc<NT, MODE>, smem), "smem attr k_fused_esc");                  \
-      prof_begin("k_fused_esc<" #NT ">");                                                      \
-      k_fused_esc<NT, MODE><<<blocks_for(cnt, 1, (long long)sms_ * (PER_SM)), NT, smem,        \
-                              stream_>>>(op, rows + (size_t)b * m, &dc->fb_count[b], row_p,    \
-                                         toff, row_span_.as<int2>(), c_cnt, t_col, t_val,      \
-                                         status);                                              \
-      SG_LAUNCHED("k_fused_esc");                                                              \
+      if (((long long)n_ << SH) <= (1ll << 32)) SG_FUSED_ESC_KEY(B, NT, SH, unsigned)          \
+      else SG_FUSED_ESC_KEY(B, NT, SH, unsigned long long)                                     \
     }                                                                                          \
   }
-  SG_FUSED_ESC(0, 128, 8) SG_FUSED_ESC(1, 256, 4) SG_FUSED_ESC(2, 512, MODE ? 1 : 2)
+  SG_FUSED_ESC(FB_ESC0 + 2, 512, 12)
+  SG_FUSED_ESC(FB_ESC0 + 1, 256, 11)
+  SG_FUSED_ESC(FB_ESC0, 128, 10)
+  SG_FUSED_ESC(FB_ESC512, 64, 9)
+  SG_FUSED_ESC(FB_ESC256, 32, 8)
 #undef SG_FUSED_ESC
+#undef SG_FUSED_ESC_KEY
   return 0;
 }
 

@@ -27,6 +27,7 @@ struct DevBuf {
 // synchronisation points.
 struct DevCounters {
   int fb_count[16];  // first-pass bins (rows per bin; mid / block lists grow on warp overflow)
+  int may_overflow[16];  // warp-bin rows that would be redone in each first-pass bin
   int num_count[16];
   int slice_count;
   int mid_count;
@@ -119,7 +120,10 @@ class Engine {
   long long nnz_c() const { return nnz_c_; }
   int m() const { return m_; }
   int n() const { return n_; }
-  int sym_bin_rows(int b) const { return fb_counts_[b]; }
+  // Rows of first-pass bin b as the statistics count them.
+  int sym_bin_rows(int b) const {
+    return fb_counts_[b] + (b == FB_ESC0 ? fb_counts_[FB_ESC256] + fb_counts_[FB_ESC512] : 0);
+  }
   int overflow_rows() const { return overflow_rows_; }
   int num_bin_rows(int b) const { return num_counts_[b]; }
   int slices() const { return nslices_; }
@@ -194,6 +198,7 @@ class Engine {
   int m_ = 0, kdim_ = 0, n_ = 0, n_chunks_ = 0;
   long long p_total_ = 0, nnz_c_ = 0;
   int fb_counts_[16] = {0};
+  int may_overflow_[16] = {0};
   long long temp_total_ = 0;
   int overflow_rows_ = 0;
   int num_counts_[16] = {0};

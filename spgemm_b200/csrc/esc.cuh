@@ -1,29 +1,22 @@
-// Fused pass by sorting: expand, sort, compress (ESC), one block per row.
+// Fused pass by sorting: expand, sort, compress (ESC), one team of threads
+// per row.
 //
 // The reference materialises every partial product of a row of C in its
 // bucket (src/mm.cu:288-312) and merges the bucket with a dense accumulator
-// (src/mm.cu:366-404). Rows of at most 4096 products whose column bound is
-// too large for a warp's hash table and whose columns spread over a wide
-// span (R-MAT rows of 2K-4K products) degrade both of this engine's other
-// fused accumulators: a block hash table sized for the bound, and a bitmap
-// over the span, which costs span/32 words per row for a few thousand
-// products. Measured on a B200, sorting costs several hash inserts per
-// product (gather, two or three radix passes, compression), so it serves
-// those rows only; rows a warp's table can hold stay hashed. Here the row's partials are written straight to shared memory at
-// their position in the row's flattened product sequence, sorted by column
-// with a stable LSD radix sort, and runs of equal columns are summed in that
-// stable order. No floating-point atomics are used, so the result is
-// deterministic: every run is summed in product order (entries of A in
-// order, each B row in order), in plain and in compensated mode.
+// (src/mm.cu:366-404). Rows of at most 4096 products whose columns hardly
+// repeat, or spread over a span too wide for a bitmap, degrade this engine's
+// other fused accumulators: a hash table fills up, and a bitmap costs its
+// span. Here the row's partials are written straight to shared memory at
+// their position in the row's flattened product sequence, ordered by (column,
+// position), and runs of equal columns are summed in that order. No
+// floating-point atomics are used, so the result is deterministic: every run
+// is summed in product order (entries of A in order, each B row in order), in
+// plain and in compensated mode.
 #pragma once
 
 #include "pipeline.cuh"
 
 namespace sg {
-
-constexpr int ESC_KPT = 8;             // products per thread: capacity NT * ESC_KPT
-constexpr int ESC_RADIX_BITS = 9;      // digit bits per radix pass (at most)
-constexpr int ESC_BUCKETS = 1 << ESC_RADIX_BITS;
 
 // Partial product as stored for the sort: plain FP32 value, or (rounded
 // product, its exact rounding error) for the compensated merge.
@@ -40,240 +33,202 @@ __device__ __forceinline__ float2 esc_value<1>(float a, float b) {
   return make_float2(p, __fmaf_rn(a, b, -p));  // TwoProduct: a*b == p + e exactly
 }
 
-// Products [f0, f1) of a row's flattened product sequence, one warp. Entry j
-// of the row holds positions aoff[j] .. aoff[j] + nnz(B(k_j,:)) - 1, so the
-// entries of a 32-entry batch cover one contiguous position range; the
-// product at position f is written to keys[f] (its column minus lo) and
-// vals[f]. Products are walked 32 at a time with the owner of each position
-// found from the OR of segment-start bits (as in run_segments), two windows
-// in flight.
-template <int MODE>
-__device__ __forceinline__ void warp_gather_range(const Operands& op, int rs, int re, int f0,
-                                                  int f1, int lo, unsigned* __restrict__ keys,
-                                                  typename EscVal<MODE>::T* __restrict__ vals,
-                                                  SegScratch* sc) {
-  const int lane = lane_id();
-  int l = rs, h = re;  // first entry whose offset is > f0
-  while (l < h) {
-    const int mid = (l + h) >> 1;
-    if (__ldg(op.aoff + mid) <= f0) l = mid + 1; else h = mid;
-  }
-  for (int base = max(l - 1, rs); base < re; base += 32) {
-    const int j = base + lane;
-    int bstart = 0, len = 0, pos0 = 0;
-    float a = 0.f;
-    bool past = true;
-    if (j < re) {
-      const int off = __ldg(op.aoff + j);
-      past = off >= f1;
-      if (!past) {
-        const int k = __ldg(op.a_col + j);
-        const int bs = __ldg(op.b_rowptr + k);
-        const int bl = __ldg(op.b_rowptr + k + 1) - bs;
-        const int s0 = max(off, f0), s1 = min(off + bl, f1);
-        if (s1 > s0) {
-          a = __ldg(op.a_val + j);
-          bstart = bs + (s0 - off);
-          len = s1 - s0;
-          pos0 = s0;
-        }
-      }
-    }
-    const bool done = __any_sync(FULL, past);
-    const unsigned ne = __ballot_sync(FULL, len > 0);
-    if (ne) {
-      const int start = __shfl_sync(FULL, pos0, __ffs(ne) - 1);
-      compact_segments(bstart, len, a, sc);
-      const int incl = warp_incl_scan(len);
-      const int total = __shfl_sync(FULL, incl, 31);
-      const int s = incl - len;
-      int nbefore = 0;
-      for (int wb = 0; wb < total; wb += 64) {
-        int col[2], dst[2];
-        float bv[2], oa[2];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int w = wb + 32 * u;
-          dst[u] = -1;
-          if (w < total) {  // warp-uniform
-            const unsigned bit = (len > 0 && s >= w && s < w + 32) ? (1u << (s - w)) : 0u;
-            const unsigned starts = __reduce_or_sync(FULL, bit);
-            const int owner = nbefore + __popc(starts & (FULL >> (31 - lane))) - 1;
-            nbefore += __popc(starts);
-            const int ob = __shfl_sync(FULL, bstart, owner);
-            const int os = __shfl_sync(FULL, s, owner);
-            oa[u] = __shfl_sync(FULL, a, owner);
-            const int fp = w + lane;
-            if (fp < total) {
-              const int pos = ob + (fp - os);
-              col[u] = __ldg(op.b_col + pos);
-              bv[u] = __ldg(op.b_val + pos);
-              dst[u] = start + fp;
-            }
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          if (dst[u] >= 0) {
-            keys[dst[u]] = (unsigned)(col[u] - lo);
-            vals[dst[u]] = esc_value<MODE>(oa[u], bv[u]);
-          }
-        }
-      }
-    }
-    if (done) break;
-  }
+// Threads that share a row: one warp (several teams to a block) or the block.
+template <int NT>
+__device__ __forceinline__ void team_sync() {
+  if (NT == 32) __syncwarp();
+  else __syncthreads();
 }
 
-// Stable LSD radix sort of (keys, vals)[0, n) by the low `bits` bits of the
-// key, one block of NT threads, n <= NT * ESC_KPT. Warp w owns groups
-// [w * gpw, (w + 1) * gpw) of 32 consecutive positions (gpw = groups per
-// warp); positions n .. NW * gpw * 32 - 1 must hold EMPTY_KEY (every digit
-// maximal, so they stay behind the row's keys). Per pass: each warp ranks
-// its keys by digit (match.any peers + per-warp counters, in position order),
-// one block scan turns the per-(digit, warp) counts into offsets, and every
-// key is scattered from registers to offset + rank. The sorted sequence ends
-// in buffer 0 or 1 (returned).
-template <int NT, class V>
-__device__ __forceinline__ int block_radix_sort(unsigned* __restrict__ k0, V* __restrict__ v0,
-                                                unsigned* __restrict__ k1, V* __restrict__ v1,
-                                                int n, int bits, int* __restrict__ hist,
-                                                long long* scan_shm) {
+// Sort key of a product: (column - lo) << SH | position, SH = log2 of the
+// row capacity, so equal columns keep their product order and the key names
+// its value, which never moves.
+//
+// Bucket of a key: the top bits of its column offset, about one bucket per
+// product. A key's place is its bucket's start plus the number of smaller
+// keys in the bucket, counted by the key's own thread: neighbouring threads
+// hold keys of the same bucket, so they read the same words. Counting is
+// quadratic in the bucket, so rows with a bucket of more than
+// esc_bucket_max(p) keys sort bitonically instead. A bitonic sort of p keys
+// is p/32 * log2(p)^2/2 * ~6 warp instructions (60K at 4096 keys, 1.7K at
+// 256); a bucket of s keys costs s^2/8 of them (41K at 576 keys, 1.2K at 96).
+__device__ __forceinline__ int esc_bucket_max(int p) { return 64 + (p >> 3); }
+
+// All products of a row into vals[pos] / keys[pos], pos = the product's
+// flattened position (entry j of the row holds aoff[j] .. aoff[j] +
+// nnz(B(k_j,:)) - 1), and their bucket counts. Entries are dealt to the
+// team's warps in turn; each warp loads 32 of them at once, then groups of
+// 2^lg lanes (about the mean B row length, so short rows do not idle a warp)
+// walk one entry each, two entries in flight. Columns beyond the row's span
+// (`width`; a replayed batch whose structure was changed) are clamped, which
+// keeps every index below in bounds.
+template <int NT, int SH, int MODE, class KEY>
+__device__ __forceinline__ void esc_gather(const Operands& op, int rs, int re, int p, int lo,
+                                           unsigned width, int shift, KEY* __restrict__ keys,
+                                           typename EscVal<MODE>::T* __restrict__ vals,
+                                           int* __restrict__ cnt) {
   constexpr int NW = NT / 32;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int groups = (n + 31) >> 5;
-  const int gpw = (groups + NW - 1) / NW;  // <= ESC_KPT
-  const int npass = (bits + ESC_RADIX_BITS - 1) / ESC_RADIX_BITS;
-  const int db = (bits + npass - 1) / npass;
-  const unsigned dmask = (1u << db) - 1u;
-  const int nb = 1 << db;
-  const unsigned lt = (1u << lane) - 1u;
-  int* wh = hist + warp * ESC_BUCKETS;
-  unsigned* sk = k0;
-  V* sv = v0;
-  unsigned* dk = k1;
-  V* dv = v1;
-  for (int pass = 0; pass < npass; ++pass) {
-    const int sh = pass * db;
-    for (int t = lane; t < nb; t += 32) wh[t] = 0;
-    __syncwarp();
-    unsigned k[ESC_KPT];
-    V v[ESC_KPT];
-    int rk[ESC_KPT];
+  const int lane = threadIdx.x & 31, warp = NT == 32 ? 0 : threadIdx.x >> 5;
+  const int mean = p / (re - rs);
+  const int lg = mean <= 4 ? 2 : (mean <= 8 ? 3 : (mean <= 16 ? 4 : 5));
+  const int groups = 32 >> lg, g = lane >> lg, gl = lane & ((1 << lg) - 1), step = 1 << lg;
+  for (int base = rs + warp; base < re; base += 32 * NW) {
+    const int j = base + NW * lane;
+    int bstart = 0, len = 0, off = 0;
+    float a = 0.f;
+    if (j < re) {
+      const int k = __ldg(op.a_col + j);
+      off = __ldg(op.aoff + j);
+      a = __ldg(op.a_val + j);
+      bstart = __ldg(op.b_rowptr + k);
+      len = __ldg(op.b_rowptr + k + 1) - bstart;
+    }
+    const int entries = min((re - base + NW - 1) / NW, 32);
+    for (int e0 = 0; e0 < entries; e0 += 2 * groups) {
+      int eb[2], el[2], eo[2], c[2];
+      float ea[2], v[2];
 #pragma unroll
-    for (int g = 0; g < ESC_KPT; ++g) {
-      if (g < gpw) {  // block-uniform
-        const int p = (warp * gpw + g) * 32 + lane;
-        k[g] = sk[p];
-        v[g] = sv[p];
-        const unsigned d = (k[g] >> sh) & dmask;
-        const unsigned peers = __match_any_sync(FULL, d);
-        const int before = wh[d];
-        rk[g] = before + __popc(peers & lt);
-        __syncwarp();
-        if ((peers & lt) == 0) wh[d] = before + __popc(peers);  // lowest peer
-        __syncwarp();
+      for (int u = 0; u < 2; ++u) {
+        const int e = e0 + u * groups + g;
+        eb[u] = __shfl_sync(FULL, bstart, e & 31);
+        el[u] = __shfl_sync(FULL, len, e & 31);
+        eo[u] = __shfl_sync(FULL, off, e & 31);
+        ea[u] = __shfl_sync(FULL, a, e & 31);
+        if (e >= entries) el[u] = 0;
       }
-    }
-    __syncthreads();
-    // exclusive scan of the counts in (digit, warp) order
-    const int E = nb * NW;
-    const int ept = (E + NT - 1) / NT;
-    const int e0 = threadIdx.x * ept;
-    int sum = 0;
-    for (int q = 0; q < ept; ++q) {
-      const int e = e0 + q;
-      if (e < E) sum += hist[(e % NW) * ESC_BUCKETS + e / NW];
-    }
-    long long tot;
-    int run = (int)block_excl_scan64(sum, scan_shm, tot);  // ends with a barrier
-    for (int q = 0; q < ept; ++q) {
-      const int e = e0 + q;
-      if (e < E) {
-        int* hp = hist + (e % NW) * ESC_BUCKETS + e / NW;
-        const int c = *hp;
-        *hp = run;
-        run += c;
-      }
-    }
-    __syncthreads();
+      for (int t = gl; t < max(el[0], el[1]); t += step) {
 #pragma unroll
-    for (int g = 0; g < ESC_KPT; ++g) {
-      if (g < gpw) {
-        const int pos = wh[(k[g] >> sh) & dmask] + rk[g];
-        dk[pos] = k[g];
-        dv[pos] = v[g];
+        for (int u = 0; u < 2; ++u) {
+          c[u] = 0;
+          v[u] = 0.f;
+          if (t < el[u]) {
+            c[u] = __ldg(op.b_col + eb[u] + t);
+            v[u] = __ldg(op.b_val + eb[u] + t);
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          if (t < el[u]) {
+            const unsigned x = min((unsigned)(c[u] - lo), width);
+            const int pos = eo[u] + t;
+            keys[pos] = ((KEY)x << SH) | (KEY)pos;
+            vals[pos] = esc_value<MODE>(ea[u], v[u]);
+            atomicAdd(cnt + (x >> shift), 1);
+          }
+        }
       }
     }
-    __syncthreads();
-    unsigned* tk = sk; sk = dk; dk = tk;
-    V* tv = sv; sv = dv; dv = tv;
   }
-  return npass & 1;
 }
 
-__device__ __forceinline__ float esc_run_sum(const float* v, const unsigned* k, int t, int n) {
-  const unsigned key = k[t];
-  float s = v[t];
-  for (int u = t + 1; u < n && k[u] == key; ++u) s = __fadd_rn(s, v[u]);
+// cnt[0, nb) to its exclusive prefix sums (nb a power of two, >= NT); returns
+// the largest count (to every thread). Ends with a barrier.
+template <int NT>
+__device__ __forceinline__ int esc_scan(int* __restrict__ cnt, int nb, int* warp_sums,
+                                        int* warp_max) {
+  constexpr int NW = NT / 32;
+  const int lane = threadIdx.x & 31, warp = NT == 32 ? 0 : threadIdx.x >> 5;
+  const int tid = NT == 32 ? lane : threadIdx.x;
+  const int per = nb / NT;
+  int* mine = cnt + tid * per;
+  int sum = 0, mx = 0;
+  for (int q = 0; q < per; ++q) {
+    const int c = mine[q];
+    sum += c;
+    mx = max(mx, c);
+  }
+  const int incl = warp_incl_scan(sum);
+  mx = __reduce_max_sync(FULL, mx);
+  int run = incl - sum;
+  if (NW > 1) {
+    if (lane == 31) {
+      warp_sums[warp] = incl;
+      warp_max[warp] = mx;
+    }
+    __syncthreads();
+    const int s = lane < NW ? warp_sums[lane] : 0;
+    const int m = lane < NW ? warp_max[lane] : 0;
+    const int wi = warp_incl_scan(s);
+    run += __shfl_sync(FULL, wi - s, warp);
+    mx = __reduce_max_sync(FULL, m);
+  }
+  for (int q = 0; q < per; ++q) {
+    const int c = mine[q];
+    mine[q] = run;
+    run += c;
+  }
+  team_sync<NT>();
+  return mx;
+}
+
+template <int SH, class KEY>
+__device__ __forceinline__ float esc_run_sum(const float* v, const KEY* k, int t, int n) {
+  constexpr unsigned MASK = (1u << SH) - 1u;
+  const KEY col = k[t] >> SH;
+  float s = v[(unsigned)k[t] & MASK];
+  for (int u = t + 1; u < n && (k[u] >> SH) == col; ++u) s = __fadd_rn(s, v[(unsigned)k[u] & MASK]);
   return s;
 }
 
 // Compensated run sum (Dot2): TwoSum of the rounded products, their rounding
 // errors and the TwoSum errors collected in a second word.
-__device__ __forceinline__ float esc_run_sum(const float2* v, const unsigned* k, int t, int n) {
-  const unsigned key = k[t];
-  float s = v[t].x, c = v[t].y;
-  for (int u = t + 1; u < n && k[u] == key; ++u) {
-    const float p = v[u].x;
-    const float ns = __fadd_rn(s, p);
-    c = __fadd_rn(c, __fadd_rn(two_sum_err(s, p, ns), v[u].y));
+template <int SH, class KEY>
+__device__ __forceinline__ float esc_run_sum(const float2* v, const KEY* k, int t, int n) {
+  constexpr unsigned MASK = (1u << SH) - 1u;
+  const KEY col = k[t] >> SH;
+  const float2 f = v[(unsigned)k[t] & MASK];
+  float s = f.x, c = f.y;
+  for (int u = t + 1; u < n && (k[u] >> SH) == col; ++u) {
+    const float2 q = v[(unsigned)k[u] & MASK];
+    const float ns = __fadd_rn(s, q.x);
+    c = __fadd_rn(c, __fadd_rn(two_sum_err(s, q.x, ns), q.y));
     s = ns;
   }
   return __fadd_rn(s, c);
 }
 
-// Compression of the sorted (keys, vals)[0, p) into one output per run of
-// equal keys (the run's key and its sum, summed in order by the run's first
-// thread), in key order. Warp w takes its groups [w * gpw, (w + 1) * gpw)
-// of 32 positions; the outputs before them come from the per-warp run
-// counts (one barrier). Returns the number of outputs.
-template <int NT, class V>
-__device__ __forceinline__ int block_compress(const unsigned* __restrict__ ks,
-                                              const V* __restrict__ vs, int p, int gpw, int lo,
-                                              int* __restrict__ out_col, float* __restrict__ out_val,
-                                              int* warp_runs) {
+// Compression of the ordered keys[0, p) into one output per run of equal
+// columns (summed in order by the run's first thread). Warp w takes its
+// groups [w * gpw, (w + 1) * gpw) of 32 positions; the outputs before them
+// come from the per-warp run counts (one barrier). Returns the number of
+// outputs.
+template <int NT, int SH, class KEY, class V>
+__device__ __forceinline__ int esc_compress(const KEY* __restrict__ ks, const V* __restrict__ vs,
+                                            int p, int lo, int* __restrict__ out_col,
+                                            float* __restrict__ out_val, int* warp_runs) {
   constexpr int NW = NT / 32;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int GPW = (1 << SH) / NT;
+  const int lane = threadIdx.x & 31, warp = NT == 32 ? 0 : threadIdx.x >> 5;
+  const int gpw = ((p + 31) / 32 + NW - 1) / NW;
   const unsigned lt = (1u << lane) - 1u;
-  unsigned hm[ESC_KPT];
+  unsigned hm[GPW];
   int mine = 0;
 #pragma unroll
-  for (int g = 0; g < ESC_KPT; ++g) {
+  for (int g = 0; g < GPW; ++g) {
     hm[g] = 0u;
-    if (g < gpw) {  // block-uniform
+    if (g < gpw) {  // team-uniform
       const int t = (warp * gpw + g) * 32 + lane;
-      hm[g] = __ballot_sync(FULL, t < p && (t == 0 || ks[t - 1] != ks[t]));
+      hm[g] = __ballot_sync(FULL, t < p && (t == 0 || (ks[t - 1] >> SH) != (ks[t] >> SH)));
       mine += __popc(hm[g]);
     }
   }
-  if (lane == 0) warp_runs[warp] = mine;
-  __syncthreads();
-  int run = 0, total = 0;
-#pragma unroll
-  for (int w = 0; w < NW; ++w) {
-    const int c = warp_runs[w];
-    run += w < warp ? c : 0;
-    total += c;
+  int run = 0, total = mine;
+  if (NW > 1) {
+    if (lane == 0) warp_runs[warp] = mine;
+    __syncthreads();
+    const int c = lane < NW ? warp_runs[lane] : 0;
+    const int incl = warp_incl_scan(c);
+    run = __shfl_sync(FULL, incl - c, warp);
+    total = __shfl_sync(FULL, incl, 31);
   }
 #pragma unroll
-  for (int g = 0; g < ESC_KPT; ++g) {
+  for (int g = 0; g < GPW; ++g) {
     if (g < gpw) {
       const int t = (warp * gpw + g) * 32 + lane;
       if ((hm[g] >> lane) & 1u) {
         const int o = run + __popc(hm[g] & lt);
-        out_col[o] = lo + (int)ks[t];
-        out_val[o] = esc_run_sum(vs, ks, t, p);
+        out_col[o] = lo + (int)(ks[t] >> SH);
+        out_val[o] = esc_run_sum<SH>(vs, ks, t, p);
       }
       run += __popc(hm[g]);
     }
@@ -281,38 +236,49 @@ __device__ __forceinline__ int block_compress(const unsigned* __restrict__ ks,
   return total;
 }
 
-// Rows of P_i <= NT * ESC_KPT products from the bin list, one block per row:
-// gather, radix sort of the column offsets (as many bits as the row's span
-// needs), compression of equal columns, sorted row written to the temporary
-// buffer at toff[i] with its length in c_cnt[i].
-//
-// Shared memory: vals[2][CAP] | keys[2][CAP] | hist[NW][ESC_BUCKETS] |
-// SegScratch[NW].
-template <int NT, int MODE>
-__global__ void __launch_bounds__(NT, NT <= 128 ? 8 : (NT <= 256 ? 4 : (MODE ? 1 : 2)))
+// Teams of one warp share a block of 128 threads; larger teams are a block.
+template <int NT>
+__host__ __device__ constexpr int esc_teams() { return NT == 32 ? 4 : 1; }
+
+// Shared memory of one team: vals[CAP] | keys[2][CAP] | buckets[CAP].
+template <int SH, int MODE, class KEY>
+__host__ __device__ constexpr size_t esc_team_bytes() {
+  return ((size_t)1 << SH) * (sizeof(typename EscVal<MODE>::T) + 2 * sizeof(KEY) + sizeof(int));
+}
+
+// Dynamic shared memory of k_fused_esc.
+template <int NT, int SH, int MODE, class KEY>
+constexpr size_t esc_smem_bytes() {
+  return esc_teams<NT>() * esc_team_bytes<SH, MODE, KEY>();
+}
+
+// Rows of P_i <= 2^SH products from the bin list: gather, order by bucket,
+// compress, sorted row written to the temporary buffer at toff[i] with its
+// length in c_cnt[i]. Eight products a thread.
+template <int NT, int SH, int MODE, class KEY>
+__global__ void __launch_bounds__(NT * esc_teams<NT>(), 1536 / (NT * esc_teams<NT>()))
 k_fused_esc(Operands op, const int* __restrict__ rows, const int* __restrict__ nrows_p,
             const long long* __restrict__ row_p, const long long* __restrict__ toff,
             const int2* __restrict__ row_span, int* __restrict__ c_cnt,
             int* __restrict__ t_col, float* __restrict__ t_val, unsigned* status) {
-  constexpr int NW = NT / 32;
-  constexpr int CAP = NT * ESC_KPT;
+  constexpr int CAP = 1 << SH, TEAMS = esc_teams<NT>();
   using V = typename EscVal<MODE>::T;
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ long long scan_shm[33];
-  __shared__ int warp_runs[NW];
-  const int warp = threadIdx.x >> 5;
-  V* v0 = reinterpret_cast<V*>(smem);
-  V* v1 = v0 + CAP;
-  unsigned* k0 = reinterpret_cast<unsigned*>(v1 + CAP);
-  unsigned* k1 = k0 + CAP;
-  int* hist = reinterpret_cast<int*>(k1 + CAP);
-  SegScratch* sc = reinterpret_cast<SegScratch*>(hist + NW * ESC_BUCKETS) + warp;
+  __shared__ int warp_a[32], warp_b[32], warp_c[32];
+  const int lane = threadIdx.x & 31;
+  const int team = TEAMS > 1 ? threadIdx.x >> 5 : 0;
+  const int tid = TEAMS > 1 ? lane : threadIdx.x;
+  unsigned char* mem = smem + team * esc_team_bytes<SH, MODE, KEY>();
+  KEY* k0 = reinterpret_cast<KEY*>(mem);
+  KEY* k1 = k0 + CAP;
+  V* vals = reinterpret_cast<V*>(k1 + CAP);
+  int* cnt = reinterpret_cast<int*>(vals + CAP);
   const int nrows = *nrows_p;
-  for (int r = blockIdx.x; r < nrows; r += gridDim.x) {
+  for (int r = blockIdx.x * TEAMS + team; r < nrows; r += gridDim.x * TEAMS) {
     const int i = rows[r];
     const long long p64 = row_p[i];
-    if (p64 > CAP || p64 <= 0) {  // the binning prevents this (block-uniform)
-      if (threadIdx.x == 0) {
+    if (p64 > CAP || p64 <= 0) {  // the binning prevents this (team-uniform)
+      if (tid == 0) {
         if (p64 > CAP) atomicOr(status, ST_SLICE_OVERFLOW);
         c_cnt[i] = 0;
       }
@@ -321,31 +287,46 @@ k_fused_esc(Operands op, const int* __restrict__ rows, const int* __restrict__ n
     const int p = (int)p64;
     const int2 sp = row_span[i];
     const int lo = sp.x;
-    const unsigned width = (unsigned)(sp.y - sp.x);  // largest key
+    const unsigned width = (unsigned)(sp.y - lo);  // largest column offset
     const int bits = width ? 32 - __clz(width) : 1;
+    const int nbits = max(p > 1 ? 32 - __clz(p - 1) : 0, 31 - __clz(NT));  // <= SH
+    const int nb = 1 << nbits;
+    const int shift = max(bits - nbits, 0);
     const int rs = op.a_rowptr[i], re = op.a_rowptr[i + 1];
-    const int U = chunk_for(p, NW, CAP);
-    for (int f = warp * U; f < p; f += NW * U)
-      warp_gather_range<MODE>(op, rs, re, f, min(f + U, p), lo, k0, v0, sc);
-    const int gpw = (((p + 31) >> 5) + NW - 1) / NW;
-    for (int t = p + threadIdx.x; t < NW * gpw * 32; t += NT) k0[t] = EMPTY_KEY;
-    __syncthreads();
-    const int which = block_radix_sort<NT>(k0, v0, k1, v1, p, bits, hist, scan_shm);
-    const unsigned* ks = which ? k1 : k0;
-    const V* vs = which ? v1 : v0;
+    for (int t = tid; t < nb; t += NT) cnt[t] = 0;
+    team_sync<NT>();
+    esc_gather<NT, SH, MODE, KEY>(op, rs, re, p, lo, width, shift, k0, vals, cnt);
+    team_sync<NT>();
+    const int mx = esc_scan<NT>(cnt, nb, warp_a, warp_b);
+    if (mx <= esc_bucket_max(p)) {  // team-uniform
+      for (int t = tid; t < p; t += NT) {
+        const KEY k = k0[t];
+        k1[atomicAdd(cnt + (int)((k >> SH) >> shift), 1)] = k;
+      }
+      team_sync<NT>();  // bucket b now ends at cnt[b]
+      for (int t = tid; t < p; t += NT) {
+        const KEY k = k1[t];
+        const int b = (int)((k >> SH) >> shift);
+        const int s0 = b ? cnt[b - 1] : 0, s1 = cnt[b];
+        int place = s0;
+        if (s1 - s0 > 1)
+          for (int q = s0; q < s1; ++q) place += k1[q] < k;
+        k0[place] = k;
+      }
+    } else {
+      int n2 = 1;
+      while (n2 < p) n2 <<= 1;
+      for (int t = p + tid; t < n2; t += NT) k0[t] = ~(KEY)0;
+      team_sync<NT>();
+      if (NT == 32) bitonic_sort_keys_rt(k0, n2, tid, NT, WarpSync());
+      else bitonic_sort_keys_rt(k0, n2, tid, NT, BlockSync());
+    }
+    team_sync<NT>();
     const long long base = toff[i];
-    const int total = block_compress<NT>(ks, vs, p, gpw, lo, t_col + base, t_val + base,
-                                         warp_runs);
-    if (threadIdx.x == 0) c_cnt[i] = total;
-    __syncthreads();  // the buffers and run counts are reused by the block's next row
+    const int total = esc_compress<NT, SH>(k0, vals, p, lo, t_col + base, t_val + base, warp_c);
+    if (tid == 0) c_cnt[i] = total;
+    team_sync<NT>();  // the buffers are reused by the team's next row
   }
-}
-
-// Dynamic shared memory of k_fused_esc<NT, MODE>.
-template <int NT, int MODE>
-constexpr size_t esc_smem_bytes() {
-  return (size_t)NT * ESC_KPT * 2 * (sizeof(typename EscVal<MODE>::T) + sizeof(unsigned)) +
-         (size_t)(NT / 32) * ESC_BUCKETS * sizeof(int) + (size_t)(NT / 32) * sizeof(SegScratch);
 }
 
 }  // namespace sg

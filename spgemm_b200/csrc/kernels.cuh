@@ -67,15 +67,18 @@ struct Operands {
 //   9     symbolic bitmap count (k_sym_long), numeric later
 // and, for rows the warp bins do not take, ahead of the mid and block bins
 // when the tuning enables it (the default):
-//   10..12 one block of 128 / 256 / 512 threads per row of at most 1024 /
-//         2048 / 4096 products, sorted instead of hashed (k_fused_esc)
+//   10..12 rows of at most 1024 / 2048 / 4096 products, sorted instead of
+//         hashed (k_fused_esc), one block of 128 / 256 / 512 threads per row;
+//         rows of at most 256 (one warp) and 512 products (64 threads) have
+//         lists of their own, 13 and 14, and count as bin 10 in the statistics
 constexpr int FB_WARP_BINS = 5;
 constexpr int FB_BLOCK0 = 5;
 constexpr int FB_MID = 8;
 constexpr int FB_LONG = 9;
 constexpr int FB_ESC0 = 10;
-constexpr int FB_ESC_BINS = 3;
-constexpr int FB_COUNT = 13;
+constexpr int FB_ESC256 = 13, FB_ESC512 = 14;
+constexpr int FB_COUNT = 15;
+constexpr int FB_STAT_COUNT = 13;  // bins of the statistics
 // Numeric bins of long rows: 4..7 block hash (2^10..2^13 slots), 8 column
 // slices, 9 bitmap of the whole span (statistics slots 0..3 stay unused).
 constexpr int NB_COUNT = 10;
@@ -129,6 +132,13 @@ __host__ __device__ inline long long row_cap(long long p, int n, int span) {
   return c < span ? c : span;
 }
 
+// Sorted bin of a row of p <= 4096 products.
+__host__ __device__ inline int esc_bin_of(long long p) {
+  if (p <= 256) return FB_ESC256;
+  if (p <= 512) return FB_ESC512;
+  return p <= 1024 ? FB_ESC0 : (p <= 2048 ? FB_ESC0 + 1 : FB_ESC0 + 2);
+}
+
 __host__ __device__ inline int first_bin_of(long long p, long long cap, int span, const Tuning& t) {
   if (p <= 0) return -1;
   if (p > t.long_p) return FB_LONG;
@@ -140,11 +150,19 @@ __host__ __device__ inline int first_bin_of(long long p, long long cap, int span
     return lg - 6;
   }
   if (p > t.esc_p_min && span > t.esc_span_min)  // p <= long_p <= 4096
-    return p <= 1024 ? FB_ESC0 : (p <= 2048 ? FB_ESC0 + 1 : FB_ESC0 + 2);
+    return esc_bin_of(p);
   if (span <= t.mid_cols) return FB_MID;
   int lg = ceil_log2_ll(2 * cap);
   if (lg < 11) lg = 11;
   return lg - 11 + FB_BLOCK0;  // cap <= p <= long_p <= 4096, so lg <= 13
+}
+
+// Where a warp-bin row whose table overflows is redone: the sorted bins when
+// the tuning sorts rows like it, else the span bitmap or the largest block
+// table. `lo`: first column of the row's span.
+__host__ __device__ inline int overflow_bin_of(long long p, int lo, int span, const Tuning& t) {
+  if (p > t.esc_p_min && span > t.esc_span_min && p <= 4096) return esc_bin_of(p);
+  return span + (lo & 31) <= t.mid_cols ? FB_MID : FB_BLOCK0 + 2;
 }
 
 // Numeric bin of a long row (P_i > long_p) with nnz_i outputs.
@@ -810,8 +828,8 @@ __device__ __forceinline__ void bitonic_sort_kv_rt(unsigned* keys, V* vals, int 
 
 // bitonic_sort_kv_rt for keys alone (n a power of two, keys unique or padded
 // with EMPTY_KEY), by the threads of one warp or block.
-template <class Sync>
-__device__ __forceinline__ void bitonic_sort_keys_rt(unsigned* keys, int n, int tid, int nthreads,
+template <class K, class Sync>
+__device__ __forceinline__ void bitonic_sort_keys_rt(K* keys, int n, int tid, int nthreads,
                                                      Sync sync) {
   for (int k = 2; k <= n; k <<= 1) {
     for (int j = k >> 1; j > 0; j >>= 1) {
@@ -819,7 +837,7 @@ __device__ __forceinline__ void bitonic_sort_keys_rt(unsigned* keys, int n, int 
         const int lo = ((t & ~(j - 1)) << 1) | (t & (j - 1));
         const int hi = lo + j;
         const bool up = (lo & k) == 0;
-        const unsigned kl = keys[lo], kh = keys[hi];
+        const K kl = keys[lo], kh = keys[hi];
         if ((kl > kh) == up) {
           keys[lo] = kh;
           keys[hi] = kl;

@@ -93,22 +93,23 @@ constexpr int RA_UNROLL = 4;  // 32-entry batches of a row in flight together
 // the flattened offset of each A entry, the column span of the row's
 // products, the first-pass bin, and tcap[i] = the column bound min(P_i, n,
 // span_i) for rows the fused pass computes (0 otherwise), which sizes their
-// slot in the temporary output buffer. Rows are appended to their bin's list
+// slot in the temporary output buffer. may_overflow[b] counts the warp-bin
+// rows that go to bin b should their table overflow. Rows are appended to their bin's list
 // with one global atomic per bin per block. B's pointers are range-checked
 // here because the validation pass's result is only read after this kernel.
 __global__ void __launch_bounds__(RA_THREADS)
 k_row_analysis(Operands op, int* __restrict__ aoff, long long* __restrict__ row_p,
                int* __restrict__ c_cnt, int* __restrict__ tcap, int* __restrict__ fb_count,
-               int* __restrict__ fb_rows, unsigned long long* __restrict__ p_total,
+               int* __restrict__ may_overflow, int* __restrict__ fb_rows, unsigned long long* __restrict__ p_total,
                int* __restrict__ max_row_len, int2* __restrict__ row_span, unsigned* status,
                Tuning tn) {
-  __shared__ int hist[FB_COUNT], base[FB_COUNT];
+  __shared__ int hist[FB_COUNT], base[FB_COUNT], ovf[FB_COUNT];
   __shared__ int rowbin[RA_ROWS], rowrank[RA_ROWS];
   __shared__ unsigned long long block_p;
   __shared__ int block_max_len;  // longest A row of the block (one global atomic per block)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row0 = blockIdx.x * RA_ROWS;
-  if (threadIdx.x < FB_COUNT) hist[threadIdx.x] = 0;
+  if (threadIdx.x < FB_COUNT) hist[threadIdx.x] = ovf[threadIdx.x] = 0;
   if (threadIdx.x == 0) {
     block_p = 0;
     block_max_len = 0;
@@ -215,12 +216,17 @@ k_row_analysis(Operands op, int* __restrict__ aoff, long long* __restrict__ row_
       tcap[i] = (bin >= 0 && bin != FB_LONG) ? (int)cap : 0;
       rowbin[lr] = bin;
       if (bin >= 0) rowrank[lr] = atomicAdd(&hist[bin], 1);
+      // a table smaller than 1.25 x the column bound may overflow
+      if (bin >= 0 && bin < FB_WARP_BINS && cap + cap / 4 + 1 > (64ll << bin))
+        atomicAdd(&ovf[overflow_bin_of(acc, lo, span, tn)], 1);
       atomicAdd(&block_p, (unsigned long long)acc);
     }
   }
   __syncthreads();
   if (threadIdx.x < FB_COUNT && hist[threadIdx.x])
     base[threadIdx.x] = atomicAdd(fb_count + threadIdx.x, hist[threadIdx.x]);
+  if (threadIdx.x < FB_COUNT && ovf[threadIdx.x])
+    atomicAdd(may_overflow + threadIdx.x, ovf[threadIdx.x]);
   if (threadIdx.x == 0) {
     atomicAdd(p_total, block_p);
     if (block_max_len > 0) atomicMax(max_row_len, block_max_len);
@@ -269,9 +275,7 @@ __global__ void __launch_bounds__(SW_THREADS, LOG2T >= 10 ? 2 : 4)
 k_fused_warp(Operands op, const int* __restrict__ rows, int nrows,
              const int2* __restrict__ row_span, const long long* __restrict__ toff,
              int* __restrict__ c_cnt, int* __restrict__ t_col, float* __restrict__ t_val,
-             int* __restrict__ mid_rows, int* __restrict__ mid_count,
-             int* __restrict__ big_rows, int* __restrict__ big_count, int mid_cols,
-             int* __restrict__ esc_rows, int* __restrict__ esc_count, Tuning tn,
+             int* fb_rows, int* fb_count, Tuning tn,
              const long long* __restrict__ row_p, int* __restrict__ overflow_count) {
   constexpr int T = 1 << LOG2T;
   constexpr int LIMIT = T * 4 / 5;
@@ -299,15 +303,8 @@ k_fused_warp(Operands op, const int* __restrict__ rows, int nrows,
     if (distinct > LIMIT) {  // redo with a larger structure
       if (lane == 0) {
         const int2 sp = row_span[i];
-        const long long p = row_p[i];
-        if (p > tn.esc_p_min && sp.y + 1 - sp.x > tn.esc_span_min && p <= 4096) {
-          const int q = p <= 1024 ? 0 : (p <= 2048 ? 1 : 2);  // sorted bins, as first_bin_of
-          esc_rows[(size_t)q * op.m + atomicAdd(esc_count + q, 1)] = i;
-        } else if (sp.y + 1 - (sp.x & ~31) <= mid_cols) {
-          mid_rows[atomicAdd(mid_count, 1)] = i;
-        } else {
-          big_rows[atomicAdd(big_count, 1)] = i;
-        }
+        const int q = overflow_bin_of(row_p[i], sp.x, sp.y + 1 - sp.x, tn);
+        fb_rows[(size_t)q * op.m + atomicAdd(fb_count + q, 1)] = i;
         atomicAdd(overflow_count, 1);
       }
       continue;

@@ -1,0 +1,70 @@
+"""Row kernels of the fused pass at the sizes where they can go wrong: every
+product count around a bin's capacity, columns spread evenly or crowded into a
+few neighbours, and column spans around the limits of the packed sort keys.
+Structure is compared exactly and values within the stated bounds of
+helpers.py, against the FP64 oracle."""
+import numpy as np
+import pytest
+
+import spgemm_b200 as sg
+from spgemm_b200 import workloads as W
+from helpers import assert_structure_equal, assert_values_close, compensated_tolerance, plain_tolerance
+from test_gpu_parity import ref_product
+
+pytestmark = pytest.mark.gpu
+
+COUNTS = [1, 2, 7, 8, 9, 15, 16, 17, 31, 32, 33, 63, 64, 65, 127, 128, 129, 204, 205, 255, 256, 257, 511, 512,
+          513, 1023, 1024, 1025, 2047, 2048, 2049, 4095, 4096]
+
+
+def rows_of(counts, n, lengths, crowd, seed, empty=0):
+    """A and B such that row i of A*B has counts[i] products, from rows of B of
+    the given lengths in turn (the last one cut to fit) and `empty` empty rows
+    of B spread among them. Columns: distinct in a row of B, uniform in [0, n),
+    or (crowd) within 64 neighbours but for one far column in each row."""
+    rng = np.random.default_rng(seed)
+    ar, ac, br, bc, k = [], [], [], [], 0
+    for i, count in enumerate(counts):
+        left, turn, used = count, 0, []
+        while left > 0:
+            size = min(lengths[turn % len(lengths)], left, 60 if crowd else n)
+            if crowd:
+                cols = np.concatenate([n // 3 + rng.choice(64, size - 1, replace=False), [n - 1 - i]])
+            else:
+                cols = rng.choice(n, size, replace=False) if n < 10000 else np.unique(rng.integers(0, n, 4 * size))
+                cols = rng.permutation(cols)[:size]
+            br += [k] * size
+            bc += sorted(cols.tolist())
+            used.append(k)
+            k += 1
+            left -= size
+            turn += 1
+        used += list(range(k, k + empty))
+        k += empty
+        ar += [i] * len(used)
+        ac += used
+    vals = lambda size: rng.uniform(-1, 1, size).astype(np.float32)
+    A = W.from_coo(len(counts), k, np.array(ar), np.array(ac), vals(len(ar)))
+    B = W.from_coo(k, n, np.array(br), np.array(bc), vals(len(br)))
+    return A, B
+
+
+def check_rows(A, B, precision, tuning):
+    ref = ref_product(A, B)
+    with sg.Handle(precision) as h:
+        h.set_tuning(**tuning)
+        C = h.multiply_host(A, B)
+        stats = h.stats()
+    assert_structure_equal(C.rowptr, C.col, ref["rowptr"], ref["col"])
+    tol = plain_tolerance(ref) if precision == sg.PLAIN else compensated_tolerance(ref)
+    assert_values_close(C.val, ref, tol)
+    return stats
+
+
+@pytest.mark.parametrize("precision", [sg.PLAIN, sg.COMPENSATED])
+@pytest.mark.parametrize("n", [5003, (1 << 20) + 77, 1 << 25])
+@pytest.mark.parametrize("lengths,crowd", [((1,), False), ((13, 40, 3), False), ((60, 5), True)])
+def test_sorted_rows_around_their_capacities(precision, n, lengths, crowd):
+    A, B = rows_of(COUNTS, n, lengths, crowd, seed=len(lengths))
+    stats = check_rows(A, B, precision, dict(warp_cap_max=0))
+    assert sum(stats["rows_per_symbolic_bin"][10:13]) == len(COUNTS), stats
