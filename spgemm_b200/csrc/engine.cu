@@ -16,6 +16,7 @@
 
 #include "esc.cuh"
 #include "pipeline.cuh"
+#include "warp_rows.cuh"
 
 namespace sg {
 
@@ -344,7 +345,7 @@ int Engine::analyze(const cm& A, const cm& B) {
   // ---- row analysis ----
   SG_CK(aoff_.ensure(sizeof(int) * (size_t)std::max(nnz_a, 1)), "alloc aoff");
   SG_CK(row_p_.ensure(sizeof(long long) * (size_t)std::max(m, 1)), "alloc row_p");
-  SG_CK(sym_rows_.ensure(sizeof(int) * (size_t)FB_COUNT * std::max(m, 1)), "alloc bin lists");
+  SG_CK(sym_rows_.ensure(sizeof(int) * (size_t)FB_LISTS * std::max(m, 1)), "alloc bin lists");
   SG_CK(row_span_.ensure(sizeof(int2) * (size_t)std::max(m, 1)), "alloc row spans");
   SG_CK(tcap_.ensure(sizeof(int) * (size_t)std::max(m, 1)), "alloc row bounds");
   SG_CK(toff_.ensure(sizeof(long long) * ((size_t)m + 1)), "alloc temp offsets");
@@ -355,8 +356,8 @@ int Engine::analyze(const cm& A, const cm& B) {
     prof_begin("k_row_analysis");
     k_row_analysis<<<(m + RA_ROWS - 1) / RA_ROWS, RA_THREADS, 0, stream_>>>(
         op_, aoff_.as<int>(), row_p_.as<long long>(), c_cnt_.as<int>(), tcap_.as<int>(),
-        dc->fb_count, dc->may_overflow, sym_rows_.as<int>(), &dc->p_total, &dc->max_row_len, row_span_.as<int2>(),
-        &dc->status, tn_);
+        dc->fb_count, dc->may_overflow, dc->warp_stat, sym_rows_.as<int>(),
+        &dc->p_total, &dc->max_row_len, row_span_.as<int2>(), &dc->status, tn_);
     SG_LAUNCHED("k_row_analysis");
   }
   // temporary-buffer slots of the fused rows (grand total = buffer size)
@@ -374,6 +375,7 @@ int Engine::analyze(const cm& A, const cm& B) {
     fb_counts_[b] = host_counters_->fb_count[b];
     may_overflow_[b] = host_counters_->may_overflow[b];
   }
+  for (int b = 0; b < FB_WARP_BINS; ++b) warp_stat_[b] = host_counters_->warp_stat[b];
   n_long_sym_ = fb_counts_[FB_LONG];
   max_row_len_ = host_counters_->max_row_len;
   temp_total_ = host_counters_->grand_total;
@@ -509,6 +511,34 @@ int Engine::launch_fused() {
   int* t_col = t_col_.as<int>();
   float* t_val = t_val_.as<float>();
   int* mid_rows = rows + (size_t)FB_MID * m;
+  // start of a list that shares another's memory from its end (fb_list_at)
+  auto shared_list = [&](int b) {
+    return rows + (fb_counts_[b] > 0 ? fb_list_at(b, fb_counts_[b] - 1, m) : 0);
+  };
+  // rows of at most 32 products, in registers
+  {
+    const int n32 = fb_counts_[FB_TINY32], n16 = fb_counts_[FB_TINY16], n8 = fb_counts_[FB_TINY8];
+    auto blocks = [&](int cnt, int g) {
+      return cnt > 0 ? blocks_for(cnt, TINY_THREADS / g, (long long)sms_ * 32) : 0;
+    };
+    const TinyLists li{shared_list(FB_TINY32), shared_list(FB_TINY16), shared_list(FB_TINY8),
+                       n32, n16, n8, blocks(n32, 32), blocks(n16, 16), blocks(n8, 8)};
+    if (n32 + n16 + n8 > 0) {
+      prof_begin("k_fused_tiny");
+      k_fused_tiny<MODE><<<li.blocks32 + li.blocks16 + li.blocks8, TINY_THREADS, 0, stream_>>>(
+          op, li, row_span_.as<int2>(), toff, c_cnt, t_col, t_val);
+      SG_LAUNCHED("k_fused_tiny");
+    }
+  }
+  // rows with a narrow span, in a warp's bitmap
+  if (const int cnt = fb_counts_[FB_BITS]) {
+    prof_begin("k_fused_bits");
+    k_fused_bits<MODE><<<blocks_for(cnt, BITS_THREADS / 32, (long long)sms_ * 32), BITS_THREADS, 0,
+                         stream_>>>(op, shared_list(FB_BITS), cnt, row_span_.as<int2>(), toff,
+                                    row_p, c_cnt, t_col, t_val, rows, dc->fb_count, tn_,
+                                    &dc->overflow_count);
+    SG_LAUNCHED("k_fused_bits");
+  }
 #define SG_FUSED_WARP(L)                                                                      \
   {                                                                                            \
     const int b = L - 6, cnt = fb_counts_[b];                                                  \

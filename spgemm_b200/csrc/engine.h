@@ -26,8 +26,9 @@ struct DevBuf {
 // Device-side counters, reset once per product and read back at the two
 // synchronisation points.
 struct DevCounters {
-  int fb_count[16];  // first-pass bins (rows per bin; mid / block lists grow on warp overflow)
-  int may_overflow[16];  // warp-bin rows that would be redone in each first-pass bin
+  int fb_count[24];  // first-pass bins (rows per bin; mid / block / sorted lists grow on overflow)
+  int may_overflow[24];  // warp-bin rows that would be redone in each first-pass bin
+  int warp_stat[8];      // rows of each warp bin listed outside it (bins 15..)
   int num_count[16];
   int slice_count;
   int mid_count;
@@ -104,7 +105,7 @@ class Engine {
   int read_status(unsigned* st);
   const long long* rowptr64() const { return c_rowptr64_.as<long long>(); }
   // After analyze(): products per row (int64) and the row list of first-pass
-  // bin b (sym_bin_rows(b) entries).
+  // bin b (mid and long rows: sym_bin_rows(b) entries).
   const long long* row_products() const { return row_p_.as<long long>(); }
   const int* bin_list(int b) const { return sym_rows_.as<int>() + (size_t)b * (size_t)m_; }
   const int* a_rowptr() const { return op_.a_rowptr; }
@@ -122,6 +123,7 @@ class Engine {
   int n() const { return n_; }
   // Rows of first-pass bin b as the statistics count them.
   int sym_bin_rows(int b) const {
+    if (b < FB_WARP_BINS) return fb_counts_[b] + warp_stat_[b];
     return fb_counts_[b] + (b == FB_ESC0 ? fb_counts_[FB_ESC256] + fb_counts_[FB_ESC512] : 0);
   }
   int overflow_rows() const { return overflow_rows_; }
@@ -197,8 +199,9 @@ class Engine {
   bool have_sym_ = false;
   int m_ = 0, kdim_ = 0, n_ = 0, n_chunks_ = 0;
   long long p_total_ = 0, nnz_c_ = 0;
-  int fb_counts_[16] = {0};
-  int may_overflow_[16] = {0};
+  int fb_counts_[24] = {0};
+  int may_overflow_[24] = {0};
+  int warp_stat_[8] = {0};
   long long temp_total_ = 0;
   int overflow_rows_ = 0;
   int num_counts_[16] = {0};

@@ -71,13 +71,21 @@ struct Operands {
 //         hashed (k_fused_esc), one block of 128 / 256 / 512 threads per row;
 //         rows of at most 256 (one warp) and 512 products (64 threads) have
 //         lists of their own, 13 and 14, and count as bin 10 in the statistics
+// Rows of the warp bins that need no hash table leave them for
+//   15..17 rows of at most 8 / 16 / 32 products, sorted in registers
+//         (k_fused_tiny)
+//   18    rows whose span fits a warp's bitmap (k_fused_bits)
+// and count as the warp bin of their column bound in the statistics.
 constexpr int FB_WARP_BINS = 5;
 constexpr int FB_BLOCK0 = 5;
 constexpr int FB_MID = 8;
 constexpr int FB_LONG = 9;
 constexpr int FB_ESC0 = 10;
 constexpr int FB_ESC256 = 13, FB_ESC512 = 14;
-constexpr int FB_COUNT = 15;
+constexpr int FB_TINY8 = 15, FB_TINY16 = 16, FB_TINY32 = 17;
+constexpr int FB_BITS = 18;
+constexpr int FB_COUNT = 19;
+constexpr int FB_LISTS = 15;  // row lists of m entries; see fb_list_at
 constexpr int FB_STAT_COUNT = 13;  // bins of the statistics
 // Numeric bins of long rows: 4..7 block hash (2^10..2^13 slots), 8 column
 // slices, 9 bitmap of the whole span (statistics slots 0..3 stay unused).
@@ -120,6 +128,13 @@ __host__ __device__ inline bool whole_row_path(int o, int2 sp, int cnt_max, int 
   return ((sp.y + 1 - lo + 31) >> 5) <= max_words;
 }
 
+// Position of entry `pos` of bin b's row list. A row is in one bin, so bins
+// 15.. (which only row analysis fills) share the lists of bins 0.., from the
+// other end.
+__host__ __device__ inline size_t fb_list_at(int b, int pos, int m) {
+  return b < FB_LISTS ? (size_t)b * m + pos : (size_t)(b - FB_LISTS + 1) * m - 1 - pos;
+}
+
 __host__ __device__ inline int ceil_log2_ll(long long v) {
   int r = 0;
   while ((1ll << r) < v) ++r;
@@ -157,12 +172,33 @@ __host__ __device__ inline int first_bin_of(long long p, long long cap, int span
   return lg - 11 + FB_BLOCK0;  // cap <= p <= long_p <= 4096, so lg <= 13
 }
 
+// Bitmap rows (k_fused_bits): words of the bitmap (spans of at most 4096
+// columns), outputs held at once, and outputs above which a row is redone by
+// the overflow bin. Wider bitmaps were slower than the other bins (27-point
+// stencil 96^3, 1165 words: 6.9 ms against 5.1 hashed): few warps fit an SM
+// and the neighbouring columns of a B row serialise on their word.
+constexpr int BITS_WORDS = 128;
+constexpr int BITS_CAP = 256;
+constexpr int BITS_OUT_MAX = 2 * BITS_CAP;
+
+// 32-column words from the word of column lo to the end of the span.
+__host__ __device__ inline int span_words(int lo, int span) { return ((lo & 31) + span + 31) >> 5; }
+
+// First-pass list of a row whose bin is `nominal` (first_bin_of): warp-bin
+// rows of at most 32 products are sorted in registers (packed keys hold a
+// 27-bit column offset), those with a narrow span use a bitmap.
+__host__ __device__ inline int row_list_of(int nominal, long long p, int lo, int span) {
+  if (nominal < 0 || nominal >= FB_WARP_BINS) return nominal;
+  if (p <= 32 && span < (1 << 27)) return p <= 8 ? FB_TINY8 : (p <= 16 ? FB_TINY16 : FB_TINY32);
+  return span_words(lo, span) <= BITS_WORDS ? FB_BITS : nominal;
+}
+
 // Where a warp-bin row whose table overflows is redone: the sorted bins when
 // the tuning sorts rows like it, else the span bitmap or the largest block
 // table. `lo`: first column of the row's span.
 __host__ __device__ inline int overflow_bin_of(long long p, int lo, int span, const Tuning& t) {
   if (p > t.esc_p_min && span > t.esc_span_min && p <= 4096) return esc_bin_of(p);
-  return span + (lo & 31) <= t.mid_cols ? FB_MID : FB_BLOCK0 + 2;
+  return (lo & 31) + span <= t.mid_cols ? FB_MID : FB_BLOCK0 + 2;
 }
 
 // Numeric bin of a long row (P_i > long_p) with nnz_i outputs.

@@ -94,22 +94,25 @@ constexpr int RA_UNROLL = 4;  // 32-entry batches of a row in flight together
 // products, the first-pass bin, and tcap[i] = the column bound min(P_i, n,
 // span_i) for rows the fused pass computes (0 otherwise), which sizes their
 // slot in the temporary output buffer. may_overflow[b] counts the warp-bin
-// rows that go to bin b should their table overflow. Rows are appended to their bin's list
+// rows that go to bin b should their table overflow; warp_stat the rows of each
+// warp bin that have a list outside it. Rows are appended to their bin's list
 // with one global atomic per bin per block. B's pointers are range-checked
 // here because the validation pass's result is only read after this kernel.
 __global__ void __launch_bounds__(RA_THREADS)
 k_row_analysis(Operands op, int* __restrict__ aoff, long long* __restrict__ row_p,
                int* __restrict__ c_cnt, int* __restrict__ tcap, int* __restrict__ fb_count,
-               int* __restrict__ may_overflow, int* __restrict__ fb_rows, unsigned long long* __restrict__ p_total,
+               int* __restrict__ may_overflow, int* __restrict__ warp_stat,
+               int* __restrict__ fb_rows, unsigned long long* __restrict__ p_total,
                int* __restrict__ max_row_len, int2* __restrict__ row_span, unsigned* status,
                Tuning tn) {
-  __shared__ int hist[FB_COUNT], base[FB_COUNT], ovf[FB_COUNT];
+  __shared__ int hist[FB_COUNT], base[FB_COUNT], ovf[FB_COUNT], nominal[FB_WARP_BINS];
   __shared__ int rowbin[RA_ROWS], rowrank[RA_ROWS];
   __shared__ unsigned long long block_p;
   __shared__ int block_max_len;  // longest A row of the block (one global atomic per block)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row0 = blockIdx.x * RA_ROWS;
   if (threadIdx.x < FB_COUNT) hist[threadIdx.x] = ovf[threadIdx.x] = 0;
+  if (threadIdx.x < FB_WARP_BINS) nominal[threadIdx.x] = 0;
   if (threadIdx.x == 0) {
     block_p = 0;
     block_max_len = 0;
@@ -211,14 +214,19 @@ k_row_analysis(Operands op, int* __restrict__ aoff, long long* __restrict__ row_
       row_p[i] = acc;
       if (acc >= (1ll << 31)) atomicOr(status, ST_ROW_TOO_LONG);
       const long long cap = row_cap(acc, op.n, span);
-      const int bin = first_bin_of(acc, cap, span, tn);
+      const int bin0 = first_bin_of(acc, cap, span, tn);
+      const int bin = row_list_of(bin0, acc, lo, span);
       if (bin < 0) c_cnt[i] = 0;
       tcap[i] = (bin >= 0 && bin != FB_LONG) ? (int)cap : 0;
       rowbin[lr] = bin;
       if (bin >= 0) rowrank[lr] = atomicAdd(&hist[bin], 1);
-      // a table smaller than 1.25 x the column bound may overflow
-      if (bin >= 0 && bin < FB_WARP_BINS && cap + cap / 4 + 1 > (64ll << bin))
-        atomicAdd(&ovf[overflow_bin_of(acc, lo, span, tn)], 1);
+      // a table smaller than 1.25 x the column bound may overflow, and so may
+      // a bitmap row of that many outputs
+      const bool over = bin == FB_BITS ? cap > BITS_OUT_MAX
+                                       : bin >= 0 && bin < FB_WARP_BINS &&
+                                             cap + cap / 4 + 1 > (64ll << bin);
+      if (over) atomicAdd(&ovf[overflow_bin_of(acc, lo, span, tn)], 1);
+      if (bin >= FB_TINY8) atomicAdd(&nominal[bin0], 1);
       atomicAdd(&block_p, (unsigned long long)acc);
     }
   }
@@ -227,6 +235,8 @@ k_row_analysis(Operands op, int* __restrict__ aoff, long long* __restrict__ row_
     base[threadIdx.x] = atomicAdd(fb_count + threadIdx.x, hist[threadIdx.x]);
   if (threadIdx.x < FB_COUNT && ovf[threadIdx.x])
     atomicAdd(may_overflow + threadIdx.x, ovf[threadIdx.x]);
+  if (threadIdx.x < FB_WARP_BINS && nominal[threadIdx.x])
+    atomicAdd(warp_stat + threadIdx.x, nominal[threadIdx.x]);
   if (threadIdx.x == 0) {
     atomicAdd(p_total, block_p);
     if (block_max_len > 0) atomicMax(max_row_len, block_max_len);
@@ -234,7 +244,7 @@ k_row_analysis(Operands op, int* __restrict__ aoff, long long* __restrict__ row_
   __syncthreads();
   for (int lr = threadIdx.x; lr < RA_ROWS; lr += RA_THREADS) {
     const int b = rowbin[lr];
-    if (b >= 0) fb_rows[(size_t)b * op.m + base[b] + rowrank[lr]] = row0 + lr;
+    if (b >= 0) fb_rows[fb_list_at(b, base[b] + rowrank[lr], op.m)] = row0 + lr;
   }
 }
 

@@ -68,3 +68,16 @@ def test_sorted_rows_around_their_capacities(precision, n, lengths, crowd):
     A, B = rows_of(COUNTS, n, lengths, crowd, seed=len(lengths))
     stats = check_rows(A, B, precision, dict(warp_cap_max=0))
     assert sum(stats["rows_per_symbolic_bin"][10:13]) == len(COUNTS), stats
+
+
+@pytest.mark.parametrize("precision", [sg.PLAIN, sg.COMPENSATED])
+@pytest.mark.parametrize("n", [4096, 4128, 40999, (1 << 27) + 5])
+@pytest.mark.parametrize("lengths,crowd,empty", [((1,), False, 0), ((2, 1), False, 40), ((11, 3, 60), False, 3),
+                                                 ((33, 200), False, 0), ((60, 5), True, 0)])
+def test_warp_rows_around_their_capacities(precision, n, lengths, crowd, empty):
+    """Default tuning: rows of at most 32 products in registers (with empty
+    rows of B among their entries), rows of at most 4096 columns in a warp's
+    bitmap, wider ones hashed; rows of more outputs than those hold are redone."""
+    A, B = rows_of([c for c in COUNTS if c <= 2048], n, lengths, crowd, seed=n % 1000, empty=empty)
+    stats = check_rows(A, B, precision, {})
+    assert sum(stats["rows_per_symbolic_bin"][:5]) == A.rows, stats
