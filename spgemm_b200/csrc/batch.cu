@@ -240,8 +240,7 @@ int Batch::execute(Engine& E, int use_graph) {
   } else {
     r = run(E);
   }
-  unsigned st = 0;
-  if (!r) r = E.read_status(&st);
+  if (!r) r = E.read_status();
   E.set_replay(false);
   E.set_batch_output(false);
   if (!user && use_graph) E.set_stream(user);

@@ -11,6 +11,7 @@
 #include "engine.h"
 
 #include <algorithm>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 
@@ -124,7 +125,7 @@ Engine::~Engine() {
                    &c_rowptr64_, &tiles_, &sym_rows_, &num_rows_, &long_slot_,
                    &chunk_cnt_, &slices_buf_, &mid_slices_, &row_span_, &counters_, &restrict_scratch_,
                    &tcap_, &toff_, &t_col_, &t_val_,
-                   &bitmaps_, &lpt_order_, &valid_starts_, &out_rowptr_,
+                   &bitmaps_, &lpt_order_, &b_info_, &out_rowptr_,
                    &out_col_, &out_val_};
   for (DevBuf* b : all) b->release();
   for (DevBuf& b : stage_) b.release();
@@ -210,7 +211,8 @@ static inline int blocks_for(long long work, int per_block, long long cap) {
   return (int)b;
 }
 
-int Engine::check_status(unsigned st) {
+int Engine::check_status(const DevCounters& c) {
+  const unsigned st = c.status | (c.descents != 0 ? ST_UNSORTED : 0u);
   if (!st) return 0;
   std::string msg = "device check failed:";
   if (st & ST_TABLE_FULL) msg += " hash-table-full";
@@ -222,21 +224,26 @@ int Engine::check_status(unsigned st) {
   return fail(st & ST_ROW_TOO_LONG ? 7 : ((st & (ST_BAD_INDEX | ST_UNSORTED)) ? 1 : 6), msg);
 }
 
-int Engine::scan_counts(const int* in, int n, long long* out) {
-  const int ntiles = (n + SCAN_TILE - 1) / SCAN_TILE;
-  SG_CK(tiles_.ensure(sizeof(long long) * (size_t)std::max(ntiles, 1)), "alloc scan tiles");
-  long long* tiles = tiles_.as<long long>();
-  long long* total = &counters_.as<DevCounters>()->grand_total;
-  if (ntiles > 0) {
-    prof_begin("k_scan_tiles");
-    k_scan_tiles<<<ntiles, SCAN_THREADS, 0, stream_>>>(in, n, tiles);
-    SG_LAUNCHED("k_scan_tiles");
+int Engine::scan_counts(const int* in, int n, long long* tiles, const ScanOut& out) {
+  const int ntiles = std::max((n + SCAN_TILE - 1) / SCAN_TILE, 1);
+  if (!tiles) {
+    SG_CK(tiles_.ensure(sizeof(long long) * (size_t)ntiles), "alloc scan tiles");
+    tiles = tiles_.as<long long>();
+    if (ntiles > 1) {  // a single tile needs no sums before it
+      prof_begin("k_scan_tiles");
+      k_scan_tiles<<<ntiles, SCAN_THREADS, 0, stream_>>>(in, n, tiles);
+      SG_LAUNCHED("k_scan_tiles");
+    }
   }
-  prof_begin("k_scan_tile_sums");
-  k_scan_tile_sums<<<1, SCAN_THREADS, 0, stream_>>>(tiles, ntiles, total);
-  SG_LAUNCHED("k_scan_tile_sums");
+  const bool scanned = ntiles > SCAN_SELF_TILES;
+  if (scanned) {
+    prof_begin("k_scan_tile_sums");
+    k_scan_tile_sums<<<1, SCAN_THREADS, 0, stream_>>>(tiles, ntiles);
+    SG_LAUNCHED("k_scan_tile_sums");
+  }
   prof_begin("k_scan_apply");
-  k_scan_apply<<<std::max(ntiles, 1), SCAN_THREADS, 0, stream_>>>(in, n, tiles, total, out);
+  k_scan_apply<<<ntiles, SCAN_THREADS, 0, stream_>>>(
+      in, n, tiles, scanned, &counters_.as<DevCounters>()->grand_total, out);
   SG_LAUNCHED("k_scan_apply");
   return 0;
 }
@@ -263,72 +270,47 @@ int Engine::analyze(const cm& A, const cm& B) {
   const int nnz_a = A.nnz;
   const int m = m_;
 
-  SG_CK(counters_.ensure(sizeof(DevCounters)), "alloc counters");
+  const size_t row_tiles = (size_t)(m + SCAN_TILE - 1) / SCAN_TILE + 1;
+  const size_t counter_bytes = ROW_TILES_OFFSET + sizeof(long long) * row_tiles;
+  SG_CK(counters_.ensure(counter_bytes), "alloc counters");
   DevCounters* dc = counters_.as<DevCounters>();
-  SG_CK(cudaMemsetAsync(dc, 0, sizeof(DevCounters), stream_), "memset counters");
+  SG_CK(cudaMemsetAsync(dc, 0, counter_bytes, stream_), "memset counters");
+  const bool a_csc = A.type == COL_MAJOR;
+  SG_CK(c_cnt_.ensure(sizeof(int) * (size_t)std::max(m, 1)), "alloc c_cnt");
+  SG_CK(c_rowptr64_.ensure(sizeof(long long) * ((size_t)m + 1)), "alloc c_rowptr64");
+  int* cnt = c_cnt_.as<int>();
+  if (a_csc)
+    SG_CK(cudaMemsetAsync(cnt, 0, sizeof(int) * (size_t)std::max(m, 1), stream_), "memset cnt");
 
   // ---- validate the operands (sync point 1 reports the result) ----
+  // The transpose and row analysis guard every index they use; their findings
+  // and the validation pass's are read at the first synchronisation below,
+  // before any kernel trusts the inputs.
   {
-    // flat passes: pointers (marking where B's rows start), then entries
-    const long long grid_cap = (long long)sms_ * 16;
-    const size_t start_words = ((size_t)std::max(B.nnz, 1) + 31) / 32;
-    SG_CK(valid_starts_.ensure(sizeof(unsigned) * start_words), "alloc validation bitmap");
-    unsigned* starts = valid_starts_.as<unsigned>();
-    SG_CK(cudaMemsetAsync(starts, 0, sizeof(unsigned) * start_words, stream_), "memset bitmap");
-    prof_begin("k_validate");
-    k_validate_ptr<<<blocks_for((long long)kdim_ + 1, 256, grid_cap), 256, 0, stream_>>>(
-        B.ptr, kdim_, B.nnz, starts, &dc->status);
-    SG_LAUNCHED("k_validate_ptr(B)");
-    if (B.nnz > 0) {
-      prof_begin("k_validate");
-      k_validate_idx<<<blocks_for(B.nnz, 256, grid_cap), 256, 0, stream_>>>(B.idx, B.nnz, n_, starts,
-                                                                           &dc->status);
-      SG_LAUNCHED("k_validate_idx(B)");
-    }
-    const int a_major = A.type == COL_MAJOR ? kdim_ : m;
-    const int a_minor = A.type == COL_MAJOR ? m : kdim_;
-    prof_begin("k_validate");
-    k_validate_ptr<<<blocks_for((long long)a_major + 1, 256, grid_cap), 256, 0, stream_>>>(
-        A.ptr, a_major, nnz_a, nullptr, &dc->status);
-    SG_LAUNCHED("k_validate_ptr(A)");
-    if (nnz_a > 0) {
-      prof_begin("k_validate");
-      k_validate_idx<<<blocks_for(nnz_a, 256, grid_cap), 256, 0, stream_>>>(A.idx, nnz_a, a_minor,
-                                                                           nullptr, &dc->status);
-      SG_LAUNCHED("k_validate_idx(A)");
-    }
-    // The transpose and row analysis guard every index they use; their
-    // findings and the validation pass's are read at the first synchronisation below,
-    // before any kernel trusts the inputs.
+    SG_CK(b_info_.ensure(sizeof(int4) * (size_t)std::max(kdim_, 1)), "alloc B row table");
+    const CheckArgs c{B.ptr, B.idx, A.ptr, A.idx, kdim_, B.nnz, n_, a_csc ? kdim_ : m, nnz_a,
+                      a_csc ? m : kdim_, b_info_.as<int4>(), a_csc ? cnt : nullptr};
+    const long long most = std::max<long long>(std::max(kdim_, m) + 1ll, std::max(B.nnz, nnz_a));
+    const dim3 grid(blocks_for(most, CHECK_THREADS, (long long)sms_ * 16), 4);
+    prof_begin("k_check");
+    k_check<<<grid, CHECK_THREADS, 0, stream_>>>(c, &dc->status, &dc->descents);
+    SG_LAUNCHED("k_check");
   }
 
   // ---- A in CSR ----
-  const int* a_rowptr;
-  const int* a_col;
-  const float* a_val;
-  SG_CK(c_cnt_.ensure(sizeof(int) * (size_t)std::max(m, 1)), "alloc c_cnt");
-  SG_CK(c_rowptr64_.ensure(sizeof(long long) * ((size_t)m + 1)), "alloc c_rowptr64");
-  if (A.type == COL_MAJOR) {
+  const int* a_rowptr = A.ptr;
+  const int* a_col = A.idx;
+  const float* a_val = A.val;
+  if (a_csc) {
     SG_CK(a_rowptr_.ensure(sizeof(int) * ((size_t)m + 1)), "alloc a_rowptr");
     SG_CK(cursor_.ensure(sizeof(int) * ((size_t)m + 1)), "alloc cursor");
     SG_CK(a_col_.ensure(sizeof(int) * (size_t)std::max(nnz_a, 1)), "alloc a_col");
     SG_CK(a_val_.ensure(sizeof(float) * (size_t)std::max(nnz_a, 1)), "alloc a_val");
-    int* cnt = c_cnt_.as<int>();
-    SG_CK(cudaMemsetAsync(cnt, 0, sizeof(int) * (size_t)std::max(m, 1), stream_), "memset cnt");
-    if (nnz_a > 0) {
-      prof_begin("k_transpose_hist");
-      k_transpose_hist<<<blocks_for(nnz_a, 256, (long long)sms_ * 16), 256, 0, stream_>>>(
-          A.idx, nnz_a, m, cnt, &dc->status);
-      SG_LAUNCHED("k_transpose_hist");
-    }
-    if (int r = scan_counts(cnt, m, c_rowptr64_.as<long long>())) return r;
-    prof_begin("k_rowptr_i64_to_i32_shift");
-    k_rowptr_i64_to_i32_shift<<<blocks_for(m + 1, 256, (long long)sms_ * 16), 256, 0, stream_>>>(
-        c_rowptr64_.as<long long>(), m + 1, a_rowptr_.as<int>(), cursor_.as<int>());
-    SG_LAUNCHED("k_rowptr_i64_to_i32_shift");
+    if (int r = scan_counts(cnt, m, nullptr, ScanOut{nullptr, a_rowptr_.as<int>(), cursor_.as<int>()}))
+      return r;
     if (nnz_a > 0) {
       prof_begin("k_transpose_scatter");
-      k_transpose_scatter<<<blocks_for(nnz_a, 256, (long long)sms_ * 16), 256, 0, stream_>>>(
+      k_transpose_scatter<<<(nnz_a - 1) / TR_ENTRIES + 1, TR_THREADS, 0, stream_>>>(
           A.ptr, A.idx, A.val, kdim_, nnz_a, m, cursor_.as<int>(), a_col_.as<int>(),
           a_val_.as<float>());
       SG_LAUNCHED("k_transpose_scatter");
@@ -336,10 +318,6 @@ int Engine::analyze(const cm& A, const cm& B) {
     a_rowptr = a_rowptr_.as<int>();
     a_col = a_col_.as<int>();
     a_val = a_val_.as<float>();
-  } else {
-    a_rowptr = A.ptr;
-    a_col = A.idx;
-    a_val = A.val;
   }
 
   // ---- row analysis ----
@@ -353,15 +331,28 @@ int Engine::analyze(const cm& A, const cm& B) {
   op_ = Operands{a_rowptr, a_col, a_val, aoff_.as<int>(), B.ptr, B.idx, B.val, m_, kdim_, n_,
                  vec_ok, B.nnz};
   if (m > 0) {
+    // lanes per row: about the mean row length; rows per block: enough blocks
+    // for the SMs when there are few rows
+    const long long mean = nnz_a / m;
+    const int g = mean <= 4 ? 4 : (mean <= 8 ? 8 : (mean <= 16 ? 16 : 32));
+    const int rpb = m >= 2 * RA_ROWS * sms_ ? RA_ROWS : RA_THREADS / g;
+    auto launch = [&](auto kernel) {
+      kernel<<<(m + rpb - 1) / rpb, RA_THREADS, 0, stream_>>>(
+          op_, b_info_.as<int4>(), rpb, aoff_.as<int>(), row_p_.as<long long>(), cnt,
+          tcap_.as<int>(), this->row_tiles(), dc->fb_count, dc->may_overflow, dc->warp_stat,
+          sym_rows_.as<int>(), &dc->p_total, &dc->max_row_len, row_span_.as<int2>(), &dc->status,
+          tn_);
+    };
     prof_begin("k_row_analysis");
-    k_row_analysis<<<(m + RA_ROWS - 1) / RA_ROWS, RA_THREADS, 0, stream_>>>(
-        op_, aoff_.as<int>(), row_p_.as<long long>(), c_cnt_.as<int>(), tcap_.as<int>(),
-        dc->fb_count, dc->may_overflow, dc->warp_stat, sym_rows_.as<int>(),
-        &dc->p_total, &dc->max_row_len, row_span_.as<int2>(), &dc->status, tn_);
+    if (g == 4) launch(k_row_analysis<4>);
+    else if (g == 8) launch(k_row_analysis<8>);
+    else if (g == 16) launch(k_row_analysis<16>);
+    else launch(k_row_analysis<32>);
     SG_LAUNCHED("k_row_analysis");
   }
   // temporary-buffer slots of the fused rows (grand total = buffer size)
-  if (int r = scan_counts(tcap_.as<int>(), m, toff_.as<long long>())) return r;
+  if (int r = scan_counts(tcap_.as<int>(), m, this->row_tiles(), ScanOut{toff_.as<long long>(), nullptr, nullptr}))
+    return r;
   if (replay_) {  // same structure as the planned run: keep its sizes
     have_analysis_ = true;
     return 0;
@@ -369,7 +360,7 @@ int Engine::analyze(const cm& A, const cm& B) {
   SG_CK(cudaMemcpyAsync(host_counters_, dc, sizeof(DevCounters), cudaMemcpyDeviceToHost, stream_),
         "read counters");
   SG_CK(cudaStreamSynchronize(stream_), "sync after row analysis");
-  if (int r = check_status(host_counters_->status)) return r;
+  if (int r = check_status(*host_counters_)) return r;
   p_total_ = (long long)host_counters_->p_total;
   for (int b = 0; b < FB_COUNT; ++b) {
     fb_counts_[b] = host_counters_->fb_count[b];
@@ -401,7 +392,8 @@ int Engine::symbolic_pass(long long* nnz_c) {
   if (int r = launch_first_pass()) return r;
 
   // ---- row pointers + numeric binning of the long rows ----
-  if (int r = scan_counts(c_cnt_.as<int>(), m, c_rowptr64_.as<long long>())) return r;
+  if (int r = scan_counts(c_cnt_.as<int>(), m, nullptr, ScanOut{c_rowptr64_.as<long long>(), nullptr, nullptr}))
+    return r;
   SG_CK(num_rows_.ensure(sizeof(int) * (size_t)NB_COUNT * std::max(m, 1)), "alloc num_rows");
   big_capacity_ = (long long)n_long_sym_ * std::max(n_chunks_, 1);
   SG_CK(slices_buf_.ensure(sizeof(Slice) * (size_t)std::max(big_capacity_, 1ll)), "alloc slices");
@@ -436,7 +428,7 @@ int Engine::symbolic_pass(long long* nnz_c) {
   SG_CK(cudaMemcpyAsync(host_counters_, dc, sizeof(DevCounters), cudaMemcpyDeviceToHost, stream_),
         "read counters");
   SG_CK(cudaStreamSynchronize(stream_), "sync after symbolic pass");
-  if (int r = check_status(host_counters_->status)) return r;
+  if (int r = check_status(*host_counters_)) return r;
   nnz_c_ = host_counters_->grand_total;
   for (int b = 0; b < NB_COUNT; ++b) num_counts_[b] = host_counters_->num_count[b];
   nslices_ = host_counters_->slice_count;
@@ -625,29 +617,41 @@ int Engine::launch_fused() {
 template int Engine::launch_fused<0>();
 template int Engine::launch_fused<1>();
 
-int Engine::numeric_values(int* c_col, float* c_val) { return numeric_rows(c_col, c_val, 0, m_); }
-
 int Engine::numeric_rows(int* c_col, float* c_val, int r0, int r1) {
+  return numeric_range(c_col, c_val, r0, r1, nullptr);
+}
+
+int Engine::numeric_range(int* c_col, float* c_val, int r0, int r1, int* c_rowptr) {
   if (!have_sym_) return fail(5, "numeric called without a successful symbolic pass");
   if (nnz_c_ > 0 && (!c_col || !c_val)) return fail(1, "null output pointer");
   if (r0 < 0 || r1 > m_ || r0 > r1) return fail(1, "numeric: row range outside [0, m]");
   if (r1 > r0 && temp_total_ > 0) {
+    // rows per warp: 32, fewer while that leaves SMs without work
+    int rpw = 32;
+    while (rpw > 1 && (long long)(r1 - r0) < (long long)rpw * sms_ * 16) rpw >>= 1;
     prof_begin("k_copy_fused");
-    k_copy_fused<<<blocks_for((long long)(r1 - r0), 256, (long long)sms_ * 16), 256, 0, stream_>>>(
-        r0, r1, tcap_.as<int>(), toff_.as<long long>(), c_cnt_.as<int>(),
-        c_rowptr64_.as<long long>(), t_col_.as<int>(), t_val_.as<float>(), c_col, c_val);
+    k_copy_fused<<<blocks_for((long long)(r1 - r0), 8 * rpw, (long long)sms_ * 16), 256, 0, stream_>>>(
+        r0, r1, m_, rpw, tcap_.as<int>(), toff_.as<long long>(), c_cnt_.as<int>(),
+        c_rowptr64_.as<long long>(), t_col_.as<int>(), t_val_.as<float>(), c_col, c_val, c_rowptr);
     SG_LAUNCHED("k_copy_fused");
+  } else if (c_rowptr) {
+    if (int r = rowptr_kernel(c_rowptr)) return r;
   }
   return launch_numeric_bins(c_col, c_val, r0, r1);
+}
+
+int Engine::rowptr_kernel(int* c_rowptr) {
+  prof_begin("k_rowptr_to_i32");
+  k_rowptr_to_i32<<<blocks_for(m_ + 1ll, 256, (long long)sms_ * 16), 256, 0, stream_>>>(
+      c_rowptr64_.as<long long>(), m_ + 1, c_rowptr);
+  SG_LAUNCHED("k_rowptr_to_i32");
+  return 0;
 }
 
 int Engine::numeric_rowptr(int* c_rowptr) {
   if (!have_sym_) return fail(5, "numeric called without a successful symbolic pass");
   if (!c_rowptr) return fail(1, "null output pointer");
-  prof_begin("k_rowptr_to_i32");
-  k_rowptr_to_i32<<<blocks_for(m_ + 1, 256, (long long)sms_ * 16), 256, 0, stream_>>>(
-      c_rowptr64_.as<long long>(), m_ + 1, c_rowptr);
-  SG_LAUNCHED("k_rowptr_to_i32");
+  if (int r = rowptr_kernel(c_rowptr)) return r;
   return finish_numeric();
 }
 
@@ -678,23 +682,13 @@ int Engine::rowptr64_to_host(long long* host) {
 
 int Engine::finish_numeric() {
   if (replay_) return 0;  // the caller reads the status after the captured work
-  DevCounters* dc = counters_.as<DevCounters>();
-  SG_CK(cudaMemcpyAsync(&host_counters_->status, &dc->status, sizeof(unsigned),
-                        cudaMemcpyDeviceToHost, stream_),
-        "read status");
-  SG_CK(cudaStreamSynchronize(stream_), "sync after numeric pass");
-  prof_collect_if_full();
-  return check_status(host_counters_->status);
+  return read_status();
 }
 
 int Engine::numeric(int* c_rowptr, int* c_col, float* c_val) {
   if (!have_sym_) return fail(5, "numeric called without a successful symbolic pass");
   if (!c_rowptr) return fail(1, "null output pointer");
-  if (int r = numeric_values(c_col, c_val)) return r;
-  prof_begin("k_rowptr_to_i32");
-  k_rowptr_to_i32<<<blocks_for(m_ + 1, 256, (long long)sms_ * 16), 256, 0, stream_>>>(
-      c_rowptr64_.as<long long>(), m_ + 1, c_rowptr);
-  SG_LAUNCHED("k_rowptr_to_i32");
+  if (int r = numeric_range(c_col, c_val, 0, m_, c_rowptr)) return r;
   return finish_numeric();
 }
 
@@ -702,7 +696,7 @@ int Engine::numeric_batch(int count, const long long* row_off_dev, long long max
                           int* c_rowptr, int* c_col, float* c_val) {
   if (!have_sym_) return fail(5, "numeric called without a successful symbolic pass");
   if (!c_rowptr) return fail(1, "null output pointer");
-  if (int r = numeric_values(c_col, c_val)) return r;
+  if (int r = numeric_range(c_col, c_val, 0, m_, nullptr)) return r;
   if (count > 0) {
     prof_begin("k_batch_rowptr");
     const dim3 grid(blocks_for(max_rows + 1, 256, 64), count);
@@ -712,15 +706,16 @@ int Engine::numeric_batch(int count, const long long* row_off_dev, long long max
   return finish_numeric();
 }
 
-int Engine::read_status(unsigned* st) {
+int Engine::read_status() {
   DevCounters* dc = counters_.as<DevCounters>();
-  SG_CK(cudaMemcpyAsync(&host_counters_->status, &dc->status, sizeof(unsigned),
+  static_assert(offsetof(DevCounters, descents) == offsetof(DevCounters, status) + sizeof(unsigned),
+                "read together");
+  SG_CK(cudaMemcpyAsync(&host_counters_->status, &dc->status, sizeof(unsigned) + sizeof(int),
                         cudaMemcpyDeviceToHost, stream_),
         "read status");
-  SG_CK(cudaStreamSynchronize(stream_), "sync after batch");
+  SG_CK(cudaStreamSynchronize(stream_), "sync to read the status");
   prof_collect_if_full();
-  *st = host_counters_->status;
-  return check_status(*st);
+  return check_status(*host_counters_);
 }
 
 int Engine::launch_numeric_bins(int* c_col, float* c_val, int r0, int r1) {
@@ -926,17 +921,15 @@ int Engine::multiply_numeric_owned(cm* C_dev) {
 
 cudaError_t scan_counts_to_ptr32(const int* cnt, int n, int* ptr, DevBuf& tmp,
                                  long long* total_dev, cudaStream_t s) {
-  const int ntiles = (n + SCAN_TILE - 1) / SCAN_TILE;
-  const size_t tiles_bytes = sizeof(long long) * (size_t)std::max(ntiles, 1);
-  const size_t ptr64_bytes = sizeof(long long) * ((size_t)n + 1);
-  cudaError_t e = tmp.ensure(tiles_bytes + ptr64_bytes);
+  const int ntiles = std::max((n + SCAN_TILE - 1) / SCAN_TILE, 1);
+  cudaError_t e = tmp.ensure(sizeof(long long) * (size_t)ntiles);
   if (e != cudaSuccess) return e;
   long long* tiles = tmp.as<long long>();
-  long long* ptr64 = tiles + std::max(ntiles, 1);
-  if (ntiles > 0) k_scan_tiles<<<ntiles, SCAN_THREADS, 0, s>>>(cnt, n, tiles);
-  k_scan_tile_sums<<<1, SCAN_THREADS, 0, s>>>(tiles, ntiles, total_dev);
-  k_scan_apply<<<std::max(ntiles, 1), SCAN_THREADS, 0, s>>>(cnt, n, tiles, total_dev, ptr64);
-  k_rowptr_to_i32<<<blocks_for(n + 1, 256, 4096), 256, 0, s>>>(ptr64, n + 1, ptr);
+  if (ntiles > 1) k_scan_tiles<<<ntiles, SCAN_THREADS, 0, s>>>(cnt, n, tiles);
+  const bool scanned = ntiles > SCAN_SELF_TILES;
+  if (scanned) k_scan_tile_sums<<<1, SCAN_THREADS, 0, s>>>(tiles, ntiles);
+  k_scan_apply<<<ntiles, SCAN_THREADS, 0, s>>>(cnt, n, tiles, scanned, total_dev,
+                                               ScanOut{nullptr, ptr, nullptr});
   return cudaGetLastError();
 }
 

@@ -14,6 +14,8 @@
 
 namespace sg {
 
+struct ScanOut;
+
 // Grow-only device buffer.
 struct DevBuf {
   void* ptr = nullptr;
@@ -33,6 +35,7 @@ struct DevCounters {
   int slice_count;
   int mid_count;
   unsigned status;
+  int descents;  // zero when B's rows are sorted (k_check); read with the status
   unsigned long long p_total;
   long long grand_total;
   int max_row_len;  // longest row of A (entries)
@@ -102,7 +105,7 @@ class Engine {
   bool replay() const { return replay_; }
   // Batch output: nnz(C) may exceed the int32 range of a single cm.
   void set_batch_output(bool on) { batch_out_ = on; }
-  int read_status(unsigned* st);
+  int read_status();
   const long long* rowptr64() const { return c_rowptr64_.as<long long>(); }
   // After analyze(): products per row (int64) and the row list of first-pass
   // bin b (mid and long rows: sym_bin_rows(b) entries).
@@ -165,7 +168,9 @@ class Engine {
   int cuda_fail(cudaError_t e, const char* what);
 
  private:
-  int numeric_values(int* c_col, float* c_val);
+  // c_rowptr non-null: also C's int32 row pointers (r0 == 0, r1 == m).
+  int numeric_range(int* c_col, float* c_val, int r0, int r1, int* c_rowptr);
+  int rowptr_kernel(int* c_rowptr);
   int finish_numeric();
   int launch_first_pass();
   template <int MODE> int launch_fused();
@@ -178,8 +183,15 @@ class Engine {
   int rows_cnt_max() const;
   int rows_smem_cap(int threads) const;
   int launch_num_rows(int* c_col, float* c_val, int r0, int r1);
-  int scan_counts(const int* in, int n, long long* out);
-  int check_status(unsigned st);
+  // Exclusive scan of in[0, n) (total to the counters' grand_total); `tiles`:
+  // the tiles' sums when a kernel has already formed them, else null.
+  int scan_counts(const int* in, int n, long long* tiles, const ScanOut& out);
+  // Zeroed long long per tile of the row counts, behind the counters.
+  long long* row_tiles() const {
+    return reinterpret_cast<long long*>(counters_.as<unsigned char>() + ROW_TILES_OFFSET);
+  }
+  static constexpr size_t ROW_TILES_OFFSET = (sizeof(DevCounters) + 15) / 16 * 16;
+  int check_status(const DevCounters& c);
   template <class K> cudaError_t smem_attr(K kernel, size_t bytes);
 
   cudaStream_t stream_ = nullptr;
@@ -217,7 +229,7 @@ class Engine {
   DevBuf sym_rows_, num_rows_, long_slot_, chunk_cnt_, slices_buf_, mid_slices_, row_span_;
   DevBuf tcap_, toff_, t_col_, t_val_;  // fused pass: row bounds, temp offsets, temp output
   DevBuf counters_, restrict_scratch_, bitmaps_, lpt_order_;
-  DevBuf valid_starts_;  // input validation: first position of every row of B (nnz(B) bits)
+  DevBuf b_info_;  // int4 per row of B: position, length, first and last column
   int bitmap_words_ = 0;  // per long row; 0 when the bitmaps are not kept
   int max_row_len_ = 0;
   DevBuf out_rowptr_, out_col_, out_val_;

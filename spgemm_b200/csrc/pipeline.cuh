@@ -6,76 +6,158 @@
 
 namespace sg {
 
+// Row counts are scanned in tiles (see k_scan_apply).
+constexpr int SCAN_THREADS = 1024;
+constexpr int SCAN_ITEMS = 4;
+constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
+
+__device__ __forceinline__ long long block_excl_scan64(long long v, long long* shm,
+                                                       long long& total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long incl = warp_incl_scan64(v);
+  if (lane == 31) shm[warp] = incl;
+  __syncthreads();
+  if (warp == 0) {
+    const long long w = (lane < (int)(blockDim.x >> 5)) ? shm[lane] : 0;
+    const long long wi = warp_incl_scan64(w);
+    shm[lane] = wi - w;
+    if (lane == 31) shm[32] = wi;
+  }
+  __syncthreads();
+  const long long r = shm[warp] + incl - v;
+  total = shm[32];
+  __syncthreads();
+  return r;
+}
+
 // ---------------------------------------------------------------------------
 // Input validation
 // ---------------------------------------------------------------------------
 
-// Input validation as two flat passes (coalesced, one thread per pointer,
-// then one per entry): pointers inside [0, nnz], non-decreasing, ptr[0] == 0
-// and ptr[n_major] == nnz, each segment's first position marked in `starts`
-// (nnz bits, zeroed by the caller; null when sortedness is not checked) ...
-__global__ void k_validate_ptr(const int* __restrict__ ptr, int n_major, int nnz,
-                               unsigned* __restrict__ starts, unsigned* status) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= n_major; i += gridDim.x * blockDim.x) {
-    const int s = ptr[i];
-    bool bad = s < 0 || s > nnz || (i == 0 && s != 0) || (i == n_major && s != nnz);
-    if (i < n_major && s > ptr[i + 1]) bad = true;
-    if (bad) atomicOr(status, ST_BAD_INDEX);
-    else if (starts && i < n_major && s < nnz) atomicOr(starts + (s >> 5), 1u << (s & 31));
-  }
+// One pass over both operands, in four roles (blockIdx.y), each flat and
+// coalesced:
+//   0  B's pointers: inside [0, nnz], non-decreasing, first 0, last nnz; each
+//      row's position, length, first and last column to b_info (an empty row
+//      for pointers that fail);
+//   1  B's columns: inside [0, n);
+//   2  A's pointers, as B's;
+//   3  A's indices: inside [0, a_minor); with `hist` (A in CSC), entries per
+//      row of A (the reference builds its CSC with the same atomic histogram
+//      but never zeroes it first, src/mm.cu:43-63, 89; the caller zeroes it).
+// B's rows must be sorted (the long-row kernels binary-search them). Every
+// entry that is not above the one before it must begin a row: `descents` gets
+// the count over all entries (role 1) minus the count over row starts (role
+// 0), so it ends at zero exactly when that holds. Violations of the ranges
+// set ST_BAD_INDEX. Nothing is read outside ptr[0..n_major] and idx[0..nnz).
+constexpr int CHECK_THREADS = 256;
+
+struct CheckArgs {
+  const int *b_ptr, *b_idx, *a_ptr, *a_idx;
+  int b_rows, b_nnz, n, a_major, a_nnz, a_minor;
+  int4* b_info;
+  int* hist;
+};
+
+__device__ __forceinline__ bool pointer_ok(const int* ptr, int i, int n_major, int nnz, int s) {
+  bool ok = s >= 0 && s <= nnz && (i > 0 || s == 0) && (i < n_major || s == nnz);
+  if (i < n_major && s > ptr[i + 1]) ok = false;
+  return ok;
 }
 
-// ... then every entry inside [0, n_minor) and, with `starts`, above the
-// entry before it unless it begins a segment (B's rows must be sorted: the
-// long-row kernels binary-search them). Violations set ST_BAD_INDEX (range)
-// or ST_UNSORTED; nothing is read outside ptr[0..n_major] and idx[0..nnz).
-__global__ void k_validate_idx(const int* __restrict__ idx, int nnz, int n_minor,
-                               const unsigned* __restrict__ starts, unsigned* status) {
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nnz; q += gridDim.x * blockDim.x) {
-    const int v = idx[q];
-    if ((unsigned)v >= (unsigned)n_minor) atomicOr(status, ST_BAD_INDEX);
-    if (starts && q > 0 && !((starts[q >> 5] >> (q & 31)) & 1u) && idx[q - 1] >= v)
-      atomicOr(status, ST_UNSORTED);
+__global__ void __launch_bounds__(CHECK_THREADS)
+k_check(CheckArgs c, unsigned* status, int* descents) {
+  const int stride = gridDim.x * CHECK_THREADS;
+  const int t0 = blockIdx.x * CHECK_THREADS + threadIdx.x;
+  bool bad = false;
+  int net = 0;
+  if (blockIdx.y == 0) {
+    for (int i = t0; i <= c.b_rows; i += stride) {
+      const int s = c.b_ptr[i];
+      const bool ok = pointer_ok(c.b_ptr, i, c.b_rows, c.b_nnz, s);
+      bad |= !ok;
+      if (i < c.b_rows) {
+        const int e = c.b_ptr[i + 1];
+        int4 info = make_int4(0, 0, 0, 0);
+        if (ok && e <= c.b_nnz && e > s) {
+          info = make_int4(s, e - s, c.b_idx[s], c.b_idx[e - 1]);
+          if (s > 0 && c.b_idx[s - 1] >= info.z) --net;
+        }
+        c.b_info[i] = info;
+      }
+    }
+  } else if (blockIdx.y == 1) {
+    for (int q = t0; q < c.b_nnz; q += stride) {
+      const int v = c.b_idx[q];
+      bad |= (unsigned)v >= (unsigned)c.n;
+      if (q > 0 && c.b_idx[q - 1] >= v) ++net;
+    }
+  } else if (blockIdx.y == 2) {
+    for (int i = t0; i <= c.a_major; i += stride)
+      bad |= !pointer_ok(c.a_ptr, i, c.a_major, c.a_nnz, c.a_ptr[i]);
+  } else {
+    for (int q = t0; q < c.a_nnz; q += stride) {
+      const int v = c.a_idx[q];
+      const bool ok = (unsigned)v < (unsigned)c.a_minor;
+      bad |= !ok;
+      if (c.hist && ok) atomicAdd(c.hist + v, 1);
+    }
   }
+  if (bad) atomicOr(status, ST_BAD_INDEX);
+  net = warp_sum(net);
+  if ((threadIdx.x & 31) == 0 && net) atomicAdd(descents, net);
 }
 
 // ---------------------------------------------------------------------------
 // A: CSC -> CSR
 // ---------------------------------------------------------------------------
 
-// Count entries per row of A. The reference builds A's CSC with the same
-// atomic histogram but never zeroes it first (src/mm.cu:43-63, 89); the
-// caller of this kernel zeroes `cnt`.
-__global__ void k_transpose_hist(const int* __restrict__ rowidx, int nnz, int m,
-                                 int* __restrict__ cnt, unsigned* status) {
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nnz;
-       e += gridDim.x * blockDim.x) {
-    const int r = rowidx[e];
-    if ((unsigned)r < (unsigned)m) atomicAdd(cnt + r, 1);
-    else atomicOr(status, ST_BAD_INDEX);
-  }
-}
-
 // Scatter CSC entries into CSR order. cursor[] starts as the CSR row
-// pointers; the entry order inside a row is the atomic arrival order.
-__global__ void k_transpose_scatter(const int* __restrict__ colptr,
-                                    const int* __restrict__ rowidx,
-                                    const float* __restrict__ val, int kdim, int nnz,
-                                    int m, int* __restrict__ cursor,
-                                    int* __restrict__ out_col,
-                                    float* __restrict__ out_val) {
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nnz;
-       e += gridDim.x * blockDim.x) {
-    // column of entry e: last k with colptr[k] <= e
-    int lo = 0, hi = kdim;
+// pointers; the entry order inside a row is the atomic arrival order. A block
+// takes TR_ENTRIES consecutive entries (balanced however long the columns
+// are) and finds their columns by searching the stretch of column pointers
+// that covers them, kept in shared memory when it fits: searching all of
+// them in global memory took 22 dependent loads an entry (27-point stencil
+// 96^3, 23.6 M entries: 485 us).
+constexpr int TR_THREADS = 256;
+constexpr int TR_ENTRIES = 2048;
+constexpr int TR_COLS = 2048;
+
+__global__ void __launch_bounds__(TR_THREADS)
+k_transpose_scatter(const int* __restrict__ colptr,
+                    const int* __restrict__ rowidx,
+                    const float* __restrict__ val, int kdim, int nnz,
+                    int m, int* __restrict__ cursor,
+                    int* __restrict__ out_col,
+                    float* __restrict__ out_val) {
+  __shared__ int sptr[TR_COLS];
+  __shared__ int edge[2];
+  const int e0 = blockIdx.x * TR_ENTRIES, e1 = min(nnz, e0 + TR_ENTRIES);
+  // last k in [lo, hi] with p(k) <= e (p(lo) <= e)
+  auto search = [](auto p, int lo, int hi, int e) {
     while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (__ldg(colptr + mid) <= e) lo = mid; else hi = mid - 1;
+      const int mid = lo + (hi - lo + 1) / 2;
+      if (p(mid) <= e) lo = mid; else hi = mid - 1;
     }
+    return lo;
+  };
+  auto global_ptr = [&](int k) { return __ldg(colptr + k); };
+  if (threadIdx.x < 2)
+    edge[threadIdx.x] = search(global_ptr, 0, kdim - 1, threadIdx.x ? e1 - 1 : e0);
+  __syncthreads();
+  const int k0 = edge[0], nk = edge[1] - k0 + 1;
+  const bool local = nk > 0 && nk <= TR_COLS;
+  if (local)
+    for (int t = threadIdx.x; t < nk; t += TR_THREADS) sptr[t] = __ldg(colptr + k0 + t);
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < TR_ENTRIES / TR_THREADS; ++u) {
+    const int e = e0 + u * TR_THREADS + threadIdx.x;
+    if (e >= e1) break;
     const int r = rowidx[e];
     if ((unsigned)r >= (unsigned)m) continue;
     const int pos = atomicAdd(cursor + r, 1);
-    out_col[pos] = lo;
+    out_col[pos] = local ? k0 + search([&](int k) { return sptr[k]; }, 0, nk - 1, e)
+                         : search(global_ptr, 0, kdim - 1, e);
     out_val[pos] = val[e];
   }
 }
@@ -85,141 +167,207 @@ __global__ void k_transpose_scatter(const int* __restrict__ colptr,
 // ---------------------------------------------------------------------------
 
 constexpr int RA_THREADS = 256;
-constexpr int RA_ROWS = 64;  // rows per block
-constexpr int RA_UNROLL = 4;  // 32-entry batches of a row in flight together
+constexpr int RA_ROWS = 64;    // most rows per block
+constexpr int RA_UNROLL = 4;   // batches of a row in flight together
+constexpr int RA_HEAVY = 1024; // rows of more entries are walked by the whole block
 
 // Per row i: P_i = sum over A(i,k) of nnz(B(k,:)) (the intermediate product
 // count the reference accumulates per row in initGEMM, src/mm.cu:138-148),
 // the flattened offset of each A entry, the column span of the row's
 // products, the first-pass bin, and tcap[i] = the column bound min(P_i, n,
 // span_i) for rows the fused pass computes (0 otherwise), which sizes their
-// slot in the temporary output buffer. may_overflow[b] counts the warp-bin
-// rows that go to bin b should their table overflow; warp_stat the rows of each
-// warp bin that have a list outside it. Rows are appended to their bin's list
-// with one global atomic per bin per block. B's pointers are range-checked
-// here because the validation pass's result is only read after this kernel.
+// slot in the temporary output buffer; tile_sum gets tcap's sum per
+// SCAN_TILE rows. may_overflow[b] counts the warp-bin rows that go to bin b
+// should their table overflow; warp_stat the rows of each warp bin that have
+// a list outside it. Rows are appended to their bin's list with one global
+// atomic per bin per block. A's indices are range-checked here because the
+// validation pass's result is only read after this kernel; b_info holds valid
+// positions only.
+//
+// G lanes walk a row, G about the mean row length of A, so the lanes of a
+// warp are busy on short rows too; one 16-byte load per entry brings the B
+// row's position, length, first and last column. Rows above RA_HEAVY entries
+// are left for the whole block (a warp took 0.9 ms over the longest row of
+// R-MAT 2^18, 15.9K entries). What follows from a row's totals is computed by
+// one thread per row.
+template <int G>
 __global__ void __launch_bounds__(RA_THREADS)
-k_row_analysis(Operands op, int* __restrict__ aoff, long long* __restrict__ row_p,
-               int* __restrict__ c_cnt, int* __restrict__ tcap, int* __restrict__ fb_count,
-               int* __restrict__ may_overflow, int* __restrict__ warp_stat,
-               int* __restrict__ fb_rows, unsigned long long* __restrict__ p_total,
-               int* __restrict__ max_row_len, int2* __restrict__ row_span, unsigned* status,
-               Tuning tn) {
+k_row_analysis(Operands op, const int4* __restrict__ b_info, int rows_per_block,
+               int* __restrict__ aoff, long long* __restrict__ row_p,
+               int* __restrict__ c_cnt, int* __restrict__ tcap, long long* __restrict__ tile_sum,
+               int* __restrict__ fb_count, int* __restrict__ may_overflow,
+               int* __restrict__ warp_stat, int* __restrict__ fb_rows,
+               unsigned long long* __restrict__ p_total, int* __restrict__ max_row_len,
+               int2* __restrict__ row_span, unsigned* status, Tuning tn) {
+  constexpr int NW = RA_THREADS / 32;
   __shared__ int hist[FB_COUNT], base[FB_COUNT], ovf[FB_COUNT], nominal[FB_WARP_BINS];
-  __shared__ int rowbin[RA_ROWS], rowrank[RA_ROWS];
-  __shared__ unsigned long long block_p;
-  __shared__ int block_max_len;  // longest A row of the block (one global atomic per block)
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int row0 = blockIdx.x * RA_ROWS;
+  __shared__ long long s_p[RA_ROWS];
+  __shared__ int s_lo[RA_ROWS], s_hi[RA_ROWS];
+  __shared__ int heavy[RA_ROWS], n_heavy;
+  __shared__ long long part_p[NW];
+  __shared__ int part_lo[NW], part_hi[NW];
+  __shared__ unsigned long long block_p, block_cap;
+  __shared__ int block_max_len;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gl = lane & (G - 1);
+  const int row0 = blockIdx.x * rows_per_block;
+  const int nrows = min(rows_per_block, op.m - row0);
   if (threadIdx.x < FB_COUNT) hist[threadIdx.x] = ovf[threadIdx.x] = 0;
   if (threadIdx.x < FB_WARP_BINS) nominal[threadIdx.x] = 0;
   if (threadIdx.x == 0) {
-    block_p = 0;
+    block_p = block_cap = 0;
     block_max_len = 0;
+    n_heavy = 0;
   }
   __syncthreads();
-  for (int lr = warp; lr < RA_ROWS; lr += RA_THREADS / 32) {
-    const int i = row0 + lr;
-    if (i >= op.m) {
-      if (lane == 0) rowbin[lr] = -1;
-      continue;
+  // B row of A's entry j (an empty one beyond `re` or for an invalid index)
+  auto entry = [&](int j, int re) {
+    if (j >= re) return make_int4(0, 0, 0, 0);
+    const int k = __ldg(op.a_col + j);
+    if ((unsigned)k >= (unsigned)op.kdim) {
+      atomicOr(status, ST_BAD_INDEX);
+      return make_int4(0, 0, 0, 0);
     }
-    const int rs = op.a_rowptr[i], re = op.a_rowptr[i + 1];
-    long long acc = 0;
-    int lo = 0x7fffffff, hi = -1;  // column span of the row's products
-    // Entry j's B row length and first/last column (invalid indices are
-    // reported and count as empty).
-    auto entry = [&](int j, int& bs, int& be) {
-      const int k = op.a_col[j];
-      bs = be = 0;
-      if ((unsigned)k >= (unsigned)op.kdim) {
-        atomicOr(status, ST_BAD_INDEX);
-        return;
+    return __ldg(b_info + k);
+  };
+  // inclusive sums over W lanes; the sum of 32 lengths fits 32 bits when B
+  // has at most 2^26 entries
+  const bool narrow = op.nnz_b <= (1 << 26);
+  auto incl_scan = [&](int len, auto width) -> long long {
+    constexpr int W = decltype(width)::value;
+    const int l = lane & (W - 1);
+    if (narrow) {
+      unsigned v = (unsigned)len;
+#pragma unroll
+      for (int d = 1; d < W; d <<= 1) {
+        const unsigned t = __shfl_up_sync(FULL, v, d, W);
+        if (l >= d) v += t;
       }
-      const int s0 = op.b_rowptr[k], s1 = op.b_rowptr[k + 1];
-      if (s0 >= 0 && s1 <= op.nnz_b && s0 <= s1) {
-        bs = s0;
-        be = s1;
-      } else {
-        atomicOr(status, ST_BAD_INDEX);
+      return (long long)v;
+    }
+    long long v = len;
+#pragma unroll
+    for (int d = 1; d < W; d <<= 1) {
+      const long long t = __shfl_up_sync(FULL, v, d, W);
+      if (l >= d) v += t;
+    }
+    return v;
+  };
+  // offsets of entries [j0, re) of a row by W lanes, RA_UNROLL batches at a
+  // time, the first batch of W entries alone when that is all there is;
+  // returns the sum
+  auto offsets = [&](int j0, int re, long long acc, int& lo, int& hi, auto width) {
+    constexpr int W = decltype(width)::value;
+    const int l = lane & (W - 1);
+    while (__any_sync(FULL, j0 < re)) {
+      const bool one = !__any_sync(FULL, re - j0 > W);
+      int4 f[RA_UNROLL];
+#pragma unroll
+      for (int u = 0; u < RA_UNROLL; ++u)
+        if (u == 0 || !one) f[u] = entry(j0 + W * u + l, re);
+#pragma unroll
+      for (int u = 0; u < RA_UNROLL; ++u) {
+        if (u == 0 || !one) {  // warp-uniform
+          const int j = j0 + W * u + l;
+          if (f[u].y > 0) {
+            lo = min(lo, f[u].z);
+            hi = max(hi, f[u].w);
+          }
+          const long long incl = incl_scan(f[u].y, width);
+          if (j < re) aoff[j] = (int)(acc + incl - f[u].y);
+          acc += __shfl_sync(FULL, incl, W - 1, W);
+        }
       }
-    };
-    if (re - rs <= 32) {  // one batch (most rows)
-      const int j = rs + lane;
-      int bs = 0, be = 0;
-      if (j < re) entry(j, bs, be);
-      if (be > bs) {
-        lo = min(lo, op.b_col[bs]);
-        hi = max(hi, op.b_col[be - 1]);
-      }
-      const long long len = be - bs;
-      const long long incl = warp_incl_scan64(len);
-      if (j < re) aoff[j] = (int)(incl - len);
-      acc = __shfl_sync(FULL, incl, 31);
-    } else {
-      // RA_UNROLL batches of 32 entries at a time, each level of the
-      // dependent loads (A's column, B's row bounds, B's first and last
-      // column) issued for all of them before the next, so a long row of A
-      // is not walked one round trip after another
-      for (int b0 = rs; b0 < re; b0 += 32 * RA_UNROLL) {
-        int k[RA_UNROLL], bs[RA_UNROLL], be[RA_UNROLL];
-        bool ok[RA_UNROLL];
-#pragma unroll
-        for (int u = 0; u < RA_UNROLL; ++u) {
-          const int j = b0 + 32 * u + lane;
-          k[u] = j < re ? op.a_col[j] : 0;
-          ok[u] = j < re;
-          if (ok[u] && (unsigned)k[u] >= (unsigned)op.kdim) {
-            atomicOr(status, ST_BAD_INDEX);
-            ok[u] = false;
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < RA_UNROLL; ++u) {
-          bs[u] = ok[u] ? op.b_rowptr[k[u]] : 0;
-          be[u] = ok[u] ? op.b_rowptr[k[u] + 1] : 0;
-          if (ok[u] && !(bs[u] >= 0 && be[u] <= op.nnz_b && bs[u] <= be[u])) {
-            atomicOr(status, ST_BAD_INDEX);
-            ok[u] = false;
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < RA_UNROLL; ++u) {
-          if (ok[u] && be[u] > bs[u]) {
-            lo = min(lo, op.b_col[bs[u]]);
-            hi = max(hi, op.b_col[be[u] - 1]);
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < RA_UNROLL; ++u) {
-          if (b0 + 32 * u < re) {  // warp-uniform
-            const int j = b0 + 32 * u + lane;
-            const long long len = ok[u] ? (long long)(be[u] - bs[u]) : 0;
-            const long long incl = warp_incl_scan64(len);
-            if (j < re) aoff[j] = (int)(acc + incl - len);
-            acc += __shfl_sync(FULL, incl, 31);
-          }
-        }
+      j0 += W * RA_UNROLL;
+    }
+    return acc;
+  };
+  constexpr int GROUPS = RA_THREADS / G;
+  for (int lr0 = 0; lr0 < nrows; lr0 += GROUPS) {
+    const int lr = lr0 + (int)threadIdx.x / G;
+    int rs = 0, re = 0;
+    if (lr < nrows) {
+      rs = op.a_rowptr[row0 + lr];
+      re = op.a_rowptr[row0 + lr + 1];
+      if (gl == 0 && re > rs) atomicMax(&block_max_len, re - rs);
+      if (re - rs > RA_HEAVY) {
+        if (gl == 0) heavy[atomicAdd(&n_heavy, 1)] = lr;
+        re = rs;
       }
     }
+    int lo = 0x7fffffff, hi = -1;
+    const long long acc = offsets(rs, re, 0ll, lo, hi, std::integral_constant<int, G>());
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1) {
+    for (int d = G / 2; d > 0; d >>= 1) {
       lo = min(lo, __shfl_xor_sync(FULL, lo, d));
       hi = max(hi, __shfl_xor_sync(FULL, hi, d));
     }
+    if (lr < nrows && gl == 0) {
+      s_p[lr] = acc;
+      s_lo[lr] = lo;
+      s_hi[lr] = hi;
+    }
+  }
+  __syncthreads();
+  for (int h = 0; h < n_heavy; ++h) {  // each warp a stretch of the row: sums, then offsets
+    const int lr = heavy[h];
+    const int rs = op.a_rowptr[row0 + lr], re = op.a_rowptr[row0 + lr + 1];
+    const int per = ((re - rs + NW - 1) / NW + 31) & ~31;
+    const int j0 = min(rs + warp * per, re), j1 = min(j0 + per, re);
+    long long sum = 0;
+    int lo = 0x7fffffff, hi = -1;
+    for (int j = j0 + lane; j < j1; j += 32) {
+      const int4 f = entry(j, j1);
+      sum += f.y;
+      if (f.y > 0) {
+        lo = min(lo, f.z);
+        hi = max(hi, f.w);
+      }
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(FULL, sum, d);
+    lo = __reduce_min_sync(FULL, lo);
+    hi = __reduce_max_sync(FULL, hi);
     if (lane == 0) {
-      if (re - rs > 0) atomicMax(&block_max_len, re - rs);
-      const int span = acc > 0 ? hi + 1 - lo : 0;
+      part_p[warp] = sum;
+      part_lo[warp] = lo;
+      part_hi[warp] = hi;
+    }
+    __syncthreads();
+    long long acc = 0, total = 0;
+    for (int w = 0; w < NW; ++w) {
+      if (w < warp) acc += part_p[w];
+      total += part_p[w];
+      lo = min(lo, part_lo[w]);
+      hi = max(hi, part_hi[w]);
+    }
+    if (threadIdx.x == 0) {
+      s_p[lr] = total;
+      s_lo[lr] = lo;
+      s_hi[lr] = hi;
+    }
+    int l2 = 0, h2 = 0;
+    offsets(j0, j1, acc, l2, h2, std::integral_constant<int, 32>());
+    __syncthreads();
+  }
+  int bin = -1, rank = 0;
+  if (threadIdx.x < RA_ROWS) {  // two whole warps
+    const int lr = threadIdx.x, i = row0 + lr;
+    long long acc = 0;
+    int slot = 0;
+    if (lr < nrows) {
+      acc = s_p[lr];
+      const int lo = s_lo[lr], hi = s_hi[lr];
+      const int span = acc > 0 ? max(hi + 1 - lo, 1) : 0;
       row_span[i] = acc > 0 ? make_int2(lo, hi) : make_int2(0, -1);
       row_p[i] = acc;
       if (acc >= (1ll << 31)) atomicOr(status, ST_ROW_TOO_LONG);
       const long long cap = row_cap(acc, op.n, span);
       const int bin0 = first_bin_of(acc, cap, span, tn);
-      const int bin = row_list_of(bin0, acc, lo, span);
+      bin = row_list_of(bin0, acc, lo, span);
       if (bin < 0) c_cnt[i] = 0;
-      tcap[i] = (bin >= 0 && bin != FB_LONG) ? (int)cap : 0;
-      rowbin[lr] = bin;
-      if (bin >= 0) rowrank[lr] = atomicAdd(&hist[bin], 1);
+      slot = (bin >= 0 && bin != FB_LONG) ? (int)cap : 0;
+      tcap[i] = slot;
+      if (bin >= 0) rank = atomicAdd(&hist[bin], 1);
       // a table smaller than 1.25 x the column bound may overflow, and so may
       // a bitmap row of that many outputs
       const bool over = bin == FB_BITS ? cap > BITS_OUT_MAX
@@ -227,7 +375,16 @@ k_row_analysis(Operands op, int* __restrict__ aoff, long long* __restrict__ row_
                                              cap + cap / 4 + 1 > (64ll << bin);
       if (over) atomicAdd(&ovf[overflow_bin_of(acc, lo, span, tn)], 1);
       if (bin >= FB_TINY8) atomicAdd(&nominal[bin0], 1);
+    }
+    long long caps = slot;
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+      acc += __shfl_xor_sync(FULL, acc, d);
+      caps += __shfl_xor_sync(FULL, caps, d);
+    }
+    if (lane == 0) {
       atomicAdd(&block_p, (unsigned long long)acc);
+      atomicAdd(&block_cap, (unsigned long long)caps);
     }
   }
   __syncthreads();
@@ -240,20 +397,17 @@ k_row_analysis(Operands op, int* __restrict__ aoff, long long* __restrict__ row_
   if (threadIdx.x == 0) {
     atomicAdd(p_total, block_p);
     if (block_max_len > 0) atomicMax(max_row_len, block_max_len);
+    // rows_per_block divides SCAN_TILE: the block's rows lie in one tile
+    if (block_cap)
+      atomicAdd(reinterpret_cast<unsigned long long*>(tile_sum) + row0 / SCAN_TILE, block_cap);
   }
   __syncthreads();
-  for (int lr = threadIdx.x; lr < RA_ROWS; lr += RA_THREADS) {
-    const int b = rowbin[lr];
-    if (b >= 0) fb_rows[fb_list_at(b, base[b] + rowrank[lr], op.m)] = row0 + lr;
-  }
+  if (bin >= 0) fb_rows[fb_list_at(bin, base[bin] + rank, op.m)] = row0 + threadIdx.x;
 }
 
 // ---------------------------------------------------------------------------
 // Symbolic pass
 // ---------------------------------------------------------------------------
-
-__device__ __forceinline__ long long block_excl_scan64(long long v, long long* shm,
-                                                       long long& total);
 
 constexpr int SW_THREADS = 256;  // warp-per-row kernels: 8 warps per block
 
@@ -697,30 +851,12 @@ k_sym_long(Operands op, const int* __restrict__ rows, int nrows,
 // Scan (row pointers of C)
 // ---------------------------------------------------------------------------
 
-constexpr int SCAN_THREADS = 1024;
-constexpr int SCAN_ITEMS = 4;
-constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
+// Exclusive prefix sums of an int32 array in two launches: per-tile sums,
+// then every block adds up the tiles before its own (SCAN_SELF_TILES at most,
+// a few loads a thread) and scans its tile. Longer arrays scan the tile sums
+// in a launch of their own in between.
+constexpr int SCAN_SELF_TILES = 8192;
 
-__device__ __forceinline__ long long block_excl_scan64(long long v, long long* shm,
-                                                       long long& total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const long long incl = warp_incl_scan64(v);
-  if (lane == 31) shm[warp] = incl;
-  __syncthreads();
-  if (warp == 0) {
-    const long long w = (lane < (int)(blockDim.x >> 5)) ? shm[lane] : 0;
-    const long long wi = warp_incl_scan64(w);
-    shm[lane] = wi - w;
-    if (lane == 31) shm[32] = wi;
-  }
-  __syncthreads();
-  const long long r = shm[warp] + incl - v;
-  total = shm[32];
-  __syncthreads();
-  return r;
-}
-
-// Phase 1: per-tile sums of an int32 array.
 __global__ void __launch_bounds__(SCAN_THREADS)
 k_scan_tiles(const int* __restrict__ in, int n, long long* __restrict__ tile_sum) {
   __shared__ long long shm[33];
@@ -728,7 +864,7 @@ k_scan_tiles(const int* __restrict__ in, int n, long long* __restrict__ tile_sum
   long long v = 0;
 #pragma unroll
   for (int q = 0; q < SCAN_ITEMS; ++q) {
-    const long long idx = base + threadIdx.x * SCAN_ITEMS + q;
+    const long long idx = base + q * SCAN_THREADS + threadIdx.x;
     if (idx < n) v += in[idx];
   }
   long long total;
@@ -736,10 +872,9 @@ k_scan_tiles(const int* __restrict__ in, int n, long long* __restrict__ tile_sum
   if (threadIdx.x == 0) tile_sum[blockIdx.x] = total;
 }
 
-// Phase 2: exclusive scan of the tile sums (single block, looping).
+// Exclusive scan of more than SCAN_SELF_TILES tile sums (single block).
 __global__ void __launch_bounds__(SCAN_THREADS)
-k_scan_tile_sums(long long* __restrict__ tile_sum, int ntiles,
-                 long long* __restrict__ grand_total) {
+k_scan_tile_sums(long long* __restrict__ tile_sum, int ntiles) {
   __shared__ long long shm[33];
   long long carry = 0;
   for (int b = 0; b < ntiles; b += SCAN_THREADS) {
@@ -750,32 +885,53 @@ k_scan_tile_sums(long long* __restrict__ tile_sum, int ntiles,
     if (idx < ntiles) tile_sum[idx] = carry + ex;
     carry += total;
   }
-  if (threadIdx.x == 0) *grand_total = carry;
 }
 
-// Phase 3: out[i] = exclusive prefix of in (int64), out[n] = total.
+// out[i] = exclusive prefix of in, out[n] = the total, also to *grand_total;
+// any of the outputs (int64, and two int32 copies) may be null. tiles: the
+// tiles' sums, or (scanned) their exclusive prefix.
+struct ScanOut {
+  long long* p64;
+  int *p32, *copy32;
+};
+
 __global__ void __launch_bounds__(SCAN_THREADS)
-k_scan_apply(const int* __restrict__ in, int n, const long long* __restrict__ tile_off,
-             const long long* __restrict__ grand_total, long long* __restrict__ out) {
+k_scan_apply(const int* __restrict__ in, int n, const long long* __restrict__ tiles, bool scanned,
+             long long* __restrict__ grand_total, ScanOut out) {
   __shared__ long long shm[33];
-  const long long base = (long long)blockIdx.x * SCAN_TILE;
+  long long before = 0, total;
+  if (scanned) {
+    before = tiles[blockIdx.x];
+  } else {
+    for (int t = threadIdx.x; t < (int)blockIdx.x; t += SCAN_THREADS) before += tiles[t];
+    block_excl_scan64(before, shm, total);
+    before = total;
+  }
+  const long long base = (long long)blockIdx.x * SCAN_TILE + threadIdx.x * SCAN_ITEMS;
   int v[SCAN_ITEMS];
   long long sum = 0;
 #pragma unroll
   for (int q = 0; q < SCAN_ITEMS; ++q) {
-    const long long idx = base + threadIdx.x * SCAN_ITEMS + q;
-    v[q] = idx < n ? in[idx] : 0;
+    v[q] = base + q < n ? in[base + q] : 0;
     sum += v[q];
   }
-  long long total;
-  long long run = block_excl_scan64(sum, shm, total) + tile_off[blockIdx.x];
+  long long run = before + block_excl_scan64(sum, shm, total);
 #pragma unroll
   for (int q = 0; q < SCAN_ITEMS; ++q) {
-    const long long idx = base + threadIdx.x * SCAN_ITEMS + q;
-    if (idx < n) out[idx] = run;
+    if (base + q < n) {
+      if (out.p64) out.p64[base + q] = run;
+      if (out.p32) out.p32[base + q] = (int)run;
+      if (out.copy32) out.copy32[base + q] = (int)run;
+    }
     run += v[q];
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) out[n] = *grand_total;
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+    const long long all = before + total;
+    if (out.p64) out.p64[n] = all;
+    if (out.p32) out.p32[n] = (int)all;
+    if (out.copy32) out.copy32[n] = (int)all;
+    *grand_total = all;
+  }
 }
 
 // int64 row pointers -> the int32 row pointers of the cm boundary.
@@ -785,7 +941,6 @@ __global__ void k_rowptr_to_i32(const long long* __restrict__ in, int n1,
     out[i] = (int)in[i];
 }
 
-// int32 CSC/CSR pointer array from counts (used by the transpose).
 // Row pointers of a block-diagonal batch, per product: product p =
 // blockIdx.y owns the global rows [row_off[p], row_off[p + 1]); its m_p + 1
 // pointers, relative to its first entry, go to out[row_off[p] + p ...].
@@ -800,57 +955,102 @@ k_batch_rowptr(const long long* __restrict__ rowptr64, const long long* __restri
     out[r + p] = (int)(rowptr64[r] - base);
 }
 
-__global__ void k_rowptr_i64_to_i32_shift(const long long* __restrict__ in, int n1,
-                                          int* __restrict__ out, int* __restrict__ out2) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n1; i += gridDim.x * blockDim.x) {
-    out[i] = (int)in[i];
-    if (out2) out2[i] = (int)in[i];
-  }
-}
-
 // Rows finished by the fused pass: copy each row's sorted entries from the
-// temporary buffer (slot toff[i], c_cnt[i] entries) to its place in C. One
-// warp per row; rows with tcap == 0 (empty or long) are skipped.
+// temporary buffer (slot toff[i], c_cnt[i] entries) to its place in C; rows
+// with tcap == 0 (empty or long) are skipped. With `out_ptr`, also C's int32
+// row pointers (rows [r0, r1), and the last pointer when r1 == m). Bound by
+// memory: 16 bytes an entry (27-point stencil 96^3: 106 M entries).
+//
+// A warp takes `rpw` rows (a power of two, at most 32; fewer when C has few
+// rows, so that every SM has some): one lane per row loads its length and
+// offsets, so those loads are in flight together. Rows of 16 entries or more
+// on average are copied one after the other, four entries a lane in flight;
+// shorter ones as one sequence of entries, each lane finding its entry's row
+// by a search of the lengths' prefix sums with shuffles.
+constexpr int COPY_UNROLL = 4;
+
 __global__ void __launch_bounds__(256)
-k_copy_fused(int r0, int r1, const int* __restrict__ tcap, const long long* __restrict__ toff,
-             const int* __restrict__ c_cnt, const long long* __restrict__ c_rowptr,
-             const int* __restrict__ t_col, const float* __restrict__ t_val,
-             int* __restrict__ c_col, float* __restrict__ c_val) {
-  // Rows [r0, r1). A warp takes 32 rows at a time: each lane loads one row's
-  // length and offsets (so the 32 rows' loads are in flight together), then
-  // the warp copies the rows one after the other, two entries per lane per
-  // step.
+k_copy_fused(int r0, int r1, int m, int rpw, const int* __restrict__ tcap,
+             const long long* __restrict__ toff, const int* __restrict__ c_cnt,
+             const long long* __restrict__ c_rowptr, const int* __restrict__ t_col,
+             const float* __restrict__ t_val, int* __restrict__ c_col,
+             float* __restrict__ c_val, int* __restrict__ out_ptr) {
   const int lane = threadIdx.x & 31;
   const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
-  for (long long i0 = r0 + (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; i0 < r1;
-       i0 += warps * 32) {
+  for (long long i0 = r0 + (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * rpw; i0 < r1;
+       i0 += warps * rpw) {
     const long long i = i0 + lane;
     int n = 0;
     long long src = 0, dst = 0;
-    if (i < r1 && tcap[i] != 0) {
-      n = c_cnt[i];
-      src = toff[i];
-      dst = c_rowptr[i];
+    if (lane < rpw && i < r1) {
+      const bool fused = tcap[i] != 0;
+      if (out_ptr || fused) dst = c_rowptr[i];
+      if (fused) {
+        n = c_cnt[i];
+        src = toff[i];
+      }
+      if (out_ptr) {
+        out_ptr[i] = (int)dst;
+        if (i == m - 1) out_ptr[m] = (int)c_rowptr[m];
+      }
     }
-    for (int r = 0; r < 32; ++r) {
-      const int nr = __shfl_sync(FULL, n, r);
-      if (nr == 0) continue;  // warp-uniform
-      const long long s = __shfl_sync(FULL, src, r), d = __shfl_sync(FULL, dst, r);
-      for (int t = lane; t < nr; t += 64) {
-        const bool two = t + 32 < nr;
-        const int c0 = __ldcs(t_col + s + t);
-        const float v0 = __ldcs(t_val + s + t);
-        int c1 = 0;
-        float v1 = 0.f;
-        if (two) {
-          c1 = __ldcs(t_col + s + t + 32);
-          v1 = __ldcs(t_val + s + t + 32);
+    const int incl = warp_incl_scan(n);
+    const int total = __shfl_sync(FULL, incl, 31);
+    if (total >= 16 * rpw) {
+      for (int r = 0; r < rpw; ++r) {
+        const int nr = __shfl_sync(FULL, n, r);
+        if (nr == 0) continue;  // warp-uniform
+        const long long s = __shfl_sync(FULL, src, r), d = __shfl_sync(FULL, dst, r);
+        for (int t = lane; t < nr; t += 32 * COPY_UNROLL) {
+          int c[COPY_UNROLL];
+          float v[COPY_UNROLL];
+#pragma unroll
+          for (int u = 0; u < COPY_UNROLL; ++u) {
+            if (t + 32 * u < nr) {
+              c[u] = __ldcs(t_col + s + t + 32 * u);
+              v[u] = __ldcs(t_val + s + t + 32 * u);
+            }
+          }
+#pragma unroll
+          for (int u = 0; u < COPY_UNROLL; ++u) {
+            if (t + 32 * u < nr) {
+              __stcs(c_col + d + t + 32 * u, c[u]);
+              __stcs(c_val + d + t + 32 * u, v[u]);
+            }
+          }
         }
-        __stcs(c_col + d + t, c0);
-        __stcs(c_val + d + t, v0);
-        if (two) {
-          __stcs(c_col + d + t + 32, c1);
-          __stcs(c_val + d + t + 32, v1);
+      }
+    } else {
+      // entry f of the sequence belongs to the first row whose inclusive sum
+      // exceeds f; from = its temporary slot minus f's row start, likewise to
+      const long long from = src - (incl - n), to = dst - (incl - n);
+      for (int f0 = 0; f0 < total; f0 += 64) {
+        int c[2];
+        float v[2];
+        long long d[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int f = f0 + 32 * u + lane;
+          int row = 0;
+#pragma unroll
+          for (int step = 16; step > 0; step >>= 1) {
+            const int below = __shfl_sync(FULL, incl, row + step - 1);
+            if (below <= f) row += step;
+          }
+          row = min(row, 31);
+          const long long s = __shfl_sync(FULL, from, row) + f;
+          d[u] = __shfl_sync(FULL, to, row) + f;
+          if (f < total) {
+            c[u] = __ldcs(t_col + s);
+            v[u] = __ldcs(t_val + s);
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          if (f0 + 32 * u + lane < total) {
+            __stcs(c_col + d[u], c[u]);
+            __stcs(c_val + d[u], v[u]);
+          }
         }
       }
     }

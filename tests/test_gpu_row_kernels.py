@@ -81,3 +81,55 @@ def test_warp_rows_around_their_capacities(precision, n, lengths, crowd, empty):
     A, B = rows_of([c for c in COUNTS if c <= 2048], n, lengths, crowd, seed=n % 1000, empty=empty)
     stats = check_rows(A, B, precision, {})
     assert sum(stats["rows_per_symbolic_bin"][:5]) == A.rows, stats
+
+
+@pytest.mark.parametrize("csc", [False, True])
+@pytest.mark.parametrize("m", [1, 63, 64, 65, 4095, 4096, 4097, 20011])
+def test_row_analysis_and_scans_by_size(m, csc):
+    """Row counts around a scan tile and a block of row analysis, A rows of a
+    few entries with some above what a group of lanes walks (1024), most
+    columns of A empty, and B rows that are often empty."""
+    rng = np.random.default_rng(m)
+    k, n = 30011, 700
+    lens = rng.integers(0, 4, m)
+    for size, i in zip((1024, 1025, 1300, 4000), rng.choice(m, min(m, 4), replace=False)):
+        lens[i] = size
+    used = np.sort(rng.choice(k, 5000, replace=False))
+    r = np.repeat(np.arange(m), lens)
+    c = np.concatenate([used[np.sort(rng.choice(5000, x, replace=False))] for x in lens]) if lens.sum() else r
+    A = W.from_coo(m, k, r, c, rng.uniform(-1, 1, len(r)).astype(np.float32))
+    blens = rng.integers(0, 3, k)
+    br = np.repeat(np.arange(k), blens)
+    bc = np.concatenate([np.sort(rng.choice(n, x, replace=False)) for x in blens])
+    B = W.from_coo(k, n, br, bc, rng.uniform(-1, 1, len(br)).astype(np.float32))
+    ref = ref_product(A, B)
+    with sg.Handle() as h:
+        C = h.multiply_host(A.to_csc() if csc else A, B)
+        assert h.stats()["intermediate_products"] == ref["products"]
+    assert_structure_equal(C.rowptr, C.col, ref["rowptr"], ref["col"])
+    assert_values_close(C.val, ref, plain_tolerance(ref))
+
+
+@pytest.mark.parametrize("seed", range(12))
+def test_unsorted_rows_are_refused(seed):
+    """Rows of B must rise strictly: a repeat or a swap inside a row is
+    refused wherever it lies, equal or falling columns across a row boundary
+    (also over empty rows) are not."""
+    rng = np.random.default_rng(seed)
+    k, n = 700, 40
+    lens = rng.integers(0, 6, k)
+    col = np.concatenate([np.sort(rng.choice(n, x, replace=False)) for x in lens]).astype(np.int32)
+    ptr = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    B = W.Csr(k, n, ptr, col, np.ones(len(col), np.float32))
+    A = W.er(300, 4.0, seed, cols=k)
+    with sg.Handle() as h:
+        assert len(h.multiply_host(A, B).col) == len(ref_product(A, B)["col"])
+        row = int(rng.choice(np.nonzero(lens >= 2)[0]))
+        at = int(ptr[row] + rng.integers(0, lens[row] - 1))
+        if seed % 2:
+            B.col[at], B.col[at + 1] = col[at + 1], col[at]
+        else:
+            B.col[at + 1] = col[at]
+        with pytest.raises(sg.SpgemmError) as e:
+            h.multiply_host(A, B)
+        assert e.value.status == 1
