@@ -339,7 +339,7 @@ int Engine::analyze(const cm& A, const cm& B) {
     auto launch = [&](auto kernel) {
       kernel<<<(m + rpb - 1) / rpb, RA_THREADS, 0, stream_>>>(
           op_, b_info_.as<int4>(), rpb, aoff_.as<int>(), row_p_.as<long long>(), cnt,
-          tcap_.as<int>(), this->row_tiles(), dc->fb_count, dc->may_overflow, dc->warp_stat,
+          tcap_.as<int>(), this->row_tiles(), dc->fb_count, dc->may_overflow, dc->nominal,
           sym_rows_.as<int>(), &dc->p_total, &dc->max_row_len, row_span_.as<int2>(), &dc->status,
           tn_);
     };
@@ -365,8 +365,8 @@ int Engine::analyze(const cm& A, const cm& B) {
   for (int b = 0; b < FB_COUNT; ++b) {
     fb_counts_[b] = host_counters_->fb_count[b];
     may_overflow_[b] = host_counters_->may_overflow[b];
+    nominal_[b] = host_counters_->nominal[b];
   }
-  for (int b = 0; b < FB_WARP_BINS; ++b) warp_stat_[b] = host_counters_->warp_stat[b];
   n_long_sym_ = fb_counts_[FB_LONG];
   max_row_len_ = host_counters_->max_row_len;
   temp_total_ = host_counters_->grand_total;
@@ -489,7 +489,7 @@ int Engine::launch_first_pass() {
 
 template <int MODE>
 int Engine::launch_fused() {
-  constexpr int WPB = SW_THREADS / 32;
+  constexpr int WPB = HASH_THREADS / 32;
   constexpr int MID_THREADS = 512;
   constexpr size_t VB = sizeof(typename SlotOf<MODE>::T);
   const Operands op = op_;
@@ -531,21 +531,22 @@ int Engine::launch_fused() {
                                     &dc->overflow_count);
     SG_LAUNCHED("k_fused_bits");
   }
-#define SG_FUSED_WARP(L)                                                                      \
-  {                                                                                            \
-    const int b = L - 6, cnt = fb_counts_[b];                                                  \
-    if (cnt > 0) {                                                                             \
-      const size_t smem = WPB * ((size_t(1) << L) * (VB + 5) + SEG_SCRATCH_BYTES);             \
-      SG_CK(smem_attr(k_fused_warp<L, MODE>, smem), "smem attr k_fused_warp");                 \
-      prof_begin("k_fused_warp<" #L ">");                                                      \
-      k_fused_warp<L, MODE><<<blocks_for(cnt, WPB, (long long)sms_ * 16), SW_THREADS, smem,    \
-                              stream_>>>(op, rows + (size_t)b * m, cnt, row_span_.as<int2>(),  \
-                                         toff, c_cnt, t_col, t_val, rows, dc->fb_count, tn_,   \
-                                         row_p, &dc->overflow_count);                          \
-      SG_LAUNCHED("k_fused_warp");                                                             \
-    }                                                                                          \
+#define SG_FUSED_WARP(B)                                                                      \
+  if (const int cnt = fb_counts_[B]) {                                                         \
+    constexpr int L = hash_slots_log2(B);                                                      \
+    const size_t smem = WPB * hash_warp_bytes<L, MODE>();                                      \
+    SG_CK((smem_attr(k_fused_warp<L, MODE>, smem)), "smem attr k_fused_warp");                 \
+    /* rows in a stretch: enough stretches for the warps that the GPU holds */                 \
+    const int stretch = std::max(1, std::min(HASH_ROWS, cnt / (sms_ * 40)));                   \
+    prof_begin("k_fused_warp<" #B ">");                                                        \
+    k_fused_warp<L, MODE><<<blocks_for(cnt, WPB * stretch, (long long)sms_ * 64),              \
+                            HASH_THREADS, smem, stream_>>>(                                    \
+        op, rows + (size_t)B * m, cnt, stretch, row_span_.as<int2>(),                          \
+                                       toff, c_cnt, t_col, t_val, rows, dc->fb_count, tn_,     \
+                                       row_p, &dc->overflow_count);                            \
+    SG_LAUNCHED("k_fused_warp");                                                               \
   }
-  SG_FUSED_WARP(6) SG_FUSED_WARP(7) SG_FUSED_WARP(8) SG_FUSED_WARP(9) SG_FUSED_WARP(10)
+  SG_FUSED_WARP(0) SG_FUSED_WARP(1) SG_FUSED_WARP(2) SG_FUSED_WARP(3) SG_FUSED_WARP(4)
 #undef SG_FUSED_WARP
   // mid bitmap rows (and warp overflow with a narrow span)
   if (fb_counts_[FB_MID] + may_overflow_[FB_MID] > 0) {

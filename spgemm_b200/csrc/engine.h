@@ -30,7 +30,7 @@ struct DevBuf {
 struct DevCounters {
   int fb_count[24];  // first-pass bins (rows per bin; mid / block / sorted lists grow on overflow)
   int may_overflow[24];  // warp-bin rows that would be redone in each first-pass bin
-  int warp_stat[8];      // rows of each warp bin listed outside it (bins 15..)
+  int nominal[24];       // rows by first_bin_of, whatever list they are on
   int num_count[16];
   int slice_count;
   int mid_count;
@@ -126,8 +126,7 @@ class Engine {
   int n() const { return n_; }
   // Rows of first-pass bin b as the statistics count them.
   int sym_bin_rows(int b) const {
-    if (b < FB_WARP_BINS) return fb_counts_[b] + warp_stat_[b];
-    return fb_counts_[b] + (b == FB_ESC0 ? fb_counts_[FB_ESC256] + fb_counts_[FB_ESC512] : 0);
+    return nominal_[b] + (b == FB_ESC0 ? nominal_[FB_ESC256] + nominal_[FB_ESC512] : 0);
   }
   int overflow_rows() const { return overflow_rows_; }
   int num_bin_rows(int b) const { return num_counts_[b]; }
@@ -213,7 +212,7 @@ class Engine {
   long long p_total_ = 0, nnz_c_ = 0;
   int fb_counts_[24] = {0};
   int may_overflow_[24] = {0};
-  int warp_stat_[8] = {0};
+  int nominal_[24] = {0};
   long long temp_total_ = 0;
   int overflow_rows_ = 0;
   int num_counts_[16] = {0};

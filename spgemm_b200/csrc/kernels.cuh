@@ -10,11 +10,13 @@
 // each own a column slice. Partials never touch HBM.
 //
 // Pipeline (kernel names):
-//   k_validate        index ranges and sortedness of the inputs
-//   k_transpose_hist / k_transpose_scatter  A CSC -> CSR (row-wise expansion)
+//   k_check           index ranges and sortedness of the inputs
+//   k_transpose_scatter  A CSC -> CSR (row-wise expansion)
 //   k_row_analysis    P_i per row, flattened offsets, column spans, bins
-//   k_fused_warp/block  rows of at most long_p products in one pass: hash
-//                     accumulate, sort, row written to a temporary buffer
+//   k_fused_tiny/bits/warp/esc/block  rows of at most long_p products in one
+//                     pass, each written sorted to a temporary buffer: products
+//                     sorted in registers, a warp's bitmap, a warp's hash table,
+//                     products sorted in shared memory, a block's hash table
 //   k_num_long<.,512,sparse> as k_fused_mid  the same for rows whose column
 //                     span fits a bitmap (two passes over the row on chip)
 //   k_sym_long        exact nnz of long rows via a shared-memory bitmap
@@ -184,13 +186,12 @@ constexpr int BITS_OUT_MAX = 2 * BITS_CAP;
 // 32-column words from the word of column lo to the end of the span.
 __host__ __device__ inline int span_words(int lo, int span) { return ((lo & 31) + span + 31) >> 5; }
 
-// First-pass list of a row whose bin is `nominal` (first_bin_of): warp-bin
-// rows of at most 32 products are sorted in registers (packed keys hold a
-// 27-bit column offset), those with a narrow span use a bitmap.
-__host__ __device__ inline int row_list_of(int nominal, long long p, int lo, int span) {
-  if (nominal < 0 || nominal >= FB_WARP_BINS) return nominal;
-  if (p <= 32 && span < (1 << 27)) return p <= 8 ? FB_TINY8 : (p <= 16 ? FB_TINY16 : FB_TINY32);
-  return span_words(lo, span) <= BITS_WORDS ? FB_BITS : nominal;
+// Slots (of four columns) of the hash table of warp bin b.
+__host__ __device__ constexpr int hash_slots_log2(int b) { return b < 2 ? 6 + b : 5 + b; }
+
+// Whether a warp-bin row may need more slots than its table gives.
+__host__ __device__ inline bool hash_may_overflow(int b, long long cap) {
+  return cap > (1 << hash_slots_log2(b)) * 4 / 5;
 }
 
 // Where a warp-bin row whose table overflows is redone: the sorted bins when
@@ -199,6 +200,20 @@ __host__ __device__ inline int row_list_of(int nominal, long long p, int lo, int
 __host__ __device__ inline int overflow_bin_of(long long p, int lo, int span, const Tuning& t) {
   if (p > t.esc_p_min && span > t.esc_span_min && p <= 4096) return esc_bin_of(p);
   return (lo & 31) + span <= t.mid_cols ? FB_MID : FB_BLOCK0 + 2;
+}
+
+// First-pass list of a row whose bin is `nominal` (first_bin_of): warp-bin
+// rows of at most 32 products are sorted in registers (packed keys hold a
+// 27-bit column offset), those with a narrow span use a bitmap, and spans too
+// wide for the table's packed order (a quarter of 2^26 columns at 64 slots)
+// go where overflowing rows do.
+__host__ __device__ inline int row_list_of(int nominal, long long p, int lo, int span,
+                                           const Tuning& t) {
+  if (nominal < 0 || nominal >= FB_WARP_BINS) return nominal;
+  if (p <= 32 && span < (1 << 27)) return p <= 8 ? FB_TINY8 : (p <= 16 ? FB_TINY16 : FB_TINY32);
+  if (span_words(lo, span) <= BITS_WORDS) return FB_BITS;
+  if ((span >> 2) + 2 >= 1 << (26 - nominal)) return overflow_bin_of(p, lo, span, t);
+  return nominal;
 }
 
 // Numeric bin of a long row (P_i > long_p) with nnz_i outputs.
@@ -233,7 +248,6 @@ struct SegScratch {
   int bstart[32];
   int len[32];
   float a[32];
-  int count;  // fused warp rows: distinct columns inserted so far
 };
 
 // Move the lanes with len > 0 to lanes 0..cnt-1 (order preserved).
@@ -437,30 +451,6 @@ __device__ __forceinline__ int chunk_for(long long p, int nwarps, int max_chunk)
   if (u < 32) u = 32;
   if (u > max_chunk) u = max_chunk;
   return (int)u;
-}
-
-// Whole row of A, one warp. With stop_limit >= 0 the walk ends early once
-// sc->count exceeds it (checked between 32-entry batches, warp-uniformly).
-template <bool NEED_VAL, class F>
-__device__ __forceinline__ void warp_expand_row(const Operands& op, int rs, int re,
-                                                F& f, SegScratch* sc, int stop_limit = -1) {
-  const int lane = lane_id();
-  for (int base = rs; base < re; base += 32) {
-    if (stop_limit >= 0) {
-      __syncwarp();
-      if (*((volatile int*)&sc->count) > stop_limit) break;
-    }
-    const int j = base + lane;
-    int bstart = 0, len = 0;
-    float a = 0.f;
-    if (j < re) {
-      const int k = __ldg(op.a_col + j);
-      a = __ldg(op.a_val + j);
-      bstart = __ldg(op.b_rowptr + k);
-      len = __ldg(op.b_rowptr + k + 1) - bstart;
-    }
-    warp_run_batch<NEED_VAL>(op, bstart, len, a, f, sc);
-  }
 }
 
 // Products [f0, f1) of the row's flattened product sequence (entries in
@@ -793,47 +783,6 @@ struct LongBits {
       (*this)(c4.z, 0.f, 0.f);
       (*this)(c4.w, 0.f, 0.f);
     }
-  }
-};
-
-// Fused-pass hash insert: like the numeric inserts, but a full table is not an
-// error (the caller redoes the row with a larger structure when it counted
-// more distinct columns than its limit), and new keys are counted.
-__device__ __forceinline__ int hash_slot_soft(unsigned* keys, int log2t, unsigned col,
-                                              bool& inserted) {
-  const unsigned mask = (1u << log2t) - 1u;
-  unsigned h = hash_col(col, log2t);
-  inserted = false;
-  for (unsigned probe = 0; probe <= mask; ++probe) {
-    const unsigned k = ((volatile unsigned*)keys)[h];
-    if (k == col) return (int)h;
-    if (k == EMPTY_KEY) {
-      const unsigned old = atomicCAS(keys + h, EMPTY_KEY, col);
-      if (old == EMPTY_KEY) { inserted = true; return (int)h; }
-      if (old == col) return (int)h;
-    }
-    h = (h + 1u) & mask;
-  }
-  return -1;
-}
-
-// `count` (per warp, shared) counts distinct columns; once it exceeds `limit`
-// the row will be redone elsewhere, so further products are skipped.
-template <int MODE>  // 0: FP32 add; 1: TwoSum-compensated FP32 pair
-struct FusedHash {
-  unsigned* keys;
-  void* vals;
-  int log2t;
-  int* count;
-  int limit;
-  __device__ __forceinline__ void operator()(int col, float a, float b) {
-    if (*((volatile int*)count) > limit) return;
-    bool ins;
-    const int h = hash_slot_soft(keys, log2t, (unsigned)col, ins);
-    if (ins) atomicAdd(count, 1);
-    if (h < 0) return;
-    if (MODE == 0) atomicAdd(static_cast<float*>(vals) + h, __fmul_rn(a, b));
-    else twosum_accumulate(static_cast<float2*>(vals) + h, a, b);
   }
 };
 

@@ -178,8 +178,8 @@ constexpr int RA_HEAVY = 1024; // rows of more entries are walked by the whole b
 // span_i) for rows the fused pass computes (0 otherwise), which sizes their
 // slot in the temporary output buffer; tile_sum gets tcap's sum per
 // SCAN_TILE rows. may_overflow[b] counts the warp-bin rows that go to bin b
-// should their table overflow; warp_stat the rows of each warp bin that have
-// a list outside it. Rows are appended to their bin's list with one global
+// should their table overflow, nominal_count the rows of each bin of
+// first_bin_of, whatever list they are on. Rows are appended to their bin's list with one global
 // atomic per bin per block. A's indices are range-checked here because the
 // validation pass's result is only read after this kernel; b_info holds valid
 // positions only.
@@ -196,27 +196,28 @@ k_row_analysis(Operands op, const int4* __restrict__ b_info, int rows_per_block,
                int* __restrict__ aoff, long long* __restrict__ row_p,
                int* __restrict__ c_cnt, int* __restrict__ tcap, long long* __restrict__ tile_sum,
                int* __restrict__ fb_count, int* __restrict__ may_overflow,
-               int* __restrict__ warp_stat, int* __restrict__ fb_rows,
+               int* __restrict__ nominal_count, int* __restrict__ fb_rows,
                unsigned long long* __restrict__ p_total, int* __restrict__ max_row_len,
                int2* __restrict__ row_span, unsigned* status, Tuning tn) {
   constexpr int NW = RA_THREADS / 32;
-  __shared__ int hist[FB_COUNT], base[FB_COUNT], ovf[FB_COUNT], nominal[FB_WARP_BINS];
+  __shared__ int hist[FB_COUNT], base[FB_COUNT], ovf[FB_COUNT], nominal[FB_COUNT];
   __shared__ long long s_p[RA_ROWS];
   __shared__ int s_lo[RA_ROWS], s_hi[RA_ROWS];
   __shared__ int heavy[RA_ROWS], n_heavy;
   __shared__ long long part_p[NW];
   __shared__ int part_lo[NW], part_hi[NW];
+  __shared__ unsigned cand[2];
+  __shared__ int s_pairs, s_hits;
   __shared__ unsigned long long block_p, block_cap;
   __shared__ int block_max_len;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gl = lane & (G - 1);
   const int row0 = blockIdx.x * rows_per_block;
   const int nrows = min(rows_per_block, op.m - row0);
-  if (threadIdx.x < FB_COUNT) hist[threadIdx.x] = ovf[threadIdx.x] = 0;
-  if (threadIdx.x < FB_WARP_BINS) nominal[threadIdx.x] = 0;
+  if (threadIdx.x < FB_COUNT) hist[threadIdx.x] = ovf[threadIdx.x] = nominal[threadIdx.x] = 0;
   if (threadIdx.x == 0) {
     block_p = block_cap = 0;
     block_max_len = 0;
-    n_heavy = 0;
+    n_heavy = s_pairs = s_hits = 0;
   }
   __syncthreads();
   // B row of A's entry j (an empty one beyond `re` or for an invalid index)
@@ -349,32 +350,73 @@ k_row_analysis(Operands op, const int4* __restrict__ b_info, int rows_per_block,
     offsets(j0, j1, acc, l2, h2, std::integral_constant<int, 32>());
     __syncthreads();
   }
-  int bin = -1, rank = 0;
-  if (threadIdx.x < RA_ROWS) {  // two whole warps
-    const int lr = threadIdx.x, i = row0 + lr;
-    long long acc = 0;
-    int slot = 0;
+  // bins, one thread per row (two whole warps); hashed rows that could be
+  // sorted instead are candidates
+  int bin = -1, bin0 = -1, rank = 0, lo = 0, span = 0;
+  long long acc = 0, cap = 0;
+  bool candidate = false;
+  if (threadIdx.x < RA_ROWS) {
+    const int lr = threadIdx.x;
     if (lr < nrows) {
       acc = s_p[lr];
-      const int lo = s_lo[lr], hi = s_hi[lr];
-      const int span = acc > 0 ? max(hi + 1 - lo, 1) : 0;
-      row_span[i] = acc > 0 ? make_int2(lo, hi) : make_int2(0, -1);
+      lo = s_lo[lr];
+      span = acc > 0 ? max(s_hi[lr] + 1 - lo, 1) : 0;
+      cap = row_cap(acc, op.n, span);
+      bin0 = first_bin_of(acc, cap, span, tn);
+      bin = row_list_of(bin0, acc, lo, span, tn);
+      candidate = bin >= 0 && bin < FB_WARP_BINS && overflow_bin_of(acc, lo, span, tn) >= FB_ESC0;
+    }
+    const unsigned c = __ballot_sync(FULL, candidate);
+    if (lane == 0) cand[warp] = c;
+  }
+  __syncthreads();
+  // Do the rows' products share columns? Each warp looks at one candidate row:
+  // is the middle column of an entry's B row also in the next entry's B row?
+  // Neighbouring rows of grid operators and meshes overlap (27-point stencil:
+  // 2 of 3 pairs, any order of the entries: 1 of 2), rows of random graphs
+  // hardly. Rows that do not repeat columns fill a hash table for nothing
+  // (random rows of 200 products: 4.6 ns each hashed, 3.4 sorted).
+  const int n0 = __popc(cand[0]), ncand = n0 + __popc(cand[1]);
+  if (ncand > 0 && warp < ncand) {  // warp-uniform
+    const int idx = ncand <= NW ? warp : warp * ncand / NW;
+    const unsigned mask = idx < n0 ? cand[0] : cand[1];
+    const int nth = idx < n0 ? idx : idx - n0;
+    const unsigned at = __ballot_sync(
+        FULL, ((mask >> lane) & 1u) && __popc(mask & ((1u << lane) - 1u)) == nth);
+    const int lr = (idx < n0 ? 0 : 32) + __ffs(at) - 1;
+    const int rs = op.a_rowptr[row0 + lr], re = op.a_rowptr[row0 + lr + 1];
+    const int4 f = entry(rs + lane, re);
+    const int next = __shfl_down_sync(FULL, f.x, 1), next_len = __shfl_down_sync(FULL, f.y, 1);
+    const bool pair = lane < 31 && f.y > 0 && next_len > 0;
+    bool hit = false;
+    if (pair) {
+      const int c = __ldg(op.b_col + f.x + f.y / 2);
+      const int p = lower_bound_i32(op.b_col, next, next + next_len, c);
+      hit = p < next + next_len && __ldg(op.b_col + p) == c;
+    }
+    const int pairs = __popc(__ballot_sync(FULL, pair)), hits = __popc(__ballot_sync(FULL, hit));
+    if (lane == 0) {
+      atomicAdd(&s_pairs, pairs);
+      atomicAdd(&s_hits, hits);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < RA_ROWS) {
+    const int i = row0 + threadIdx.x;
+    int slot = 0;
+    if (threadIdx.x < nrows) {
+      if (candidate && 4 * s_hits < max(s_pairs, 1)) bin = overflow_bin_of(acc, lo, span, tn);
+      row_span[i] = acc > 0 ? make_int2(lo, lo + span - 1) : make_int2(0, -1);
       row_p[i] = acc;
       if (acc >= (1ll << 31)) atomicOr(status, ST_ROW_TOO_LONG);
-      const long long cap = row_cap(acc, op.n, span);
-      const int bin0 = first_bin_of(acc, cap, span, tn);
-      bin = row_list_of(bin0, acc, lo, span);
       if (bin < 0) c_cnt[i] = 0;
       slot = (bin >= 0 && bin != FB_LONG) ? (int)cap : 0;
       tcap[i] = slot;
       if (bin >= 0) rank = atomicAdd(&hist[bin], 1);
-      // a table smaller than 1.25 x the column bound may overflow, and so may
-      // a bitmap row of that many outputs
       const bool over = bin == FB_BITS ? cap > BITS_OUT_MAX
-                                       : bin >= 0 && bin < FB_WARP_BINS &&
-                                             cap + cap / 4 + 1 > (64ll << bin);
+                                       : bin >= 0 && bin < FB_WARP_BINS && hash_may_overflow(bin, cap);
       if (over) atomicAdd(&ovf[overflow_bin_of(acc, lo, span, tn)], 1);
-      if (bin >= FB_TINY8) atomicAdd(&nominal[bin0], 1);
+      if (bin0 >= 0) atomicAdd(&nominal[bin0], 1);
     }
     long long caps = slot;
 #pragma unroll
@@ -392,8 +434,8 @@ k_row_analysis(Operands op, const int4* __restrict__ b_info, int rows_per_block,
     base[threadIdx.x] = atomicAdd(fb_count + threadIdx.x, hist[threadIdx.x]);
   if (threadIdx.x < FB_COUNT && ovf[threadIdx.x])
     atomicAdd(may_overflow + threadIdx.x, ovf[threadIdx.x]);
-  if (threadIdx.x < FB_WARP_BINS && nominal[threadIdx.x])
-    atomicAdd(warp_stat + threadIdx.x, nominal[threadIdx.x]);
+  if (threadIdx.x < FB_COUNT && nominal[threadIdx.x])
+    atomicAdd(nominal_count + threadIdx.x, nominal[threadIdx.x]);
   if (threadIdx.x == 0) {
     atomicAdd(p_total, block_p);
     if (block_max_len > 0) atomicMax(max_row_len, block_max_len);
@@ -409,227 +451,11 @@ k_row_analysis(Operands op, const int4* __restrict__ b_info, int rows_per_block,
 // Symbolic pass
 // ---------------------------------------------------------------------------
 
-constexpr int SW_THREADS = 256;  // warp-per-row kernels: 8 warps per block
-
 // Value slot type of each precision mode (0 plain, 1 compensated).
 template <int MODE> struct SlotOf { using T = float; };
 template <> struct SlotOf<1> { using T = unsigned long long; };  // float2 or double bits
 
-// Fused pass, one warp per row: hash accumulate, compact the table in place,
-// sort the occupied entries by column, write the sorted row to the temporary
-// buffer at toff[i] and its length to c_cnt[i]. A row that turns out to have
-// more distinct columns than 4/5 of the table is pushed to the sorted bins
-// (when the tuning sorts rows like it), else to the mid list (span within
-// mid_cols) or the largest block list, and redone there.
-//
-// Sorting: tables of 256 slots and more sort packed keys (column offset in
-// the row's span above the slot index; the values stay in their slots) by a
-// bucket pass -- NB = T/4 buckets on the column offset's top bits, counts,
-// scan, scatter with the keys held in registers -- and an insertion sort of
-// each bucket by one lane. Rows whose columns crowd one bucket (more than
-// BUCKET_MAX entries: skewed column popularity) take LSD radix passes over
-// the column offset instead. Rows of at most SMALL_SORT entries (and small
-// tables) sort the packed keys bitonically; rows whose span is too wide to
-// pack sort key/value pairs bitonically.
-constexpr int BUCKET_MAX = 24;
-constexpr int SMALL_SORT = 128;  // rows with at most this many entries sort bitonically
-
-template <int LOG2T, int MODE>
-__global__ void __launch_bounds__(SW_THREADS, LOG2T >= 10 ? 2 : 4)
-k_fused_warp(Operands op, const int* __restrict__ rows, int nrows,
-             const int2* __restrict__ row_span, const long long* __restrict__ toff,
-             int* __restrict__ c_cnt, int* __restrict__ t_col, float* __restrict__ t_val,
-             int* fb_rows, int* fb_count, Tuning tn,
-             const long long* __restrict__ row_p, int* __restrict__ overflow_count) {
-  constexpr int T = 1 << LOG2T;
-  constexpr int LIMIT = T * 4 / 5;
-  constexpr int WPB = SW_THREADS / 32;
-  using V = typename SlotOf<MODE>::T;
-  extern __shared__ __align__(16) unsigned char smem[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  V* vals = reinterpret_cast<V*>(smem) + warp * T;
-  unsigned* keys = reinterpret_cast<unsigned*>(smem + WPB * T * sizeof(V)) + warp * T;
-  SegScratch* sc = reinterpret_cast<SegScratch*>(smem + WPB * T * (sizeof(V) + 4)) + warp;
-  constexpr int NB = T / 4;                   // sort buckets (tables of >= 256 slots)
-  constexpr int E = (LIMIT + 31) / 32;        // entries per lane
-  int* bucket = reinterpret_cast<int*>(smem + WPB * (T * (sizeof(V) + 4) + sizeof(SegScratch))) +
-                warp * NB;
-  for (int r = blockIdx.x * WPB + warp; r < nrows; r += gridDim.x * WPB) {
-    const int i = rows[r];
-    for (int t = lane; t < T; t += 32) { keys[t] = EMPTY_KEY; vals[t] = V(0); }
-    if (lane == 0) sc->count = 0;
-    __syncwarp();
-    FusedHash<MODE> f{keys, vals, LOG2T, &sc->count, LIMIT};
-    warp_expand_row<true>(op, op.a_rowptr[i], op.a_rowptr[i + 1], f, sc, LIMIT);
-    __syncwarp();
-    const int distinct = *((volatile int*)&sc->count);
-    __syncwarp();
-    if (distinct > LIMIT) {  // redo with a larger structure
-      if (lane == 0) {
-        const int2 sp = row_span[i];
-        const int q = overflow_bin_of(row_p[i], sp.x, sp.y + 1 - sp.x, tn);
-        fb_rows[(size_t)q * op.m + atomicAdd(fb_count + q, 1)] = i;
-        atomicAdd(overflow_count, 1);
-      }
-      continue;
-    }
-    // compact in place: entries move to lower slots only, after the whole
-    // 32-slot group has been read
-    int o = 0;
-    for (int g = 0; g < T; g += 32) {
-      const unsigned k = keys[g + lane];
-      const V v = vals[g + lane];
-      const bool valid = k != EMPTY_KEY;
-      const unsigned bal = __ballot_sync(FULL, valid);
-      const int pos = o + __popc(bal & ((1u << lane) - 1u));
-      __syncwarp();
-      if (valid) { keys[pos] = k; vals[pos] = v; }
-      o += __popc(bal);
-      __syncwarp();
-    }
-    int n2 = 1;
-    while (n2 < o) n2 <<= 1;
-    const long long base = toff[i];
-    const int2 sp = row_span[i];
-    const unsigned lo = (unsigned)(sp.x & ~31);
-    const unsigned span = (unsigned)(sp.y + 1) - lo;
-    if (span <= (1u << (32 - LOG2T)) && (LOG2T < 8 || o <= SMALL_SORT)) {
-      // packed keys, (column - lo) << LOG2T | slot, sorted bitonically
-      for (int t = lane; t < n2; t += 32)
-        keys[t] = t < o ? ((keys[t] - lo) << LOG2T) | (unsigned)t : EMPTY_KEY;
-      __syncwarp();
-      bitonic_sort_keys_rt(keys, n2, lane, 32, WarpSync());
-      for (int t = lane; t < o; t += 32) {
-        const unsigned p = keys[t];
-        const int slot = (int)(p & (T - 1));
-        t_col[base + t] = (int)(lo + (p >> LOG2T));
-        if (MODE == 0) t_val[base + t] = finalize_value(reinterpret_cast<float*>(vals)[slot]);
-        else t_val[base + t] = finalize_value(reinterpret_cast<float2*>(vals)[slot]);
-      }
-    } else if (LOG2T >= 8 && span <= (1u << (32 - LOG2T))) {
-      // packed keys: (column - lo) << LOG2T | slot
-      unsigned pk[E];
-#pragma unroll
-      for (int e = 0; e < E; ++e) {
-        const int t = lane + 32 * e;
-        pk[e] = t < o ? ((keys[t] - lo) << LOG2T) | (unsigned)t : EMPTY_KEY;
-      }
-      const int bits = 32 - __clz(span > 1 ? span - 1 : 1);
-      const int shift = bits > LOG2T - 2 ? bits - (LOG2T - 2) : 0;
-      for (int t = lane; t < NB; t += 32) bucket[t] = 0;
-      __syncwarp();
-#pragma unroll
-      for (int e = 0; e < E; ++e)
-        if (pk[e] != EMPTY_KEY) atomicAdd(&bucket[(pk[e] >> LOG2T) >> shift], 1);
-      __syncwarp();
-      constexpr int PER = NB / 32 > 0 ? NB / 32 : 1;
-      int cnt[PER];
-      int sum = 0, mx = 0;
-#pragma unroll
-      for (int q = 0; q < PER; ++q) {
-        cnt[q] = bucket[lane * PER + q];
-        sum += cnt[q];
-        mx = max(mx, cnt[q]);
-      }
-#pragma unroll
-      for (int d = 16; d > 0; d >>= 1) mx = max(mx, __shfl_xor_sync(FULL, mx, d));
-      if (mx <= BUCKET_MAX) {
-        int run = warp_incl_scan(sum) - sum;
-#pragma unroll
-        for (int q = 0; q < PER; ++q) {
-          bucket[lane * PER + q] = run;
-          run += cnt[q];
-        }
-        __syncwarp();
-        // every key is in registers: scatter into the key array by bucket
-#pragma unroll
-        for (int e = 0; e < E; ++e)
-          if (pk[e] != EMPTY_KEY) keys[atomicAdd(&bucket[(pk[e] >> LOG2T) >> shift], 1)] = pk[e];
-        __syncwarp();
-        // bucket b now ends at bucket[b]; each lane sorts its buckets in place
-        for (int b = lane; b < NB; b += 32) {
-          const int s0 = b ? bucket[b - 1] : 0, s1 = bucket[b];
-          for (int x = s0 + 1; x < s1; ++x) {
-            const unsigned v = keys[x];
-            int y = x - 1;
-            while (y >= s0 && keys[y] > v) {
-              keys[y + 1] = keys[y];
-              --y;
-            }
-            keys[y + 1] = v;
-          }
-        }
-      } else {
-        // crowded buckets (skewed columns): LSD radix sort of the column
-        // offset, LOG2T - 2 bits (NB counters) a pass, stable by array order;
-        // each pass scatters from registers into the key array, then reloads
-        // the keys in the new order
-        constexpr int DIG = LOG2T - 2;
-        for (int d0 = 0; d0 < bits; d0 += DIG) {
-          for (int t = lane; t < NB; t += 32) bucket[t] = 0;
-          __syncwarp();
-#pragma unroll
-          for (int e = 0; e < E; ++e)
-            if (pk[e] != EMPTY_KEY) atomicAdd(&bucket[((pk[e] >> LOG2T) >> d0) & (NB - 1)], 1);
-          __syncwarp();
-          int tot = 0;
-#pragma unroll
-          for (int q = 0; q < PER; ++q) {
-            cnt[q] = bucket[lane * PER + q];
-            tot += cnt[q];
-          }
-          int run = warp_incl_scan(tot) - tot;
-#pragma unroll
-          for (int q = 0; q < PER; ++q) {
-            bucket[lane * PER + q] = run;
-            run += cnt[q];
-          }
-          __syncwarp();
-#pragma unroll
-          for (int e = 0; e < E; ++e) {
-            const bool valid = pk[e] != EMPTY_KEY;
-            const unsigned dig = valid ? ((pk[e] >> LOG2T) >> d0) & (NB - 1) : (unsigned)(NB + lane);
-            const unsigned peers = __match_any_sync(FULL, dig);
-            const int rank = __popc(peers & ((1u << lane) - 1u));
-            int pos = 0;
-            if (valid) pos = bucket[dig] + rank;
-            __syncwarp();
-            if (valid) {
-              keys[pos] = pk[e];
-              if (rank == __popc(peers) - 1) bucket[dig] = pos + 1;
-            }
-            __syncwarp();
-          }
-#pragma unroll
-          for (int e = 0; e < E; ++e) {
-            const int t = lane + 32 * e;
-            pk[e] = t < o ? keys[t] : EMPTY_KEY;
-          }
-          __syncwarp();
-        }
-      }
-      __syncwarp();
-      for (int t = lane; t < o; t += 32) {
-        const unsigned p = keys[t];
-        const int slot = (int)(p & (T - 1));
-        t_col[base + t] = (int)(lo + (p >> LOG2T));
-        if (MODE == 0) t_val[base + t] = finalize_value(reinterpret_cast<float*>(vals)[slot]);
-        else t_val[base + t] = finalize_value(reinterpret_cast<float2*>(vals)[slot]);
-      }
-    } else {
-      for (int t = o + lane; t < n2; t += 32) keys[t] = EMPTY_KEY;
-      __syncwarp();
-      bitonic_sort_kv_rt(keys, vals, n2, lane, 32, WarpSync());
-      for (int t = lane; t < o; t += 32) {
-        t_col[base + t] = (int)keys[t];
-        if (MODE == 0) t_val[base + t] = finalize_value(reinterpret_cast<float*>(vals)[t]);
-        else t_val[base + t] = finalize_value(reinterpret_cast<float2*>(vals)[t]);
-      }
-    }
-    if (lane == 0) c_cnt[i] = o;
-    __syncwarp();
-  }
-}
+constexpr int BUCKET_MAX = 24;  // entries of a sort bucket one thread orders by insertion
 
 // Fused pass, one block per row (rows whose column bound needs more than a
 // warp's table and whose span is too wide for the bitmap): hash accumulate

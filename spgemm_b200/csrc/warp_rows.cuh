@@ -1,6 +1,7 @@
 // Fused pass, rows merged by a warp or less: rows of at most 32 products
-// (sorted in registers by 8, 16 or 32 lanes), and rows whose column span is
-// narrow enough for a bitmap in shared memory (one warp per row).
+// (sorted in registers by 8, 16 or 32 lanes), rows whose column span is narrow
+// enough for a bitmap in shared memory (one warp per row), and rows hashed in
+// shared memory (one warp per row).
 //
 // The reference scatters every partial product of a row into its bucket in
 // global memory (src/mm.cu:288-312) and merges the bucket in a dense array
@@ -387,6 +388,389 @@ k_fused_bits(Operands op, const int* __restrict__ rows, int nrows,
     }
     *my_bits = make_uint4(0u, 0u, 0u, 0u);  // clean for the next row
     __syncwarp();
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Rows in a warp's hash table
+// ---------------------------------------------------------------------------
+
+// Bitonic sort of N = 32 * R keys held by a warp, key e = 32 * r + lane in
+// k[r]: exchanges over fewer than 32 positions are shuffles, the rest are
+// between a lane's own registers.
+template <int R>
+__device__ __forceinline__ void warp_sort_regs(unsigned (&k)[R], int lane) {
+#pragma unroll
+  for (int size = 2; size <= 32 * R; size <<= 1) {
+#pragma unroll
+    for (int j = size >> 1; j > 0; j >>= 1) {
+      if (j >= 32) {
+        const int jr = j >> 5;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          if ((r & jr) == 0) {
+            const bool up = ((r << 5) & size) == 0;
+            const unsigned lo = min(k[r], k[r + jr]), hi = max(k[r], k[r + jr]);
+            k[r] = up ? lo : hi;
+            k[r + jr] = up ? hi : lo;
+          }
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const unsigned o = __shfl_xor_sync(FULL, k[r], j);
+          const bool up = size >= 32 ? ((r << 5) & size) == 0 : (lane & size) == 0;
+          const bool low = (lane & j) == 0;
+          k[r] = low == up ? min(k[r], o) : max(k[r], o);
+        }
+      }
+    }
+  }
+}
+
+// keys[0, o) (shared memory, o <= 32 * R) to ascending order.
+template <int R>
+__device__ __forceinline__ void warp_sort_shared(unsigned* keys, int o, int lane) {
+  unsigned k[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) k[r] = 32 * r + lane < o ? keys[32 * r + lane] : EMPTY_KEY;
+  warp_sort_regs<R>(k, lane);
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (32 * r + lane < o) keys[32 * r + lane] = k[r];
+}
+
+// A warp's table: 2^LOG2T slots in buckets of four, each slot for a group of
+// four neighbouring columns (key: column offset from the row's first column,
+// / 4) with a value per column. Columns of structured rows come in runs, so a
+// step's lanes look up few distinct keys and a run claims one or two slots;
+// one 16-byte read covers a bucket, so nearly every look-up ends at the first
+// (single-key probing walked 3 to 5 keys for the worst of 32 lanes). A value
+// that no product has reached holds ABSENT, a NaN pattern that no FP32
+// operation returns.
+//
+// Keys are relative to the row, and they stay in the table from one row to
+// the next: rows of grid operators repeat their neighbours' pattern, so after
+// the first row nothing is claimed, compacted or sorted any more. Slots that
+// the row at hand does not reach are all ABSENT and are passed over.
+constexpr int GROUP_COLS = 4;
+constexpr unsigned ABSENT = 0xffffffffu;
+
+template <int MODE> struct GroupVals;  // the four values of a slot
+template <> struct alignas(16) GroupVals<0> { float v[GROUP_COLS]; };
+template <> struct alignas(16) GroupVals<1> { float2 v[GROUP_COLS]; };
+
+// Bucket of a group: two multiplications with a shift between them. A single
+// one maps the regular strides of grid operators onto few places (27-point
+// stencil 60^3: planes and rows next to each other, 2.1x the time of 61^3).
+__device__ __forceinline__ unsigned hash_group(unsigned g, int log2t) {
+  g *= 0x9e3779b1u;
+  g ^= g >> 15;
+  return ((g * 0x85ebca6bu) >> (34 - log2t)) * 4u;  // the bucket's first slot
+}
+
+// The four keys of a bucket as they are now (other lanes claim slots).
+__device__ __forceinline__ uint4 bucket_keys(const unsigned* bucket) {
+  uint4 k;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(k.x), "=r"(k.y), "=r"(k.z), "=r"(k.w)
+               : "r"((unsigned)__cvta_generic_to_shared(bucket))
+               : "memory");
+  return k;
+}
+
+// Place of g among a bucket's keys, or -1.
+__device__ __forceinline__ int way_of(uint4 k, unsigned g) {
+  return k.x == g ? 0 : (k.y == g ? 1 : (k.z == g ? 2 : (k.w == g ? 3 : -1)));
+}
+
+__device__ __forceinline__ void add_product(float* v, float a, float b) {
+  const float old = *v;
+  *v = __fadd_rn(__float_as_uint(old) == ABSENT ? 0.f : old, __fmul_rn(a, b));
+}
+
+// Dot2 step: the rounded product by TwoSum, both rounding errors into .y.
+__device__ __forceinline__ void add_product(float2* v, float a, float b) {
+  float2 old = *v;
+  if (__float_as_uint(old.x) == ABSENT) old = make_float2(0.f, 0.f);
+  const float p = __fmul_rn(a, b);
+  const float s = __fadd_rn(old.x, p);
+  *v = make_float2(s, __fadd_rn(old.y, __fadd_rn(two_sum_err(old.x, p, s), __fmaf_rn(a, b, -p))));
+}
+
+// Products of up to 32 segments (lane j: B positions [bstart, bstart + len)
+// scaled by a) into the table, 2^LG entries of one segment to each group of
+// 2^LG lanes, 32 >> LG segments a step. The columns of a segment are distinct
+// and the warp owns the table, so values are added with plain loads and
+// stores, one lane group after the other; only claiming a slot takes an
+// atomic. HASH_UNROLL steps go together, so their loads are in flight at
+// once; more of them, or loads a round ahead, cost the warps that hide the
+// latency better (27-point stencil 96^3: 2 steps and 40 warps an SM 2.77 ms,
+// 4 and 28 3.08, loads ahead 2.92 to 3.92). Adds the number of new slots to `slots`, and stops once it exceeds
+// `limit` (or a group finds every bucket full).
+constexpr int HASH_UNROLL = 2;
+
+template <int LG, int LOG2T, int MODE>
+__device__ __forceinline__ void hash_segments(const Operands& op, int bstart, int len, float a,
+                                              int lo, unsigned* keys, GroupVals<MODE>* vals,
+                                              int& slots, int limit) {
+  constexpr int SUB = 32 >> LG, W = 1 << LG;
+  constexpr unsigned MASK = (1u << LOG2T) - 1u;
+  const int lane = lane_id(), sub = lane >> LG, gl = lane & (W - 1);
+  // a segment no longer than a step is step number `lane`; else the steps of
+  // a segment are found from the inclusive sum of their counts
+  const bool simple = !__any_sync(FULL, len > W);
+  const int chunks = (len + W - 1) >> LG;
+  const int incl = simple ? lane + 1 : warp_incl_scan(chunks);
+  const int total = simple ? 32 - __clz(__ballot_sync(FULL, len > 0)) : __shfl_sync(FULL, incl, 31);
+  const int before = W * (simple ? lane : incl - chunks);  // W * steps of earlier segments
+  const int pos0 = bstart - before, end0 = len + before;
+  bool full = false;
+  for (int q0 = 0; q0 < total; q0 += SUB * HASH_UNROLL) {
+    unsigned x[HASH_UNROLL], slot[HASH_UNROLL];
+    float sa[HASH_UNROLL], bv[HASH_UNROLL];
+    bool act[HASH_UNROLL];
+#pragma unroll
+    for (int u = 0; u < HASH_UNROLL; ++u) {
+      const int q = q0 + u * SUB + sub;
+      int owner = q;
+      if (!simple) {
+#pragma unroll
+        for (int s = 0; s < SUB; ++s) {
+          const unsigned past = __ballot_sync(FULL, incl <= q0 + u * SUB + s);
+          if (s == sub) owner = __popc(past);
+        }
+      }
+      const int t = W * q + gl;
+      const int pos = __shfl_sync(FULL, pos0, owner & 31) + t;
+      const int end = __shfl_sync(FULL, end0, owner & 31);
+      sa[u] = __shfl_sync(FULL, a, owner & 31);
+      act[u] = q < total && t < end;
+      x[u] = 0u;
+      bv[u] = 0.f;
+      if (act[u]) {
+        x[u] = (unsigned)(__ldg(op.b_col + pos) - lo);
+        bv[u] = __ldg(op.b_val + pos);
+      }
+    }
+    uint4 k[HASH_UNROLL];
+#pragma unroll
+    for (int u = 0; u < HASH_UNROLL; ++u) {
+      slot[u] = hash_group(x[u] / GROUP_COLS, LOG2T);
+      k[u] = bucket_keys(keys + slot[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < HASH_UNROLL; ++u) {
+      const unsigned g = x[u] / GROUP_COLS;
+      int way = way_of(k[u], g);
+      bool miss = act[u] && way < 0;
+      int passed = 0;  // full buckets
+      while (__any_sync(FULL, miss)) {
+        bool claimed = false;
+        if (miss) {
+          const int empty = way_of(k[u], EMPTY_KEY);
+          if (empty >= 0) {
+            const unsigned old = atomicCAS(keys + slot[u] + empty, EMPTY_KEY, g);
+            claimed = old == EMPTY_KEY;
+            if (claimed || old == g) {
+              way = empty;
+              miss = false;
+            }
+          } else {
+            slot[u] = (slot[u] + 4u) & MASK;
+            full = ++passed > (1 << LOG2T) / 4;
+            miss = !full;
+          }
+        }
+        slots += __popc(__ballot_sync(FULL, claimed));
+        if (miss) {
+          k[u] = bucket_keys(keys + slot[u]);
+          way = way_of(k[u], g);
+          miss = way < 0;
+        }
+      }
+      act[u] = act[u] && way >= 0;
+      slot[u] += way & 3;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < HASH_UNROLL; ++u) {
+      auto* v = &vals[slot[u]].v[x[u] % GROUP_COLS];
+#pragma unroll
+      for (int s = 0; s < SUB; ++s) {
+        if (act[u] && s == sub) add_product(v, sa[u], bv[u]);
+        __syncwarp();
+      }
+    }
+    if (__any_sync(FULL, full)) slots = limit + 1;
+    if (slots > limit) break;
+  }
+}
+
+// BYTES of shared memory to all ones, by one warp.
+template <int BYTES>
+__device__ __forceinline__ void clear_shared(void* p, int lane) {
+#pragma unroll
+  for (int t = 0; t < BYTES / 16; t += 32)
+    if (t + lane < BYTES / 16)
+      reinterpret_cast<uint4*>(p)[t + lane] = make_uint4(ABSENT, ABSENT, ABSENT, ABSENT);
+  __syncwarp();
+}
+
+// Rows of the warp bins that the kernels above do not take, one warp per row,
+// `stretch` rows of the list in a row: accumulate in the table, then write the
+// present columns of the slots in the order of their groups. The order (packed
+// keys, group above slot index, sorted in registers) is renewed only when the
+// row claimed slots. A row that needs more than 4/5 of the slots is pushed to
+// the bin that redoes it (overflow_bin_of). Rows that reuse little of the
+// table switch the reuse off for the rest of the stretch. The table of bin b
+// has 2^hash_slots_log2(b) slots. Results are summed in product order, so
+// they are reproducible when A's entries come in a fixed order.
+//
+// Bound by instruction issue (59% of the slots, 2,350 warp instructions per
+// 27-point row of 690 products) and shared-memory wavefronts (60%); with
+// atomic adds, an owner search per product and a sort per row it took 5,800
+// (stencil 96^3: 5.10 ms, now 2.77; compensated 61^3: 1.53, now 0.94).
+constexpr int HASH_THREADS = 128;
+constexpr int HASH_ROWS = 16;  // most rows in a stretch
+
+template <int LOG2T, int MODE>
+constexpr size_t hash_warp_bytes() {
+  return ((size_t)1 << LOG2T) * (sizeof(GroupVals<MODE>) + 2 * sizeof(unsigned));
+}
+
+template <int LOG2T, int MODE>
+__global__ void __launch_bounds__(HASH_THREADS, 10)
+k_fused_warp(Operands op, const int* __restrict__ rows, int nrows, int stretch,
+             const int2* __restrict__ row_span, const long long* __restrict__ toff,
+             int* __restrict__ c_cnt, int* __restrict__ t_col, float* __restrict__ t_val,
+             int* fb_rows, int* fb_count, Tuning tn, const long long* __restrict__ row_p,
+             int* __restrict__ overflow_count) {
+  constexpr int T = 1 << LOG2T;
+  constexpr int LIMIT = T * 4 / 5;
+  constexpr int WPB = HASH_THREADS / 32;
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  GroupVals<MODE>* vals = reinterpret_cast<GroupVals<MODE>*>(smem) + warp * T;
+  unsigned* keys = reinterpret_cast<unsigned*>(smem + WPB * T * sizeof(GroupVals<MODE>)) + 2 * warp * T;
+  unsigned* order = keys + T;
+  static_assert(EMPTY_KEY == ABSENT, "one pattern clears keys and values");
+  int slots = 0, ordered = 0;
+  auto clear_keys = [&]() {
+    clear_shared<T * (int)sizeof(unsigned)>(keys, lane);
+    slots = ordered = 0;
+  };
+  auto clear_vals = [&]() { clear_shared<T * (int)sizeof(GroupVals<MODE>)>(vals, lane); };
+  clear_keys();
+  clear_vals();
+  for (int r0 = (blockIdx.x * WPB + warp) * stretch; r0 < nrows;
+       r0 += gridDim.x * WPB * stretch) {
+    bool reuse = true;
+    const int r1 = min(r0 + stretch, nrows);
+    for (int r = r0; r < r1; ++r) {
+      const int i = rows[r];
+      const int2 sp = row_span[i];
+      const int rs = op.a_rowptr[i], re = op.a_rowptr[i + 1];
+      if (!reuse && slots > 0) clear_keys();
+      int kept = slots;
+      for (;;) {
+        for (int base = rs; base < re && slots <= LIMIT; base += 32) {
+          const int j = base + lane;
+          int bstart = 0, len = 0;
+          float a = 0.f;
+          if (j < re) {
+            const int k = __ldg(op.a_col + j);
+            a = __ldg(op.a_val + j);
+            bstart = __ldg(op.b_rowptr + k);
+            len = __ldg(op.b_rowptr + k + 1) - bstart;
+          }
+          const int longest = __reduce_max_sync(FULL, len);
+          if (longest > 16)
+            hash_segments<5, LOG2T, MODE>(op, bstart, len, a, sp.x, keys, vals, slots, LIMIT);
+          else if (longest > 8)
+            hash_segments<4, LOG2T, MODE>(op, bstart, len, a, sp.x, keys, vals, slots, LIMIT);
+          else
+            hash_segments<3, LOG2T, MODE>(op, bstart, len, a, sp.x, keys, vals, slots, LIMIT);
+        }
+        if (slots <= LIMIT || kept == 0) break;
+        // the earlier rows' slots were in the way: once more with none
+        clear_keys();
+        clear_vals();
+        kept = 0;
+        reuse = false;
+      }
+      if (slots > LIMIT) {  // redo with a larger structure
+        if (lane == 0) {
+          const int q = overflow_bin_of(row_p[i], sp.x, sp.y + 1 - sp.x, tn);
+          fb_rows[(size_t)q * op.m + atomicAdd(fb_count + q, 1)] = i;
+          atomicAdd(overflow_count, 1);
+        }
+        clear_keys();
+        clear_vals();
+        continue;
+      }
+      if (slots != ordered) {
+        int o = 0;
+#pragma unroll
+        for (int g = 0; g < T; g += 32) {
+          const unsigned k = keys[g + lane];
+          const bool valid = k != EMPTY_KEY;
+          const unsigned bal = __ballot_sync(FULL, valid);
+          if (valid) order[o + __popc(bal & ((1u << lane) - 1u))] = (k << LOG2T) | (unsigned)(g + lane);
+          o += __popc(bal);
+        }
+        __syncwarp();
+        if (o <= 32) warp_sort_shared<1>(order, o, lane);
+        else if (o <= 64) warp_sort_shared<2>(order, o, lane);
+        else if (o <= 128) warp_sort_shared<4>(order, o, lane);
+        else if (o <= 256) warp_sort_shared<8>(order, o, lane);
+        else {
+          int n2 = 512;
+          while (n2 < o) n2 <<= 1;
+          for (int t = o + lane; t < n2; t += 32) order[t] = EMPTY_KEY;
+          __syncwarp();
+          bitonic_sort_keys_rt(order, n2, lane, 32, WarpSync());
+        }
+        ordered = o;
+        __syncwarp();
+      }
+      const long long base = toff[i];
+      int written = 0, reached = 0;
+      for (int t0 = 0; t0 < ordered; t0 += 32) {
+        unsigned present = 0u, group = 0u;
+        GroupVals<MODE> v;
+        if (t0 + lane < ordered) {
+          const unsigned key = order[t0 + lane];
+          group = key >> LOG2T;
+          GroupVals<MODE>* at = vals + (key & (T - 1));
+          v = *at;  // and clean for the next row
+#pragma unroll
+          for (int q = 0; q < (int)sizeof(GroupVals<MODE>) / 16; ++q)
+            reinterpret_cast<uint4*>(at)[q] = make_uint4(ABSENT, ABSENT, ABSENT, ABSENT);
+#pragma unroll
+          for (int c = 0; c < GROUP_COLS; ++c) {
+            const float f = *reinterpret_cast<const float*>(&v.v[c]);
+            present |= __float_as_uint(f) != ABSENT ? 1u << c : 0u;
+          }
+        }
+        const int n = __popc(present);
+        reached += __popc(__ballot_sync(FULL, n > 0));
+        const int incl = warp_incl_scan(n);
+        long long pos = base + written + incl - n;
+#pragma unroll
+        for (int c = 0; c < GROUP_COLS; ++c) {
+          if ((present >> c) & 1u) {
+            t_col[pos] = sp.x + (int)(group * GROUP_COLS) + c;
+            t_val[pos] = finalize_value(v.v[c]);
+            ++pos;
+          }
+        }
+        written += __shfl_sync(FULL, incl, 31);
+      }
+      if (lane == 0) c_cnt[i] = written;
+      if (kept > 0 && 2 * (slots - kept) > reached) reuse = false;
+      __syncwarp();
+    }
   }
 }
 

@@ -133,3 +133,36 @@ def test_unsorted_rows_are_refused(seed):
         with pytest.raises(sg.SpgemmError) as e:
             h.multiply_host(A, B)
         assert e.value.status == 1
+
+
+@pytest.mark.parametrize("precision", [sg.PLAIN, sg.COMPENSATED])
+@pytest.mark.parametrize("table", [64, 256, 1024])
+@pytest.mark.parametrize("stride", [1, 3, 700])
+def test_hashed_rows_reuse_and_overflow(precision, table, stride):
+    """Rows of a 27-point operator (their pattern stays in a warp's table from
+    row to row) with random rows among them, which switch the reuse off or
+    overflow; columns next to each other, or apart so that every slot holds
+    one column. Runs twice, with the same bits: A is in CSR."""
+    rng = np.random.default_rng(table + stride)
+    S = W.stencil27(33, seed=stride)
+    n, keep = S.rows, 9000
+    lens = np.diff(S.rowptr)[:keep].astype(np.int64)
+    r, c = np.repeat(np.arange(keep), lens), S.col[:lens.sum()].astype(np.int64)
+    odd = rng.choice(keep, 400, replace=False)
+    own = ~np.isin(r, odd)
+    extra = [np.sort(rng.choice(n, rng.integers(2, 60), replace=False)) for _ in odd]
+    r = np.concatenate([r[own], np.repeat(odd, [len(x) for x in extra])])
+    c = np.concatenate([c[own], *extra])
+    A = W.from_coo(keep, n, r, c, rng.uniform(-1, 1, len(r)).astype(np.float32))
+    B = W.Csr(n, n * stride, S.rowptr, (S.col.astype(np.int64) * stride).astype(np.int32), S.val)
+    ref = ref_product(A, B)
+    out = []
+    for _ in range(2):
+        with sg.Handle(precision) as h:
+            h.set_tuning(warp_table_max=table)
+            out.append(h.multiply_host(A, B))
+    assert_structure_equal(out[0].rowptr, out[0].col, ref["rowptr"], ref["col"])
+    tol = plain_tolerance(ref) if precision == sg.PLAIN else compensated_tolerance(ref)
+    assert_values_close(out[0].val, ref, tol)
+    assert np.array_equal(out[0].col, out[1].col)
+    assert np.array_equal(out[0].val.view(np.uint32), out[1].val.view(np.uint32))
