@@ -2,58 +2,191 @@
 // rows or CSC over columns), replacing the host qsort the reference's
 // protocol puts before cudaCOO2CM (src/coo.cpp:73-79, src/main.cu:27-30).
 //
-// Counting sort by the major index (histogram, scan, scatter), then a sort of
+// Counting sort by the major index -- the histogram's atomics return each
+// entry's place in its segment, so the scatter needs none -- then a sort of
 // each major index's segment by (minor index, input position): 64-bit keys
 // minor << 32 | position, unique, so the result is deterministic and entries
-// with equal indices keep their input order. Segments of up to 1024 entries
-// are sorted by one warp in shared memory, up to 8192 by one block, longer
-// ones by one block as sorted 8192-entry runs merged pairwise in global
-// memory (merge-path partitions). Values are gathered from the input by
-// position at the end.
+// with equal indices keep their input order. Segments of up to 32 entries are
+// sorted in registers by 8, 16 or 32 lanes; up to CS_RANGE in shared memory
+// by a warp or a block, by one bucket pass and a count within the bucket;
+// longer ones by several blocks, each a range of the buckets, or (segments
+// beyond CS_SPLIT_MAX or with most entries on few indices) by one block as
+// sorted 8192-entry runs merged pairwise in global memory (merge-path
+// partitions). Every sort writes the minor indices
+// and gathers the values from the input by position.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "engine.h"
+#include "kernels.cuh"
 
 namespace sg {
 namespace {
 
-constexpr int CS_WARP_MAX = 1024;   // entries a warp sorts in shared memory
-constexpr int CS_BLOCK_MAX = 8192;  // entries a block sorts in shared memory
+constexpr int CS_RUN = 8192;    // entries of one sorted run of the merge kernel
+constexpr int CS_RANGE = 6144;  // entries of a long segment that one block sorts
 constexpr int CS_THREADS = 1024;
 constexpr unsigned long long CS_PAD = ~0ull;
 
+// Segments by length, each with a list: at most 8, 16, 32, 256, 2048, 8192
+// entries, and longer.
+constexpr int CS_CLASSES = 7;
+constexpr int CS_LONG = 6;
+
 struct CsCounters {
   unsigned flags;  // bit 0: an index outside its dimension
-  int n_mid;       // segments of (CS_WARP_MAX, CS_BLOCK_MAX] entries
-  int n_big;       // segments of more than CS_BLOCK_MAX entries
+  int count[CS_CLASSES];
+  int n_merge;  // segments for the merge kernel
   long long total;
 };
 
-__global__ void k_cs_hist(const triplet* __restrict__ t, int nnz, int row_major, int n_major,
-                          int n_minor, int* __restrict__ cnt, CsCounters* cc) {
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += gridDim.x * blockDim.x) {
-    const triplet x = t[e];
-    const int major = row_major ? x.ridx : x.cidx;
-    const int minor = row_major ? x.cidx : x.ridx;
-    if ((unsigned)major >= (unsigned)n_major || (unsigned)minor >= (unsigned)n_minor) {
-      atomicOr(&cc->flags, 1u);
-      continue;
+__device__ __forceinline__ int cs_class(int len) {
+  if (len <= 32) return len <= 8 ? 0 : (len <= 16 ? 1 : 2);
+  if (len <= 2048) return len <= 256 ? 3 : 4;
+  return len <= 8192 ? 5 : CS_LONG;
+}
+
+// Entry `pos` of a class's list: a segment is on one list, so two classes
+// share an array of n from both ends.
+constexpr int CS_LISTS = 4;
+__device__ __forceinline__ size_t cs_at(int c, int pos, int n) {
+  const size_t base = (size_t)(c / 2) * n;
+  return c & 1 ? base + pos : base + n - 1 - pos;
+}
+
+__device__ __forceinline__ bool cs_entry(const triplet& x, int row_major, int n_major, int n_minor,
+                                         int& major, int& minor) {
+  major = row_major ? x.ridx : x.cidx;
+  minor = row_major ? x.cidx : x.ridx;
+  return (unsigned)major < (unsigned)n_major && (unsigned)minor < (unsigned)n_minor;
+}
+
+// Entries per major index, and each entry's place in its segment. A block
+// gathers its entries (`items` a thread) by major index in a shared-memory
+// table first and then adds one count per major index to global memory: the
+// entries of one hub of a power-law graph would otherwise queue for one
+// address (R-MAT 2^18, 4.2 M entries, longest segment 28K: 150 us).
+constexpr int CS_HIST_ITEMS = 8;
+constexpr int CS_HIST_SLOTS = 2 * CS_THREADS * CS_HIST_ITEMS;  // at most half full
+
+__global__ void __launch_bounds__(CS_THREADS)
+k_cs_hist(const triplet* __restrict__ t, int nnz, int items, int row_major, int n_major,
+          int n_minor, int* __restrict__ cnt, int* __restrict__ rank, CsCounters* cc) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  unsigned* key = reinterpret_cast<unsigned*>(smem);
+  int* count = reinterpret_cast<int*>(key + CS_HIST_SLOTS);
+  for (int q = threadIdx.x; q < CS_HIST_SLOTS; q += CS_THREADS) {
+    key[q] = EMPTY_KEY;
+    count[q] = 0;
+  }
+  __syncthreads();
+  const long long e0 = (long long)blockIdx.x * CS_THREADS * items + threadIdx.x;
+  int slot[CS_HIST_ITEMS], place[CS_HIST_ITEMS];
+#pragma unroll
+  for (int u = 0; u < CS_HIST_ITEMS; ++u) {
+    slot[u] = -1;
+    const long long e = e0 + (long long)u * CS_THREADS;
+    if (u < items && e < nnz) {
+      int major, minor;
+      if (cs_entry(t[e], row_major, n_major, n_minor, major, minor)) {
+        unsigned h = ((unsigned)major * 0x9e3779b1u) >> 18;  // 14 bits
+        for (;;) {
+          const unsigned old = atomicCAS(key + h, EMPTY_KEY, (unsigned)major);
+          if (old == EMPTY_KEY || old == (unsigned)major) break;
+          h = (h + 1) & (CS_HIST_SLOTS - 1);
+        }
+        slot[u] = (int)h;
+        place[u] = atomicAdd(count + h, 1);
+      } else {
+        atomicOr(&cc->flags, 1u);
+      }
     }
-    atomicAdd(cnt + major, 1);
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < CS_HIST_SLOTS; q += CS_THREADS)
+    if (key[q] != EMPTY_KEY) count[q] = atomicAdd(cnt + key[q], count[q]);
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < CS_HIST_ITEMS; ++u)
+    if (slot[u] >= 0) rank[e0 + (long long)u * CS_THREADS] = count[slot[u]] + place[u];
+}
+static_assert(CS_HIST_SLOTS == 1 << 14, "the hash keeps 14 bits");
+
+__global__ void k_cs_scatter(const triplet* __restrict__ t, int nnz, int row_major, int n_major,
+                             int n_minor, const int* __restrict__ ptr, const int* __restrict__ rank,
+                             unsigned long long* __restrict__ keys) {
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += gridDim.x * blockDim.x) {
+    int major, minor;
+    if (!cs_entry(t[e], row_major, n_major, n_minor, major, minor)) continue;
+    keys[__ldg(ptr + major) + rank[e]] = ((unsigned long long)(unsigned)minor << 32) | (unsigned)e;
   }
 }
 
-__global__ void k_cs_scatter(const triplet* __restrict__ t, int nnz, int row_major, int n_major,
-                             int n_minor, int* __restrict__ cursor,
-                             unsigned long long* __restrict__ keys) {
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += gridDim.x * blockDim.x) {
-    const triplet x = t[e];
-    const int major = row_major ? x.ridx : x.cidx;
-    const int minor = row_major ? x.cidx : x.ridx;
-    if ((unsigned)major >= (unsigned)n_major || (unsigned)minor >= (unsigned)n_minor) continue;
-    const int pos = atomicAdd(cursor + major, 1);
-    keys[pos] = ((unsigned long long)(unsigned)minor << 32) | (unsigned)e;
+__global__ void __launch_bounds__(256)
+k_cs_bins(const int* __restrict__ cnt, int n_major, int* __restrict__ lists, CsCounters* cc) {
+  __shared__ int hist[CS_CLASSES], base[CS_CLASSES];
+  if (threadIdx.x < CS_CLASSES) hist[threadIdx.x] = 0;
+  __syncthreads();
+  const int s = blockIdx.x * 256 + threadIdx.x;
+  const int len = s < n_major ? cnt[s] : 0;
+  const int c = cs_class(len);
+  const int rank = len > 0 ? atomicAdd(&hist[c], 1) : 0;
+  __syncthreads();
+  if (threadIdx.x < CS_CLASSES && hist[threadIdx.x])
+    base[threadIdx.x] = atomicAdd(&cc->count[threadIdx.x], hist[threadIdx.x]);
+  __syncthreads();
+  if (len > 0) lists[cs_at(c, base[c] + rank, n_major)] = s;
+}
+
+// Output entry p: the minor index of its key, the value of its input entry.
+struct CsOut {
+  const triplet* t;
+  int* idx;
+  float* val;
+  __device__ __forceinline__ void put(int p, unsigned long long k) const {
+    idx[p] = (int)(k >> 32);
+    val[p] = __ldg(&t[(unsigned)k].val);
   }
+};
+
+// Segments of at most G entries, G lanes each: bitonic in registers.
+template <int G>
+__device__ __forceinline__ void cs_tiny(const int* __restrict__ ptr, const int* __restrict__ lists,
+                                        int c, int n_major, int count,
+                                        const unsigned long long* __restrict__ keys,
+                                        const CsOut& out) {
+  const int lane = threadIdx.x & 31, gl = lane & (G - 1);
+  const int group = (blockIdx.x * blockDim.x + threadIdx.x) / G, groups = gridDim.x * blockDim.x / G;
+  const int rounds = (count + groups - 1) / groups;
+  for (int q = 0; q < rounds; ++q) {
+    const int r = q * groups + group;
+    int b = 0, len = 0;
+    if (r < count) {
+      const int s = lists[cs_at(c, r, n_major)];
+      b = ptr[s];
+      len = ptr[s + 1] - b;
+    }
+    unsigned long long k = gl < len ? keys[b + gl] : CS_PAD;
+#pragma unroll
+    for (int size = 2; size <= G; size <<= 1) {
+#pragma unroll
+      for (int j = size >> 1; j > 0; j >>= 1) {
+        const unsigned long long o = __shfl_xor_sync(FULL, k, j);
+        const bool up = (gl & size) == 0, low = (lane & j) == 0;
+        k = ((k < o) == (low == up)) ? k : o;
+      }
+    }
+    if (gl < len) out.put(b + gl, k);
+  }
+}
+
+__global__ void __launch_bounds__(256)
+k_cs_sort_tiny(const int* __restrict__ ptr, const int* __restrict__ lists, int n_major,
+               const CsCounters* cc, const unsigned long long* __restrict__ keys, CsOut out) {
+  cs_tiny<32>(ptr, lists, 2, n_major, cc->count[2], keys, out);
+  cs_tiny<16>(ptr, lists, 1, n_major, cc->count[1], keys, out);
+  cs_tiny<8>(ptr, lists, 0, n_major, cc->count[0], keys, out);
 }
 
 // In-place bitonic sort of n (a power of two) keys by `nthreads` threads.
@@ -84,52 +217,83 @@ struct CsBlockSync {
   __device__ void operator()() const { __syncthreads(); }
 };
 
-// One warp per segment of 2..CS_WARP_MAX entries; longer segments are listed
-// for the block kernels.
-constexpr int CS_WARPS = 4;  // warps per block of the warp kernel (32 KB of keys)
-
-__global__ void __launch_bounds__(CS_WARPS * 32)
-k_cs_sort_warp(const int* __restrict__ ptr, int n_major, unsigned long long* __restrict__ keys,
-               int* __restrict__ mid, int* __restrict__ big, CsCounters* cc) {
-  __shared__ unsigned long long buf[CS_WARPS][CS_WARP_MAX];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  unsigned long long* k = buf[warp];
-  for (int s = blockIdx.x * CS_WARPS + warp; s < n_major; s += gridDim.x * CS_WARPS) {
-    const int b = ptr[s], len = ptr[s + 1] - b;
-    if (len <= 1) continue;
-    if (len > CS_WARP_MAX) {
-      if (lane == 0) {
-        if (len > CS_BLOCK_MAX) big[atomicAdd(&cc->n_big, 1)] = s;
-        else mid[atomicAdd(&cc->n_mid, 1)] = s;
-      }
-      continue;
-    }
-    int n2 = 2;
-    while (n2 < len) n2 <<= 1;
-    for (int t = lane; t < n2; t += 32) k[t] = t < len ? keys[b + t] : CS_PAD;
-    __syncwarp();
-    bitonic64(k, n2, lane, 32, CsWarpSync());
-    for (int t = lane; t < len; t += 32) keys[b + t] = k[t];
-    __syncwarp();
-  }
+// Segments of class `c` (at most CAP entries), one team of NT threads each:
+// keys to buckets by the top bits of the minor index within the segment's
+// range, about one bucket per entry, then each key counts the smaller keys of
+// its bucket. A segment with a crowded bucket is sorted bitonically.
+template <int NT, int CAP, int NB>
+__host__ __device__ constexpr size_t cs_team_bytes() {
+  return CAP * sizeof(unsigned long long) + NB * sizeof(int);
 }
 
-// One block per segment of (CS_WARP_MAX, CS_BLOCK_MAX] entries.
-__global__ void __launch_bounds__(CS_THREADS)
-k_cs_sort_block(const int* __restrict__ ptr, const int* __restrict__ list, const CsCounters* cc,
-                unsigned long long* __restrict__ keys) {
-  extern __shared__ unsigned long long sk[];
-  const int count = cc->n_mid;
-  for (int q = blockIdx.x; q < count; q += gridDim.x) {
-    const int s = list[q];
+template <int NT, int CAP, int NB>
+__global__ void __launch_bounds__(NT == 32 ? 128 : NT)
+k_cs_sort(const int* __restrict__ ptr, const int* __restrict__ lists, int c, int n_major,
+          const CsCounters* cc, const unsigned long long* __restrict__ keys, CsOut out) {
+  constexpr int TEAMS = NT == 32 ? 4 : 1;
+  static_assert((CAP & (CAP - 1)) == 0, "the bitonic sort pads to a power of two");
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ int warp_a[32], warp_b[32];
+  const int lane = threadIdx.x & 31, team = TEAMS > 1 ? threadIdx.x >> 5 : 0;
+  const int warp = TEAMS > 1 ? 0 : threadIdx.x >> 5;
+  const int tid = TEAMS > 1 ? lane : threadIdx.x;
+  unsigned long long* k = reinterpret_cast<unsigned long long*>(smem + team * cs_team_bytes<NT, CAP, NB>());
+  int* cnt = reinterpret_cast<int*>(k + CAP);
+  const int count = cc->count[c];
+  for (int q = blockIdx.x * TEAMS + team; q < count; q += gridDim.x * TEAMS) {
+    const int s = lists[cs_at(c, q, n_major)];
     const int b = ptr[s], len = ptr[s + 1] - b;
-    int n2 = 2;
-    while (n2 < len) n2 <<= 1;
-    for (int t = threadIdx.x; t < n2; t += CS_THREADS) sk[t] = t < len ? keys[b + t] : CS_PAD;
-    __syncthreads();
-    bitonic64(sk, n2, threadIdx.x, CS_THREADS, CsBlockSync());
-    for (int t = threadIdx.x; t < len; t += CS_THREADS) keys[b + t] = sk[t];
-    __syncthreads();
+    // range of the minor index
+    unsigned lo = FULL, hi = 0u;
+    for (int t = tid; t < len; t += NT) {
+      const unsigned m = (unsigned)(keys[b + t] >> 32);
+      lo = min(lo, m);
+      hi = max(hi, m);
+    }
+    lo = __reduce_min_sync(FULL, lo);
+    hi = __reduce_max_sync(FULL, hi);
+    if (NT > 32) {
+      if (lane == 0) {
+        warp_a[warp] = (int)lo;
+        warp_b[warp] = (int)hi;
+      }
+      __syncthreads();
+      lo = __reduce_min_sync(FULL, lane < NT / 32 ? (unsigned)warp_a[lane] : FULL);
+      hi = __reduce_max_sync(FULL, lane < NT / 32 ? (unsigned)warp_b[lane] : 0u);
+    }
+    const int bits = hi > lo ? 32 - __clz(hi - lo) : 1;
+    const int nbits = min(max(len > 1 ? 32 - __clz(len - 1) : 0, 31 - __clz(NT)), 31 - __clz(NB));
+    const int shift = max(bits - nbits, 0);
+    for (int t = tid; t < (1 << nbits); t += NT) cnt[t] = 0;
+    team_sync<NT>();
+    auto bucket = [&](unsigned long long key) { return (int)(((unsigned)(key >> 32) - lo) >> shift); };
+    for (int t = tid; t < len; t += NT) atomicAdd(cnt + bucket(keys[b + t]), 1);
+    team_sync<NT>();
+    const int mx = bucket_scan<NT>(cnt, 1 << nbits, warp_a, warp_b);
+    if (mx <= 64 + (len >> 3)) {  // as esc_bucket_max
+      for (int t = tid; t < len; t += NT) {
+        const unsigned long long key = keys[b + t];
+        k[atomicAdd(cnt + bucket(key), 1)] = key;
+      }
+      team_sync<NT>();  // bucket j now ends at cnt[j]
+      for (int t = tid; t < len; t += NT) {
+        const unsigned long long key = k[t];
+        const int j = bucket(key), s0 = j ? cnt[j - 1] : 0, s1 = cnt[j];
+        int place = s0;
+        if (s1 - s0 > 1)
+          for (int u = s0; u < s1; ++u) place += k[u] < key;
+        out.put(b + place, key);
+      }
+    } else {
+      int n2 = 2;
+      while (n2 < len) n2 <<= 1;
+      for (int t = tid; t < n2; t += NT) k[t] = t < len ? keys[b + t] : CS_PAD;
+      team_sync<NT>();
+      if (NT == 32) bitonic64(k, n2, tid, NT, CsWarpSync());
+      else bitonic64(k, n2, tid, NT, CsBlockSync());
+      for (int t = tid; t < len; t += NT) out.put(b + t, k[t]);
+    }
+    team_sync<NT>();
   }
 }
 
@@ -146,29 +310,136 @@ __device__ __forceinline__ int merge_split(const unsigned long long* a, int na,
   return lo;
 }
 
-// One block per segment of more than CS_BLOCK_MAX entries: sorted runs of
-// CS_BLOCK_MAX in shared memory, then pairwise merges between the segment
-// and its scratch copy; the result ends in `keys`.
+// Segments of up to CS_SPLIT_MAX entries: each of several blocks
+// (blockIdx.y) counts the whole segment's buckets, cuts them into ranges of
+// at most CS_RANGE entries -- the same cut in every block -- and sorts one
+// range as k_cs_sort does. Segments that do not cut so (a bucket of more than
+// CS_CROWD entries) go to the merge kernel, as do longer ones.
+constexpr int CS_SPLIT_MAX = 1 << 20;
+constexpr int CS_CROWD = 3072;
+
 __global__ void __launch_bounds__(CS_THREADS)
-k_cs_sort_big(const int* __restrict__ ptr, const int* __restrict__ list, const CsCounters* cc,
-              unsigned long long* __restrict__ keys, unsigned long long* __restrict__ tmp) {
-  extern __shared__ unsigned long long sk[];
-  const int count = cc->n_big;
+k_cs_sort_split(const int* __restrict__ ptr, const int* __restrict__ lists, int n_major,
+                const CsCounters* cc, int* __restrict__ merge, int* __restrict__ n_merge,
+                const unsigned long long* __restrict__ keys, CsOut out) {
+  constexpr int NB = 4096;
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ int warp_a[32], warp_b[32];
+  __shared__ int cut[2];  // first and last bucket + 1 of this block's range
+  unsigned long long* k = reinterpret_cast<unsigned long long*>(smem);
+  int* cnt = reinterpret_cast<int*>(k + CS_RANGE);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int count = cc->count[CS_LONG];
   for (int q = blockIdx.x; q < count; q += gridDim.x) {
-    const int s = list[q];
+    const int s = lists[cs_at(CS_LONG, q, n_major)];
+    const int b = ptr[s], len = ptr[s + 1] - b;
+    bool fits = len <= CS_SPLIT_MAX;
+    if (fits) {
+      // two neighbouring ranges exceed CS_RANGE, so there are at most this many
+      if ((int)blockIdx.y > 2 * (len / CS_RANGE) + 1) continue;
+      unsigned lo = FULL, hi = 0u;
+      // f(key) for this thread's keys of the segment, four loads in flight
+      auto each_key = [&](auto f) {
+        for (int t = threadIdx.x; t < len; t += 4 * CS_THREADS) {
+          unsigned long long x[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (t + u * CS_THREADS < len) x[u] = keys[b + t + u * CS_THREADS];
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (t + u * CS_THREADS < len) f(x[u]);
+        }
+      };
+      each_key([&](unsigned long long key) {
+        lo = min(lo, (unsigned)(key >> 32));
+        hi = max(hi, (unsigned)(key >> 32));
+      });
+      lo = __reduce_min_sync(FULL, lo);
+      hi = __reduce_max_sync(FULL, hi);
+      if (lane == 0) {
+        warp_a[warp] = (int)lo;
+        warp_b[warp] = (int)hi;
+      }
+      for (int t = threadIdx.x; t < NB; t += CS_THREADS) cnt[t] = 0;
+      __syncthreads();
+      lo = __reduce_min_sync(FULL, (unsigned)warp_a[lane]);
+      hi = __reduce_max_sync(FULL, (unsigned)warp_b[lane]);
+      const int shift = max((hi > lo ? 32 - __clz(hi - lo) : 1) - 12, 0);
+      auto bucket = [&](unsigned long long key) { return (int)(((unsigned)(key >> 32) - lo) >> shift); };
+      each_key([&](unsigned long long key) { atomicAdd(cnt + bucket(key), 1); });
+      __syncthreads();
+      const int mx = bucket_scan<CS_THREADS>(cnt, NB, warp_a, warp_b);
+      fits = mx <= CS_CROWD;
+      if (fits) {
+        if (threadIdx.x == 0) {  // ranges end before the bucket that would overfill them
+          int first = 0;
+          for (int r = 0;; ++r) {
+            int l = first + 1, h = NB;  // most buckets whose entries fit: cnt[l] - cnt[first]
+            while (l < h) {
+              const int mid = (l + h + 1) >> 1;
+              if ((mid < NB ? cnt[mid] : len) - cnt[first] <= CS_RANGE) l = mid;
+              else h = mid - 1;
+            }
+            cut[0] = first;
+            cut[1] = l;
+            if (r == (int)blockIdx.y) break;
+            first = l;
+            if (first >= NB) {
+              cut[0] = cut[1] = NB;
+              break;
+            }
+          }
+        }
+        __syncthreads();
+        const int b0 = cut[0], b1 = cut[1];
+        if (b0 < NB) {
+          const int base = cnt[b0];
+          __syncthreads();
+          each_key([&](unsigned long long key) {
+            const int j = bucket(key);
+            if (j >= b0 && j < b1) k[atomicAdd(cnt + j, 1) - base] = key;
+          });
+          __syncthreads();  // bucket j of the range now ends at cnt[j]
+          const int end = cnt[b1 - 1] - base;
+          for (int t = threadIdx.x; t < end; t += CS_THREADS) {
+            const unsigned long long key = k[t];
+            const int j = bucket(key);
+            const int s0 = j > b0 ? cnt[j - 1] - base : 0, s1 = cnt[j] - base;
+            int place = s0;
+            for (int u = s0; u < s1; ++u) place += k[u] < key;
+            out.put(b + base + place, key);
+          }
+        }
+      }
+    }
+    if (!fits && blockIdx.y == 0 && threadIdx.x == 0) merge[atomicAdd(n_merge, 1)] = s;
+    __syncthreads();
+  }
+}
+
+// One block per segment of the merge list: sorted runs of CS_RUN entries in
+// shared memory, then pairwise merges between the segment and its scratch
+// copy.
+__global__ void __launch_bounds__(CS_THREADS)
+k_cs_sort_merge(const int* __restrict__ ptr, const int* __restrict__ merge,
+                const int* __restrict__ n_merge, unsigned long long* __restrict__ keys,
+                unsigned long long* __restrict__ tmp, CsOut out) {
+  extern __shared__ unsigned long long sk[];
+  const int count = *n_merge;
+  for (int q = blockIdx.x; q < count; q += gridDim.x) {
+    const int s = merge[q];
     const int b = ptr[s], len = ptr[s + 1] - b;
     unsigned long long* src = keys + b;
     unsigned long long* dst = tmp + b;
-    for (int r0 = 0; r0 < len; r0 += CS_BLOCK_MAX) {
-      const int rl = min(CS_BLOCK_MAX, len - r0);
-      for (int t = threadIdx.x; t < CS_BLOCK_MAX; t += CS_THREADS)
-        sk[t] = t < rl ? src[r0 + t] : CS_PAD;
+    for (int r0 = 0; r0 < len; r0 += CS_RUN) {
+      const int rl = min(CS_RUN, len - r0);
+      for (int t = threadIdx.x; t < CS_RUN; t += CS_THREADS) sk[t] = t < rl ? src[r0 + t] : CS_PAD;
       __syncthreads();
-      bitonic64(sk, CS_BLOCK_MAX, threadIdx.x, CS_THREADS, CsBlockSync());
+      bitonic64(sk, CS_RUN, threadIdx.x, CS_THREADS, CsBlockSync());
       for (int t = threadIdx.x; t < rl; t += CS_THREADS) src[r0 + t] = sk[t];
       __syncthreads();
     }
-    for (long long w = CS_BLOCK_MAX; w < len; w <<= 1) {
+    for (long long w = CS_RUN; w < len; w <<= 1) {
       for (long long p0 = 0; p0 < len; p0 += 2 * w) {
         const int na = (int)min(w, (long long)len - p0);
         const int nb = (int)max(0ll, min(w, (long long)len - p0 - w));
@@ -189,24 +460,8 @@ k_cs_sort_big(const int* __restrict__ ptr, const int* __restrict__ list, const C
       src = dst;
       dst = x;
     }
-    if (src != keys + b)
-      for (int t = threadIdx.x; t < len; t += CS_THREADS) keys[b + t] = src[t];
+    for (int t = threadIdx.x; t < len; t += CS_THREADS) out.put(b + t, src[t]);
     __syncthreads();
-  }
-}
-
-// Entries placed by the scatter (cc->total: indices out of range are left
-// out) to the output: minor index from the key, value from the input entry.
-__global__ void k_cs_write(const unsigned long long* __restrict__ keys, const CsCounters* cc,
-                           int nnz, const triplet* __restrict__ t, int* __restrict__ idx,
-                           float* __restrict__ val) {
-  const long long placed = cc->total;
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < placed;
-       p += (long long)gridDim.x * blockDim.x) {
-    const unsigned long long k = keys[p];
-    const unsigned e = (unsigned)(k & 0xffffffffu);
-    idx[p] = (int)(k >> 32);
-    val[p] = e < (unsigned)nnz ? t[e].val : 0.f;
   }
 }
 
@@ -215,54 +470,85 @@ int grid_for(long long work, int per_block, int cap) {
   return (int)(g < 1 ? 1 : (g > cap ? cap : g));
 }
 
+// k_cs_sort for one class; a segment of the class has more than `over`
+// entries, so there are none unless nnz exceeds it.
+template <int NT, int CAP, int NB>
+cudaError_t sort_class(int c, int over, int nnz, int grid, const int* ptr, const int* lists,
+                       int n_major, const CsCounters* cc, const unsigned long long* keys, const CsOut& out,
+                       cudaStream_t s) {
+  if (nnz <= over) return cudaSuccess;
+  constexpr int TEAMS = NT == 32 ? 4 : 1;
+  const size_t smem = TEAMS * cs_team_bytes<NT, CAP, NB>();
+  cudaError_t e = cudaFuncSetAttribute(k_cs_sort<NT, CAP, NB>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  k_cs_sort<NT, CAP, NB><<<grid, NT * TEAMS, smem, s>>>(ptr, lists, c, n_major, cc, keys, out);
+  return cudaGetLastError();
+}
+
 }  // namespace
 
 cudaError_t coo_compress(const triplet* t, int nnz, bool row_major, int n_major, int n_minor,
                          int* ptr, int* idx, float* val, DevBuf& scratch, DevBuf& scan_tmp,
                          unsigned* flags_host, cudaStream_t s) {
+  auto padded = [](size_t b) { return (b + 255) & ~size_t(255); };
   const size_t cnt_bytes = sizeof(int) * ((size_t)n_major + 1);
   const size_t key_bytes = sizeof(unsigned long long) * (size_t)(nnz > 0 ? nnz : 1);
-  const size_t list_bytes = sizeof(int) * ((size_t)n_major + 1);
-  size_t off_cc = 0, off_cnt = 256, off_keys = off_cnt + ((cnt_bytes + 255) & ~size_t(255));
-  size_t off_tmp = off_keys + ((key_bytes + 255) & ~size_t(255));
-  size_t off_mid = off_tmp + ((key_bytes + 255) & ~size_t(255));
-  size_t off_big = off_mid + ((list_bytes + 255) & ~size_t(255));
-  const size_t total = off_big + ((list_bytes + 255) & ~size_t(255));
+  const size_t off_cnt = padded(sizeof(CsCounters));
+  const size_t off_keys = off_cnt + padded(cnt_bytes);
+  const size_t off_tmp = off_keys + padded(key_bytes);
+  const size_t off_lists = off_tmp + padded(key_bytes);
+  const size_t total = off_lists + CS_LISTS * sizeof(int) * (size_t)n_major + 256;
   cudaError_t e = scratch.ensure(total);
   if (e != cudaSuccess) return e;
   unsigned char* base = scratch.as<unsigned char>();
-  CsCounters* cc = reinterpret_cast<CsCounters*>(base + off_cc);
+  CsCounters* cc = reinterpret_cast<CsCounters*>(base);
   int* cnt = reinterpret_cast<int*>(base + off_cnt);
   unsigned long long* keys = reinterpret_cast<unsigned long long*>(base + off_keys);
   unsigned long long* tmp = reinterpret_cast<unsigned long long*>(base + off_tmp);
-  int* mid = reinterpret_cast<int*>(base + off_mid);
-  int* big = reinterpret_cast<int*>(base + off_big);
+  int* rank = reinterpret_cast<int*>(tmp);  // until the scatter; the merges use tmp after it
+  int* lists = reinterpret_cast<int*>(base + off_lists);
 
-  if ((e = cudaMemsetAsync(cc, 0, sizeof(CsCounters), s)) != cudaSuccess) return e;
-  if ((e = cudaMemsetAsync(cnt, 0, cnt_bytes, s)) != cudaSuccess) return e;
-  if (nnz > 0) k_cs_hist<<<grid_for(nnz, 256, 4096), 256, 0, s>>>(t, nnz, row_major ? 1 : 0,
-                                                                   n_major, n_minor, cnt, cc);
+  if ((e = cudaMemsetAsync(base, 0, off_cnt + cnt_bytes, s)) != cudaSuccess) return e;
+  if (nnz > 0) {
+    const int items = grid_for(nnz / (148 * CS_THREADS), 1, CS_HIST_ITEMS);
+    const size_t smem = CS_HIST_SLOTS * (sizeof(unsigned) + sizeof(int));
+    if ((e = cudaFuncSetAttribute(k_cs_hist, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)smem)) != cudaSuccess)
+      return e;
+    k_cs_hist<<<(nnz - 1) / (CS_THREADS * items) + 1, CS_THREADS, smem, s>>>(
+        t, nnz, items, row_major ? 1 : 0, n_major, n_minor, cnt, rank, cc);
+  }
   if ((e = scan_counts_to_ptr32(cnt, n_major, ptr, scan_tmp, &cc->total, s)) != cudaSuccess)
     return e;
-  if (nnz > 0) {
-    // the counts are free again: reuse them as the scatter cursors
-    if ((e = cudaMemcpyAsync(cnt, ptr, sizeof(int) * (size_t)n_major, cudaMemcpyDeviceToDevice, s)) !=
-        cudaSuccess)
-      return e;
+  if (nnz > 0 && n_major > 0) {
     k_cs_scatter<<<grid_for(nnz, 256, 4096), 256, 0, s>>>(t, nnz, row_major ? 1 : 0, n_major,
-                                                          n_minor, cnt, keys);
-    k_cs_sort_warp<<<grid_for(n_major, CS_WARPS, 8192), CS_WARPS * 32, 0, s>>>(ptr, n_major, keys,
-                                                                              mid, big, cc);
-    const size_t smem = sizeof(unsigned long long) * CS_BLOCK_MAX;
-    if ((e = cudaFuncSetAttribute(k_cs_sort_block, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem)) != cudaSuccess)
+                                                          n_minor, ptr, rank, keys);
+    k_cs_bins<<<(n_major - 1) / 256 + 1, 256, 0, s>>>(cnt, n_major, lists, cc);
+    const CsOut out{t, idx, val};
+    if ((e = sort_class<1024, 8192, 4096>(5, 2048, nnz, 296, ptr, lists, n_major, cc, keys, out, s)) != cudaSuccess)
       return e;
-    if ((e = cudaFuncSetAttribute(k_cs_sort_big, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem)) != cudaSuccess)
+    if ((e = sort_class<256, 2048, 2048>(4, 256, nnz, 1184, ptr, lists, n_major, cc, keys, out, s)) != cudaSuccess)
       return e;
-    k_cs_sort_block<<<296, CS_THREADS, smem, s>>>(ptr, mid, cc, keys);
-    k_cs_sort_big<<<148, CS_THREADS, smem, s>>>(ptr, big, cc, keys, tmp);
-    k_cs_write<<<grid_for(nnz, 256, 8192), 256, 0, s>>>(keys, cc, nnz, t, idx, val);
+    if ((e = sort_class<32, 256, 256>(3, 32, nnz, 2368, ptr, lists, n_major, cc, keys, out, s)) != cudaSuccess)
+      return e;
+    k_cs_sort_tiny<<<grid_for(n_major, 8, 2368), 256, 0, s>>>(ptr, lists, n_major, cc, keys, out);
+    if (nnz > 8192) {
+      const size_t split = cs_team_bytes<CS_THREADS, CS_RANGE, 4096>();
+      const size_t smem = sizeof(unsigned long long) * CS_RUN;
+      int* merge = cnt;  // the counts are not needed any more
+      if ((e = cudaFuncSetAttribute(k_cs_sort_split, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)split)) != cudaSuccess)
+        return e;
+      if ((e = cudaFuncSetAttribute(k_cs_sort_merge, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)smem)) != cudaSuccess)
+        return e;
+      const int ranges = 2 * (std::min(nnz, CS_SPLIT_MAX) / CS_RANGE) + 2;
+      k_cs_sort_split<<<dim3(grid_for(nnz, 8192, 64), ranges), CS_THREADS, split, s>>>(
+          ptr, lists, n_major, cc, merge, &cc->n_merge, keys, out);
+      k_cs_sort_merge<<<grid_for(nnz, 8192, 148), CS_THREADS, smem, s>>>(ptr, merge, &cc->n_merge,
+                                                                        keys, tmp, out);
+    }
   }
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if (flags_host) {

@@ -33,13 +33,6 @@ __device__ __forceinline__ float2 esc_value<1>(float a, float b) {
   return make_float2(p, __fmaf_rn(a, b, -p));  // TwoProduct: a*b == p + e exactly
 }
 
-// Threads that share a row: one warp (several teams to a block) or the block.
-template <int NT>
-__device__ __forceinline__ void team_sync() {
-  if (NT == 32) __syncwarp();
-  else __syncthreads();
-}
-
 // Sort key of a product: (column - lo) << SH | position, SH = log2 of the
 // row capacity, so equal columns keep their product order and the key names
 // its value, which never moves.
@@ -119,46 +112,6 @@ __device__ __forceinline__ void esc_gather(const Operands& op, int rs, int re, i
       }
     }
   }
-}
-
-// cnt[0, nb) to its exclusive prefix sums (nb a power of two, >= NT); returns
-// the largest count (to every thread). Ends with a barrier.
-template <int NT>
-__device__ __forceinline__ int esc_scan(int* __restrict__ cnt, int nb, int* warp_sums,
-                                        int* warp_max) {
-  constexpr int NW = NT / 32;
-  const int lane = threadIdx.x & 31, warp = NT == 32 ? 0 : threadIdx.x >> 5;
-  const int tid = NT == 32 ? lane : threadIdx.x;
-  const int per = nb / NT;
-  int* mine = cnt + tid * per;
-  int sum = 0, mx = 0;
-  for (int q = 0; q < per; ++q) {
-    const int c = mine[q];
-    sum += c;
-    mx = max(mx, c);
-  }
-  const int incl = warp_incl_scan(sum);
-  mx = __reduce_max_sync(FULL, mx);
-  int run = incl - sum;
-  if (NW > 1) {
-    if (lane == 31) {
-      warp_sums[warp] = incl;
-      warp_max[warp] = mx;
-    }
-    __syncthreads();
-    const int s = lane < NW ? warp_sums[lane] : 0;
-    const int m = lane < NW ? warp_max[lane] : 0;
-    const int wi = warp_incl_scan(s);
-    run += __shfl_sync(FULL, wi - s, warp);
-    mx = __reduce_max_sync(FULL, m);
-  }
-  for (int q = 0; q < per; ++q) {
-    const int c = mine[q];
-    mine[q] = run;
-    run += c;
-  }
-  team_sync<NT>();
-  return mx;
 }
 
 template <int SH, class KEY>
@@ -297,7 +250,7 @@ k_fused_esc(Operands op, const int* __restrict__ rows, const int* __restrict__ n
     team_sync<NT>();
     esc_gather<NT, SH, MODE, KEY>(op, rs, re, p, lo, width, shift, k0, vals, cnt);
     team_sync<NT>();
-    const int mx = esc_scan<NT>(cnt, nb, warp_a, warp_b);
+    const int mx = bucket_scan<NT>(cnt, nb, warp_a, warp_b);
     if (mx <= esc_bucket_max(p)) {  // team-uniform
       for (int t = tid; t < p; t += NT) {
         const KEY k = k0[t];

@@ -946,6 +946,57 @@ struct LongValF64 {
 };
 
 // ---------------------------------------------------------------------------
+// Teams of threads that sort by buckets
+// ---------------------------------------------------------------------------
+
+// Threads that share a row: one warp (several teams to a block) or the block.
+template <int NT>
+__device__ __forceinline__ void team_sync() {
+  if (NT == 32) __syncwarp();
+  else __syncthreads();
+}
+
+// cnt[0, nb) to its exclusive prefix sums (nb a power of two, >= NT); returns
+// the largest count (to every thread). Ends with a barrier.
+template <int NT>
+__device__ __forceinline__ int bucket_scan(int* __restrict__ cnt, int nb, int* warp_sums,
+                                        int* warp_max) {
+  constexpr int NW = NT / 32;
+  const int lane = threadIdx.x & 31, warp = NT == 32 ? 0 : threadIdx.x >> 5;
+  const int tid = NT == 32 ? lane : threadIdx.x;
+  const int per = nb / NT;
+  int* mine = cnt + tid * per;
+  int sum = 0, mx = 0;
+  for (int q = 0; q < per; ++q) {
+    const int c = mine[q];
+    sum += c;
+    mx = max(mx, c);
+  }
+  const int incl = warp_incl_scan(sum);
+  mx = __reduce_max_sync(FULL, mx);
+  int run = incl - sum;
+  if (NW > 1) {
+    if (lane == 31) {
+      warp_sums[warp] = incl;
+      warp_max[warp] = mx;
+    }
+    __syncthreads();
+    const int s = lane < NW ? warp_sums[lane] : 0;
+    const int m = lane < NW ? warp_max[lane] : 0;
+    const int wi = warp_incl_scan(s);
+    run += __shfl_sync(FULL, wi - s, warp);
+    mx = __reduce_max_sync(FULL, m);
+  }
+  for (int q = 0; q < per; ++q) {
+    const int c = mine[q];
+    mine[q] = run;
+    run += c;
+  }
+  team_sync<NT>();
+  return mx;
+}
+
+// ---------------------------------------------------------------------------
 // Bitonic sort of a power-of-two key/value array in shared memory
 // ---------------------------------------------------------------------------
 

@@ -70,3 +70,35 @@ def test_empty_and_out_of_range():
         with pytest.raises(sg.SpgemmError) as e:
             run(h, np.array([0, 5]), np.array([1, 1]), np.ones(2, np.float32), 4, 4, sg.ROW_MAJOR)
         assert e.value.status == 1
+
+
+@pytest.mark.parametrize("kind", [sg.ROW_MAJOR, sg.COL_MAJOR])
+@pytest.mark.parametrize("spread", ["even", "band", "crowd"])
+def test_segment_lengths_around_the_sorts_limits(kind, spread):
+    """Segments of every length around the limits of the register, warp, block
+    and merge sorts: minor indices spread evenly, within a narrow band, or with
+    most entries on a few indices (one bucket holds most of the segment, and
+    equal entries keep their input order)."""
+    rng = np.random.default_rng(len(spread))
+    lens = [0, 1, 2, 7, 8, 9, 15, 16, 17, 31, 32, 33, 255, 256, 257, 2047, 2048, 2049, 8191, 8192, 8193,
+            24575, 24576, 24577, 0, 5, 24576, 9000]
+    major = np.repeat(np.arange(len(lens)), lens)
+    n_minor = 100_000
+    if spread == "even":
+        minor = rng.integers(0, n_minor, len(major))
+    elif spread == "band":
+        minor = major * 3000 + rng.integers(0, 900, len(major))
+    else:
+        minor = np.where(rng.random(len(major)) < 0.8, 5000 + rng.integers(0, 3, len(major)),
+                         rng.integers(0, n_minor, len(major)))
+    perm = rng.permutation(len(major))
+    major, minor = major[perm], minor[perm]
+    v = rng.uniform(-1, 1, len(major)).astype(np.float32)
+    rows, cols = (len(lens), n_minor) if kind == sg.ROW_MAJOR else (n_minor, len(lens))
+    r, c = (major, minor) if kind == sg.ROW_MAJOR else (minor, major)
+    with sg.Handle() as h:
+        got = run(h, r, c, v, rows, cols, kind)
+    exp = expected(r, c, v, rows, cols, kind)
+    assert np.array_equal(got[0], exp[0])
+    assert np.array_equal(got[1], exp[1])
+    assert np.array_equal(got[2], exp[2])
