@@ -121,7 +121,7 @@ int Engine::prof_collect() {
 }
 
 Engine::~Engine() {
-  DevBuf* all[] = {&a_rowptr_, &a_col_, &a_val_, &cursor_, &aoff_, &row_p_, &c_cnt_,
+  DevBuf* all[] = {&a_rowptr_, &a_col_, &a_val_, &cursor_, &aoff_, &row_p_,
                    &c_rowptr64_, &tiles_, &sym_rows_, &num_rows_, &long_slot_,
                    &chunk_cnt_, &slices_buf_, &mid_slices_, &row_span_, &counters_, &restrict_scratch_,
                    &tcap_, &toff_, &t_col_, &t_val_,
@@ -248,6 +248,22 @@ int Engine::scan_counts(const int* in, int n, long long* tiles, const ScanOut& o
   return 0;
 }
 
+size_t Engine::row_counts_offset() const {
+  const size_t tiles = (size_t)(m_ + SCAN_TILE - 1) / SCAN_TILE + 1;
+  return ROW_TILES_OFFSET + (sizeof(long long) * tiles + 15) / 16 * 16;
+}
+
+int* Engine::c_cnt() const {
+  return reinterpret_cast<int*>(counters_.as<unsigned char>() + row_counts_offset());
+}
+
+void Engine::publish_counters(ScanOut* out) const {
+  static_assert(sizeof(DevCounters) % sizeof(unsigned) == 0, "copied by words");
+  out->counters = reinterpret_cast<const unsigned*>(counters_.as<DevCounters>());
+  out->publish = reinterpret_cast<unsigned*>(host_counters_);
+  out->publish_words = (int)(sizeof(DevCounters) / sizeof(unsigned));
+}
+
 int Engine::symbolic(const cm& A, const cm& B, long long* nnz_c) {
   if (int r = analyze(A, B)) return r;
   return symbolic_pass(nnz_c);
@@ -270,17 +286,17 @@ int Engine::analyze(const cm& A, const cm& B) {
   const int nnz_a = A.nnz;
   const int m = m_;
 
-  const size_t row_tiles = (size_t)(m + SCAN_TILE - 1) / SCAN_TILE + 1;
-  const size_t counter_bytes = ROW_TILES_OFFSET + sizeof(long long) * row_tiles;
-  SG_CK(counters_.ensure(counter_bytes), "alloc counters");
-  DevCounters* dc = counters_.as<DevCounters>();
-  SG_CK(cudaMemsetAsync(dc, 0, counter_bytes, stream_), "memset counters");
+  if (!host_counters_) return fail(3, "no pinned host memory for the counters");
+  // counters, row tiles and row counts in one buffer: one memset (the row
+  // counts need it only as the transpose's histogram)
   const bool a_csc = A.type == COL_MAJOR;
-  SG_CK(c_cnt_.ensure(sizeof(int) * (size_t)std::max(m, 1)), "alloc c_cnt");
+  const size_t cnt_bytes = sizeof(int) * (size_t)std::max(m, 1);
+  SG_CK(counters_.ensure(row_counts_offset() + cnt_bytes), "alloc counters");
+  DevCounters* dc = counters_.as<DevCounters>();
+  SG_CK(cudaMemsetAsync(dc, 0, row_counts_offset() + (a_csc ? cnt_bytes : 0), stream_),
+        "memset counters");
   SG_CK(c_rowptr64_.ensure(sizeof(long long) * ((size_t)m + 1)), "alloc c_rowptr64");
-  int* cnt = c_cnt_.as<int>();
-  if (a_csc)
-    SG_CK(cudaMemsetAsync(cnt, 0, sizeof(int) * (size_t)std::max(m, 1), stream_), "memset cnt");
+  int* cnt = c_cnt();
 
   // ---- validate the operands (sync point 1 reports the result) ----
   // The transpose and row analysis guard every index they use; their findings
@@ -351,14 +367,14 @@ int Engine::analyze(const cm& A, const cm& B) {
     SG_LAUNCHED("k_row_analysis");
   }
   // temporary-buffer slots of the fused rows (grand total = buffer size)
-  if (int r = scan_counts(tcap_.as<int>(), m, this->row_tiles(), ScanOut{toff_.as<long long>(), nullptr, nullptr}))
-    return r;
+  // and everything counted so far to the host
+  ScanOut slots{toff_.as<long long>(), nullptr, nullptr};
+  if (!replay_) publish_counters(&slots);
+  if (int r = scan_counts(tcap_.as<int>(), m, this->row_tiles(), slots)) return r;
   if (replay_) {  // same structure as the planned run: keep its sizes
     have_analysis_ = true;
     return 0;
   }
-  SG_CK(cudaMemcpyAsync(host_counters_, dc, sizeof(DevCounters), cudaMemcpyDeviceToHost, stream_),
-        "read counters");
   SG_CK(cudaStreamSynchronize(stream_), "sync after row analysis");
   if (int r = check_status(*host_counters_)) return r;
   p_total_ = (long long)host_counters_->p_total;
@@ -392,8 +408,10 @@ int Engine::symbolic_pass(long long* nnz_c) {
   if (int r = launch_first_pass()) return r;
 
   // ---- row pointers + numeric binning of the long rows ----
-  if (int r = scan_counts(c_cnt_.as<int>(), m, nullptr, ScanOut{c_rowptr64_.as<long long>(), nullptr, nullptr}))
-    return r;
+  ScanOut rowptr{c_rowptr64_.as<long long>(), nullptr, nullptr};
+  const bool last = n_long_sym_ == 0;  // nothing more is counted without long rows
+  if (last && !replay_) publish_counters(&rowptr);
+  if (int r = scan_counts(c_cnt(), m, nullptr, rowptr)) return r;
   SG_CK(num_rows_.ensure(sizeof(int) * (size_t)NB_COUNT * std::max(m, 1)), "alloc num_rows");
   big_capacity_ = (long long)n_long_sym_ * std::max(n_chunks_, 1);
   SG_CK(slices_buf_.ensure(sizeof(Slice) * (size_t)std::max(big_capacity_, 1ll)), "alloc slices");
@@ -414,7 +432,7 @@ int Engine::symbolic_pass(long long* nnz_c) {
   if (m > 0 && n_long_sym_ > 0) {
     prof_begin("k_num_bin");
     k_num_bin<<<(m + NBIN_THREADS - 1) / NBIN_THREADS, NBIN_THREADS, 0, stream_>>>(
-        m, n_, c_cnt_.as<int>(), row_p_.as<long long>(), c_rowptr64_.as<long long>(),
+        m, n_, c_cnt(), row_p_.as<long long>(), c_rowptr64_.as<long long>(),
         row_span_.as<int2>(), dc->num_count, num_rows_.as<int>(), chunk_cnt_.as<int>(),
         n_chunks_, long_slot_.as<int>(), slices_buf_.as<Slice>(), &dc->slice_count,
         (int)big_capacity_, mid_slices_.as<Slice>(), &dc->mid_count, bitmap_words_ > 0 ? 1 : 0,
@@ -425,8 +443,9 @@ int Engine::symbolic_pass(long long* nnz_c) {
     have_sym_ = true;
     return 0;
   }
-  SG_CK(cudaMemcpyAsync(host_counters_, dc, sizeof(DevCounters), cudaMemcpyDeviceToHost, stream_),
-        "read counters");
+  if (!last)
+    SG_CK(cudaMemcpyAsync(host_counters_, dc, sizeof(DevCounters), cudaMemcpyDeviceToHost, stream_),
+          "read counters");
   SG_CK(cudaStreamSynchronize(stream_), "sync after symbolic pass");
   if (int r = check_status(*host_counters_)) return r;
   nnz_c_ = host_counters_->grand_total;
@@ -446,7 +465,7 @@ int Engine::launch_first_pass() {
   DevCounters* dc = counters_.as<DevCounters>();
   unsigned* status = &dc->status;
   const int m = m_;
-  int* c_cnt = c_cnt_.as<int>();
+  int* c_cnt = this->c_cnt();
   const long long* row_p = row_p_.as<long long>();
   int* rows = sym_rows_.as<int>();
   if (!replay_) bitmap_words_ = 0;
@@ -497,7 +516,7 @@ int Engine::launch_fused() {
   unsigned* status = &dc->status;
   const int m = m_;
   int* rows = sym_rows_.as<int>();
-  int* c_cnt = c_cnt_.as<int>();
+  int* c_cnt = this->c_cnt();
   const long long* row_p = row_p_.as<long long>();
   const long long* toff = toff_.as<long long>();
   int* t_col = t_col_.as<int>();
@@ -632,7 +651,7 @@ int Engine::numeric_range(int* c_col, float* c_val, int r0, int r1, int* c_rowpt
     while (rpw > 1 && (long long)(r1 - r0) < (long long)rpw * sms_ * 16) rpw >>= 1;
     prof_begin("k_copy_fused");
     k_copy_fused<<<blocks_for((long long)(r1 - r0), 8 * rpw, (long long)sms_ * 16), 256, 0, stream_>>>(
-        r0, r1, m_, rpw, tcap_.as<int>(), toff_.as<long long>(), c_cnt_.as<int>(),
+        r0, r1, m_, rpw, tcap_.as<int>(), toff_.as<long long>(), c_cnt(),
         c_rowptr64_.as<long long>(), t_col_.as<int>(), t_val_.as<float>(), c_col, c_val, c_rowptr);
     SG_LAUNCHED("k_copy_fused");
   } else if (c_rowptr) {
@@ -683,7 +702,11 @@ int Engine::rowptr64_to_host(long long* host) {
 
 int Engine::finish_numeric() {
   if (replay_) return 0;  // the caller reads the status after the captured work
-  return read_status();
+  if (n_long_sym_ > 0) return read_status();
+  // only long rows have numeric kernels that check anything
+  SG_CK(cudaStreamSynchronize(stream_), "sync after numeric pass");
+  prof_collect_if_full();
+  return 0;
 }
 
 int Engine::numeric(int* c_rowptr, int* c_col, float* c_val) {
@@ -848,12 +871,12 @@ int Engine::launch_num_rows(int* c_col, float* c_val, int r0, int r1) {
     const int cmin = plan[g].cmin, cmax = plan[g].cmax;
     int* order = lpt_order_.as<int>() + (size_t)g * cnt;
     prof_begin("k_lpt_hist");
-    k_lpt_hist<<<lb, 256, 0, stream_>>>(rows, cnt, r0, r1, row_p_.as<long long>(), c_cnt_.as<int>(),
+    k_lpt_hist<<<lb, 256, 0, stream_>>>(rows, cnt, r0, r1, row_p_.as<long long>(), c_cnt(),
                                         row_span_.as<int2>(), cmin, cmax, ROWS_MAX_WORDS,
                                         dc->lpt_hist[g]);
     SG_LAUNCHED("k_lpt_hist");
     prof_begin("k_lpt_scatter");
-    k_lpt_scatter<<<lb, 256, 0, stream_>>>(rows, cnt, r0, r1, row_p_.as<long long>(), c_cnt_.as<int>(),
+    k_lpt_scatter<<<lb, 256, 0, stream_>>>(rows, cnt, r0, r1, row_p_.as<long long>(), c_cnt(),
                                            row_span_.as<int2>(), cmin, cmax, ROWS_MAX_WORDS,
                                            dc->lpt_hist[g], dc->lpt_cursor[g], order,
                                            &dc->rows_listed[g]);

@@ -185,6 +185,11 @@ class Engine {
   // Exclusive scan of in[0, n) (total to the counters' grand_total); `tiles`:
   // the tiles' sums when a kernel has already formed them, else null.
   int scan_counts(const int* in, int n, long long* tiles, const ScanOut& out);
+  // Entries per row of C (of A, while it is transposed), behind the tiles.
+  int* c_cnt() const;
+  size_t row_counts_offset() const;
+  // The scan copies the counters to host_counters_ (see ScanOut).
+  void publish_counters(ScanOut* out) const;
   // Zeroed long long per tile of the row counts, behind the counters.
   long long* row_tiles() const {
     return reinterpret_cast<long long*>(counters_.as<unsigned char>() + ROW_TILES_OFFSET);
@@ -224,7 +229,7 @@ class Engine {
   Operands op_{};
 
   DevBuf a_rowptr_, a_col_, a_val_, cursor_, aoff_;
-  DevBuf row_p_, c_cnt_, c_rowptr64_, tiles_;
+  DevBuf row_p_, c_rowptr64_, tiles_;
   DevBuf sym_rows_, num_rows_, long_slot_, chunk_cnt_, slices_buf_, mid_slices_, row_span_;
   DevBuf tcap_, toff_, t_col_, t_val_;  // fused pass: row bounds, temp offsets, temp output
   DevBuf counters_, restrict_scratch_, bitmaps_, lpt_order_;
@@ -233,7 +238,7 @@ class Engine {
   int max_row_len_ = 0;
   DevBuf out_rowptr_, out_col_, out_val_;
   DevBuf stage_[6];
-  DevCounters* host_counters_ = nullptr;  // pinned
+  DevCounters* host_counters_ = nullptr;  // pinned, written by kernels
 
   bool prof_on_ = false;
   struct ProfRec { std::string name; cudaEvent_t a, b; };

@@ -715,10 +715,17 @@ k_scan_tile_sums(long long* __restrict__ tile_sum, int ntiles) {
 
 // out[i] = exclusive prefix of in, out[n] = the total, also to *grand_total;
 // any of the outputs (int64, and two int32 copies) may be null. tiles: the
-// tiles' sums, or (scanned) their exclusive prefix.
+// tiles' sums, or (scanned) their exclusive prefix. With `publish`, the last
+// block then copies publish_words words from `counters` (which hold
+// *grand_total and what earlier kernels counted) to `publish`, mapped host
+// memory that is read after the next synchronisation: a copy of its own cost
+// a small product 4 us.
 struct ScanOut {
   long long* p64;
   int *p32, *copy32;
+  const unsigned* counters = nullptr;
+  unsigned* publish = nullptr;
+  int publish_words = 0;
 };
 
 __global__ void __launch_bounds__(SCAN_THREADS)
@@ -757,6 +764,11 @@ k_scan_apply(const int* __restrict__ in, int n, const long long* __restrict__ ti
     if (out.p32) out.p32[n] = (int)all;
     if (out.copy32) out.copy32[n] = (int)all;
     *grand_total = all;
+  }
+  if (out.publish && blockIdx.x == gridDim.x - 1) {
+    __syncthreads();
+    for (int t = threadIdx.x; t < out.publish_words; t += SCAN_THREADS)
+      out.publish[t] = __ldcg(out.counters + t);
   }
 }
 
