@@ -646,9 +646,10 @@ int Engine::numeric_range(int* c_col, float* c_val, int r0, int r1, int* c_rowpt
   if (nnz_c_ > 0 && (!c_col || !c_val)) return fail(1, "null output pointer");
   if (r0 < 0 || r1 > m_ || r0 > r1) return fail(1, "numeric: row range outside [0, m]");
   if (r1 > r0 && temp_total_ > 0) {
-    // rows per warp: 32, fewer while that leaves SMs without work
+    // rows per warp: 32, fewer while that makes less than two waves of warps
+    // (100003 rows of 207 entries: 88 us with 32 rows a warp, 21 warps an SM)
     int rpw = 32;
-    while (rpw > 1 && (long long)(r1 - r0) < (long long)rpw * sms_ * 16) rpw >>= 1;
+    while (rpw > 1 && (long long)(r1 - r0) < (long long)rpw * sms_ * 128) rpw >>= 1;
     prof_begin("k_copy_fused");
     k_copy_fused<<<blocks_for((long long)(r1 - r0), 8 * rpw, (long long)sms_ * 16), 256, 0, stream_>>>(
         r0, r1, m_, rpw, tcap_.as<int>(), toff_.as<long long>(), c_cnt(),
