@@ -453,6 +453,22 @@ __device__ __forceinline__ int chunk_for(long long p, int nwarps, int max_chunk)
   return (int)u;
 }
 
+// Number of entries j in [lo, hi) with at(j) <= f, added to lo (at rises with
+// j), by a whole warp: 32 probes a round, so a row of 1000 entries takes two
+// dependent loads instead of ten.
+template <class At>
+__device__ __forceinline__ int warp_upper_bound(int lo, int hi, int f, At at) {
+  const int lane = lane_id();
+  while (hi - lo > 32) {
+    const int step = (hi - lo + 31) >> 5;
+    const int p = lo + (lane + 1) * step - 1;
+    const int c = __popc(__ballot_sync(FULL, p < hi && at(p) <= f));
+    lo += c * step;
+    hi = min(hi, lo + step - 1);
+  }
+  return lo + __popc(__ballot_sync(FULL, lo + lane < hi && at(lo + lane) <= f));
+}
+
 // Products [f0, f1) of the row's flattened product sequence (entries in
 // order, each contributing nnz(B(k,:)) products), one warp. Uses the
 // per-entry flattened offsets `aoff` written by k_row_analysis.
@@ -462,11 +478,7 @@ __device__ __forceinline__ void warp_expand_range(const Operands& op, int rs, in
                                                   SegScratch* sc) {
   const int lane = lane_id();
   // Last entry whose offset is <= f0 holds product f0.
-  int lo = rs, hi = re;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (__ldg(op.aoff + mid) <= f0) lo = mid + 1; else hi = mid;
-  }
+  const int lo = warp_upper_bound(rs, re, f0, [&](int j) { return __ldg(op.aoff + j); });
   for (int base = lo - 1; base < re; base += 32) {
     const int j = base + lane;
     int bstart = 0, len = 0;
@@ -554,11 +566,8 @@ __device__ __forceinline__ void warp_expand_explicit(const Operands& op, int rs,
                                                      const int* seg_start, const int* roff,
                                                      int f0, int f1, F& f, SegScratch* sc) {
   const int lane = lane_id();
-  int lo = 0, hi = d;  // last entry whose offset is <= f0
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (roff[mid] <= f0) lo = mid + 1; else hi = mid;
-  }
+  // last entry whose offset is <= f0
+  const int lo = warp_upper_bound(0, d, f0, [&](int j) { return roff[j]; });
   for (int base = lo - 1; base < d; base += 32) {
     const int j = base + lane;
     int bstart = 0, len = 0;
