@@ -49,12 +49,13 @@ __device__ __forceinline__ int esc_bucket_max(int p) { return 64 + (p >> 3); }
 
 // All products of a row into vals[pos] / keys[pos], pos = the product's
 // flattened position (entry j of the row holds aoff[j] .. aoff[j] +
-// nnz(B(k_j,:)) - 1), and their bucket counts. Entries are dealt to the
-// team's warps in turn; each warp loads 32 of them at once, then groups of
-// 2^lg lanes (about the mean B row length, so short rows do not idle a warp)
-// walk one entry each, two entries in flight. Columns beyond the row's span
-// (`width`; a replayed batch whose structure was changed) are clamped, which
-// keeps every index below in bounds.
+// nnz(B(k_j,:)) - 1), and their bucket counts. Entries are dealt in turn to
+// the team's warps, or, when there are fewer, to groups of warps that walk an
+// entry together (a power-law row of 3000 products may be one hub row of B:
+// one warp alone took 38 us over it). Each warp loads 32 of its entries at
+// once, then groups of 2^lg lanes (about the mean B row length, so short rows
+// do not idle a warp) walk one entry each, two entries in flight. Columns beyond the row's span (`width`; a replayed batch whose
+// structure was changed) are clamped, which keeps every index below in bounds.
 template <int NT, int SH, int MODE, class KEY>
 __device__ __forceinline__ void esc_gather(const Operands& op, int rs, int re, int p, int lo,
                                            unsigned width, int shift, KEY* __restrict__ keys,
@@ -63,10 +64,18 @@ __device__ __forceinline__ void esc_gather(const Operands& op, int rs, int re, i
   constexpr int NW = NT / 32;
   const int lane = threadIdx.x & 31, warp = NT == 32 ? 0 : threadIdx.x >> 5;
   const int mean = p / (re - rs);
-  const int lg = mean <= 4 ? 2 : (mean <= 8 ? 3 : (mean <= 16 ? 4 : 5));
-  const int groups = 32 >> lg, g = lane >> lg, gl = lane & ((1 << lg) - 1), step = 1 << lg;
-  for (int base = rs + warp; base < re; base += 32 * NW) {
-    const int j = base + NW * lane;
+  int share = 1;  // warps to an entry
+  if (NT >= 256)  // smaller teams lose more to the registers than they gain
+    while (2 * share * (re - rs) <= NW) share <<= 1;
+  const int dealt = NW / share;  // entries walked at once
+  auto put = [&](int col, float av, float bv, int pos) {
+    const unsigned x = min((unsigned)(col - lo), width);
+    keys[pos] = ((KEY)x << SH) | (KEY)pos;
+    vals[pos] = esc_value<MODE>(av, bv);
+    atomicAdd(cnt + (x >> shift), 1);
+  };
+  for (int base = rs + warp / share; base < re; base += 32 * dealt) {
+    const int j = base + dealt * lane;
     int bstart = 0, len = 0, off = 0;
     float a = 0.f;
     if (j < re) {
@@ -76,7 +85,32 @@ __device__ __forceinline__ void esc_gather(const Operands& op, int rs, int re, i
       bstart = __ldg(op.b_rowptr + k);
       len = __ldg(op.b_rowptr + k + 1) - bstart;
     }
-    const int entries = min((re - base + NW - 1) / NW, 32);
+    const int entries = min((re - base + dealt - 1) / dealt, 32);
+    if (NT >= 256 && share > 1) {  // team-uniform: four steps of one entry in flight
+      const int step = 32 * share;
+      for (int e = 0; e < entries; ++e) {
+        const int eb = __shfl_sync(FULL, bstart, e), el = __shfl_sync(FULL, len, e);
+        const int eo = __shfl_sync(FULL, off, e);
+        const float ea = __shfl_sync(FULL, a, e);
+        for (int t = (warp % share) * 32 + lane; t < el; t += 4 * step) {
+          int c[4];
+          float v[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            if (t + u * step < el) {
+              c[u] = __ldg(op.b_col + eb + t + u * step);
+              v[u] = __ldg(op.b_val + eb + t + u * step);
+            }
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (t + u * step < el) put(c[u], ea, v[u], eo + t + u * step);
+        }
+      }
+      continue;
+    }
+    const int lg = mean <= 4 ? 2 : (mean <= 8 ? 3 : (mean <= 16 ? 4 : 5));
+    const int groups = 32 >> lg, g = lane >> lg, gl = lane & ((1 << lg) - 1), step = 1 << lg;
     for (int e0 = 0; e0 < entries; e0 += 2 * groups) {
       int eb[2], el[2], eo[2], c[2];
       float ea[2], v[2];
@@ -100,15 +134,8 @@ __device__ __forceinline__ void esc_gather(const Operands& op, int rs, int re, i
           }
         }
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          if (t < el[u]) {
-            const unsigned x = min((unsigned)(c[u] - lo), width);
-            const int pos = eo[u] + t;
-            keys[pos] = ((KEY)x << SH) | (KEY)pos;
-            vals[pos] = esc_value<MODE>(ea[u], v[u]);
-            atomicAdd(cnt + (x >> shift), 1);
-          }
-        }
+        for (int u = 0; u < 2; ++u)
+          if (t < el[u]) put(c[u], ea[u], v[u], eo[u] + t);
       }
     }
   }

@@ -166,3 +166,26 @@ def test_hashed_rows_reuse_and_overflow(precision, table, stride):
     assert_values_close(out[0].val, ref, tol)
     assert np.array_equal(out[0].col, out[1].col)
     assert np.array_equal(out[0].val.view(np.uint32), out[1].val.view(np.uint32))
+
+
+@pytest.mark.parametrize("precision", [sg.PLAIN, sg.COMPENSATED])
+@pytest.mark.parametrize("lengths", [(4096,), (1500, 700, 1), (513, 90), (260,), (130, 7)])
+def test_sorted_rows_of_few_long_entries(precision, lengths):
+    """Rows of 1025 to 4096 products from one to some thirty entries: several
+    warps of the team walk an entry together."""
+    counts = [1025, 1500, 1537, 2047, 2048, 2049, 3000, 3073, 4095, 4096]
+    A, B = rows_of(counts, 300_000, lengths, False, seed=lengths[0], empty=1)
+    check_rows(A, B, precision, dict(warp_cap_max=0))
+
+
+@pytest.mark.parametrize("m,k", [(1, 5), (37, 1), (300, 4000), (19000, 3)])
+def test_copy_by_rows_per_warp(m, k):
+    """C of few or many rows, short and long, so that a warp of the copy takes
+    from 1 to 32 of them, with empty rows between."""
+    rng = np.random.default_rng(m + k)
+    rows = np.repeat(np.arange(m), rng.integers(0, min(k, 4) + 1, m))
+    cols = np.concatenate([np.sort(rng.choice(k, n, replace=False)) for n in np.bincount(rows, minlength=m)]) \
+        if len(rows) else rows
+    A = W.from_coo(m, k, rows, cols, rng.uniform(-1, 1, len(rows)).astype(np.float32))
+    B = W.er(k, 30.0, m, cols=900)
+    check_rows(A, B, sg.PLAIN, {})
