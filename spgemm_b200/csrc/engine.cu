@@ -125,7 +125,7 @@ Engine::~Engine() {
                    &c_rowptr64_, &tiles_, &sym_rows_, &num_rows_, &long_slot_,
                    &chunk_cnt_, &slices_buf_, &mid_slices_, &row_span_, &counters_, &restrict_scratch_,
                    &tcap_, &toff_, &t_col_, &t_val_,
-                   &bitmaps_, &lpt_order_, &b_info_, &out_rowptr_,
+                   &bitmaps_, &lpt_order_, &b_info_, &route_, &out_rowptr_,
                    &out_col_, &out_val_};
   for (DevBuf* b : all) b->release();
   for (DevBuf& b : stage_) b.release();
@@ -352,12 +352,14 @@ int Engine::analyze(const cm& A, const cm& B) {
     const long long mean = nnz_a / m;
     const int g = mean <= 4 ? 4 : (mean <= 8 ? 8 : (mean <= 16 ? 16 : 32));
     const int rpb = m >= 2 * RA_ROWS * sms_ ? RA_ROWS : RA_THREADS / g;
+    const int blocks = (m + rpb - 1) / rpb;
+    SG_CK(route_.ensure((size_t)blocks), "alloc row routes");
     auto launch = [&](auto kernel) {
-      kernel<<<(m + rpb - 1) / rpb, RA_THREADS, 0, stream_>>>(
+      kernel<<<blocks, RA_THREADS, 0, stream_>>>(
           op_, b_info_.as<int4>(), rpb, aoff_.as<int>(), row_p_.as<long long>(), cnt,
           tcap_.as<int>(), this->row_tiles(), dc->fb_count, dc->may_overflow, dc->nominal,
-          sym_rows_.as<int>(), &dc->p_total, &dc->max_row_len, row_span_.as<int2>(), &dc->status,
-          tn_);
+          sym_rows_.as<int>(), &dc->p_total, &dc->max_row_len, row_span_.as<int2>(),
+          route_.as<unsigned char>(), replay_, &dc->status, tn_);
     };
     prof_begin("k_row_analysis");
     if (g == 4) launch(k_row_analysis<4>);

@@ -198,7 +198,8 @@ k_row_analysis(Operands op, const int4* __restrict__ b_info, int rows_per_block,
                int* __restrict__ fb_count, int* __restrict__ may_overflow,
                int* __restrict__ nominal_count, int* __restrict__ fb_rows,
                unsigned long long* __restrict__ p_total, int* __restrict__ max_row_len,
-               int2* __restrict__ row_span, unsigned* status, Tuning tn) {
+               int2* __restrict__ row_span, unsigned char* __restrict__ route, bool routed,
+               unsigned* status, Tuning tn) {
   constexpr int NW = RA_THREADS / 32;
   __shared__ int hist[FB_COUNT], base[FB_COUNT], ovf[FB_COUNT], nominal[FB_COUNT];
   __shared__ long long s_p[RA_ROWS];
@@ -376,8 +377,11 @@ k_row_analysis(Operands op, const int4* __restrict__ b_info, int rows_per_block,
   // 2 of 3 pairs, any order of the entries: 1 of 2), rows of random graphs
   // hardly. Rows that do not repeat columns fill a hash table for nothing
   // (random rows of 200 products: 4.6 ns each hashed, 3.4 sorted).
+  // The answer depends on the order of A's entries, which the transpose leaves
+  // to chance, so a replayed product takes the planned run's (`routed`): its
+  // launches are sized for those lists.
   const int n0 = __popc(cand[0]), ncand = n0 + __popc(cand[1]);
-  if (ncand > 0 && warp < ncand) {  // warp-uniform
+  if (ncand > 0 && warp < ncand && !routed) {  // warp-uniform
     const int idx = ncand <= NW ? warp : warp * ncand / NW;
     const unsigned mask = idx < n0 ? cand[0] : cand[1];
     const int nth = idx < n0 ? idx : idx - n0;
@@ -401,11 +405,13 @@ k_row_analysis(Operands op, const int4* __restrict__ b_info, int rows_per_block,
     }
   }
   __syncthreads();
+  const bool repeats = routed ? route[blockIdx.x] != 0 : 4 * s_hits >= max(s_pairs, 1);
+  if (!routed && threadIdx.x == 0) route[blockIdx.x] = repeats;
   if (threadIdx.x < RA_ROWS) {
     const int i = row0 + threadIdx.x;
     int slot = 0;
     if (threadIdx.x < nrows) {
-      if (candidate && 4 * s_hits < max(s_pairs, 1)) bin = overflow_bin_of(acc, lo, span, tn);
+      if (candidate && !repeats) bin = overflow_bin_of(acc, lo, span, tn);
       row_span[i] = acc > 0 ? make_int2(lo, lo + span - 1) : make_int2(0, -1);
       row_p[i] = acc;
       if (acc >= (1ll << 31)) atomicOr(status, ST_ROW_TOO_LONG);

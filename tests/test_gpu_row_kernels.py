@@ -9,6 +9,7 @@ import pytest
 import spgemm_b200 as sg
 from spgemm_b200 import workloads as W
 from helpers import assert_structure_equal, assert_values_close, compensated_tolerance, plain_tolerance
+from test_gpu_batch import DeviceBatch, check_all
 from test_gpu_parity import ref_product
 
 pytestmark = pytest.mark.gpu
@@ -189,3 +190,37 @@ def test_copy_by_rows_per_warp(m, k):
     A = W.from_coo(m, k, rows, cols, rng.uniform(-1, 1, len(rows)).astype(np.float32))
     B = W.er(k, 30.0, m, cols=900)
     check_rows(A, B, sg.PLAIN, {})
+
+
+def grouped_rows(m, seed, n=60_000):
+    """Rows of A with nine entries, three on each of three rows of B that share
+    all their columns: how often neighbouring entries meet the same columns
+    lies at the limit between hashed and sorted rows and depends on the order
+    in which A's entries are taken."""
+    rng = np.random.default_rng(seed)
+    cols = np.sort(np.stack([rng.choice(n, 6, replace=False) for _ in range(3 * m)]), axis=1)
+    B = W.from_coo(9 * m, n, np.repeat(np.arange(9 * m), 6), np.repeat(cols, 3, axis=0).ravel(),
+                   rng.uniform(-1, 1, 54 * m).astype(np.float32))
+    A = W.from_coo(m, 9 * m, np.repeat(np.arange(m), 9), np.arange(9 * m),
+                   rng.uniform(-1, 1, 9 * m).astype(np.float32))
+    perm = rng.permutation(9 * m)  # A's columns in any order: groups mixed
+    order = np.argsort(perm, kind="stable")
+    A = W.from_coo(m, 9 * m, np.repeat(np.arange(m), 9), perm, A.val)
+    B = W.from_coo(9 * m, n, np.repeat(np.arange(9 * m), 6), B.col.reshape(-1, 6)[order].ravel(),
+                   B.val.reshape(-1, 6)[order].ravel())
+    return A, B
+
+
+@pytest.mark.parametrize("a_format", ["csc", "csr"])
+@pytest.mark.parametrize("m", [5, 40, 700])
+def test_replayed_rows_keep_their_kernels(m, a_format):
+    """The transpose of a CSC A leaves the entries of a row in any order, so a
+    replay must not decide anew between hashing and sorting: its launches are
+    sized for the planned run's lists."""
+    db = DeviceBatch([grouped_rows(m, seed) for seed in (m, m + 1)], a_format)
+    with sg.Handle() as h:
+        h.batch_plan(db.A, db.B)
+        refs = check_all(h, db.pairs)
+        for graph in (True, True, True, False, False):
+            h.batch_execute(graph=graph)
+            check_all(h, db.pairs, refs=refs)
