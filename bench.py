@@ -142,29 +142,35 @@ def product_stats(A, B):
 # Mirrors of the engine's default bin rules (kernels.cuh), used only to
 # attribute algorithmic bytes to the kernel that processed each row.
 LONG_P, WARP_CAP, WARP_TMAX, MID_COLS, LONG_O, MID_O = 4096, 2048, 256, 1 << 18, 4096, 256
-ESC_P_MIN, ESC_SPAN_MIN = 0, 0  # rows outside the warp bins merged by sorting
+ESC_P = {32: 256, 64: 512, 128: 1024, 256: 2048, 512: 4096}  # products of a sorted row, by block size
 # output capacities of the whole-row kernel's two block sizes (engine.cu:
 # (shared-memory budget - per-warp scratch - directory) / 4 bytes)
-ROWS_CAP_512 = (111 * 1024 - 16 * 388 - 8193 * 8) // 4
-ROWS_CAP_1024 = (225 * 1024 - 32 * 388 - 8193 * 8) // 4
+ROWS_CAP_512 = (111 * 1024 - 16 * 384 - 8193 * 8) // 4
+ROWS_CAP_1024 = (225 * 1024 - 32 * 384 - 8193 * 8) // 4
 
 
-def first_bin(p, cap, span):
+def row_kernel(p, cap, span):
+    """Kernel of each row's first pass, as the profile names it. Warp-table
+    rows are put down as hashed: the engine sorts those of a neighbourhood
+    whose products hardly share columns, which only a sample of A's entries
+    tells."""
     lg = np.ceil(np.log2(np.maximum(cap + cap // 4 + 1, 1))).astype(np.int64)
-    warp = np.clip(lg, 6, int(np.log2(WARP_TMAX))) - 6
-    blk = np.maximum(np.ceil(np.log2(np.maximum(2 * cap, 1))).astype(np.int64), 11) - 11 + 5
-    esc = (p > ESC_P_MIN) & (span > ESC_SPAN_MIN)
-    esc_bin = np.where(p <= 1024, 10, np.where(p <= 2048, 11, 12))
-    b = np.where(cap <= WARP_CAP, warp, np.where(esc, esc_bin, np.where(span <= MID_COLS, 8, blk)))
-    b = np.where(p > LONG_P, 9, b)
-    return np.where(p <= 0, -1, b)
+    bin_ = np.clip(lg, 6, int(np.log2(WARP_TMAX))) - 6
+    name = np.array([f"k_fused_warp<{b}>" for b in range(5)], dtype=object)[bin_]
+    name[span <= 4096 - 31] = "k_fused_bits"
+    name[p <= 32] = "k_fused_tiny"
+    wide = cap > WARP_CAP
+    below = 0
+    for nt, most in ESC_P.items():
+        name[wide & (p > below) & (p <= most)] = f"k_fused_esc<{nt}>"
+        below = most
+    name[(p > LONG_P) | (p <= 0)] = ""
+    return name
 
 
 def kernel_rows(name, p_i, o_i, span, n):
     """Rows processed by an engine kernel (mask), and whether it writes C."""
-    import re
     cap = np.minimum(np.minimum(p_i, n), span)
-    fb = first_bin(p_i, cap, span)
     long_rows = p_i > LONG_P
     if name == "k_sym_long":
         return long_rows, False
@@ -179,15 +185,9 @@ def kernel_rows(name, p_i, o_i, span, n):
         return long_rows & (o_i > LONG_O) & ((o_i > ROWS_CAP_1024) | (span > (1 << 18))), True
     if name == "k_num_mid":
         return long_rows & (o_i > MID_O) & (o_i <= LONG_O) & (span <= MID_COLS), True
-    if name == "k_fused_mid":
-        return fb == 8, True
-    m = re.match(r"k_fused_esc<(\d+)>", name)
-    if m:
-        return fb == {128: 10, 256: 11, 512: 12}[int(m.group(1))], True
-    m = re.match(r"k_fused_(warp|block)<(\d+)>", name)
-    if m:
-        lg = int(m.group(2))
-        return fb == (lg - 6 if m.group(1) == "warp" else lg - 11 + 5), True
+    if name.startswith("k_fused_"):
+        sel = row_kernel(p_i, cap, span) == name
+        return (sel, True) if sel.any() else (None, False)
     return None, False
 
 

@@ -56,31 +56,37 @@ typedef struct spgemm_context* spgemm_handle_t;
 typedef struct spgemm_stats {
     long long intermediate_products;   /* P = sum_k nnz(A(:,k)) * nnz(B(k,:)) */
     long long nnz_c;                   /* exact nnz(C) */
-    int rows_per_symbolic_bin[16];     /* rows per first-pass bin: 0..4 warp hash
-                                          (64..1024 slots), 5..7 block hash
-                                          (2048..8192), 8 span bitmap, 9 long,
-                                          10..12 sorted (rows of <= 1024, 2048,
-                                          4096 products) */
+    int rows_per_symbolic_bin[16];     /* rows per first-pass bin: 0..4 warp rows
+                                          (by table size, 64..1024), 5..7 block
+                                          hash (2048..8192), 8 span bitmap, 9
+                                          long, 10..12 sorted (rows of <= 1024,
+                                          2048, 4096 products) */
     int rows_per_numeric_bin[16];      /* long rows per numeric bin: 4..7 block
                                           hash, 8 column slices, 9 span bitmap */
     int long_row_slices;               /* column slices of the long-row path */
     long long kernel_launches;         /* engine kernels launched by the handle so far */
-    int warp_overflow_rows;            /* warp-bin rows redone by a block kernel */
+    int warp_overflow_rows;            /* warp rows whose table or bitmap was full,
+                                          redone by another kernel */
 } spgemm_stats;
 
 /* Bin thresholds and slice shapes of the engine (spgemm_get_tuning returns
  * the defaults of a new handle). Row i of C has P_i partial products, nnz_i
  * outputs and a column bound cap_i = min(P_i, columns of C, column span of its
- * products). Rows with P_i <= long_p are computed in one fused pass: one warp
- * per row with a hash table of at most warp_table_max slots (a row with more
- * distinct columns than 4/5 of its table is redone by a block), or one block
- * per row with a bitmap over the column span (span <= mid_cols) or a larger
+ * products). Rows with P_i <= long_p are computed in one fused pass. Warp rows
+ * (P_i <= warp_p_max, cap_i <= warp_cap_max) have a hash table of the size
+ * that fits cap_i, at most warp_table_max; of those, rows of at most 32
+ * products are sorted in registers, rows whose columns span at most 4096 use
+ * a bitmap, and rows whose products hardly share columns, or whose table or
+ * bitmap is full, are handled like the rows outside the warp limits: their
+ * products are sorted in shared memory, or (esc_p_min, esc_span_min) one block
+ * per row takes a bitmap over the column span (span <= mid_cols) or a larger
  * hash table. Rows with P_i > long_p take two passes: a bitmap count, then
  * column-slice blocks (nnz_i > long_o_num), a span bitmap block
  * (nnz_i > mid_o_min) or a block hash table. */
 typedef struct spgemm_tuning {
     int warp_p_max;       /* fused warp path only when P_i <= this */
-    int warp_table_max;   /* largest per-warp hash table: power of two, 64..1024 */
+    int warp_table_max;   /* largest table size of the warp rows: power of two,
+                             64..1024 */
     int warp_cap_max;     /* rows with cap_i above this skip the warp path */
     int long_p;           /* two-pass long path when P_i > this (1..4096) */
     int long_o_num;       /* long rows: column slices when nnz_i > this (1..4096) */
@@ -99,12 +105,12 @@ typedef struct spgemm_tuning {
                              shared-memory accumulation for rows of up to ~38K
                              outputs (longer rows take column slices); 3 = as 2,
                              with the longer rows reduced into C in L2 */
-    int esc_p_min;        /* rows outside the warp bins (column bound above
-                             warp_cap_max) with esc_p_min < P_i <= long_p and a
+    int esc_p_min;        /* rows outside the warp limits, and warp rows better
+                             not hashed, with esc_p_min < P_i <= long_p and a
                              column span above esc_span_min are merged by
-                             sorting their products (one block per row) instead
-                             of the span bitmap / block hash; esc_p_min >=
-                             long_p turns this off */
+                             sorting their products (32 to 512 threads per row)
+                             instead of the span bitmap / block hash;
+                             esc_p_min >= long_p turns this off */
     int esc_span_min;
 } spgemm_tuning;
 
@@ -221,8 +227,9 @@ int spgemm_get_kernel_times(spgemm_handle_t handle, char* names, int names_len,
  * device triplets; type ROW_MAJOR -> CSR (d_ptr[num_rows + 1]), COL_MAJOR ->
  * CSC (d_ptr[num_cols + 1]); d_idx / d_val [nnz]. Minor indices come out
  * ascending within each row (column), entries with equal indices in input
- * order. Counting sort on the major index, then per-row sorts in shared
- * memory (warp, block, or block-merged runs for rows above 8192 entries).
+ * order. Counting sort on the major index, then per-row sorts: in registers
+ * (up to 32 entries), in shared memory by a warp or a block (up to 8192), by
+ * several blocks, or as block-merged runs.
  * Uses handle-owned scratch (about 16 bytes per entry) and synchronises the
  * handle's stream once. An index outside its dimension: SPGEMM_ERR_INVALID
  * (the output then omits those entries). cudaCOO2CM takes this path by
