@@ -234,7 +234,13 @@ constexpr size_t esc_smem_bytes() {
 
 // Rows of P_i <= 2^SH products from the bin list: gather, order by bucket,
 // compress, sorted row written to the temporary buffer at toff[i] with its
-// length in c_cnt[i]. Eight products a thread.
+// length in c_cnt[i]. Eight products a thread. Bound by shared-memory
+// wavefronts (80%) and issue (72%) with 32 threads, by issue and the row's
+// barriers with 512. Against a radix sort by 128 threads and more: 100003 rows
+// of 223 products 666 us (half of the rows), now 231 (all); R-MAT 2^18 rows of
+// 2K to 4K products 1.98 ms, now 0.92; 48 random products of 184 M partials
+// 4.3 ms and 1.8 lost in full hash tables, now 2.2. Eight products a thread:
+// 48 warps an SM then fit both the registers (40) and the shared memory.
 template <int NT, int SH, int MODE, class KEY>
 __global__ void __launch_bounds__(NT * esc_teams<NT>(), 1536 / (NT * esc_teams<NT>()))
 k_fused_esc(Operands op, const int* __restrict__ rows, const int* __restrict__ nrows_p,

@@ -204,9 +204,10 @@ __host__ __device__ inline int overflow_bin_of(long long p, int lo, int span, co
 
 // First-pass list of a row whose bin is `nominal` (first_bin_of): warp-bin
 // rows of at most 32 products are sorted in registers (packed keys hold a
-// 27-bit column offset), those with a narrow span use a bitmap, and spans too
-// wide for the table's packed order (a quarter of 2^26 columns at 64 slots)
-// go where overflowing rows do.
+// 27-bit column offset; one lane a product, so no more fit a warp: 10^6 rows
+// of 9 products 120 us, 837 hashed), those with a narrow span use a bitmap
+// (see BITS_WORDS), and spans too wide for the table's packed order (a quarter
+// of 2^26 columns at 64 slots) go where overflowing rows do.
 __host__ __device__ inline int row_list_of(int nominal, long long p, int lo, int span,
                                            const Tuning& t) {
   if (nominal < 0 || nominal >= FB_WARP_BINS) return nominal;

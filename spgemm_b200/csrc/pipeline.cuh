@@ -49,6 +49,8 @@ __device__ __forceinline__ long long block_excl_scan64(long long v, long long* s
 // the count over all entries (role 1) minus the count over row starts (role
 // 0), so it ends at zero exactly when that holds. Violations of the ranges
 // set ST_BAD_INDEX. Nothing is read outside ptr[0..n_major] and idx[0..nnz).
+// Bound by the histogram's atomics and the reads (R-MAT 2^18: two passes of
+// their own and the histogram 140 us, together 74; 27-point stencil 96^3 137).
 constexpr int CHECK_THREADS = 256;
 
 struct CheckArgs {
@@ -117,7 +119,8 @@ k_check(CheckArgs c, unsigned* status, int* descents) {
 // are) and finds their columns by searching the stretch of column pointers
 // that covers them, kept in shared memory when it fits: searching all of
 // them in global memory took 22 dependent loads an entry (27-point stencil
-// 96^3, 23.6 M entries: 485 us).
+// 96^3, 23.6 M entries: 485 us, now 305). Bound by the returning atomics and
+// the scattered stores.
 constexpr int TR_THREADS = 256;
 constexpr int TR_ENTRIES = 2048;
 constexpr int TR_COLS = 2048;
@@ -189,7 +192,9 @@ constexpr int RA_HEAVY = 1024; // rows of more entries are walked by the whole b
 // row's position, length, first and last column. Rows above RA_HEAVY entries
 // are left for the whole block (a warp took 0.9 ms over the longest row of
 // R-MAT 2^18, 15.9K entries). What follows from a row's totals is computed by
-// one thread per row.
+// one thread per row. Bound by the latency of the loads of b_info, which L2
+// serves (a warp per row: 10^6 rows of 3 entries 361 us, now 68; R-MAT 2^18
+// 1.05 ms, now 0.46; stencil 96^3 380 us, now 238).
 template <int G>
 __global__ void __launch_bounds__(RA_THREADS)
 k_row_analysis(Operands op, const int4* __restrict__ b_info, int rows_per_block,
