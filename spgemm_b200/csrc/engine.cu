@@ -295,6 +295,7 @@ int Engine::analyze(const cm& A, const cm& B) {
   DevCounters* dc = counters_.as<DevCounters>();
   SG_CK(cudaMemsetAsync(dc, 0, row_counts_offset() + (a_csc ? cnt_bytes : 0), stream_),
         "memset counters");
+  row_orders_clean_ = true;
   SG_CK(c_rowptr64_.ensure(sizeof(long long) * ((size_t)m + 1)), "alloc c_rowptr64");
   int* cnt = c_cnt();
 
@@ -847,11 +848,12 @@ int Engine::rows_cnt_max() const {
 // reductions into C above the 1024-thread capacity.
 int Engine::launch_num_rows(int* c_col, float* c_val, int r0, int r1) {
   DevCounters* dc = counters_.as<DevCounters>();
-  if (r0 != 0 || r1 != m_) {  // one of several row ranges: fresh work orders and queues
+  if (!row_orders_clean_) {  // analyze() cleared the counters for one use
     unsigned char* first = reinterpret_cast<unsigned char*>(&dc->lpt_hist);
     unsigned char* last = reinterpret_cast<unsigned char*>(&dc->row_queue) + sizeof(dc->row_queue);
     SG_CK(cudaMemsetAsync(first, 0, (size_t)(last - first), stream_), "reset row orders");
   }
+  row_orders_clean_ = false;
   const int cnt = n_long_sym_;
   const int* rows = sym_rows_.as<int>() + (size_t)FB_LONG * m_;
   SG_CK(lpt_order_.ensure(sizeof(int) * ROWS_LAUNCHES * (size_t)cnt), "alloc row order");

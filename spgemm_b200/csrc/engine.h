@@ -225,6 +225,9 @@ class Engine {
   long long big_capacity_ = 0;
   int n_long_sym_ = 0;
   int tn_run_slice_cap_ = 0;
+  // The whole-row kernels' work orders and queues are zero: every launch of
+  // them (another numeric pass, another row range) starts from zero.
+  bool row_orders_clean_ = false;
   bool have_analysis_ = false;
   Operands op_{};
 
