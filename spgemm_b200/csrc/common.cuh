@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "index_math.h"
+
 namespace sg {
 
 constexpr unsigned FULL = 0xffffffffu;

@@ -300,9 +300,9 @@ int Engine::analyze(const cm& A, const cm& B) {
   int* cnt = c_cnt();
 
   // ---- validate the operands (sync point 1 reports the result) ----
-  // The transpose and row analysis guard every index they use; their findings
-  // and the validation pass's are read at the first synchronisation below,
-  // before any kernel trusts the inputs.
+  // The transpose and row analysis guard every pointer and index they use
+  // (entry_range, b_info); their findings and the validation pass's are read
+  // at the first synchronisation below, before any kernel trusts the inputs.
   {
     SG_CK(b_info_.ensure(sizeof(int4) * (size_t)std::max(kdim_, 1)), "alloc B row table");
     const CheckArgs c{B.ptr, B.idx, A.ptr, A.idx, kdim_, B.nnz, n_, a_csc ? kdim_ : m, nnz_a,
@@ -346,7 +346,7 @@ int Engine::analyze(const cm& A, const cm& B) {
   SG_CK(toff_.ensure(sizeof(long long) * ((size_t)m + 1)), "alloc temp offsets");
   const int vec_ok = ((reinterpret_cast<uintptr_t>(B.idx) | reinterpret_cast<uintptr_t>(B.val)) & 15) == 0;
   op_ = Operands{a_rowptr, a_col, a_val, aoff_.as<int>(), B.ptr, B.idx, B.val, m_, kdim_, n_,
-                 vec_ok, B.nnz};
+                 vec_ok, B.nnz, nnz_a};
   if (m > 0) {
     // lanes per row: about the mean row length; rows per block: enough blocks
     // for the SMs when there are few rows

@@ -57,6 +57,7 @@ struct Operands {
   int m, kdim, n;
   int vec_ok;  // b_col and b_val are 16-byte aligned: 128-bit loads allowed
   int nnz_b;
+  int nnz_a;
 };
 
 // First-pass bins (k_row_analysis). Rows of at most long_p products are

@@ -183,9 +183,9 @@ constexpr int RA_HEAVY = 1024; // rows of more entries are walked by the whole b
 // SCAN_TILE rows. may_overflow[b] counts the warp-bin rows that go to bin b
 // should their table overflow, nominal_count the rows of each bin of
 // first_bin_of, whatever list they are on. Rows are appended to their bin's list with one global
-// atomic per bin per block. A's indices are range-checked here because the
-// validation pass's result is only read after this kernel; b_info holds valid
-// positions only.
+// atomic per bin per block. A's pointers and indices are range-checked here
+// because the validation pass's result is only read after this kernel; b_info
+// holds valid positions only.
 //
 // G lanes walk a row, G about the mean row length of A, so the lanes of a
 // warp are busy on short rows too; one 16-byte load per entry brings the B
@@ -226,6 +226,9 @@ k_row_analysis(Operands op, const int4* __restrict__ b_info, int rows_per_block,
     n_heavy = s_pairs = s_hits = 0;
   }
   __syncthreads();
+  auto row_entries = [&](int lr) {
+    return entry_range(op.a_rowptr[row0 + lr], op.a_rowptr[row0 + lr + 1], op.nnz_a);
+  };
   // B row of A's entry j (an empty one beyond `re` or for an invalid index)
   auto entry = [&](int j, int re) {
     if (j >= re) return make_int4(0, 0, 0, 0);
@@ -293,8 +296,9 @@ k_row_analysis(Operands op, const int4* __restrict__ b_info, int rows_per_block,
     const int lr = lr0 + (int)threadIdx.x / G;
     int rs = 0, re = 0;
     if (lr < nrows) {
-      rs = op.a_rowptr[row0 + lr];
-      re = op.a_rowptr[row0 + lr + 1];
+      const EntryRange e = row_entries(lr);
+      rs = e.begin;
+      re = e.end;
       if (gl == 0 && re > rs) atomicMax(&block_max_len, re - rs);
       if (re - rs > RA_HEAVY) {
         if (gl == 0) heavy[atomicAdd(&n_heavy, 1)] = lr;
@@ -317,7 +321,7 @@ k_row_analysis(Operands op, const int4* __restrict__ b_info, int rows_per_block,
   __syncthreads();
   for (int h = 0; h < n_heavy; ++h) {  // each warp a stretch of the row: sums, then offsets
     const int lr = heavy[h];
-    const int rs = op.a_rowptr[row0 + lr], re = op.a_rowptr[row0 + lr + 1];
+    const auto [rs, re] = row_entries(lr);
     const int per = ((re - rs + NW - 1) / NW + 31) & ~31;
     const int j0 = min(rs + warp * per, re), j1 = min(j0 + per, re);
     long long sum = 0;
@@ -393,7 +397,7 @@ k_row_analysis(Operands op, const int4* __restrict__ b_info, int rows_per_block,
     const unsigned at = __ballot_sync(
         FULL, ((mask >> lane) & 1u) && __popc(mask & ((1u << lane) - 1u)) == nth);
     const int lr = (idx < n0 ? 0 : 32) + __ffs(at) - 1;
-    const int rs = op.a_rowptr[row0 + lr], re = op.a_rowptr[row0 + lr + 1];
+    const auto [rs, re] = row_entries(lr);
     const int4 f = entry(rs + lane, re);
     const int next = __shfl_down_sync(FULL, f.x, 1), next_len = __shfl_down_sync(FULL, f.y, 1);
     const bool pair = lane < 31 && f.y > 0 && next_len > 0;

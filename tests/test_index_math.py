@@ -1,0 +1,33 @@
+"""csrc/index_math.h on the host: the kernels' index arithmetic at the ends of
+the int32 range, where no test would allocate the arrays, and on pointers that
+no kernel may follow."""
+import subprocess
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parents[1] / "spgemm_b200" / "csrc"
+
+
+def run_cpp(tmp_path, body):
+    src = tmp_path / "check.cpp"
+    src.write_text('#include <cstdio>\n#include "index_math.h"\nusing namespace sg;\n' + body)
+    exe = tmp_path / "check"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fsanitize=undefined", "-fno-sanitize-recover=all",
+                    f"-I{CSRC}", str(src), "-o", str(exe)], check=True)
+    return subprocess.run([str(exe)], capture_output=True, text=True, check=True).stdout.split()
+
+
+@pytest.mark.parametrize("nnz", [0, 1, 100, 2 ** 31 - 1])
+def test_entry_ranges_stay_inside_the_arrays(tmp_path, nnz):
+    ends = [-2 ** 31, -2 ** 31 + 1, -7, -1, 0, 1, 2, 50, 99, 100, 101, 2 ** 30, 2 ** 31 - 2, 2 ** 31 - 1]
+    lit = ", ".join(f"(int)({v}ll)" for v in ends)
+    out = run_cpp(tmp_path, f"""int main() {{
+  const int v[] = {{{lit}}};
+  for (int s : v) for (int e : v) {{ EntryRange r = entry_range(s, e, {nnz}); std::printf("%d %d ", r.begin, r.end); }}
+}}""")
+    got = [(int(out[i]), int(out[i + 1])) for i in range(0, len(out), 2)]
+    for (s, e), (b, t) in zip([(s, e) for s in ends for e in ends], got):
+        assert 0 <= b <= t <= nnz, (s, e, b, t)
+        if 0 <= s <= e <= nnz:
+            assert (b, t) == (s, e)
