@@ -69,11 +69,7 @@ __device__ __forceinline__ float two_sum_err(float a, float b, float s) {
 // Lower bound of `key` in the sorted array v[lo, hi).
 __device__ __forceinline__ int lower_bound_i32(const int* __restrict__ v, int lo,
                                                int hi, int key) {
-  while (lo < hi) {
-    int mid = (lo + hi) >> 1;
-    if (__ldg(v + mid) < key) lo = mid + 1; else hi = mid;
-  }
-  return lo;
+  return lower_bound_at(lo, hi, key, [&](int p) { return __ldg(v + p); });
 }
 
 }  // namespace sg

@@ -23,4 +23,15 @@ SG_HOST_DEVICE EntryRange entry_range(int begin, int end, int nnz) {
   return EntryRange{b, e};
 }
 
+// First position of [lo, hi) whose value at(position) is not below `key` (at
+// rises); positions may lie anywhere in the int32 range.
+template <class At>
+SG_HOST_DEVICE int lower_bound_at(int lo, int hi, int key, At at) {
+  while (lo < hi) {
+    const int mid = lo + ((hi - lo) >> 1);
+    if (at(mid) < key) lo = mid + 1; else hi = mid;
+  }
+  return lo;
+}
+
 }  // namespace sg

@@ -31,3 +31,22 @@ def test_entry_ranges_stay_inside_the_arrays(tmp_path, nnz):
         assert 0 <= b <= t <= nnz, (s, e, b, t)
         if 0 <= s <= e <= nnz:
             assert (b, t) == (s, e)
+
+
+@pytest.mark.parametrize("lo,hi", [(0, 0), (0, 1), (5, 1000), (2 ** 30 - 3, 2 ** 30 + 900), (0, 2 ** 31 - 1),
+                                   (2 ** 30 + 1, 2 ** 31 - 1), (2 ** 31 - 40, 2 ** 31 - 1)])
+def test_lower_bound_at_any_position(tmp_path, lo, hi):
+    """A row of B may begin anywhere below 2^31: lo + hi must not wrap. The
+    value at position p is (p - lo) / 2, every value twice."""
+    keys = sorted({0, 1, 2, (hi - lo) // 4, (hi - lo) // 2, max((hi - lo) // 2 - 1, 0), (hi - lo) // 2 + 1})
+    out = run_cpp(tmp_path, f"""int main() {{
+  const int lo = {lo}, hi = {hi}, keys[] = {{{', '.join(map(str, keys))}}};
+  for (int key : keys) {{
+    bool inside = true;
+    const int r = lower_bound_at(lo, hi, key, [&](int p) {{ inside &= p >= lo && p < hi; return (p - lo) / 2; }});
+    std::printf("%d %d ", r, (int)inside);
+  }}
+}}""")
+    for k, key in enumerate(keys):
+        assert out[2 * k + 1] == "1", key
+        assert int(out[2 * k]) == min(lo + 2 * key, hi), key
