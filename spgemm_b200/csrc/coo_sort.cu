@@ -117,11 +117,11 @@ static_assert(CS_HIST_SLOTS == 1 << 14, "the hash keeps 14 bits");
 __global__ void k_cs_scatter(const triplet* __restrict__ t, int nnz, int row_major, int n_major,
                              int n_minor, const int* __restrict__ ptr, const int* __restrict__ rank,
                              unsigned long long* __restrict__ keys) {
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += gridDim.x * blockDim.x) {
+  strided(blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, nnz, [&](int e) {
     int major, minor;
-    if (!cs_entry(t[e], row_major, n_major, n_minor, major, minor)) continue;
+    if (!cs_entry(t[e], row_major, n_major, n_minor, major, minor)) return;
     keys[__ldg(ptr + major) + rank[e]] = ((unsigned long long)(unsigned)minor << 32) | (unsigned)e;
-  }
+  });
 }
 
 __global__ void __launch_bounds__(256)
@@ -519,7 +519,7 @@ cudaError_t coo_compress(const triplet* t, int nnz, bool row_major, int n_major,
     if ((e = cudaFuncSetAttribute(k_cs_hist, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)smem)) != cudaSuccess)
       return e;
-    k_cs_hist<<<(nnz - 1) / (CS_THREADS * items) + 1, CS_THREADS, smem, s>>>(
+    k_cs_hist<<<blocks_over(nnz, CS_THREADS * items), CS_THREADS, smem, s>>>(
         t, nnz, items, row_major ? 1 : 0, n_major, n_minor, cnt, rank, cc);
   }
   if ((e = scan_counts_to_ptr32(cnt, n_major, ptr, scan_tmp, &cc->total, s)) != cudaSuccess)
@@ -527,7 +527,7 @@ cudaError_t coo_compress(const triplet* t, int nnz, bool row_major, int n_major,
   if (nnz > 0 && n_major > 0) {
     k_cs_scatter<<<grid_for(nnz, 256, 4096), 256, 0, s>>>(t, nnz, row_major ? 1 : 0, n_major,
                                                           n_minor, ptr, rank, keys);
-    k_cs_bins<<<(n_major - 1) / 256 + 1, 256, 0, s>>>(cnt, n_major, lists, cc);
+    k_cs_bins<<<blocks_over(n_major, 256), 256, 0, s>>>(cnt, n_major, lists, cc);
     const CsOut out{t, idx, val};
     if ((e = sort_class<1024, 8192, 4096>(5, 2048, nnz, 296, ptr, lists, n_major, cc, keys, out, s)) != cudaSuccess)
       return e;

@@ -225,7 +225,7 @@ int Engine::check_status(const DevCounters& c) {
 }
 
 int Engine::scan_counts(const int* in, int n, long long* tiles, const ScanOut& out) {
-  const int ntiles = std::max((n + SCAN_TILE - 1) / SCAN_TILE, 1);
+  const int ntiles = std::max(blocks_over(n, SCAN_TILE), 1);
   if (!tiles) {
     SG_CK(tiles_.ensure(sizeof(long long) * (size_t)ntiles), "alloc scan tiles");
     tiles = tiles_.as<long long>();
@@ -249,7 +249,7 @@ int Engine::scan_counts(const int* in, int n, long long* tiles, const ScanOut& o
 }
 
 size_t Engine::row_counts_offset() const {
-  const size_t tiles = (size_t)(m_ + SCAN_TILE - 1) / SCAN_TILE + 1;
+  const size_t tiles = (size_t)blocks_over(m_, SCAN_TILE) + 1;
   return ROW_TILES_OFFSET + (sizeof(long long) * tiles + 15) / 16 * 16;
 }
 
@@ -327,7 +327,7 @@ int Engine::analyze(const cm& A, const cm& B) {
       return r;
     if (nnz_a > 0) {
       prof_begin("k_transpose_scatter");
-      k_transpose_scatter<<<(nnz_a - 1) / TR_ENTRIES + 1, TR_THREADS, 0, stream_>>>(
+      k_transpose_scatter<<<blocks_over(nnz_a, TR_ENTRIES), TR_THREADS, 0, stream_>>>(
           A.ptr, A.idx, A.val, kdim_, nnz_a, m, cursor_.as<int>(), a_col_.as<int>(),
           a_val_.as<float>());
       SG_LAUNCHED("k_transpose_scatter");
@@ -353,7 +353,7 @@ int Engine::analyze(const cm& A, const cm& B) {
     const long long mean = nnz_a / m;
     const int g = mean <= 4 ? 4 : (mean <= 8 ? 8 : (mean <= 16 ? 16 : 32));
     const int rpb = m >= 2 * RA_ROWS * sms_ ? RA_ROWS : RA_THREADS / g;
-    const int blocks = (m + rpb - 1) / rpb;
+    const int blocks = blocks_over(m, rpb);
     SG_CK(route_.ensure((size_t)blocks), "alloc row routes");
     auto launch = [&](auto kernel) {
       kernel<<<blocks, RA_THREADS, 0, stream_>>>(
@@ -950,7 +950,7 @@ int Engine::multiply_numeric_owned(cm* C_dev) {
 
 cudaError_t scan_counts_to_ptr32(const int* cnt, int n, int* ptr, DevBuf& tmp,
                                  long long* total_dev, cudaStream_t s) {
-  const int ntiles = std::max((n + SCAN_TILE - 1) / SCAN_TILE, 1);
+  const int ntiles = std::max(blocks_over(n, SCAN_TILE), 1);
   cudaError_t e = tmp.ensure(sizeof(long long) * (size_t)ntiles);
   if (e != cudaSuccess) return e;
   long long* tiles = tmp.as<long long>();

@@ -34,4 +34,18 @@ SG_HOST_DEVICE int lower_bound_at(int lo, int hi, int key, At at) {
   return lo;
 }
 
+// f(p) for p = first, first + stride, ... below n; p stays in range where an
+// int counter would wrap at the last step (n near 2^31).
+template <class F>
+SG_HOST_DEVICE void strided(long long first, long long stride, long long n, F f) {
+  for (long long p = first; p < n; p += stride) f((int)p);
+}
+
+// Blocks of `per` items that cover n, and the end of the block that begins at
+// item `begin` (< n).
+SG_HOST_DEVICE int blocks_over(int n, int per) { return n > 0 ? (n - 1) / per + 1 : 0; }
+SG_HOST_DEVICE int block_end(int begin, int per, int n) {
+  return n - begin < per ? n : begin + per;
+}
+
 }  // namespace sg

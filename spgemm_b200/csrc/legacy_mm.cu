@@ -54,13 +54,13 @@ __global__ void k_coo_split(const triplet* __restrict__ t, int nnz, bool row_maj
                             int n_major, int n_minor, int* __restrict__ cnt,
                             int* __restrict__ idx, float* __restrict__ val,
                             unsigned* __restrict__ flags) {
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += gridDim.x * blockDim.x) {
+  sg::strided(blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, nnz, [&](int e) {
     const triplet x = t[e];
     const int major = row_major ? x.ridx : x.cidx;
     const int minor = row_major ? x.cidx : x.ridx;
     if ((unsigned)major >= (unsigned)n_major || (unsigned)minor >= (unsigned)n_minor) {
       atomicOr(flags, 1u);
-      continue;
+      return;
     }
     if (e > 0) {
       const triplet y = t[e - 1];
@@ -71,7 +71,7 @@ __global__ void k_coo_split(const triplet* __restrict__ t, int nnz, bool row_maj
     idx[e] = minor;
     val[e] = x.val;
     atomicAdd(cnt + major, 1);
-  }
+  });
 }
 
 __global__ void k_count_above(const float* __restrict__ v, long long n, float thr,

@@ -21,6 +21,7 @@
 
 #include "../../include/coo.h"
 #include "../../include/spgemm_b200.h"
+#include "index_math.h"
 
 namespace {
 
@@ -75,13 +76,13 @@ __device__ __forceinline__ long long na_block_excl(long long v, long long* shm, 
 __global__ void na_split(const triplet* __restrict__ t, int nnz, int row_major, int n_major,
                          int n_minor, int* __restrict__ ptr, int* __restrict__ idx,
                          float* __restrict__ val, long long* scratch) {
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += gridDim.x * blockDim.x) {
+  sg::strided(blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, nnz, [&](int e) {
     const triplet x = t[e];
     const int major = row_major ? x.ridx : x.cidx;
     const int minor = row_major ? x.cidx : x.ridx;
     if ((unsigned)major >= (unsigned)n_major || (unsigned)minor >= (unsigned)n_minor) {
       atomicOr(reinterpret_cast<unsigned long long*>(scratch + NA_STATUS), 1ull);
-      continue;
+      return;
     }
     if (e > 0) {
       const triplet y = t[e - 1];
@@ -93,7 +94,7 @@ __global__ void na_split(const triplet* __restrict__ t, int nnz, int row_major, 
     idx[e] = minor;
     val[e] = x.val;
     atomicAdd(ptr + major + 1, 1);
-  }
+  });
 }
 
 // Tile sums of ptr[0..n) (n = n_major + 1 counts; ptr[0] is 0).

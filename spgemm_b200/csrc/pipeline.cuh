@@ -73,7 +73,7 @@ k_check(CheckArgs c, unsigned* status, int* descents) {
   bool bad = false;
   int net = 0;
   if (blockIdx.y == 0) {
-    for (int i = t0; i <= c.b_rows; i += stride) {
+    strided(t0, stride, c.b_rows + 1ll, [&](int i) {
       const int s = c.b_ptr[i];
       const bool ok = pointer_ok(c.b_ptr, i, c.b_rows, c.b_nnz, s);
       bad |= !ok;
@@ -86,23 +86,23 @@ k_check(CheckArgs c, unsigned* status, int* descents) {
         }
         c.b_info[i] = info;
       }
-    }
+    });
   } else if (blockIdx.y == 1) {
-    for (int q = t0; q < c.b_nnz; q += stride) {
+    strided(t0, stride, c.b_nnz, [&](int q) {
       const int v = c.b_idx[q];
       bad |= (unsigned)v >= (unsigned)c.n;
       if (q > 0 && c.b_idx[q - 1] >= v) ++net;
-    }
+    });
   } else if (blockIdx.y == 2) {
-    for (int i = t0; i <= c.a_major; i += stride)
-      bad |= !pointer_ok(c.a_ptr, i, c.a_major, c.a_nnz, c.a_ptr[i]);
+    strided(t0, stride, c.a_major + 1ll,
+            [&](int i) { bad |= !pointer_ok(c.a_ptr, i, c.a_major, c.a_nnz, c.a_ptr[i]); });
   } else {
-    for (int q = t0; q < c.a_nnz; q += stride) {
+    strided(t0, stride, c.a_nnz, [&](int q) {
       const int v = c.a_idx[q];
       const bool ok = (unsigned)v < (unsigned)c.a_minor;
       bad |= !ok;
       if (c.hist && ok) atomicAdd(c.hist + v, 1);
-    }
+    });
   }
   if (bad) atomicOr(status, ST_BAD_INDEX);
   net = warp_sum(net);
@@ -134,7 +134,7 @@ k_transpose_scatter(const int* __restrict__ colptr,
                     float* __restrict__ out_val) {
   __shared__ int sptr[TR_COLS];
   __shared__ int edge[2];
-  const int e0 = blockIdx.x * TR_ENTRIES, e1 = min(nnz, e0 + TR_ENTRIES);
+  const int e0 = blockIdx.x * TR_ENTRIES, e1 = block_end(e0, TR_ENTRIES, nnz);
   // last k in [lo, hi] with p(k) <= e (p(lo) <= e)
   auto search = [](auto p, int lo, int hi, int e) {
     while (lo < hi) {

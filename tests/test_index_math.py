@@ -50,3 +50,30 @@ def test_lower_bound_at_any_position(tmp_path, lo, hi):
     for k, key in enumerate(keys):
         assert out[2 * k + 1] == "1", key
         assert int(out[2 * k]) == min(lo + 2 * key, hi), key
+
+
+LAST = 2 ** 31 - 1
+
+
+@pytest.mark.parametrize("n", [0, 1, 255, 256, 257, LAST - 606208, LAST - 1, LAST, LAST + 1])
+@pytest.mark.parametrize("first,stride", [(0, 606208), (606207, 606208), (77, 1 << 20)])
+def test_strided_walk_ends(tmp_path, first, stride, n):
+    """The walk over an array of n entries, or n - 1 rows and their last
+    pointer, meets each position once and stops."""
+    out = run_cpp(tmp_path, f"""int main() {{
+  long long count = 0, bad = 0; int last = -1;
+  strided({first}, {stride}, {n}ll, [&](int p) {{ bad += p < 0 || p >= {n}ll || p % {stride} != {first} % {stride}; ++count; last = p; }});
+  std::printf("%lld %lld %d", count, bad, last);
+}}""")
+    count = len(range(first, n, stride))
+    assert out == [str(count), "0", str(range(first, n, stride)[-1] if count else -1)]
+
+
+@pytest.mark.parametrize("per", [32, 256, 2048, 4096])
+@pytest.mark.parametrize("n", [0, 1, 31, 2048, 2049, LAST - 2048, LAST - 1, LAST])
+def test_blocks_cover_their_items(tmp_path, per, n):
+    out = run_cpp(tmp_path, f"""int main() {{
+  const int b = blocks_over({n}, {per});
+  std::printf("%d %d %d", b, b ? block_end(0, {per}, {n}) : 0, b ? block_end((b - 1) * {per}, {per}, {n}) : 0);
+}}""")
+    assert out == [str(-(-n // per)), str(min(per, n)), str(n)]
