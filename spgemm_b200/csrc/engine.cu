@@ -295,7 +295,7 @@ int Engine::analyze(const cm& A, const cm& B) {
   DevCounters* dc = counters_.as<DevCounters>();
   SG_CK(cudaMemsetAsync(dc, 0, row_counts_offset() + (a_csc ? cnt_bytes : 0), stream_),
         "memset counters");
-  row_orders_clean_ = true;
+  row_orders_clean_ = sym_counters_clean_ = true;
   SG_CK(c_rowptr64_.ensure(sizeof(long long) * ((size_t)m + 1)), "alloc c_rowptr64");
   int* cnt = c_cnt();
 
@@ -399,6 +399,17 @@ int Engine::symbolic_pass(long long* nnz_c) {
   have_sym_ = false;
   const int m = m_;
   DevCounters* dc = counters_.as<DevCounters>();
+  if (!sym_counters_clean_) {
+    // this analysis's symbolic pass again: the lists and counts as analyze()
+    // left them, without the overflowing rows and slices of the pass before
+    SG_CK(cudaMemcpyAsync(dc->fb_count, fb_counts_, sizeof(fb_counts_), cudaMemcpyHostToDevice, stream_),
+          "reset row lists");
+    SG_CK(cudaMemsetAsync(dc->num_count, 0, offsetof(DevCounters, status) - offsetof(DevCounters, num_count),
+                          stream_),
+          "reset numeric bins");
+    SG_CK(cudaMemsetAsync(&dc->overflow_count, 0, sizeof(int), stream_), "reset overflow count");
+  }
+  sym_counters_clean_ = false;
 
   // ---- first pass: fused rows to the temporary buffer, long rows counted ----
   SG_CK(t_col_.ensure(sizeof(int) * (size_t)std::max(temp_total_, 1ll)), "alloc temp columns");

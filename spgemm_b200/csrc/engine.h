@@ -228,6 +228,8 @@ class Engine {
   // The whole-row kernels' work orders and queues are zero: every launch of
   // them (another numeric pass, another row range) starts from zero.
   bool row_orders_clean_ = false;
+  // The symbolic pass's counters are as analyze() left them.
+  bool sym_counters_clean_ = false;
   bool have_analysis_ = false;
   Operands op_{};
 

@@ -1,5 +1,7 @@
 """Calls repeated on one handle within a product: what one call leaves behind
 must not reach the next one's result."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -7,6 +9,7 @@ import spgemm_b200 as sg
 from spgemm_b200 import workloads as W
 from helpers import assert_structure_equal, assert_values_close, compensated_tolerance, plain_tolerance
 from test_gpu_batch import DeviceBatch, ref_product
+from test_gpu_legacy import _coo_of
 
 pytestmark = pytest.mark.gpu
 
@@ -53,3 +56,57 @@ def test_host_call_with_empty_row_ranges():
             C = h.multiply_host(A, A)
             assert_structure_equal(C.rowptr, C.col, ref["rowptr"], ref["col"])
             assert_values_close(C.val, ref, plain_tolerance(ref))
+
+
+def overflowing(m=600, n=40_000, seed=8):
+    """Rows of about 400 distinct columns, each product's column met about
+    three times (so the rows are hashed, and overflow the table), with some
+    long rows."""
+    rng = np.random.default_rng(seed)
+    groups = [np.sort(rng.choice(n, 20, replace=False)) for _ in range(200)]
+    B = W.from_coo(600, n, np.repeat(np.arange(600), 20), np.concatenate([groups[k // 3] for k in range(600)]),
+                   rng.uniform(-1, 1, 12000).astype(np.float32))
+    r, c = [], []
+    for i in range(m):
+        g = np.arange(200) if i % 50 == 0 else np.sort(rng.choice(200, 20, replace=False))
+        r += [i] * (3 * len(g))
+        c += np.sort(np.concatenate([3 * g, 3 * g + 1, 3 * g + 2])).tolist()
+    return W.from_coo(m, 600, np.array(r), np.array(c), rng.uniform(-1, 1, len(r)).astype(np.float32)), B
+
+
+@pytest.mark.parametrize("operands", ["overflowing", "rmat"])
+def test_symbolic_pass_again_after_one_analysis(operands):
+    """mm.h: cudaBinGEMM (or cudaSimpleGEMM) again after one cudaInitGEMM, and
+    cudaMergeGEMM again, leave the same C as one call of each."""
+    L = sg.lib()
+    L.spgemm_set_verbose(0)
+    L.spgemm_set_exit_on_error(0)
+    try:
+        A, B = overflowing() if operands == "overflowing" else (W.rmat(12, 12, 8, values="sym"),) * 2
+        ref = ref_product(A, B)
+        if operands == "overflowing":
+            with sg.Handle() as h:
+                h.multiply_host(A, B)
+                assert h.stats()["warp_overflow_rows"] > 400
+        ta, tb = _coo_of(A, True), _coo_of(B, False)
+        Ah = L.cudaCOO2CM(sg.COO(C.cast(ta, C.POINTER(sg.Triplet)), A.nnz, A.cols, A.rows, sg.COL_MAJOR))
+        Bh = L.cudaCOO2CM(sg.COO(C.cast(tb, C.POINTER(sg.Triplet)), B.nnz, B.cols, B.rows, sg.ROW_MAJOR))
+        Cm = L.cudaInitGEMM(Ah, Bh)
+        for again in range(4):
+            (L.cudaSimpleGEMM if again == 2 else L.cudaBinGEMM)(Ah, Bh, Cm)
+            assert L.spgemm_legacy_status() == 0
+            for _ in range(1 + again % 2):
+                L.cudaMergeGEMM(Cm)
+                assert L.spgemm_legacy_status() == 0
+                R = sg.CM()
+                assert L.spgemm_get_result(C.byref(R)) == 0
+                got = [np.ctypeslib.as_array(p, (k,)).copy()
+                       for p, k in ((R.ptr, R.num_rows + 1), (R.idx, R.nnz), (R.val, R.nnz))]
+                L.cmFree(C.byref(R))
+                assert_structure_equal(got[0], got[1], ref["rowptr"], ref["col"])
+                assert_values_close(got[2], ref, plain_tolerance(ref))
+        for M in (Ah, Bh):
+            L.cmFree(C.byref(M))
+    finally:
+        L.spgemm_set_verbose(1)
+        L.spgemm_set_exit_on_error(1)
