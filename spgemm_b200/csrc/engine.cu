@@ -564,22 +564,27 @@ int Engine::launch_fused() {
                                     &dc->overflow_count);
     SG_LAUNCHED("k_fused_bits");
   }
-#define SG_FUSED_WARP(B)                                                                      \
-  if (const int cnt = fb_counts_[B]) {                                                         \
-    constexpr int L = hash_slots_log2(B);                                                      \
-    const size_t smem = WPB * hash_warp_bytes<L, MODE>();                                      \
-    SG_CK((smem_attr(k_fused_warp<L, MODE>, smem)), "smem attr k_fused_warp");                 \
+#define SG_FUSED_WARP(NAME, BIN, LIST, L, G)                                                  \
+  if (const int cnt = fb_counts_[BIN]) {                                                       \
+    const size_t smem = WPB * hash_warp_bytes<L, G, MODE>();                                   \
+    SG_CK((smem_attr(k_fused_warp<L, G, MODE>, smem)), "smem attr k_fused_warp");              \
     /* rows in a stretch: enough stretches for the warps that the GPU holds */                 \
     const int stretch = std::max(1, std::min(HASH_ROWS, cnt / (sms_ * 40)));                   \
-    prof_begin("k_fused_warp<" #B ">");                                                        \
-    k_fused_warp<L, MODE><<<blocks_for(cnt, WPB * stretch, (long long)sms_ * 64),              \
-                            HASH_THREADS, smem, stream_>>>(                                    \
-        op, rows + (size_t)B * m, cnt, stretch, row_span_.as<int2>(),                          \
-                                       toff, c_cnt, t_col, t_val, rows, dc->fb_count, tn_,     \
-                                       row_p, &dc->overflow_count);                            \
+    prof_begin(NAME);                                                                          \
+    k_fused_warp<L, G, MODE><<<blocks_for(cnt, WPB * stretch, (long long)sms_ * 64),           \
+                               HASH_THREADS, smem, stream_>>>(                                 \
+        op, LIST, cnt, stretch, row_span_.as<int2>(), toff, c_cnt, t_col, t_val, rows,         \
+        dc->fb_count, tn_, row_p, &dc->overflow_count);                                        \
     SG_LAUNCHED("k_fused_warp");                                                               \
   }
-  SG_FUSED_WARP(0) SG_FUSED_WARP(1) SG_FUSED_WARP(2) SG_FUSED_WARP(3) SG_FUSED_WARP(4)
+#define SG_FUSED_GROUPS(B) \
+  SG_FUSED_WARP("k_fused_warp<" #B ">", B, rows + (size_t)(B) * m, hash_slots_log2(B), (group_cols(MODE, B)))
+#define SG_FUSED_COLS(B) \
+  SG_FUSED_WARP("k_fused_cols<" #B ">", FB_COLS2 + B - 2, shared_list(FB_COLS2 + B - 2), cols_slots_log2(B), 1)
+  SG_FUSED_GROUPS(0) SG_FUSED_GROUPS(1) SG_FUSED_GROUPS(2) SG_FUSED_GROUPS(3) SG_FUSED_GROUPS(4)
+  SG_FUSED_COLS(2) SG_FUSED_COLS(3) SG_FUSED_COLS(4)
+#undef SG_FUSED_COLS
+#undef SG_FUSED_GROUPS
 #undef SG_FUSED_WARP
   // mid bitmap rows (and warp overflow with a narrow span)
   if (fb_counts_[FB_MID] + may_overflow_[FB_MID] > 0) {

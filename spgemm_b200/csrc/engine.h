@@ -238,7 +238,7 @@ class Engine {
   DevBuf sym_rows_, num_rows_, long_slot_, chunk_cnt_, slices_buf_, mid_slices_, row_span_;
   DevBuf tcap_, toff_, t_col_, t_val_;  // fused pass: row bounds, temp offsets, temp output
   DevBuf counters_, restrict_scratch_, bitmaps_, lpt_order_;
-  DevBuf route_;   // byte per block of row analysis: its rows repeat columns (hashed, not sorted)
+  DevBuf route_;   // byte per block of row analysis: ROUTE_* answers of its sample
   DevBuf b_info_;  // int4 per row of B: position, length, first and last column
   int bitmap_words_ = 0;  // per long row; 0 when the bitmaps are not kept
   int max_row_len_ = 0;

@@ -62,8 +62,9 @@ struct Operands {
 
 // First-pass bins (k_row_analysis). Rows of at most long_p products are
 // computed in one fused pass (sorted output into a temporary buffer):
-//   0..4  one warp per row, hash table of 2^6..2^10 slots (optimistic: a row
-//         with more distinct columns than 4/5 of the table is redone below)
+//   0..4  one warp per row, hash table of 64, 128, 128, 256, 512 slots of a
+//         group of neighbouring columns (optimistic: a row that needs more
+//         than 4/5 of the slots is redone below)
 //   5..7  one block per row, hash table of 2^11..2^13 slots
 //   8     one block per row, bitmap over the row's column span ("mid")
 // Rows with more products take the two-phase long path:
@@ -78,6 +79,8 @@ struct Operands {
 //   15..17 rows of at most 8 / 16 / 32 products, sorted in registers
 //         (k_fused_tiny)
 //   18    rows whose span fits a warp's bitmap (k_fused_bits)
+// or take a table of the same bytes with one column a slot:
+//   19..21 rows of bins 2..4 whose columns lie apart, 256, 512, 1024 slots
 // and count as the warp bin of their column bound in the statistics.
 constexpr int FB_WARP_BINS = 5;
 constexpr int FB_BLOCK0 = 5;
@@ -87,7 +90,8 @@ constexpr int FB_ESC0 = 10;
 constexpr int FB_ESC256 = 13, FB_ESC512 = 14;
 constexpr int FB_TINY8 = 15, FB_TINY16 = 16, FB_TINY32 = 17;
 constexpr int FB_BITS = 18;
-constexpr int FB_COUNT = 19;
+constexpr int FB_COLS2 = 19;  // .. FB_COLS2 + 2
+constexpr int FB_COUNT = 22;
 constexpr int FB_LISTS = 15;  // row lists of m entries; see fb_list_at
 constexpr int FB_STAT_COUNT = 13;  // bins of the statistics
 // Numeric bins of long rows: 4..7 block hash (2^10..2^13 slots), 8 column
@@ -187,12 +191,27 @@ constexpr int BITS_OUT_MAX = 2 * BITS_CAP;
 // 32-column words from the word of column lo to the end of the span.
 __host__ __device__ inline int span_words(int lo, int span) { return ((lo & 31) + span + 31) >> 5; }
 
-// Slots (of four columns) of the hash table of warp bin b.
+// log2 of the slots of warp bin b's hash table when a slot holds a group of
+// neighbouring columns, and (bins 2.., the rows of list FB_COLS2 + b - 2) when
+// it holds one.
 __host__ __device__ constexpr int hash_slots_log2(int b) { return b < 2 ? 6 + b : 5 + b; }
+__host__ __device__ constexpr int cols_slots_log2(int b) { return 6 + b; }
 
-// Whether a warp-bin row may need more slots than its table gives.
-__host__ __device__ inline bool hash_may_overflow(int b, long long cap) {
-  return cap > (1 << hash_slots_log2(b)) * 4 / 5;
+// Columns of a group: four, but two in the larger tables of compensated
+// values, where four of eight bytes leave an SM 20 and 8 warps (27-point
+// stencil 61^3 with tables up to 512: 1.55 ms, now 1.19; 1024: 2.82, 1.82).
+constexpr int group_cols(int mode, int b) { return mode == 1 && b >= 3 ? 2 : 4; }
+
+// Whether a row of hash list `bin` may need more slots than its table gives.
+__host__ __device__ inline bool hash_may_overflow(int bin, long long cap) {
+  const int lg = bin < FB_WARP_BINS ? hash_slots_log2(bin) : cols_slots_log2(bin - FB_COLS2 + 2);
+  return cap > (1 << lg) * 4 / 5;
+}
+
+// Whether a row of warp bin `b` may take the table of single columns (the
+// columns must fit the packed order, as in row_list_of).
+__host__ __device__ inline bool cols_table_takes(int b, int span) {
+  return b >= 2 && b < FB_WARP_BINS && span + 2 < 1 << (32 - cols_slots_log2(b));
 }
 
 // Where a warp-bin row whose table overflows is redone: the sorted bins when

@@ -174,6 +174,10 @@ constexpr int RA_ROWS = 64;    // most rows per block
 constexpr int RA_UNROLL = 4;   // batches of a row in flight together
 constexpr int RA_HEAVY = 1024; // rows of more entries are walked by the whole block
 
+// What the sample of a block of row analysis found (bits of its route byte).
+constexpr int ROUTE_REPEATS = 1;  // products share columns: hash rather than sort
+constexpr int ROUTE_RUNS = 2;     // columns come in runs: several to a slot
+
 // Per row i: P_i = sum over A(i,k) of nnz(B(k,:)) (the intermediate product
 // count the reference accumulates per row in initGEMM, src/mm.cu:138-148),
 // the flattened offset of each A entry, the column span of the row's
@@ -213,7 +217,7 @@ k_row_analysis(Operands op, const int4* __restrict__ b_info, int rows_per_block,
   __shared__ long long part_p[NW];
   __shared__ int part_lo[NW], part_hi[NW];
   __shared__ unsigned cand[2];
-  __shared__ int s_pairs, s_hits;
+  __shared__ int s_pairs, s_hits, s_steps, s_next;
   __shared__ unsigned long long block_p, block_cap;
   __shared__ int block_max_len;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gl = lane & (G - 1);
@@ -223,7 +227,7 @@ k_row_analysis(Operands op, const int4* __restrict__ b_info, int rows_per_block,
   if (threadIdx.x == 0) {
     block_p = block_cap = 0;
     block_max_len = 0;
-    n_heavy = s_pairs = s_hits = 0;
+    n_heavy = s_pairs = s_hits = s_steps = s_next = 0;
   }
   __syncthreads();
   auto row_entries = [&](int lr) {
@@ -361,7 +365,7 @@ k_row_analysis(Operands op, const int4* __restrict__ b_info, int rows_per_block,
     __syncthreads();
   }
   // bins, one thread per row (two whole warps); hashed rows that could be
-  // sorted instead are candidates
+  // sorted, or hashed by single columns, are candidates
   int bin = -1, bin0 = -1, rank = 0, lo = 0, span = 0;
   long long acc = 0, cap = 0;
   bool candidate = false;
@@ -374,7 +378,8 @@ k_row_analysis(Operands op, const int4* __restrict__ b_info, int rows_per_block,
       cap = row_cap(acc, op.n, span);
       bin0 = first_bin_of(acc, cap, span, tn);
       bin = row_list_of(bin0, acc, lo, span, tn);
-      candidate = bin >= 0 && bin < FB_WARP_BINS && overflow_bin_of(acc, lo, span, tn) >= FB_ESC0;
+      candidate = bin >= 0 && bin < FB_WARP_BINS &&
+                  (overflow_bin_of(acc, lo, span, tn) >= FB_ESC0 || cols_table_takes(bin, span));
     }
     const unsigned c = __ballot_sync(FULL, candidate);
     if (lane == 0) cand[warp] = c;
@@ -386,7 +391,12 @@ k_row_analysis(Operands op, const int4* __restrict__ b_info, int rows_per_block,
   // 2 of 3 pairs, any order of the entries: 1 of 2), rows of random graphs
   // hardly. Rows that do not repeat columns fill a hash table for nothing
   // (random rows of 200 products: 4.6 ns each hashed, 3.4 sorted).
-  // The answer depends on the order of A's entries, which the transpose leaves
+  // And do its columns come in runs? Is the column after one of the B row's
+  // (another place for each lane) its neighbour? Grids: 2 of 3; two unknowns a
+  // point: 1 of 2 or more; points in any order: hardly. The line at a sixth
+  // (points in cell order, 0.4 to 0.5, k = 30 nearest of 150000: grouped 1.16
+  // ms, single columns 1.50; in any order 3.28 and 1.41).
+  // The answers depend on the order of A's entries, which the transpose leaves
   // to chance, so a replayed product takes the planned run's (`routed`): its
   // launches are sized for those lists.
   const int n0 = __popc(cand[0]), ncand = n0 + __popc(cand[1]);
@@ -407,20 +417,34 @@ k_row_analysis(Operands op, const int4* __restrict__ b_info, int rows_per_block,
       const int p = lower_bound_i32(op.b_col, next, next + next_len, c);
       hit = p < next + next_len && __ldg(op.b_col + p) == c;
     }
+    bool neighbour = false;
+    if (f.y > 1) {
+      const int* at = op.b_col + f.x + ((lane * (f.y - 1)) >> 5);
+      neighbour = __ldg(at + 1) == __ldg(at) + 1;
+    }
     const int pairs = __popc(__ballot_sync(FULL, pair)), hits = __popc(__ballot_sync(FULL, hit));
+    const int steps = __popc(__ballot_sync(FULL, f.y > 1)), near = __popc(__ballot_sync(FULL, neighbour));
     if (lane == 0) {
       atomicAdd(&s_pairs, pairs);
       atomicAdd(&s_hits, hits);
+      atomicAdd(&s_steps, steps);
+      atomicAdd(&s_next, near);
     }
   }
   __syncthreads();
-  const bool repeats = routed ? route[blockIdx.x] != 0 : 4 * s_hits >= max(s_pairs, 1);
-  if (!routed && threadIdx.x == 0) route[blockIdx.x] = repeats;
+  const int answers = routed ? route[blockIdx.x]
+                             : (4 * s_hits >= max(s_pairs, 1) ? ROUTE_REPEATS : 0) |
+                                   (6 * s_next >= max(s_steps, 1) ? ROUTE_RUNS : 0);
+  if (!routed && threadIdx.x == 0) route[blockIdx.x] = (unsigned char)answers;
   if (threadIdx.x < RA_ROWS) {
     const int i = row0 + threadIdx.x;
     int slot = 0;
     if (threadIdx.x < nrows) {
-      if (candidate && !repeats) bin = overflow_bin_of(acc, lo, span, tn);
+      if (candidate) {
+        const int sorted = overflow_bin_of(acc, lo, span, tn);
+        if (!(answers & ROUTE_REPEATS) && sorted >= FB_ESC0) bin = sorted;
+        else if (!(answers & ROUTE_RUNS) && cols_table_takes(bin, span)) bin += FB_COLS2 - 2;
+      }
       row_span[i] = acc > 0 ? make_int2(lo, lo + span - 1) : make_int2(0, -1);
       row_p[i] = acc;
       if (acc >= (1ll << 31)) atomicOr(status, ST_ROW_TOO_LONG);
@@ -428,8 +452,8 @@ k_row_analysis(Operands op, const int4* __restrict__ b_info, int rows_per_block,
       slot = (bin >= 0 && bin != FB_LONG) ? (int)cap : 0;
       tcap[i] = slot;
       if (bin >= 0) rank = atomicAdd(&hist[bin], 1);
-      const bool over = bin == FB_BITS ? cap > BITS_OUT_MAX
-                                       : bin >= 0 && bin < FB_WARP_BINS && hash_may_overflow(bin, cap);
+      const bool hashed = (bin >= 0 && bin < FB_WARP_BINS) || bin >= FB_COLS2;
+      const bool over = bin == FB_BITS ? cap > BITS_OUT_MAX : hashed && hash_may_overflow(bin, cap);
       if (over) atomicAdd(&ovf[overflow_bin_of(acc, lo, span, tn)], 1);
       if (bin0 >= 0) atomicAdd(&nominal[bin0], 1);
     }

@@ -443,25 +443,47 @@ __device__ __forceinline__ void warp_sort_shared(unsigned* keys, int o, int lane
     if (32 * r + lane < o) keys[32 * r + lane] = k[r];
 }
 
-// A warp's table: 2^LOG2T slots in buckets of four, each slot for a group of
-// four neighbouring columns (key: column offset from the row's first column,
-// / 4) with a value per column. Columns of structured rows come in runs, so a
-// step's lanes look up few distinct keys and a run claims one or two slots;
-// one 16-byte read covers a bucket, so nearly every look-up ends at the first
-// (single-key probing walked 3 to 5 keys for the worst of 32 lanes). A value
-// that no product has reached holds ABSENT, a NaN pattern that no FP32
+// A warp's table: 2^LOG2T slots in buckets of four, each slot for a group of G
+// neighbouring columns (key: column offset from the row's first column, / G)
+// with a value per column. Columns of structured rows come in runs, so with
+// four columns a slot a step's lanes look up few distinct keys and a run claims
+// one or two slots; one 16-byte read covers a bucket, so nearly every look-up
+// ends at the first (single-key probing walked 3 to 5 keys for the worst of 32
+// lanes). Rows whose columns lie apart would leave all but one column of a slot
+// unused and fill the table at half the columns (or fewer) that it takes by
+// itself: theirs has G = 1 and, for about the same bytes, twice the slots
+// (27-point stencil 61^3 with its points numbered at random, 118 columns a
+// row: 3.71 ms with four columns a slot, as most rows overflow and are sorted,
+// now 1.67; k nearest neighbours of 150000 random points, k = 30: 3.28, 1.41).
+// A value that no product has reached holds ABSENT, a NaN pattern that no FP32
 // operation returns.
 //
 // Keys are relative to the row, and they stay in the table from one row to
 // the next: rows of grid operators repeat their neighbours' pattern, so after
 // the first row nothing is claimed, compacted or sorted any more. Slots that
 // the row at hand does not reach are all ABSENT and are passed over.
-constexpr int GROUP_COLS = 4;
 constexpr unsigned ABSENT = 0xffffffffu;
 
-template <int MODE> struct GroupVals;  // the four values of a slot
-template <> struct alignas(16) GroupVals<0> { float v[GROUP_COLS]; };
-template <> struct alignas(16) GroupVals<1> { float2 v[GROUP_COLS]; };
+template <int MODE, int G> struct GroupVals;  // the values of a slot
+template <> struct alignas(16) GroupVals<0, 4> { float v[4]; };
+template <> struct alignas(16) GroupVals<1, 4> { float2 v[4]; };
+template <> struct alignas(16) GroupVals<1, 2> { float2 v[2]; };
+template <> struct GroupVals<0, 1> { float v[1]; };
+template <> struct alignas(8) GroupVals<1, 1> { float2 v[1]; };
+
+template <int MODE, int G>
+__device__ __forceinline__ void set_absent(GroupVals<MODE, G>* at) {
+  constexpr int BYTES = sizeof(GroupVals<MODE, G>);
+  if constexpr (BYTES == 4) {
+    *reinterpret_cast<unsigned*>(at) = ABSENT;
+  } else if constexpr (BYTES == 8) {
+    *reinterpret_cast<uint2*>(at) = make_uint2(ABSENT, ABSENT);
+  } else {
+#pragma unroll
+    for (int q = 0; q < BYTES / 16; ++q)
+      reinterpret_cast<uint4*>(at)[q] = make_uint4(ABSENT, ABSENT, ABSENT, ABSENT);
+  }
+}
 
 // Bucket of a group: two multiplications with a shift between them. A single
 // one maps the regular strides of grid operators onto few places (27-point
@@ -513,9 +535,9 @@ __device__ __forceinline__ void add_product(float2* v, float a, float b) {
 // `limit` (or a group finds every bucket full).
 constexpr int HASH_UNROLL = 2;
 
-template <int LG, int LOG2T, int MODE>
+template <int LG, int LOG2T, int G, int MODE>
 __device__ __forceinline__ void hash_segments(const Operands& op, int bstart, int len, float a,
-                                              int lo, unsigned* keys, GroupVals<MODE>* vals,
+                                              int lo, unsigned* keys, GroupVals<MODE, G>* vals,
                                               int& slots, int limit) {
   constexpr int SUB = 32 >> LG, W = 1 << LG;
   constexpr unsigned MASK = (1u << LOG2T) - 1u;
@@ -559,12 +581,12 @@ __device__ __forceinline__ void hash_segments(const Operands& op, int bstart, in
     uint4 k[HASH_UNROLL];
 #pragma unroll
     for (int u = 0; u < HASH_UNROLL; ++u) {
-      slot[u] = hash_group(x[u] / GROUP_COLS, LOG2T);
+      slot[u] = hash_group(x[u] / G, LOG2T);
       k[u] = bucket_keys(keys + slot[u]);
     }
 #pragma unroll
     for (int u = 0; u < HASH_UNROLL; ++u) {
-      const unsigned g = x[u] / GROUP_COLS;
+      const unsigned g = x[u] / G;
       int way = way_of(k[u], g);
       bool miss = act[u] && way < 0;
       int passed = 0;  // full buckets
@@ -598,7 +620,7 @@ __device__ __forceinline__ void hash_segments(const Operands& op, int bstart, in
     __syncwarp();
 #pragma unroll
     for (int u = 0; u < HASH_UNROLL; ++u) {
-      auto* v = &vals[slot[u]].v[x[u] % GROUP_COLS];
+      auto* v = &vals[slot[u]].v[x[u] % G];
 #pragma unroll
       for (int s = 0; s < SUB; ++s) {
         if (act[u] && s == sub) add_product(v, sa[u], bv[u]);
@@ -637,12 +659,12 @@ __device__ __forceinline__ void clear_shared(void* p, int lane) {
 constexpr int HASH_THREADS = 128;
 constexpr int HASH_ROWS = 16;  // most rows in a stretch
 
-template <int LOG2T, int MODE>
+template <int LOG2T, int G, int MODE>
 constexpr size_t hash_warp_bytes() {
-  return ((size_t)1 << LOG2T) * (sizeof(GroupVals<MODE>) + 2 * sizeof(unsigned));
+  return ((size_t)1 << LOG2T) * (sizeof(GroupVals<MODE, G>) + 2 * sizeof(unsigned));
 }
 
-template <int LOG2T, int MODE>
+template <int LOG2T, int G, int MODE>
 __global__ void __launch_bounds__(HASH_THREADS, 10)
 k_fused_warp(Operands op, const int* __restrict__ rows, int nrows, int stretch,
              const int2* __restrict__ row_span, const long long* __restrict__ toff,
@@ -654,8 +676,9 @@ k_fused_warp(Operands op, const int* __restrict__ rows, int nrows, int stretch,
   constexpr int WPB = HASH_THREADS / 32;
   extern __shared__ __align__(16) unsigned char smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  GroupVals<MODE>* vals = reinterpret_cast<GroupVals<MODE>*>(smem) + warp * T;
-  unsigned* keys = reinterpret_cast<unsigned*>(smem + WPB * T * sizeof(GroupVals<MODE>)) + 2 * warp * T;
+  using Vals = GroupVals<MODE, G>;
+  Vals* vals = reinterpret_cast<Vals*>(smem) + warp * T;
+  unsigned* keys = reinterpret_cast<unsigned*>(smem + WPB * T * sizeof(Vals)) + 2 * warp * T;
   unsigned* order = keys + T;
   static_assert(EMPTY_KEY == ABSENT, "one pattern clears keys and values");
   int slots = 0, ordered = 0;
@@ -663,7 +686,7 @@ k_fused_warp(Operands op, const int* __restrict__ rows, int nrows, int stretch,
     clear_shared<T * (int)sizeof(unsigned)>(keys, lane);
     slots = ordered = 0;
   };
-  auto clear_vals = [&]() { clear_shared<T * (int)sizeof(GroupVals<MODE>)>(vals, lane); };
+  auto clear_vals = [&]() { clear_shared<T * (int)sizeof(Vals)>(vals, lane); };
   clear_keys();
   clear_vals();
   for (int r0 = (blockIdx.x * WPB + warp) * stretch; r0 < nrows;
@@ -689,11 +712,11 @@ k_fused_warp(Operands op, const int* __restrict__ rows, int nrows, int stretch,
           }
           const int longest = __reduce_max_sync(FULL, len);
           if (longest > 16)
-            hash_segments<5, LOG2T, MODE>(op, bstart, len, a, sp.x, keys, vals, slots, LIMIT);
+            hash_segments<5, LOG2T, G, MODE>(op, bstart, len, a, sp.x, keys, vals, slots, LIMIT);
           else if (longest > 8)
-            hash_segments<4, LOG2T, MODE>(op, bstart, len, a, sp.x, keys, vals, slots, LIMIT);
+            hash_segments<4, LOG2T, G, MODE>(op, bstart, len, a, sp.x, keys, vals, slots, LIMIT);
           else
-            hash_segments<3, LOG2T, MODE>(op, bstart, len, a, sp.x, keys, vals, slots, LIMIT);
+            hash_segments<3, LOG2T, G, MODE>(op, bstart, len, a, sp.x, keys, vals, slots, LIMIT);
         }
         if (slots <= LIMIT || kept == 0) break;
         // the earlier rows' slots were in the way: once more with none
@@ -741,17 +764,15 @@ k_fused_warp(Operands op, const int* __restrict__ rows, int nrows, int stretch,
       int written = 0, reached = 0;
       for (int t0 = 0; t0 < ordered; t0 += 32) {
         unsigned present = 0u, group = 0u;
-        GroupVals<MODE> v;
+        Vals v;
         if (t0 + lane < ordered) {
           const unsigned key = order[t0 + lane];
           group = key >> LOG2T;
-          GroupVals<MODE>* at = vals + (key & (T - 1));
-          v = *at;  // and clean for the next row
+          Vals* at = vals + (key & (T - 1));
+          v = *at;
+          set_absent(at);  // clean for the next row
 #pragma unroll
-          for (int q = 0; q < (int)sizeof(GroupVals<MODE>) / 16; ++q)
-            reinterpret_cast<uint4*>(at)[q] = make_uint4(ABSENT, ABSENT, ABSENT, ABSENT);
-#pragma unroll
-          for (int c = 0; c < GROUP_COLS; ++c) {
+          for (int c = 0; c < G; ++c) {
             const float f = *reinterpret_cast<const float*>(&v.v[c]);
             present |= __float_as_uint(f) != ABSENT ? 1u << c : 0u;
           }
@@ -761,9 +782,9 @@ k_fused_warp(Operands op, const int* __restrict__ rows, int nrows, int stretch,
         const int incl = warp_incl_scan(n);
         long long pos = base + written + incl - n;
 #pragma unroll
-        for (int c = 0; c < GROUP_COLS; ++c) {
+        for (int c = 0; c < G; ++c) {
           if ((present >> c) & 1u) {
-            t_col[pos] = sp.x + (int)(group * GROUP_COLS) + c;
+            t_col[pos] = sp.x + (int)(group * G) + c;
             t_val[pos] = finalize_value(v.v[c]);
             ++pos;
           }

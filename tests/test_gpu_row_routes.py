@@ -1,0 +1,150 @@
+"""Which kernel merges a row: the names the profile reports, so that a change
+of the rules cannot leave a kernel, or a table's overflow, untested. Structure
+exactly, values within the bounds of helpers.py, against the FP64 oracle."""
+import numpy as np
+import pytest
+
+import spgemm_b200 as sg
+from spgemm_b200 import workloads as W
+from helpers import assert_structure_equal, assert_values_close, compensated_tolerance, plain_tolerance
+from test_gpu_batch import DeviceBatch, check_all, ref_product
+
+pytestmark = pytest.mark.gpu
+
+
+def product(A, B, precision=sg.PLAIN, csc=False, **tuning):
+    """The checked product; returns the launched first-pass kernels and the
+    rows that overflowed their table or bitmap."""
+    ref = ref_product(A, B)
+    with sg.Handle(precision) as h:
+        h.set_tuning(**tuning)
+        h.set_profiling(True)
+        C = h.multiply_host(A.to_csc() if csc else A, B)
+        names = {n for n in h.kernel_times() if n.startswith("k_fused_")}
+        overflow = h.stats()["warp_overflow_rows"]
+    assert_structure_equal(C.rowptr, C.col, ref["rowptr"], ref["col"])
+    tol = plain_tolerance(ref) if precision == sg.PLAIN else compensated_tolerance(ref)
+    assert_values_close(C.val, ref, tol)
+    return names, overflow
+
+
+def renumbered(M, seed):
+    """M with its rows and columns numbered at random."""
+    perm = np.random.default_rng(seed).permutation(M.rows)
+    r = perm[np.repeat(np.arange(M.rows), np.diff(M.rowptr))]
+    return W.from_coo(M.rows, M.cols, r, perm[M.col], M.val)
+
+
+def rows_sharing(outputs, sharing, run, n, seed=0):
+    """A and B such that row i of A*B has outputs[i] columns, `sharing`
+    products each: A's entries are that many B rows of one pattern, whose
+    columns come in runs of `run`, the runs apart, spread over [0, n)."""
+    rng = np.random.default_rng(seed)
+    br, bc, k = [], [], 0
+    for o in outputs:
+        starts = np.sort(rng.choice(n // (3 * run) - 1, -(-o // run), replace=False)) * (3 * run)
+        cols = (starts[:, None] + np.arange(run)).ravel()[:o]
+        for _ in range(sharing):
+            br.append(np.full(o, k))
+            bc.append(cols)
+            k += 1
+    m = len(outputs)
+    br, bc = np.concatenate(br), np.concatenate(bc)
+    A = W.from_coo(m, k, np.repeat(np.arange(m), sharing), np.arange(k), rng.uniform(-1, 1, k).astype(np.float32))
+    return A, W.from_coo(k, n, br, bc, rng.uniform(-1, 1, len(br)).astype(np.float32))
+
+
+@pytest.mark.parametrize("precision", [sg.PLAIN, sg.COMPENSATED])
+@pytest.mark.parametrize("csc", [False, True])
+def test_grids_are_grouped_and_numbered_at_random_are_not(precision, csc):
+    S = W.stencil27(36, seed=1)
+    names, overflow = product(S, S, precision, csc)
+    assert "k_fused_warp<2>" in names and "k_fused_cols<2>" not in names, names
+    assert overflow == 0
+    R = renumbered(S, 2)
+    names, overflow = product(R, R, precision, csc)
+    assert "k_fused_cols<2>" in names, names
+    assert overflow == 0
+
+
+@pytest.mark.parametrize("precision", [sg.PLAIN, sg.COMPENSATED])
+@pytest.mark.parametrize("table,bin_", [(256, 2), (512, 3), (1024, 4)])
+@pytest.mark.parametrize("run", [1, 4])
+def test_outputs_around_a_tables_limit(precision, table, bin_, run):
+    """Rows of up to 4/5 of the slots stay, one more and they are redone."""
+    slots = table if run == 1 else table // 2
+    per_slot = 1 if run == 1 else (4 if precision == sg.PLAIN or bin_ == 2 else 2)
+    limit = slots * 4 // 5
+    fits = [limit * per_slot - d for d in (0, 1, 2, 3)] + [table // 2, 30, limit // 2]
+    fits = [o for o in fits if 2 * o <= 2048]
+    beyond = [o for o in (limit * per_slot + d for d in (1, 2, 40)) if 2 * o <= 2048]
+    outputs = (fits + beyond) * 5
+    A, B = rows_sharing(outputs, 2, run, 90_000, seed=table + run)
+    names, overflow = product(A, B, precision, warp_table_max=table)
+    assert ("k_fused_cols<%d>" if run == 1 else "k_fused_warp<%d>") % bin_ in names, names
+    assert overflow == 5 * len(beyond), (names, overflow)
+
+
+@pytest.mark.parametrize("table,bin_", [(256, 2), (512, 3), (1024, 4)])
+@pytest.mark.parametrize("over", [-70, -1, 0, 1, 70])
+@pytest.mark.parametrize("run", [1, 4])
+def test_spans_around_the_packed_order(table, bin_, over, run):
+    """The table's order packs a column (or group) offset above a slot index;
+    rows whose span leaves no room take another kernel."""
+    limit = 1 << ((26 - bin_) if run == 1 else (28 - bin_))
+    n = limit + over
+    A, B = rows_sharing([300, 101, 150, 203], 3, run, 50_000, seed=bin_)
+    stretched = B.col.astype(np.int64)
+    stretched[stretched >= 25_000] += n - 50_000  # spans up to n
+    last = np.isin(np.arange(len(B.col)), B.rowptr[1:] - 1)
+    stretched[last] = n - 1
+    first = np.isin(np.arange(len(B.col)), B.rowptr[:-1])
+    stretched[first] = 0
+    B = W.Csr(B.rows, n, B.rowptr, stretched.astype(np.int32), B.val)
+    assert (np.diff(stretched)[np.diff(np.repeat(np.arange(B.rows), np.diff(B.rowptr))) == 0] > 0).all()
+    product(A, B, sg.PLAIN, warp_table_max=table)
+    product(A, B, sg.COMPENSATED, warp_table_max=table)
+
+
+@pytest.mark.parametrize("esc", [True, False])
+def test_every_first_pass_kernel_runs(esc):
+    """One product with rows for each kernel of the default tuning, and (with
+    sorting off) for the block kernels."""
+    rng = np.random.default_rng(1)
+    n = 50_000
+    parts = [rows_sharing([3] * 40, 2, 1, n), rows_sharing([7] * 40, 2, 1, n), rows_sharing([12] * 40, 2, 1, n),
+             rows_sharing([100] * 64, 3, 1, 4000), rows_sharing([20] * 64, 2, 1, n), rows_sharing([60] * 64, 3, 1, n),
+             rows_sharing([120] * 64, 3, 4, n), rows_sharing([150] * 64, 3, 1, n),
+             rows_sharing([200] * 64, 1, 1, n), rows_sharing([400] * 64, 1, 1, n), rows_sharing([900] * 64, 1, 1, n),
+             rows_sharing([1900] * 64, 1, 1, n), rows_sharing([4000] * 64, 1, 1, n)]
+    m = k = 0
+    ar, ac, br, bc = [], [], [], []
+    for A, B in parts:
+        m0 = -(-m // 64) * 64  # a block of row analysis each
+        ar.append(np.repeat(np.arange(A.rows), np.diff(A.rowptr)) + m0)
+        ac.append(A.col + k)
+        br.append(np.repeat(np.arange(B.rows), np.diff(B.rowptr)) + k)
+        bc.append(B.col)
+        m, k = m0 + A.rows, k + B.rows
+    ar, ac, br, bc = (np.concatenate(x) for x in (ar, ac, br, bc))
+    val = lambda x: rng.uniform(-1, 1, len(x)).astype(np.float32)
+    A, B = W.from_coo(m, k, ar, ac, val(ar)), W.from_coo(k, n, br, bc, val(br))
+    names, overflow = product(A, B, **({} if esc else dict(esc_p_min=4096)))
+    want = {"k_fused_tiny", "k_fused_bits", "k_fused_warp<0>", "k_fused_warp<2>", "k_fused_cols<2>"}
+    want |= {f"k_fused_esc<{t}>" for t in (32, 64, 128, 256, 512)} if esc else {"k_fused_mid"}
+    assert want <= names, want - names
+    if not esc:
+        names, _ = product(A, B, esc_p_min=4096, mid_cols=0, warp_p_max=100)
+        assert {"k_fused_block<11>", "k_fused_block<12>", "k_fused_block<13>"} <= names, names
+
+
+@pytest.mark.parametrize("a_format", ["csc", "csr"])
+def test_replays_of_both_tables(a_format):
+    S = W.stencil27(14, seed=3)
+    db = DeviceBatch([(S, S), (renumbered(S, 4),) * 2, (renumbered(S, 5),) * 2], a_format)
+    with sg.Handle() as h:
+        h.batch_plan(db.A, db.B)
+        refs = check_all(h, db.pairs)
+        for graph in (True, True, False):
+            h.batch_execute(graph=graph)
+            check_all(h, db.pairs, refs=refs)
