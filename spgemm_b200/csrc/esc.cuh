@@ -41,11 +41,97 @@ __device__ __forceinline__ float2 esc_value<1>(float a, float b) {
 // product. A key's place is its bucket's start plus the number of smaller
 // keys in the bucket, counted by the key's own thread: neighbouring threads
 // hold keys of the same bucket, so they read the same words. Counting is
-// quadratic in the bucket, so rows with a bucket of more than
-// esc_bucket_max(p) keys sort bitonically instead. A bitonic sort of p keys
-// is p/32 * log2(p)^2/2 * ~6 warp instructions (60K at 4096 keys, 1.7K at
-// 256); a bucket of s keys costs s^2/8 of them (41K at 576 keys, 1.2K at 96).
-__device__ __forceinline__ int esc_bucket_max(int p) { return 64 + (p >> 3); }
+// quadratic in the bucket, so what is done depends on the sum of the squared
+// sizes: up to esc_mean_max(p) * p the row's keys are counted as they lie;
+// above it, columns lie in clusters or repeat, and the buckets are cut finer
+// where the keys are (esc_refine); rows that crowd those as well, a column in
+// most of their products, sort bitonically. 60000 rows of 3844 products whose
+// columns lie in 4 windows of 60: 4.85 ms with the radix passes of old, 7.07
+// with the bitonic sort for any bucket above 64 + p/8 keys, now 3.97; grids
+// with a tenth of the entries at random 6.01, 6.40, 5.23 (most rows overflow
+// the hash); 60 nearest of 150000 points in cell order 18.0, 21.5, 16.5.
+// The line between the first two: 16 or 32 instead of 48 took 27-point rows
+// from 3.36 to 3.98 ms, 96 and 128 the windows' rows of 1024 products from
+// 0.95 to 1.30 and 1.54. Teams of one warp (at most 256 products) go without
+// the finer buckets: the registers they take (spills) cost all their rows 1%.
+template <int NT>
+__device__ __forceinline__ int esc_mean_max() { return NT == 32 ? 96 : 48; }
+
+// Whether a bitonic sort of p keys costs less than counting in buckets with
+// this sum of squared sizes: about p/32 * log2(p)^2/2 * 6 warp instructions
+// and a barrier a stage, against 1/11 of one for each of the sum.
+__device__ __forceinline__ bool esc_sorts(int squares, int p) {
+  const int lg = p > 1 ? 32 - __clz(p - 1) : 1;
+  return squares > (lg * lg * 2) << lg;
+}
+
+// Keys below k among four consecutive ones (16-byte aligned for 32-bit keys).
+__device__ __forceinline__ int smaller_of_four(const unsigned* at, unsigned k) {
+  const uint4 v = *reinterpret_cast<const uint4*>(at);
+  return (v.x < k) + (v.y < k) + (v.z < k) + (v.w < k);
+}
+__device__ __forceinline__ int smaller_of_four(const unsigned long long* at, unsigned long long k) {
+  const ulonglong2 v = reinterpret_cast<const ulonglong2*>(at)[0], w = reinterpret_cast<const ulonglong2*>(at)[1];
+  return (v.x < k) + (v.y < k) + (w.x < k) + (w.y < k);
+}
+
+// The same order for a row that crowds a few buckets (columns in clusters, or
+// repeated often): each bucket is cut into as many as it has keys, by linear
+// interpolation within its columns, so k0[0, p) goes through p buckets that
+// follow the columns' density. cnt: the starts of the nb buckets. Leaves the
+// keys ordered in k1, or returns false with k0 as it was if these buckets are
+// crowded as well.
+template <int NT, int SH, class KEY>
+__device__ __forceinline__ bool esc_refine(const KEY* __restrict__ k0, KEY* __restrict__ k1,
+                                           int* __restrict__ cnt, int nb, int p, int shift, int tid,
+                                           int* warp_a, int* warp_b) {
+  constexpr int KEYS = (1 << SH) / NT;  // of a thread, 16 bits of `at` each
+  static_assert(KEYS % 2 == 0 && SH <= 16, "two places to a register");
+  unsigned at[KEYS / 2] = {};
+  auto place_of = [&](int u) { return (int)((at[u / 2] >> (16 * (u & 1))) & 0xffffu); };
+  auto set_place = [&](int u, int v) {
+    at[u / 2] = u & 1 ? (at[u / 2] & 0xffffu) | ((unsigned)v << 16) : (at[u / 2] & ~0xffffu) | (unsigned)v;
+  };
+#pragma unroll
+  for (int u = 0; u < KEYS; ++u) {
+    const int t = tid + u * NT;
+    int m = 0;
+    if (t < p) {
+      const unsigned x = (unsigned)(k0[t] >> SH);
+      const int b = (int)(x >> shift), s0 = cnt[b], size = (b + 1 < nb ? cnt[b + 1] : p) - s0;
+      m = s0 + (int)(((unsigned long long)(x & ((1u << shift) - 1u)) * (unsigned)size) >> shift);
+    }
+    set_place(u, m);
+  }
+  team_sync<NT>();
+  for (int t = tid; t < nb; t += NT) cnt[t] = 0;
+  team_sync<NT>();
+#pragma unroll
+  for (int u = 0; u < KEYS; ++u)
+    if (tid + u * NT < p) atomicAdd(cnt + place_of(u), 1);
+  team_sync<NT>();
+  if (esc_sorts(bucket_scan<NT, true>(cnt, nb, warp_a, warp_b), p)) return false;
+  if (tid < ((-p) & 3)) k1[p + tid] = ~(KEY)0;  // the last keys are read four at a time
+#pragma unroll
+  for (int u = 0; u < KEYS; ++u)
+    if (tid + u * NT < p) k1[atomicAdd(cnt + place_of(u), 1)] = k0[tid + u * NT];
+  team_sync<NT>();  // bucket m now ends at cnt[m]
+#pragma unroll
+  for (int u = 0; u < KEYS; ++u) {
+    if (tid + u * NT < p) {
+      const KEY k = k0[tid + u * NT];
+      const int m = place_of(u), s1 = cnt[m];
+      int place = (m ? cnt[m - 1] : 0) & ~3;  // the keys before the bucket are smaller
+      for (int q = place; q < s1; q += 4) place += smaller_of_four(k1 + q, k);
+      set_place(u, place);
+    }
+  }
+  team_sync<NT>();
+#pragma unroll
+  for (int u = 0; u < KEYS; ++u)
+    if (tid + u * NT < p) k1[place_of(u)] = k0[tid + u * NT];
+  return true;
+}
 
 // All products of a row into vals[pos] / keys[pos], pos = the product's
 // flattened position (entry j of the row holds aoff[j] .. aoff[j] +
@@ -240,7 +326,8 @@ constexpr size_t esc_smem_bytes() {
 // of 223 products 666 us (half of the rows), now 231 (all); R-MAT 2^18 rows of
 // 2K to 4K products 1.98 ms, now 0.92; 48 random products of 184 M partials
 // 4.3 ms and 1.8 lost in full hash tables, now 2.2. Eight products a thread:
-// 48 warps an SM then fit both the registers (40) and the shared memory.
+// 48 warps an SM then fit both the registers (40, with 40 to 48 bytes spilled
+// by 256 threads and more) and the shared memory.
 template <int NT, int SH, int MODE, class KEY>
 __global__ void __launch_bounds__(NT * esc_teams<NT>(), 1536 / (NT * esc_teams<NT>()))
 k_fused_esc(Operands op, const int* __restrict__ rows, const int* __restrict__ nrows_p,
@@ -283,8 +370,8 @@ k_fused_esc(Operands op, const int* __restrict__ rows, const int* __restrict__ n
     team_sync<NT>();
     esc_gather<NT, SH, MODE, KEY>(op, rs, re, p, lo, width, shift, k0, vals, cnt);
     team_sync<NT>();
-    const int mx = bucket_scan<NT>(cnt, nb, warp_a, warp_b);
-    if (mx <= esc_bucket_max(p)) {  // team-uniform
+    const KEY* ordered = k0;
+    if (bucket_scan<NT, true>(cnt, nb, warp_a, warp_b) <= esc_mean_max<NT>() * p) {  // team-uniform
       for (int t = tid; t < p; t += NT) {
         const KEY k = k0[t];
         k1[atomicAdd(cnt + (int)((k >> SH) >> shift), 1)] = k;
@@ -299,6 +386,8 @@ k_fused_esc(Operands op, const int* __restrict__ rows, const int* __restrict__ n
           for (int q = s0; q < s1; ++q) place += k1[q] < k;
         k0[place] = k;
       }
+    } else if (NT > 32 && esc_refine<NT, SH, KEY>(k0, k1, cnt, nb, p, shift, tid, warp_a, warp_b)) {
+      ordered = k1;
     } else {
       int n2 = 1;
       while (n2 < p) n2 <<= 1;
@@ -309,7 +398,7 @@ k_fused_esc(Operands op, const int* __restrict__ rows, const int* __restrict__ n
     }
     team_sync<NT>();
     const long long base = toff[i];
-    const int total = esc_compress<NT, SH>(k0, vals, p, lo, t_col + base, t_val + base, warp_c);
+    const int total = esc_compress<NT, SH>(ordered, vals, p, lo, t_col + base, t_val + base, warp_c);
     if (tid == 0) c_cnt[i] = total;
     team_sync<NT>();  // the buffers are reused by the team's next row
   }

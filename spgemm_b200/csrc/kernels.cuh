@@ -1020,7 +1020,7 @@ __device__ __forceinline__ void store_counters(int* p, const int (&c)[8]) {
 }
 
 // bucket_scan with nb = N * NT.
-template <int NT, int N>
+template <int NT, bool SQUARES, int N>
 __device__ __forceinline__ int bucket_scan_n(int* __restrict__ cnt, int* warp_sums, int* warp_max) {
   constexpr int NW = NT / 32;
   const int lane = threadIdx.x & 31, warp = NT == 32 ? 0 : threadIdx.x >> 5;
@@ -1031,10 +1031,10 @@ __device__ __forceinline__ int bucket_scan_n(int* __restrict__ cnt, int* warp_su
 #pragma unroll
   for (int q = 0; q < N; ++q) {
     sum += c[q];
-    mx = max(mx, c[q]);
+    mx = SQUARES ? mx + c[q] * c[q] : max(mx, c[q]);
   }
   const int incl = warp_incl_scan(sum);
-  mx = __reduce_max_sync(FULL, mx);
+  mx = SQUARES ? __reduce_add_sync(FULL, mx) : __reduce_max_sync(FULL, mx);
   int run = incl - sum;
   if (NW > 1) {
     if (lane == 31) {
@@ -1046,7 +1046,7 @@ __device__ __forceinline__ int bucket_scan_n(int* __restrict__ cnt, int* warp_su
     const int m = lane < NW ? warp_max[lane] : 0;
     const int wi = warp_incl_scan(s);
     run += __shfl_sync(FULL, wi - s, warp);
-    mx = __reduce_max_sync(FULL, m);
+    mx = SQUARES ? __reduce_add_sync(FULL, m) : __reduce_max_sync(FULL, m);
   }
 #pragma unroll
   for (int q = 0; q < N; ++q) {
@@ -1060,15 +1060,15 @@ __device__ __forceinline__ int bucket_scan_n(int* __restrict__ cnt, int* warp_su
 }
 
 // cnt[0, nb) to its exclusive prefix sums (nb = NT, 2, 4 or 8 times NT; cnt
-// 16-byte aligned); returns the largest count (to every thread). Ends with a
-// barrier.
-template <int NT>
+// 16-byte aligned); returns, to every thread, the largest count, or (SQUARES)
+// the sum of the counts' squares, which must fit an int. Ends with a barrier.
+template <int NT, bool SQUARES = false>
 __device__ __forceinline__ int bucket_scan(int* __restrict__ cnt, int nb, int* warp_sums,
                                            int* warp_max) {
-  if (nb == 8 * NT) return bucket_scan_n<NT, 8>(cnt, warp_sums, warp_max);
-  if (nb == 4 * NT) return bucket_scan_n<NT, 4>(cnt, warp_sums, warp_max);
-  if (nb == 2 * NT) return bucket_scan_n<NT, 2>(cnt, warp_sums, warp_max);
-  return bucket_scan_n<NT, 1>(cnt, warp_sums, warp_max);
+  if (nb == 8 * NT) return bucket_scan_n<NT, SQUARES, 8>(cnt, warp_sums, warp_max);
+  if (nb == 4 * NT) return bucket_scan_n<NT, SQUARES, 4>(cnt, warp_sums, warp_max);
+  if (nb == 2 * NT) return bucket_scan_n<NT, SQUARES, 2>(cnt, warp_sums, warp_max);
+  return bucket_scan_n<NT, SQUARES, 1>(cnt, warp_sums, warp_max);
 }
 
 // ---------------------------------------------------------------------------

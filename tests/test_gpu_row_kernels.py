@@ -224,3 +224,34 @@ def test_replayed_rows_keep_their_kernels(m, a_format):
         for graph in (True, True, True, False, False):
             h.batch_execute(graph=graph)
             check_all(h, db.pairs, refs=refs)
+
+
+@pytest.mark.parametrize("precision", [sg.PLAIN, sg.COMPENSATED])
+@pytest.mark.parametrize("n", [40_000, (1 << 22) + 3])
+@pytest.mark.parametrize("windows,width", [(1, 40), (2, 60), (4, 30), (16, 9), (5, 400), (3, 1)])
+def test_sorted_rows_of_crowded_columns(precision, n, windows, width):
+    """Rows of up to 4096 products whose columns lie in a few narrow windows
+    far apart, each met many times (in most products, when a window is one
+    column wide), with a few columns elsewhere: crowded buckets, cut finer or
+    sorted as a whole."""
+    rng = np.random.default_rng(windows * 1000 + width)
+    counts = [c for c in COUNTS if c > 30] + [300, 700, 1500, 3001, 3999]
+    starts = np.sort(rng.choice(n // 500 - 1, windows, replace=False)) * 500
+    near = (starts[:, None] + np.arange(width)).ravel()
+    ar, br, bc, k = [], [], [], 0
+    for i, count in enumerate(counts):
+        left = count
+        while left > 0:
+            cols = np.unique(np.concatenate([rng.choice(near, min(len(near), 45), replace=False),
+                                             rng.integers(0, n, rng.integers(0, 3))]))[:left]
+            br.append(np.full(len(cols), k))
+            bc.append(cols)
+            ar.append(i)
+            k += 1
+            left -= len(cols)
+    br, bc = np.concatenate(br), np.concatenate(bc)
+    vals = lambda x: rng.uniform(-1, 1, len(x)).astype(np.float32)
+    A = W.from_coo(len(counts), k, np.array(ar), np.arange(k), vals(ar))
+    B = W.from_coo(k, n, br, bc, vals(br))
+    stats = check_rows(A, B, precision, dict(warp_cap_max=0))
+    assert sum(stats["rows_per_symbolic_bin"][10:13]) == len(counts), stats
