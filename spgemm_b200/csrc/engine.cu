@@ -564,28 +564,44 @@ int Engine::launch_fused() {
                                     &dc->overflow_count);
     SG_LAUNCHED("k_fused_bits");
   }
-#define SG_FUSED_WARP(NAME, BIN, LIST, L, G)                                                  \
-  if (const int cnt = fb_counts_[BIN]) {                                                       \
-    const size_t smem = WPB * hash_warp_bytes<L, G, MODE>();                                   \
-    SG_CK((smem_attr(k_fused_warp<L, G, MODE>, smem)), "smem attr k_fused_warp");              \
-    /* rows in a stretch: enough stretches for the warps that the GPU holds */                 \
-    const int stretch = std::max(1, std::min(HASH_ROWS, cnt / (sms_ * 40)));                   \
-    prof_begin(NAME);                                                                          \
-    k_fused_warp<L, G, MODE><<<blocks_for(cnt, WPB * stretch, (long long)sms_ * 64),           \
-                               HASH_THREADS, smem, stream_>>>(                                 \
-        op, LIST, cnt, stretch, row_span_.as<int2>(), toff, c_cnt, t_col, t_val, rows,         \
-        dc->fb_count, tn_, row_p, &dc->overflow_count);                                        \
+  // hashed rows: stretches of the list, enough of them for the warps that the
+  // GPU holds
+  auto hash_list = [&](const int* list, int cnt) {
+    const int stretch = std::max(1, std::min(HASH_ROWS, cnt / (sms_ * 40)));
+    return HashList{list, cnt, stretch,
+                    cnt > 0 ? blocks_for(cnt, WPB * stretch, (long long)sms_ * 64) : 0};
+  };
+#define SG_HASH(NAME, B, GROUPS, COLS)                                                        \
+  {                                                                                            \
+    const size_t smem =                                                                        \
+        WPB * std::max((GROUPS) ? hash_warp_bytes<hash_slots_log2(B), group_cols(MODE, B), MODE>() : (size_t)0, \
+                       (COLS) ? hash_warp_bytes<cols_slots_log2(B), 1, MODE>() : (size_t)0);   \
+    SG_CK((smem_attr(k_fused_warp<B, MODE, GROUPS, COLS>, smem)), "smem attr k_fused_warp");   \
+    prof_begin(NAME "<" #B ">");                                                               \
+    k_fused_warp<B, MODE, GROUPS, COLS>                                                        \
+        <<<groups.blocks + cols.blocks, HASH_THREADS, smem, stream_>>>(                        \
+            op, groups, cols, row_span_.as<int2>(), toff, c_cnt, t_col, t_val, rows,           \
+            dc->fb_count, tn_, row_p, &dc->overflow_count);                                    \
     SG_LAUNCHED("k_fused_warp");                                                               \
   }
-#define SG_FUSED_GROUPS(B) \
-  SG_FUSED_WARP("k_fused_warp<" #B ">", B, rows + (size_t)(B) * m, hash_slots_log2(B), (group_cols(MODE, B)))
-#define SG_FUSED_COLS(B) \
-  SG_FUSED_WARP("k_fused_cols<" #B ">", FB_COLS2 + B - 2, shared_list(FB_COLS2 + B - 2), cols_slots_log2(B), 1)
-  SG_FUSED_GROUPS(0) SG_FUSED_GROUPS(1) SG_FUSED_GROUPS(2) SG_FUSED_GROUPS(3) SG_FUSED_GROUPS(4)
-  SG_FUSED_COLS(2) SG_FUSED_COLS(3) SG_FUSED_COLS(4)
-#undef SG_FUSED_COLS
+#define SG_FUSED_GROUPS(B)                                                                    \
+  {                                                                                            \
+    const HashList groups = hash_list(rows + (size_t)(B) * m, fb_counts_[B]), cols{};          \
+    if (groups.n) SG_HASH("k_fused_warp", B, true, false)                                      \
+  }
+#define SG_FUSED_BOTH(B)                                                                      \
+  {                                                                                            \
+    constexpr int C = FB_COLS2 + (B) - 2;                                                      \
+    const HashList groups = hash_list(rows + (size_t)(B) * m, fb_counts_[B]);                  \
+    const HashList cols = hash_list(shared_list(C), fb_counts_[C]);                            \
+    if (groups.n && cols.n) SG_HASH("k_fused_warp+cols", B, true, true)                        \
+    else if (groups.n) SG_HASH("k_fused_warp", B, true, false)                                 \
+    else if (cols.n) SG_HASH("k_fused_cols", B, false, true)                                   \
+  }
+  SG_FUSED_GROUPS(0) SG_FUSED_GROUPS(1) SG_FUSED_BOTH(2) SG_FUSED_BOTH(3) SG_FUSED_BOTH(4)
+#undef SG_HASH
 #undef SG_FUSED_GROUPS
-#undef SG_FUSED_WARP
+#undef SG_FUSED_BOTH
   // mid bitmap rows (and warp overflow with a narrow span)
   if (fb_counts_[FB_MID] + may_overflow_[FB_MID] > 0) {
     const int width = std::min(n_, tn_.mid_cols) + 32;  // + alignment of lo down to 32

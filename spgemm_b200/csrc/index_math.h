@@ -11,16 +11,15 @@
 
 namespace sg {
 
-// Entries [begin, end) of a row whose pointers have not been validated: inside
-// [0, nnz] and not reversed whatever they hold, so that nothing is read or
+// Entries [begin, end) of a row whose pointers have not been validated: as they
+// are when 0 <= begin <= end <= nnz, else none, so that nothing is read or
 // written outside the arrays before the validation's findings are known.
 struct EntryRange {
   int begin, end;
 };
 SG_HOST_DEVICE EntryRange entry_range(int begin, int end, int nnz) {
-  const int b = begin < 0 ? 0 : (begin > nnz ? nnz : begin);
-  const int e = end < b ? b : (end > nnz ? nnz : end);
-  return EntryRange{b, e};
+  const bool ok = (unsigned)begin <= (unsigned)end && (unsigned)end <= (unsigned)nnz;
+  return EntryRange{ok ? begin : 0, ok ? end : 0};
 }
 
 // First position of [lo, hi) whose value at(position) is not below `key` (at
@@ -34,11 +33,12 @@ SG_HOST_DEVICE int lower_bound_at(int lo, int hi, int key, At at) {
   return lo;
 }
 
-// f(p) for p = first, first + stride, ... below n; p stays in range where an
-// int counter would wrap at the last step (n near 2^31).
+// f(p) for p = first, first + stride, ... below n <= 2^31; the counter is
+// unsigned, since an int would wrap at the last step when n is near 2^31
+// (first, stride < 2^31).
 template <class F>
-SG_HOST_DEVICE void strided(long long first, long long stride, long long n, F f) {
-  for (long long p = first; p < n; p += stride) f((int)p);
+SG_HOST_DEVICE void strided(unsigned first, unsigned stride, unsigned n, F f) {
+  for (unsigned p = first; p < n; p += stride) f((int)p);
 }
 
 // Blocks of `per` items that cover n, and the end of the block that begins at

@@ -200,7 +200,7 @@ __host__ __device__ constexpr int cols_slots_log2(int b) { return 6 + b; }
 // Columns of a group: four, but two in the larger tables of compensated
 // values, where four of eight bytes leave an SM 20 and 8 warps (27-point
 // stencil 61^3 with tables up to 512: 1.55 ms, now 1.19; 1024: 2.82, 1.82).
-constexpr int group_cols(int mode, int b) { return mode == 1 && b >= 3 ? 2 : 4; }
+__host__ __device__ constexpr int group_cols(int mode, int b) { return mode == 1 && b >= 3 ? 2 : 4; }
 
 // Whether a row of hash list `bin` may need more slots than its table gives.
 __host__ __device__ inline bool hash_may_overflow(int bin, long long cap) {

@@ -73,7 +73,7 @@ k_check(CheckArgs c, unsigned* status, int* descents) {
   bool bad = false;
   int net = 0;
   if (blockIdx.y == 0) {
-    strided(t0, stride, c.b_rows + 1ll, [&](int i) {
+    strided(t0, stride, c.b_rows + 1u, [&](int i) {
       const int s = c.b_ptr[i];
       const bool ok = pointer_ok(c.b_ptr, i, c.b_rows, c.b_nnz, s);
       bad |= !ok;
@@ -94,7 +94,7 @@ k_check(CheckArgs c, unsigned* status, int* descents) {
       if (q > 0 && c.b_idx[q - 1] >= v) ++net;
     });
   } else if (blockIdx.y == 2) {
-    strided(t0, stride, c.a_major + 1ll,
+    strided(t0, stride, c.a_major + 1u,
             [&](int i) { bad |= !pointer_ok(c.a_ptr, i, c.a_major, c.a_nnz, c.a_ptr[i]); });
   } else {
     strided(t0, stride, c.a_nnz, [&](int q) {
@@ -391,11 +391,12 @@ k_row_analysis(Operands op, const int4* __restrict__ b_info, int rows_per_block,
   // 2 of 3 pairs, any order of the entries: 1 of 2), rows of random graphs
   // hardly. Rows that do not repeat columns fill a hash table for nothing
   // (random rows of 200 products: 4.6 ns each hashed, 3.4 sorted).
-  // And do its columns come in runs? Is the column after one of the B row's
-  // (another place for each lane) its neighbour? Grids: 2 of 3; two unknowns a
-  // point: 1 of 2 or more; points in any order: hardly. The line at a sixth
-  // (points in cell order, 0.4 to 0.5, k = 30 nearest of 150000: grouped 1.16
-  // ms, single columns 1.50; in any order 3.28 and 1.41).
+  // And do its columns come in runs? Do two neighbours in the middle of the B
+  // row fall into the same group of four? Grids: 3 of 4; points in cell order:
+  // 1 of 3; points in any order: hardly. The line lies at an eighth (the 30
+  // nearest of 150000 points, in cell order: grouped 1.15 ms, single columns
+  // 1.50; in any order 3.28 and 1.41); a few B rows say too little, and such
+  // blocks are grouped.
   // The answers depend on the order of A's entries, which the transpose leaves
   // to chance, so a replayed product takes the planned run's (`routed`): its
   // launches are sized for those lists.
@@ -411,19 +412,20 @@ k_row_analysis(Operands op, const int4* __restrict__ b_info, int rows_per_block,
     const int4 f = entry(rs + lane, re);
     const int next = __shfl_down_sync(FULL, f.x, 1), next_len = __shfl_down_sync(FULL, f.y, 1);
     const bool pair = lane < 31 && f.y > 0 && next_len > 0;
+    int c0 = 0, c1 = 0;  // neighbours in the middle of the B row, one place earlier for odd lanes
+    if (f.y > 1) {
+      const int* at = op.b_col + f.x + max(min(f.y / 2, f.y - 2) - (lane & 1), 0);
+      c0 = __ldg(at) - s_lo[lr];
+      c1 = __ldg(at + 1) - s_lo[lr];
+    }
     bool hit = false;
     if (pair) {
       const int c = __ldg(op.b_col + f.x + f.y / 2);
       const int p = lower_bound_i32(op.b_col, next, next + next_len, c);
       hit = p < next + next_len && __ldg(op.b_col + p) == c;
     }
-    bool neighbour = false;
-    if (f.y > 1) {
-      const int* at = op.b_col + f.x + ((lane * (f.y - 1)) >> 5);
-      neighbour = __ldg(at + 1) == __ldg(at) + 1;
-    }
     const int pairs = __popc(__ballot_sync(FULL, pair)), hits = __popc(__ballot_sync(FULL, hit));
-    const int steps = __popc(__ballot_sync(FULL, f.y > 1)), near = __popc(__ballot_sync(FULL, neighbour));
+    const int steps = __popc(__ballot_sync(FULL, f.y > 1)), near = __popc(__ballot_sync(FULL, f.y > 1 && c0 >> 2 == c1 >> 2));
     if (lane == 0) {
       atomicAdd(&s_pairs, pairs);
       atomicAdd(&s_hits, hits);
@@ -434,7 +436,7 @@ k_row_analysis(Operands op, const int4* __restrict__ b_info, int rows_per_block,
   __syncthreads();
   const int answers = routed ? route[blockIdx.x]
                              : (4 * s_hits >= max(s_pairs, 1) ? ROUTE_REPEATS : 0) |
-                                   (6 * s_next >= max(s_steps, 1) ? ROUTE_RUNS : 0);
+                                   (s_steps > 0 && (8 * s_next >= s_steps || s_steps < 16) ? ROUTE_RUNS : 0);
   if (!routed && threadIdx.x == 0) route[blockIdx.x] = (unsigned char)answers;
   if (threadIdx.x < RA_ROWS) {
     const int i = row0 + threadIdx.x;

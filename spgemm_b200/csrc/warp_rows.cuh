@@ -660,17 +660,24 @@ constexpr int HASH_THREADS = 128;
 constexpr int HASH_ROWS = 16;  // most rows in a stretch
 
 template <int LOG2T, int G, int MODE>
-constexpr size_t hash_warp_bytes() {
+__host__ __device__ constexpr size_t hash_warp_bytes() {
   return ((size_t)1 << LOG2T) * (sizeof(GroupVals<MODE, G>) + 2 * sizeof(unsigned));
 }
 
+// A list of such rows, and the blocks of the launch that take them.
+struct HashList {
+  const int* rows;
+  int n, stretch, blocks;
+};
+
 template <int LOG2T, int G, int MODE>
-__global__ void __launch_bounds__(HASH_THREADS, 10)
-k_fused_warp(Operands op, const int* __restrict__ rows, int nrows, int stretch,
-             const int2* __restrict__ row_span, const long long* __restrict__ toff,
-             int* __restrict__ c_cnt, int* __restrict__ t_col, float* __restrict__ t_val,
-             int* fb_rows, int* fb_count, Tuning tn, const long long* __restrict__ row_p,
-             int* __restrict__ overflow_count) {
+__device__ __forceinline__ void hash_rows(const Operands& op, const HashList& li, int block,
+                                          const int2* __restrict__ row_span,
+                                          const long long* __restrict__ toff,
+                                          int* __restrict__ c_cnt, int* __restrict__ t_col,
+                                          float* __restrict__ t_val, int* fb_rows, int* fb_count,
+                                          const Tuning& tn, const long long* __restrict__ row_p,
+                                          int* __restrict__ overflow_count) {
   constexpr int T = 1 << LOG2T;
   constexpr int LIMIT = T * 4 / 5;
   constexpr int WPB = HASH_THREADS / 32;
@@ -689,12 +696,11 @@ k_fused_warp(Operands op, const int* __restrict__ rows, int nrows, int stretch,
   auto clear_vals = [&]() { clear_shared<T * (int)sizeof(Vals)>(vals, lane); };
   clear_keys();
   clear_vals();
-  for (int r0 = (blockIdx.x * WPB + warp) * stretch; r0 < nrows;
-       r0 += gridDim.x * WPB * stretch) {
+  for (int r0 = (block * WPB + warp) * li.stretch; r0 < li.n; r0 += li.blocks * WPB * li.stretch) {
     bool reuse = true;
-    const int r1 = min(r0 + stretch, nrows);
+    const int r1 = min(r0 + li.stretch, li.n);
     for (int r = r0; r < r1; ++r) {
-      const int i = rows[r];
+      const int i = li.rows[r];
       const int2 sp = row_span[i];
       const int rs = op.a_rowptr[i], re = op.a_rowptr[i + 1];
       if (!reuse && slots > 0) clear_keys();
@@ -795,6 +801,27 @@ k_fused_warp(Operands op, const int* __restrict__ rows, int nrows, int stretch,
       if (kept > 0 && 2 * (slots - kept) > reached) reuse = false;
       __syncwarp();
     }
+  }
+}
+
+// The rows of warp bin B in tables of groups (GROUPS), of single columns
+// (COLS), or both in one launch, the single columns, which take longer, in the
+// first blocks: the longest row of a short list is what its launch takes
+// (R-MAT 30011: 33 and 46 us one after the other).
+template <int B, int MODE, bool GROUPS, bool COLS>
+__global__ void __launch_bounds__(HASH_THREADS, 10)
+k_fused_warp(Operands op, HashList groups, HashList cols, const int2* __restrict__ row_span,
+             const long long* __restrict__ toff, int* __restrict__ c_cnt, int* __restrict__ t_col,
+             float* __restrict__ t_val, int* fb_rows, int* fb_count, Tuning tn,
+             const long long* __restrict__ row_p, int* __restrict__ overflow_count) {
+  const int block = blockIdx.x - (COLS ? cols.blocks : 0);
+  if (GROUPS && block >= 0) {
+    hash_rows<hash_slots_log2(B), group_cols(MODE, B), MODE>(
+        op, groups, block, row_span, toff, c_cnt, t_col, t_val, fb_rows, fb_count, tn, row_p,
+        overflow_count);
+  } else if constexpr (COLS) {
+    hash_rows<cols_slots_log2(B), 1, MODE>(op, cols, blockIdx.x, row_span, toff, c_cnt, t_col, t_val,
+                                           fb_rows, fb_count, tn, row_p, overflow_count);
   }
 }
 
