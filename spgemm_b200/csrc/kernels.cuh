@@ -237,6 +237,21 @@ __host__ __device__ inline int row_list_of(int nominal, long long p, int lo, int
   return nominal;
 }
 
+// The same for a row of more entries of A than a warp should walk (RA_HEAVY,
+// RA_HEAVY_ROWS): however few its products, a block of 512 threads sorts it, or,
+// when the tuning sorts no rows like it, a whole warp hashes it. Ten rows of
+// 100000 entries and 2000 products took 2.42 ms in a warp's bitmap each, which
+// walked all of them before it found too many outputs (and 0.67 sorted after
+// that), now 0.47. Many such rows keep more warps busy one to a warp: 20000 of
+// 1100 entries and 50 products 0.06 ms, 0.68 with a block each.
+__host__ __device__ inline int heavy_list_of(int nominal, long long p, int lo, int span,
+                                             const Tuning& t) {
+  if (nominal < 0 || nominal == FB_LONG) return nominal;
+  if (overflow_bin_of(p, lo, span, t) >= FB_ESC0) return FB_ESC0 + 2;
+  const bool packs = nominal < FB_WARP_BINS && (span >> 2) + 2 < 1 << (26 - nominal);
+  return packs ? nominal : row_list_of(nominal, p, lo, span, t);
+}
+
 // Numeric bin of a long row (P_i > long_p) with nnz_i outputs.
 __host__ __device__ inline int num_bin_of(int o, long long p, const Tuning& t) {
   (void)p;

@@ -173,6 +173,10 @@ constexpr int RA_THREADS = 256;
 constexpr int RA_ROWS = 64;    // most rows per block
 constexpr int RA_UNROLL = 4;   // batches of a row in flight together
 constexpr int RA_HEAVY = 1024; // rows of more entries are walked by the whole block
+// ... and, when A has room for at most so many rows of their length, merged by
+// a block too (heavy_list_of); marked in the row's product count.
+constexpr int RA_HEAVY_ROWS = 512;
+constexpr long long RA_HEAVY_ROW = 1ll << 62;
 
 // What the sample of a block of row analysis found (bits of its route byte).
 constexpr int ROUTE_REPEATS = 1;  // products share columns: hash rather than sort
@@ -356,7 +360,8 @@ k_row_analysis(Operands op, const int4* __restrict__ b_info, int rows_per_block,
       hi = max(hi, part_hi[w]);
     }
     if (threadIdx.x == 0) {
-      s_p[lr] = total;
+      const bool few = (long long)(re - rs) * RA_HEAVY_ROWS > op.nnz_a;
+      s_p[lr] = few ? total | RA_HEAVY_ROW : total;
       s_lo[lr] = lo;
       s_hi[lr] = hi;
     }
@@ -372,12 +377,13 @@ k_row_analysis(Operands op, const int4* __restrict__ b_info, int rows_per_block,
   if (threadIdx.x < RA_ROWS) {
     const int lr = threadIdx.x;
     if (lr < nrows) {
-      acc = s_p[lr];
+      acc = s_p[lr] & ~RA_HEAVY_ROW;
       lo = s_lo[lr];
       span = acc > 0 ? max(s_hi[lr] + 1 - lo, 1) : 0;
       cap = row_cap(acc, op.n, span);
       bin0 = first_bin_of(acc, cap, span, tn);
-      bin = row_list_of(bin0, acc, lo, span, tn);
+      bin = s_p[lr] & RA_HEAVY_ROW ? heavy_list_of(bin0, acc, lo, span, tn)
+                                   : row_list_of(bin0, acc, lo, span, tn);
       candidate = bin >= 0 && bin < FB_WARP_BINS &&
                   (overflow_bin_of(acc, lo, span, tn) >= FB_ESC0 || cols_table_takes(bin, span));
     }

@@ -150,3 +150,26 @@ def test_replays_of_both_tables(a_format):
         for graph in (True, True, False):
             h.batch_execute(graph=graph)
             check_all(h, db.pairs, refs=refs)
+
+
+@pytest.mark.parametrize("esc", [True, False])
+@pytest.mark.parametrize("precision", [sg.PLAIN, sg.COMPENSATED])
+def test_rows_of_many_entries_and_few_products(precision, esc):
+    """Rows of A with thousands of entries of which few meet a product (most
+    rows of B are empty), from one product to 4096: a block walks them."""
+    rng = np.random.default_rng(4)
+    k, n = 60_000, 30_000
+    blens = np.where(rng.random(k) < 0.1, rng.integers(1, 9, k), 0)
+    br = np.repeat(np.arange(k), blens)
+    bc = np.concatenate([np.sort(rng.choice(n, x, replace=False)) for x in blens])
+    empty, full = np.nonzero(blens == 0)[0], np.nonzero(blens)[0]
+    lists = []
+    for entries in (1024, 1025, 3000, 9000):  # at most 512 rows of 1025 fit A
+        for used in (0, 1, 4, 20, 60, 200, 500, 800):
+            lists.append(np.sort(np.concatenate([rng.choice(empty, entries - used, replace=False),
+                                                 rng.choice(full, used, replace=False)])))
+    val = lambda x: rng.uniform(-1, 1, len(x)).astype(np.float32)
+    ar, ac = np.repeat(np.arange(len(lists)), [len(x) for x in lists]), np.concatenate(lists)
+    A, B = W.from_coo(len(lists), k, ar, ac, val(ar)), W.from_coo(k, n, br, bc, val(br))
+    names, _ = product(A, B, precision, **({} if esc else dict(esc_p_min=4096)))
+    assert ("k_fused_esc<512>" in names) == esc, names
