@@ -102,3 +102,21 @@ def test_segment_lengths_around_the_sorts_limits(kind, spread):
     assert np.array_equal(got[0], exp[0])
     assert np.array_equal(got[1], exp[1])
     assert np.array_equal(got[2], exp[2])
+
+
+@pytest.mark.parametrize("lens", [[1 << 20], [(1 << 20) + 1, 70_000], [400_000, 5, 300_000, 24_577],
+                                  [9_000] * 230 + [20_000] * 3, [8_193] * 460 + [60_000]])
+def test_few_and_many_long_segments(lens):
+    """The longest segment that several blocks sort and one beyond it, a few
+    long ones, and about as many as there are blocks or more."""
+    rng = np.random.default_rng(len(lens))
+    major = np.repeat(np.arange(len(lens)), lens)
+    minor = rng.integers(0, 1 << 22, len(major))
+    perm = rng.permutation(len(major))
+    major, minor = major[perm], minor[perm]
+    v = rng.uniform(-1, 1, len(major)).astype(np.float32)
+    with sg.Handle() as h:
+        got = run(h, major, minor, v, len(lens), 1 << 22, sg.ROW_MAJOR)
+    exp = expected(major, minor, v, len(lens), 1 << 22, sg.ROW_MAJOR)
+    for g, e in zip(got, exp):
+        assert np.array_equal(g, e)
