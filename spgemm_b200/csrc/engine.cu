@@ -121,12 +121,8 @@ int Engine::prof_collect() {
 }
 
 Engine::~Engine() {
-  DevBuf* all[] = {&a_rowptr_, &a_col_, &a_val_, &cursor_, &aoff_, &row_p_,
-                   &c_rowptr64_, &tiles_, &sym_rows_, &num_rows_, &long_slot_,
-                   &chunk_cnt_, &slices_buf_, &mid_slices_, &row_span_, &counters_, &restrict_scratch_,
-                   &tcap_, &toff_, &t_col_, &t_val_,
-                   &bitmaps_, &lpt_order_, &b_info_, &route_, &out_rowptr_,
-                   &out_col_, &out_val_};
+  DevBuf* all[] = {&analysis_, &temp_, &num_rows_, &long_slot_, &chunk_cnt_, &slices_buf_, &mid_slices_,
+                   &restrict_scratch_, &bitmaps_, &lpt_order_, &out_rowptr_, &out_col_, &out_val_};
   for (DevBuf* b : all) b->release();
   for (DevBuf& b : stage_) b.release();
   if (host_counters_) cudaFreeHost(host_counters_);
@@ -224,10 +220,22 @@ int Engine::check_status(const DevCounters& c) {
   return fail(st & ST_ROW_TOO_LONG ? 7 : ((st & (ST_BAD_INDEX | ST_UNSORTED)) ? 1 : 6), msg);
 }
 
+int Engine::carve(DevBuf& buf, std::initializer_list<Part> parts, const char* what) {
+  auto padded = [](size_t b) { return (b + 255) & ~size_t(255); };
+  size_t total = 0;
+  for (const Part& p : parts) total += padded(p.bytes);
+  SG_CK(buf.ensure(total), what);
+  unsigned char* at = buf.as<unsigned char>();
+  for (const Part& p : parts) {
+    p.view->ptr = at;
+    at += padded(p.bytes);
+  }
+  return 0;
+}
+
 int Engine::scan_counts(const int* in, int n, long long* tiles, const ScanOut& out) {
   const int ntiles = std::max(blocks_over(n, SCAN_TILE), 1);
   if (!tiles) {
-    SG_CK(tiles_.ensure(sizeof(long long) * (size_t)ntiles), "alloc scan tiles");
     tiles = tiles_.as<long long>();
     if (ntiles > 1) {  // a single tile needs no sums before it
       prof_begin("k_scan_tiles");
@@ -290,13 +298,31 @@ int Engine::analyze(const cm& A, const cm& B) {
   // counters, row tiles and row counts in one buffer: one memset (the row
   // counts need it only as the transpose's histogram)
   const bool a_csc = A.type == COL_MAJOR;
-  const size_t cnt_bytes = sizeof(int) * (size_t)std::max(m, 1);
-  SG_CK(counters_.ensure(row_counts_offset() + cnt_bytes), "alloc counters");
+  const size_t rows = (size_t)std::max(m, 1), entries = (size_t)std::max(nnz_a, 1);
+  const size_t cnt_bytes = sizeof(int) * rows;
+  const size_t csr = a_csc ? 1 : 0;  // A's transpose
+  if (int r = carve(analysis_,
+                    {{&counters_, row_counts_offset() + cnt_bytes},
+                     {&c_rowptr64_, sizeof(long long) * ((size_t)m + 1)},
+                     {&toff_, sizeof(long long) * ((size_t)m + 1)},
+                     {&row_p_, sizeof(long long) * rows},
+                     {&row_span_, sizeof(int2) * rows},
+                     {&tcap_, sizeof(int) * rows},
+                     {&sym_rows_, sizeof(int) * FB_LISTS * rows},
+                     {&tiles_, sizeof(long long) * (size_t)std::max(blocks_over(m, SCAN_TILE), 1)},
+                     {&route_, (size_t)std::max(blocks_over(m, RA_THREADS / 32), 1)},
+                     {&b_info_, sizeof(int4) * (size_t)std::max(kdim_, 1)},
+                     {&aoff_, sizeof(int) * entries},
+                     {&a_rowptr_, csr * sizeof(int) * ((size_t)m + 1)},
+                     {&cursor_, csr * sizeof(int) * ((size_t)m + 1)},
+                     {&a_col_, csr * sizeof(int) * entries},
+                     {&a_val_, csr * sizeof(float) * entries}},
+                    "alloc workspace"))
+    return r;
   DevCounters* dc = counters_.as<DevCounters>();
   SG_CK(cudaMemsetAsync(dc, 0, row_counts_offset() + (a_csc ? cnt_bytes : 0), stream_),
         "memset counters");
   row_orders_clean_ = sym_counters_clean_ = true;
-  SG_CK(c_rowptr64_.ensure(sizeof(long long) * ((size_t)m + 1)), "alloc c_rowptr64");
   int* cnt = c_cnt();
 
   // ---- validate the operands (sync point 1 reports the result) ----
@@ -304,7 +330,6 @@ int Engine::analyze(const cm& A, const cm& B) {
   // (entry_range, b_info); their findings and the validation pass's are read
   // at the first synchronisation below, before any kernel trusts the inputs.
   {
-    SG_CK(b_info_.ensure(sizeof(int4) * (size_t)std::max(kdim_, 1)), "alloc B row table");
     const CheckArgs c{B.ptr, B.idx, A.ptr, A.idx, kdim_, B.nnz, n_, a_csc ? kdim_ : m, nnz_a,
                       a_csc ? m : kdim_, b_info_.as<int4>(), a_csc ? cnt : nullptr};
     const long long most = std::max<long long>(std::max(kdim_, m) + 1ll, std::max(B.nnz, nnz_a));
@@ -319,10 +344,6 @@ int Engine::analyze(const cm& A, const cm& B) {
   const int* a_col = A.idx;
   const float* a_val = A.val;
   if (a_csc) {
-    SG_CK(a_rowptr_.ensure(sizeof(int) * ((size_t)m + 1)), "alloc a_rowptr");
-    SG_CK(cursor_.ensure(sizeof(int) * ((size_t)m + 1)), "alloc cursor");
-    SG_CK(a_col_.ensure(sizeof(int) * (size_t)std::max(nnz_a, 1)), "alloc a_col");
-    SG_CK(a_val_.ensure(sizeof(float) * (size_t)std::max(nnz_a, 1)), "alloc a_val");
     if (int r = scan_counts(cnt, m, nullptr, ScanOut{nullptr, a_rowptr_.as<int>(), cursor_.as<int>()}))
       return r;
     if (nnz_a > 0) {
@@ -338,12 +359,6 @@ int Engine::analyze(const cm& A, const cm& B) {
   }
 
   // ---- row analysis ----
-  SG_CK(aoff_.ensure(sizeof(int) * (size_t)std::max(nnz_a, 1)), "alloc aoff");
-  SG_CK(row_p_.ensure(sizeof(long long) * (size_t)std::max(m, 1)), "alloc row_p");
-  SG_CK(sym_rows_.ensure(sizeof(int) * (size_t)FB_LISTS * std::max(m, 1)), "alloc bin lists");
-  SG_CK(row_span_.ensure(sizeof(int2) * (size_t)std::max(m, 1)), "alloc row spans");
-  SG_CK(tcap_.ensure(sizeof(int) * (size_t)std::max(m, 1)), "alloc row bounds");
-  SG_CK(toff_.ensure(sizeof(long long) * ((size_t)m + 1)), "alloc temp offsets");
   const int vec_ok = ((reinterpret_cast<uintptr_t>(B.idx) | reinterpret_cast<uintptr_t>(B.val)) & 15) == 0;
   op_ = Operands{a_rowptr, a_col, a_val, aoff_.as<int>(), B.ptr, B.idx, B.val, m_, kdim_, n_,
                  vec_ok, B.nnz, nnz_a};
@@ -354,7 +369,6 @@ int Engine::analyze(const cm& A, const cm& B) {
     const int g = mean <= 4 ? 4 : (mean <= 8 ? 8 : (mean <= 16 ? 16 : 32));
     const int rpb = m >= 2 * RA_ROWS * sms_ ? RA_ROWS : RA_THREADS / g;
     const int blocks = blocks_over(m, rpb);
-    SG_CK(route_.ensure((size_t)blocks), "alloc row routes");
     auto launch = [&](auto kernel) {
       kernel<<<blocks, RA_THREADS, 0, stream_>>>(
           op_, b_info_.as<int4>(), rpb, aoff_.as<int>(), row_p_.as<long long>(), cnt,
@@ -412,8 +426,9 @@ int Engine::symbolic_pass(long long* nnz_c) {
   sym_counters_clean_ = false;
 
   // ---- first pass: fused rows to the temporary buffer, long rows counted ----
-  SG_CK(t_col_.ensure(sizeof(int) * (size_t)std::max(temp_total_, 1ll)), "alloc temp columns");
-  SG_CK(t_val_.ensure(sizeof(float) * (size_t)std::max(temp_total_, 1ll)), "alloc temp values");
+  const size_t temp = (size_t)std::max(temp_total_, 1ll);
+  if (int r = carve(temp_, {{&t_col_, sizeof(int) * temp}, {&t_val_, sizeof(float) * temp}}, "alloc temporary rows"))
+    return r;
   if (n_long_sym_ > 0) {
     SG_CK(long_slot_.ensure(sizeof(int) * (size_t)std::max(m, 1)), "alloc long_slot");
     SG_CK(chunk_cnt_.ensure(sizeof(int) * (size_t)n_long_sym_ * std::max(n_chunks_, 1)),
@@ -426,10 +441,12 @@ int Engine::symbolic_pass(long long* nnz_c) {
   const bool last = n_long_sym_ == 0;  // nothing more is counted without long rows
   if (last && !replay_) publish_counters(&rowptr);
   if (int r = scan_counts(c_cnt(), m, nullptr, rowptr)) return r;
-  SG_CK(num_rows_.ensure(sizeof(int) * (size_t)NB_COUNT * std::max(m, 1)), "alloc num_rows");
   big_capacity_ = (long long)n_long_sym_ * std::max(n_chunks_, 1);
-  SG_CK(slices_buf_.ensure(sizeof(Slice) * (size_t)std::max(big_capacity_, 1ll)), "alloc slices");
-  SG_CK(mid_slices_.ensure(sizeof(Slice) * (size_t)std::max(n_long_sym_, 1)), "alloc mid slices");
+  if (n_long_sym_ > 0) {
+    SG_CK(num_rows_.ensure(sizeof(int) * (size_t)NB_COUNT * std::max(m, 1)), "alloc num_rows");
+    SG_CK(slices_buf_.ensure(sizeof(Slice) * (size_t)big_capacity_), "alloc slices");
+    SG_CK(mid_slices_.ensure(sizeof(Slice) * (size_t)n_long_sym_), "alloc mid slices");
+  }
   // output capacity of one big slice: what the shared-memory budget leaves
   Tuning tr = tn_;
   {

@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <initializer_list>
 #include <map>
 #include <string>
 #include <unordered_map>
@@ -23,6 +24,13 @@ struct DevBuf {
   cudaError_t ensure(size_t want);
   void release();
   template <class T> T* as() const { return static_cast<T*>(ptr); }
+};
+
+// One array of a buffer that several share: the first call on a handle makes a
+// few device allocations instead of one per array.
+struct DevView {
+  unsigned char* ptr = nullptr;
+  template <class T> T* as() const { return reinterpret_cast<T*>(ptr); }
 };
 
 // Device-side counters, reset once per product and read back at the two
@@ -233,13 +241,21 @@ class Engine {
   bool have_analysis_ = false;
   Operands op_{};
 
-  DevBuf a_rowptr_, a_col_, a_val_, cursor_, aoff_;
-  DevBuf row_p_, c_rowptr64_, tiles_;
-  DevBuf sym_rows_, num_rows_, long_slot_, chunk_cnt_, slices_buf_, mid_slices_, row_span_;
-  DevBuf tcap_, toff_, t_col_, t_val_;  // fused pass: row bounds, temp offsets, temp output
-  DevBuf counters_, restrict_scratch_, bitmaps_, lpt_order_;
-  DevBuf route_;   // byte per block of row analysis: ROUTE_* answers of its sample
-  DevBuf b_info_;  // int4 per row of B: position, length, first and last column
+  // `views` one behind another in `buf`, each aligned to 256 bytes
+  struct Part { DevView* view; size_t bytes; };
+  int carve(DevBuf& buf, std::initializer_list<Part> parts, const char* what);
+  DevBuf analysis_;  // what analyze() sizes from the operands:
+  DevView a_rowptr_, a_col_, a_val_, cursor_, aoff_;
+  DevView row_p_, c_rowptr64_, tiles_, sym_rows_, row_span_;
+  DevView tcap_, toff_;  // fused pass: row bounds, temp offsets
+  DevView counters_;
+  DevView route_;   // byte per block of row analysis: ROUTE_* answers of its sample
+  DevView b_info_;  // int4 per row of B: position, length, first and last column
+  DevBuf temp_;     // the fused pass's output, by toff_
+  DevView t_col_, t_val_;
+  // long rows only
+  DevBuf num_rows_, long_slot_, chunk_cnt_, slices_buf_, mid_slices_;
+  DevBuf restrict_scratch_, bitmaps_, lpt_order_;
   int bitmap_words_ = 0;  // per long row; 0 when the bitmaps are not kept
   int max_row_len_ = 0;
   DevBuf out_rowptr_, out_col_, out_val_;

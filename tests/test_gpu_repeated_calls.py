@@ -110,3 +110,40 @@ def test_symbolic_pass_again_after_one_analysis(operands):
     finally:
         L.spgemm_set_verbose(1)
         L.spgemm_set_exit_on_error(1)
+
+
+def test_workspace_without_long_rows():
+    """A product without long rows allocates nothing for them: 4 M rows of one
+    entry take at most 130 bytes a row beside operands and output."""
+    import torch
+    m = 1 << 22
+    ptr = torch.arange(m + 1, dtype=torch.int32, device="cuda")
+    idx = torch.randint(0, m, (m,), dtype=torch.int32, device="cuda")
+    val = torch.ones(m, device="cuda")
+    a = sg.device_cm(ptr.data_ptr(), idx.data_ptr(), val.data_ptr(), m, m, m, sg.ROW_MAJOR)
+    with sg.Handle() as warm:  # kernels loaded, contexts made
+        assert warm.symbolic(a, a) == m
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    with sg.Handle() as h:
+        assert h.symbolic(a, a) == m
+        used = free - torch.cuda.mem_get_info()[0]
+    assert used <= 130 * m + (8 << 20), used / m
+
+
+def test_products_of_changing_shapes_on_one_handle():
+    """The workspace's arrays move when a product of another shape comes:
+    larger and smaller rows, columns and entries, both formats of A, with and
+    without long rows."""
+    rng = np.random.default_rng(9)
+    shapes = [(50, 4000, 3000, 40.0), (30_000, 60, 500, 2.0), (700, 700, 700, 9.0), (1, 50_000, 2000, 3000.0),
+              (9000, 9000, 9000, 6.0), (64, 64, 64, 60.0), (20_000, 20_000, 40_000, 3.0)]
+    pairs = [(W.er(m, d, i, cols=k), W.er(k, 8.0, 50 + i, cols=n)) for i, (m, k, n, d) in enumerate(shapes)]
+    pairs.append((W.rmat(11, 16, 3),) * 2)
+    refs = [ref_product(A, B) for A, B in pairs]
+    with sg.Handle() as h:
+        for i in rng.permutation(np.repeat(np.arange(len(pairs)), 3)):
+            A, B = pairs[i]
+            C = h.multiply_host(A.to_csc() if rng.random() < 0.5 else A, B)
+            assert_structure_equal(C.rowptr, C.col, refs[i]["rowptr"], refs[i]["col"])
+            assert_values_close(C.val, refs[i], plain_tolerance(refs[i]))
