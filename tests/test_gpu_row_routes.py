@@ -108,11 +108,9 @@ def test_spans_around_the_packed_order(table, bin_, over, run):
     product(A, B, sg.COMPENSATED, warp_table_max=table)
 
 
-@pytest.mark.parametrize("esc", [True, False])
-def test_every_first_pass_kernel_runs(esc):
-    """One product with rows for each kernel of the default tuning, and (with
+def one_of_each(rng):
+    """One product with rows for each kernel of the default tuning and (with
     sorting off) for the block kernels."""
-    rng = np.random.default_rng(1)
     n = 50_000
     parts = [rows_sharing([3] * 40, 2, 1, n), rows_sharing([7] * 40, 2, 1, n), rows_sharing([12] * 40, 2, 1, n),
              rows_sharing([100] * 64, 3, 1, 4000), rows_sharing([20] * 64, 2, 1, n), rows_sharing([60] * 64, 3, 1, n),
@@ -131,6 +129,12 @@ def test_every_first_pass_kernel_runs(esc):
     ar, ac, br, bc = (np.concatenate(x) for x in (ar, ac, br, bc))
     val = lambda x: rng.uniform(-1, 1, len(x)).astype(np.float32)
     A, B = W.from_coo(m, k, ar, ac, val(ar)), W.from_coo(k, n, br, bc, val(br))
+    return A, B
+
+
+@pytest.mark.parametrize("esc", [True, False])
+def test_every_first_pass_kernel_runs(esc):
+    A, B = one_of_each(np.random.default_rng(1))
     names, overflow = product(A, B, **({} if esc else dict(esc_p_min=4096)))
     want = {"k_fused_tiny", "k_fused_bits", "k_fused_warp<0>", "k_fused_warp<2>", "k_fused_cols<2>"}
     want |= {f"k_fused_esc<{t}>" for t in (32, 64, 128, 256, 512)} if esc else {"k_fused_mid"}
@@ -173,3 +177,91 @@ def test_rows_of_many_entries_and_few_products(precision, esc):
     A, B = W.from_coo(len(lists), k, ar, ac, val(ar)), W.from_coo(k, n, br, bc, val(br))
     names, _ = product(A, B, precision, **({} if esc else dict(esc_p_min=4096)))
     assert ("k_fused_esc<512>" in names) == esc, names
+
+
+def expanded(A, B):
+    """Every product of A*B in order: (row, column, 64-bit value)."""
+    lens = np.diff(B.rowptr).astype(np.int64)[A.col]
+    own = np.repeat(np.arange(len(A.col)), lens)
+    pos = np.repeat(B.rowptr[A.col].astype(np.int64) - (np.cumsum(lens) - lens), lens) + np.arange(lens.sum())
+    row = np.repeat(np.arange(A.rows), np.diff(A.rowptr))[own]
+    return row, B.col[pos], A.val.astype(np.float64)[own] * B.val.astype(np.float64)[pos]
+
+
+@pytest.mark.parametrize("esc", [True, False])
+@pytest.mark.parametrize("precision", [sg.PLAIN, sg.COMPENSATED])
+def test_infinities_and_nans(precision, esc):
+    """Operands with infinities and NaNs, the all-ones pattern (the hash's mark
+    of an absent value) among them, in every kernel: the structure is kept; a
+    sum with a NaN, or infinities of both signs, is NaN; one with infinities of
+    one sign is that infinity (the compensated forms may make it NaN); all
+    other sums stay within the bounds."""
+    rng = np.random.default_rng(2)
+    A, B = one_of_each(rng)
+    for M, share in ((A, 0.02), (B, 0.003)):
+        bad = rng.random(len(M.val)) < share
+        kinds = np.array([np.inf, -np.inf, np.nan, 0.0], np.float32)
+        kinds[3:] = np.array([0xffffffff], np.uint32).view(np.float32)
+        bits = M.val.view(np.uint32)
+        bits[bad] = kinds.view(np.uint32)[rng.integers(0, 4, bad.sum())]
+    row, col, val = expanded(A, B)
+    key = row.astype(np.int64) * B.cols + col
+    order = np.argsort(key, kind="stable")
+    start = np.nonzero(np.diff(key[order], prepend=-1))[0]
+    with np.errstate(all="ignore"):
+        total = np.add.reduceat(val[order], start)
+        absum = np.add.reduceat(np.abs(val[order]), start)
+    ref = {"val": total, "absum": absum, "nterms": np.diff(np.append(start, len(key)))}
+    with sg.Handle(precision) as h:
+        h.set_tuning(**({} if esc else dict(esc_p_min=4096)))
+        C = h.multiply_host(A, B)
+    ptr = np.concatenate([[0], np.cumsum(np.bincount(row[order][start], minlength=A.rows))])
+    assert_structure_equal(C.rowptr, C.col, ptr, col[order][start])
+    finite = np.isfinite(total)
+    assert 0.05 < finite.mean() < 1.0
+    one_sign = np.isinf(total)
+    assert np.isnan(C.val[np.isnan(total)]).all()
+    if precision == sg.PLAIN:
+        assert np.array_equal(C.val[one_sign], total[one_sign].astype(np.float32))
+    else:
+        assert not np.isfinite(C.val[one_sign]).any()
+    part = {k: v[finite] for k, v in ref.items()}
+    tol = plain_tolerance(part) if precision == sg.PLAIN else compensated_tolerance(part)
+    assert_values_close(C.val[finite], part, tol)
+
+
+@pytest.mark.parametrize("csc", [False, True])
+def test_more_rows_than_the_scan_sums_by_itself(csc):
+    """33.6 million rows: above 8192 tiles of row counts the tile sums are
+    scanned in a launch of their own. Every third row is empty, the others have
+    one entry of A, and every row of B has two."""
+    import torch
+    m, k = 33_600_001, 1000
+    i = torch.arange(m, device="cuda")
+    has = i % 3 != 0
+    rows = i[has]
+    kk = (rows * 7919) % k
+    ptr = torch.zeros(m + 1, dtype=torch.int32, device="cuda")
+    ptr[1:] = torch.cumsum(has, 0).int()
+    val = (rows % 13 + 1).float()
+    bptr = (2 * torch.arange(k + 1, device="cuda")).int()
+    bcol = torch.stack([torch.arange(k, device="cuda") % 50, 60 + torch.arange(k, device="cuda") % 40], 1).int().reshape(-1)
+    bval = (torch.arange(2 * k, device="cuda") % 11 - 5).float()
+    if csc:
+        order = torch.argsort(kk, stable=True)
+        cptr = torch.zeros(k + 1, dtype=torch.int32, device="cuda")
+        cptr[1:] = torch.cumsum(torch.bincount(kk, minlength=k), 0).int()
+        arrays = (cptr, rows[order].int(), val[order])
+    else:
+        arrays = (ptr, kk.int(), val)
+    a = sg.device_cm(*(t.data_ptr() for t in arrays), len(rows), m, k, sg.COL_MAJOR if csc else sg.ROW_MAJOR)
+    b = sg.device_cm(bptr.data_ptr(), bcol.data_ptr(), bval.data_ptr(), 2 * k, k, 100, sg.ROW_MAJOR)
+    with sg.Handle() as h:
+        nnz = h.symbolic(a, b)
+        assert nnz == 2 * len(rows)
+        out = (torch.empty(m + 1, dtype=torch.int32, device="cuda"), torch.empty(nnz, dtype=torch.int32, device="cuda"),
+               torch.empty(nnz, device="cuda"))
+        h.numeric(*(t.data_ptr() for t in out))
+    assert torch.equal(out[0], 2 * ptr)
+    assert torch.equal(out[1].view(-1, 2), bcol.view(-1, 2)[kk])
+    assert torch.equal(out[2].view(-1, 2), val[:, None] * bval.view(-1, 2)[kk])
