@@ -664,11 +664,11 @@ __device__ __forceinline__ void block_walk_row(const Operands& op, int rs, int r
                                                const int* seg_start, const int* roff, int p,
                                                F& f, SegScratch* sc, int warp, int nwarps) {
   const int U = chunk_for(p, nwarps, 1 << 20);
-  for (int c0 = warp * U; c0 < p; c0 += nwarps * U) {
-    const int c1 = min(c0 + U, p);
+  strided(warp * U, nwarps * U, p, [&](int c0) {
+    const int c1 = block_end(c0, U, p);
     if (whole) warp_expand_range<VALUES>(op, rs, re, c0, c1, f, sc);
     else warp_expand_explicit<VALUES>(op, rs, re - rs, seg_start, roff, c0, c1, f, sc);
-  }
+  });
 }
 
 // ---------------------------------------------------------------------------

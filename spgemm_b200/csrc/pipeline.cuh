@@ -539,12 +539,14 @@ k_fused_block(Operands op, const int* __restrict__ rows, const int* __restrict__
     const int U = chunk_for(p, NW, 1 << 20);
     if (MODE == 0) {
       NumHashPlain f{keys, reinterpret_cast<float*>(vals), LOG2T, status};
-      for (int c0 = warp * U; c0 < p; c0 += NW * U)
-        warp_expand_range<true>(op, rs, re, c0, (int)min((long long)c0 + U, p), f, sc);
+      strided(warp * U, NW * U, p, [&](int c0) {
+        warp_expand_range<true>(op, rs, re, c0, block_end(c0, U, p), f, sc);
+      });
     } else {
       NumHashTwoSum f{keys, reinterpret_cast<float2*>(vals), LOG2T, status};
-      for (int c0 = warp * U; c0 < p; c0 += NW * U)
-        warp_expand_range<true>(op, rs, re, c0, (int)min((long long)c0 + U, p), f, sc);
+      strided(warp * U, NW * U, p, [&](int c0) {
+        warp_expand_range<true>(op, rs, re, c0, block_end(c0, U, p), f, sc);
+      });
     }
     __syncthreads();
     // compaction: read my PER slots, scan the counts, write after a barrier
@@ -679,7 +681,7 @@ k_sym_long(Operands op, const int* __restrict__ rows, int nrows,
     const int rs = op.a_rowptr[i], re = op.a_rowptr[i + 1];
     int* roff = seg_start + (re - rs);
     if (threadIdx.x == 0) { total = 0; long_slot[i] = r; }
-    for (int w0 = 0; w0 < n; w0 += tn.sym_window) {
+    strided(0, tn.sym_window, n, [&](int w0) {
       const int wcols = min(n - w0, tn.sym_window);
       const int nw = (wcols + 31) >> 5;
       for (int t = threadIdx.x; t < nw; t += LONG_THREADS) bits[t] = 0u;
@@ -691,8 +693,9 @@ k_sym_long(Operands op, const int* __restrict__ rows, int nrows,
         const int pw = block_restrict_row(op, rs, re, w0, w0 + wcols, seg_start, roff,
                                           scan_shm, &carry_shm);
         const int U = chunk_for(pw, NW, 1 << 20);
-        for (int c0 = warp * U; c0 < pw; c0 += NW * U)
-          warp_expand_explicit<false>(op, rs, re - rs, seg_start, roff, c0, min(c0 + U, pw), f, sc);
+        strided(warp * U, NW * U, pw, [&](int c0) {
+          warp_expand_explicit<false>(op, rs, re - rs, seg_start, roff, c0, block_end(c0, U, pw), f, sc);
+        });
       }
       __syncthreads();
       // keep the presence bitmap for the numeric pass (when memory allows)
@@ -715,7 +718,7 @@ k_sym_long(Operands op, const int* __restrict__ rows, int nrows,
         }
       }
       __syncthreads();
-    }
+    });
     if (threadIdx.x == 0) c_cnt[i] = total;
   }
 }
@@ -1059,16 +1062,19 @@ k_num_block(Operands op, const int* __restrict__ rows, int nrows, int r0, int r1
     const int U = chunk_for(p, NW, 1 << 20);
     if (MODE == 0) {
       NumHashPlain f{keys, reinterpret_cast<float*>(vals), LOG2T, status};
-      for (int c0 = warp * U; c0 < p; c0 += NW * U)
-        warp_expand_range<true>(op, rs, re, c0, (int)min((long long)c0 + U, p), f, sc);
+      strided(warp * U, NW * U, p, [&](int c0) {
+        warp_expand_range<true>(op, rs, re, c0, block_end(c0, U, p), f, sc);
+      });
     } else if (fp64) {
       NumHashF64 f{keys, reinterpret_cast<double*>(vals), LOG2T, status};
-      for (int c0 = warp * U; c0 < p; c0 += NW * U)
-        warp_expand_range<true>(op, rs, re, c0, (int)min((long long)c0 + U, p), f, sc);
+      strided(warp * U, NW * U, p, [&](int c0) {
+        warp_expand_range<true>(op, rs, re, c0, block_end(c0, U, p), f, sc);
+      });
     } else {
       NumHashTwoSum f{keys, reinterpret_cast<float2*>(vals), LOG2T, status};
-      for (int c0 = warp * U; c0 < p; c0 += NW * U)
-        warp_expand_range<true>(op, rs, re, c0, (int)min((long long)c0 + U, p), f, sc);
+      strided(warp * U, NW * U, p, [&](int c0) {
+        warp_expand_range<true>(op, rs, re, c0, block_end(c0, U, p), f, sc);
+      });
     }
     __syncthreads();
     bitonic_sort_kv<T, NT>(keys, vals, threadIdx.x, BlockSync());
