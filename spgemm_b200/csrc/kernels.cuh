@@ -628,34 +628,6 @@ __device__ __forceinline__ void warp_expand_explicit(const Operands& op, int rs,
   }
 }
 
-// Entries [jb, min(jb + 32, re)) of a row, each restricted to the columns
-// [clo, chi) of its B row (binary search), one warp.
-template <bool NEED_VAL, class F>
-__device__ __forceinline__ void warp_expand_restricted(const Operands& op, int jb, int re,
-                                                       int clo, int chi, F& f,
-                                                       SegScratch* sc) {
-  const int lane = lane_id();
-  const int j = jb + lane;
-  int bstart = 0, len = 0;
-  float a = 0.f;
-  if (j < re) {
-    const int k = __ldg(op.a_col + j);
-    const int bs = __ldg(op.b_rowptr + k);
-    const int be = __ldg(op.b_rowptr + k + 1);
-    if (be > bs) {
-      const int first = __ldg(op.b_col + bs), last = __ldg(op.b_col + be - 1);
-      if (first < chi && last >= clo) {
-        const int s0 = first >= clo ? bs : lower_bound_i32(op.b_col, bs, be, clo);
-        const int s1 = last < chi ? be : lower_bound_i32(op.b_col, s0, be, chi);
-        bstart = s0;
-        len = s1 - s0;
-        a = __ldg(op.a_val + j);
-      }
-    }
-  }
-  warp_run_batch<NEED_VAL>(op, bstart, len, a, f, sc);
-}
-
 // All products of one row (whole: every entry's whole B row; otherwise the
 // slice prepared by block_restrict_row) by the nwarps warps of a block, in
 // equal per-warp ranges of the row's flattened product sequence.
@@ -695,18 +667,6 @@ __device__ __forceinline__ int hash_slot(unsigned* keys, int log2t, unsigned col
   atomicOr(status, ST_TABLE_FULL);
   return -1;
 }
-
-struct SymHash {
-  unsigned* keys;
-  int log2t;
-  unsigned* status;
-  int nnew;
-  __device__ __forceinline__ void operator()(int col, float, float) {
-    bool ins;
-    hash_slot(keys, log2t, (unsigned)col, ins, status);
-    nnew += ins;
-  }
-};
 
 // Columns outside [lo, lo + width) cannot occur for validated inputs; the
 // range test keeps a malformed input from writing outside the bitmap.

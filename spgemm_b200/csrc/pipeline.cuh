@@ -577,7 +577,7 @@ k_fused_block(Operands op, const int* __restrict__ rows, const int* __restrict__
     if (o > 256 && span <= (1u << (32 - LOG2T))) {
       // packed keys (column - lo) << LOG2T | slot, held in registers; the
       // values stay in their compacted slots. Bucket pass on the column
-      // offset's top bits + per-bucket insertion, as in k_fused_warp.
+      // offset's top bits, then each bucket ordered by insertion.
       unsigned pk[PER];
       int j = pos0;
 #pragma unroll
@@ -1392,10 +1392,9 @@ k_lpt_scatter(const int* __restrict__ rows, int nrows, int r0, int r1,
   }
 }
 
-// Value functors of k_num_rows: the product lands in the output slot given by
-// its column's rank in the row's directory, either as a reduction into C in
-// global memory (performed in L2; nothing is returned to the SM) or as a
-// shared-memory atomic add.
+// Value functor of k_num_rows's L2 form: the product lands in the output slot
+// given by its column's rank in the row's directory, as a reduction into C in
+// global memory (performed in L2; nothing is returned to the SM).
 __device__ __forceinline__ void red_add_f32(float* p, float v) {
   asm volatile("red.global.add.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
 }
@@ -1407,16 +1406,6 @@ struct RowValRed {
   unsigned width;
   __device__ __forceinline__ void operator()(int col, float a, float b) {
     if ((unsigned)(col - lo) < width) red_add_f32(out + long_slot(dir, lo, col), __fmul_rn(a, b));
-  }
-};
-
-struct RowValSmem {
-  const uint2* dir;
-  float* vals;  // shared memory, one slot per output
-  int lo;
-  unsigned width;
-  __device__ __forceinline__ void operator()(int col, float a, float b) {
-    if ((unsigned)(col - lo) < width) atomicAdd(vals + long_slot(dir, lo, col), __fmul_rn(a, b));
   }
 };
 
