@@ -186,6 +186,8 @@ def kernel_rows(name, p_i, o_i, span, n):
     if name == "k_num_mid":
         return long_rows & (o_i > MID_O) & (o_i <= LONG_O) & (span <= MID_COLS), True
     if name.startswith("k_fused_"):
+        # one column a slot, or both forms of the table in one launch
+        name = name.replace("warp+cols", "warp").replace("k_fused_cols", "k_fused_warp")
         sel = row_kernel(p_i, cap, span) == name
         return (sel, True) if sel.any() else (None, False)
     return None, False

@@ -74,12 +74,13 @@ typedef struct spgemm_stats {
  * outputs and a column bound cap_i = min(P_i, columns of C, column span of its
  * products). Rows with P_i <= long_p are computed in one fused pass. Warp rows
  * (P_i <= warp_p_max, cap_i <= warp_cap_max) have a hash table of the size
- * that fits cap_i, at most warp_table_max; of those, rows of at most 32
- * products are sorted in registers, rows whose columns span at most 4096 use
- * a bitmap, and rows whose products hardly share columns, or whose table or
- * bitmap is full, are handled like the rows outside the warp limits: their
- * products are sorted in shared memory, or (esc_p_min, esc_span_min) one block
- * per row takes a bitmap over the column span (span <= mid_cols) or a larger
+ * that fits cap_i, at most warp_table_max columns when they lie apart, more
+ * when they come in runs; of those, rows of at most 32 products are sorted in
+ * registers, rows whose columns span at most 4096 use a bitmap, and rows whose
+ * products hardly share columns, or whose table or bitmap is full, are handled
+ * like the rows outside the warp limits: their products are sorted in shared
+ * memory, or (esc_p_min, esc_span_min) one block per row takes a bitmap over
+ * the column span (span <= mid_cols) or a larger
  * hash table. Rows with P_i > long_p take two passes: a bitmap count, then
  * column-slice blocks (nnz_i > long_o_num), a span bitmap block
  * (nnz_i > mid_o_min) or a block hash table. */

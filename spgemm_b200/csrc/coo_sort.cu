@@ -151,9 +151,10 @@ struct CsOut {
   }
 };
 
-// Segments of at most G entries, G lanes each: bitonic in registers. All the
-// sorts together took 846 us on R-MAT 2^18 with a bitonic sort per warp or
-// block and one block for a hub, now 210: bound by latency, the hubs' blocks last.
+// Segments of at most G entries, G lanes each: bitonic in registers. On R-MAT
+// 2^18 all the sorts together took 846 us with a bitonic sort per warp or block
+// and one block for a hub, 227 with these, and some 20 less since the longer
+// segments' keys are read once. Bound by latency, the hubs' blocks last.
 template <int G>
 __device__ __forceinline__ void cs_tiny(const int* __restrict__ ptr, const int* __restrict__ lists,
                                         int c, int n_major, int count,

@@ -326,7 +326,7 @@ constexpr size_t esc_smem_bytes() {
 // of 223 products 666 us (half of the rows), now 231 (all); R-MAT 2^18 rows of
 // 2K to 4K products 1.98 ms, now 0.92; 48 random products of 184 M partials
 // 4.3 ms and 1.8 lost in full hash tables, now 2.2. Eight products a thread:
-// 48 warps an SM then fit both the registers (40, with 40 to 48 bytes spilled
+// 48 warps an SM then fit both the registers (40, with 52 bytes spilled
 // by 256 threads and more) and the shared memory.
 template <int NT, int SH, int MODE, class KEY>
 __global__ void __launch_bounds__(NT * esc_teams<NT>(), 1536 / (NT * esc_teams<NT>()))

@@ -485,8 +485,9 @@ __device__ __forceinline__ void set_absent(GroupVals<MODE, G>* at) {
   }
 }
 
-// Bucket of a group: two multiplications with a shift between them. A single
-// one maps the regular strides of grid operators onto few places (27-point
+// Bucket of a group: two multiplications with a shift between them, by 2^32
+// over the golden ratio (Knuth's multiplicative hashing, as a prime) and by the
+// first constant of MurmurHash3's 32-bit finaliser. A single one maps the regular strides of grid operators onto few places (27-point
 // stencil 60^3: planes and rows next to each other, 2.1x the time of 61^3).
 __device__ __forceinline__ unsigned hash_group(unsigned g, int log2t) {
   g *= 0x9e3779b1u;
@@ -648,14 +649,15 @@ __device__ __forceinline__ void clear_shared(void* p, int lane) {
 // keys, group above slot index, sorted in registers) is renewed only when the
 // row claimed slots. A row that needs more than 4/5 of the slots is pushed to
 // the bin that redoes it (overflow_bin_of). Rows that reuse little of the
-// table switch the reuse off for the rest of the stretch. The table of bin b
-// has 2^hash_slots_log2(b) slots. Results are summed in product order, so
-// they are reproducible when A's entries come in a fixed order.
+// table switch the reuse off for the rest of the stretch. Results are summed
+// in product order, so they are reproducible when A's entries come in a fixed
+// order.
 //
-// Bound by instruction issue (59% of the slots, 2,350 warp instructions per
-// 27-point row of 690 products) and shared-memory wavefronts (60%); with
-// atomic adds, an owner search per product and a sort per row it took 5,800
-// (stencil 96^3: 5.10 ms, now 2.53; compensated 61^3: 1.53, now 0.94).
+// Bound by instruction issue (69% of the slots, 2,440 warp instructions per
+// 27-point row of 690 products) and shared-memory wavefronts (68%; stencil
+// 61^3); with atomic adds, an owner search per product and a sort per row it
+// took 5,800 (96^3: 5.10 ms, now 2.53; compensated 61^3: 1.53, now 0.89). At
+// ten blocks an SM a thread has 48 registers and spills 28 bytes.
 constexpr int HASH_THREADS = 128;
 constexpr int HASH_ROWS = 16;  // most rows in a stretch
 
